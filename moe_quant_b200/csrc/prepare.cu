@@ -165,7 +165,38 @@ __global__ void __launch_bounds__(256) absmax_scales_kernel(const float* __restr
 // src/quant_utils.py:104-139).  |d|^norm is exp(norm * log|d|) as in tl_pow (src/quant_utils.py:25-27),
 // which is 0 for d == 0.  Of equal losses the first candidate wins; candidates with equal losses
 // almost always have equal rounded scales, so the choice among them does not change the result.
+//
+// What bounds it is the number of (element, candidate) terms: two special-function operations and
+// about fifteen fp32 operations each.  Three things keep that number and the cost of a term down,
+// none of which changes a loss that decides anything:
+//  * every term is non-negative and fp32 addition is monotone, so a candidate whose largest terms
+//    alone reach the best loss so far cannot win.  The terms of the segment's largest and smallest
+//    element, which the shrunk grids clip, are computed for 32 candidates at a time (one candidate
+//    per lane); two thirds of the 100 candidates of a 128-wide group fall to them.  Wide groups
+//    also compare the partial sum every eight elements per lane.
+//  * the elements of a 32-, 64- or 128-wide group stay in registers over all candidates.
+//  * x / s goes through the reciprocal of s, which the whole warp shares, and one residual correction
+//    (Markstein 1990); scales so small or large that the residual could underflow keep the division.
+// 7168 x 2048 bf16, groups of 128, 100 candidates: 2826 us before, about 715 us now (4394 -> 2283 us for the whole quantize call).
 template <int DT>
+__device__ __forceinline__ float mse_term(float x, float s, float rs, bool plain, float zero, float maxq, float norm) {
+  float d;
+  if (plain) {
+    d = x * rs;
+    d = fmaf(fmaf(-s, d, x), rs, d);
+  } else {
+    d = __fdiv_rn(x, s);
+  }
+  // clamp first, then floor (the bounds are whole numbers, so the order does not matter; NaN becomes 0
+  // either way): adding 2^23 with rounding towards minus infinity leaves the whole part
+  const float v = fminf(fmaxf(__fadd_rn(__fadd_rn(d, zero), 0.5f), 0.0f), maxq);
+  const float q = __fadd_rd(v, 8388608.0f) - 8388608.0f;
+  const float y = round_through<DT>(__fmul_rn(q - zero, s));
+  return __expf(__logf(fabsf(y - x)) * norm);
+}
+
+// EPL: elements per lane of a group of 32 * EPL columns, held in registers; 0: any group size.
+template <int DT, int EPL>
 __global__ void __launch_bounds__(256) mse_scales_kernel(const float* __restrict__ W, int64_t R, int64_t C, int64_t ldw,
                                                          int64_t group, float maxq, float zero,
                                                          const float* __restrict__ p, int p_size, float norm,
@@ -179,22 +210,86 @@ __global__ void __launch_bounds__(256) mse_scales_kernel(const float* __restrict
     const int64_t r = seg / G, gi = seg - r * G;
     const float* x = W + r * ldw + gi * group;
     const float s0 = scale[seg];
-    float best = 0.0f;
-    int best_i = -1;
-    for (int i = 0; i < p_size; ++i) {
-      const float s = round_through<DT>(__fmul_rn(s0, __ldg(p + i)));
-      float loss = 0.0f;
+    float xr[EPL > 0 ? EPL : 1];
+    float hi = -INFINITY, lo = INFINITY;
+    if constexpr (EPL > 0) {
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) {
+        xr[e] = __ldg(x + lane + 32 * e);
+        hi = fmaxf(hi, xr[e]);
+        lo = fminf(lo, xr[e]);
+      }
+    } else {
       for (int64_t k = lane; k < group; k += 32) {
         const float xv = __ldg(x + k);
-        const float q = fminf(fmaxf(floorf(__fadd_rn(__fadd_rn(__fdiv_rn(xv, s), zero), 0.5f)), 0.0f), maxq);
-        const float y = round_through<DT>(__fmul_rn(q - zero, s));
-        loss += __expf(__logf(fabsf(y - xv)) * norm);
+        hi = fmaxf(hi, xv);
+        lo = fminf(lo, xv);
       }
-      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-      if (best_i < 0 || loss < best) { best = loss; best_i = i; }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    }
+    float best = 0.0f;
+    int best_i = -1;
+    for (int i0 = 0; i0 < p_size; i0 += 32) {
+      // A lower bound of candidate i0 + lane's loss.  The two terms may be summed in another order than in
+      // the loss itself: the factor is far below the rounding of any sum over a row.  (A group of one
+      // element has one term; an all-NaN segment leaves +-inf here, whose terms compare as NaN.)
+      float bound = INFINITY, s_lane = 1.0f, rs_lane = 1.0f;
+      if (i0 + lane < p_size) {
+        s_lane = round_through<DT>(__fmul_rn(s0, __ldg(p + i0 + lane)));
+        rs_lane = 1.0f / s_lane;
+        const bool plain = s_lane > 1e-18f && s_lane < 1e18f;
+        const float a = mse_term<DT>(hi, s_lane, rs_lane, plain, zero, maxq, norm);
+        const float b = mse_term<DT>(lo, s_lane, rs_lane, plain, zero, maxq, norm);
+        bound = hi != lo ? (a + b) * 0.9995f : a;
+      }
+      unsigned alive = __ballot_sync(0xffffffffu, bound < best);
+      if (best_i < 0) alive = __ballot_sync(0xffffffffu, i0 + lane < p_size);
+      while (alive) {
+        const int j = __ffs(alive) - 1;
+        alive &= alive - 1;
+        const int i = i0 + j;
+        const float s = __shfl_sync(0xffffffffu, s_lane, j), rs = __shfl_sync(0xffffffffu, rs_lane, j);
+        const bool plain = s > 1e-18f && s < 1e18f;
+        float loss = 0.0f;
+        bool beaten = false;
+        if constexpr (EPL > 0) {
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) loss += mse_term<DT>(xr[e], s, rs, plain, zero, maxq, norm);
+        } else {
+          int n = 0;
+          for (int64_t k0 = 0; k0 < group; k0 += 32) {
+            if (k0 + lane < group) loss += mse_term<DT>(__ldg(x + k0 + lane), s, rs, plain, zero, maxq, norm);
+            if (best_i >= 0 && (++n & 7) == 0 && k0 + 32 < group) {
+              float part = loss;
+              for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+              beaten = part >= best;   // the same tree as below, over smaller numbers: never above the final sum
+              if (beaten) break;
+            }
+          }
+        }
+        if (beaten) continue;
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        if (best_i < 0 || loss < best) {
+          best = loss;
+          best_i = i;
+          alive &= __ballot_sync(0xffffffffu, bound < best);
+        }
+      }
     }
     if (lane == 0 && best_i >= 0) scale[seg] = round_through<DT>(__fmul_rn(s0, __ldg(p + best_i)));
   }
+}
+
+template <int DT>
+void launch_mse_scales(int grid, cudaStream_t st, const float* W, int64_t R, int64_t C, int64_t ldw, int64_t group, float maxq, float zero,
+                       const float* p, int p_size, float norm, float* scale) {
+  if (group == 128) mse_scales_kernel<DT, 4><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
+  else if (group == 64) mse_scales_kernel<DT, 2><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
+  else if (group == 32) mse_scales_kernel<DT, 1><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
+  else mse_scales_kernel<DT, 0><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
 }
 
 // ---------------------------------------------------------------- fp32 working copy
@@ -321,13 +416,13 @@ extern "C" int mq_mse_scales(const float* W, int64_t R, int64_t C, int64_t ldw, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (out_dtype) {
     case MQ_F32:
-      mse_scales_kernel<MQ_F32><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, shrink, n_shrink, norm, scale);
+      launch_mse_scales<MQ_F32>(grid, st, W, R, C, ldw, group, maxq, zero, shrink, n_shrink, norm, scale);
       break;
     case MQ_BF16:
-      mse_scales_kernel<MQ_BF16><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, shrink, n_shrink, norm, scale);
+      launch_mse_scales<MQ_BF16>(grid, st, W, R, C, ldw, group, maxq, zero, shrink, n_shrink, norm, scale);
       break;
     default:
-      mse_scales_kernel<MQ_F16><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, shrink, n_shrink, norm, scale);
+      launch_mse_scales<MQ_F16>(grid, st, W, R, C, ldw, group, maxq, zero, shrink, n_shrink, norm, scale);
   }
   MQ_LAUNCH_CHECK();
   return MQ_OK;

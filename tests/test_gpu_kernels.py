@@ -446,6 +446,43 @@ def test_mse_scales_match_oracle(cuda, R, C, g, dtype):
     torch.testing.assert_close(loss(got), loss(want), rtol=1e-3, atol=0)
 
 
+@pytest.mark.parametrize("R,C,g,factor,dtype", [
+    (16, 384, 384, 1.0, torch.bfloat16),      # wide groups: partial sums are compared on the way
+    (9, 1056, 1056, 1e-6, torch.float32),     # a last trip of the lanes that is not full
+    (16, 96, 24, 1.0, torch.float16),         # fewer elements than lanes
+    (12, 256, 32, 1e-10, torch.bfloat16),
+    (12, 512, 128, 1e4, torch.float32),
+    (12, 512, 64, 1e-20, torch.float32),      # scales below the range of the reciprocal: the division
+])
+@pytest.mark.parametrize("outliers", [False, True])
+def test_mse_scales_skip_no_winner(cuda, R, C, g, factor, dtype, outliers):
+    """The search drops candidates by a lower bound of their loss.  No candidate may have a smaller
+    loss in fp64 than the chosen one by more than fp32 sums allow: terms of one sign, g additions,
+    about ten roundings in a term, |d|^norm of a d that cancels against x with |x| / |d| up to 2^8
+    on the elements that matter: 1e-4 covers them."""
+    norm = 1.0 if factor < 1e-12 else 2.4        # |d|^2.4 would leave fp32's range
+    W = synthetic.layer_weight(R, C, 17 + g, torch.float32)
+    if outliers:
+        W[:, ::max(g // 2, 1)] *= 6.0
+        W[0] = 0.0
+    W = W * factor
+    base = ops.absmax_scales(W.to(cuda), g, 4, dtype)
+    s0 = base.cpu()
+    got = ops.mse_scales(W.to(cuda), base, g, 4, dtype, norm=norm).cpu()
+    cands = O.round_fp(s0[..., None] * torch.linspace(1, 0.2, 100), dtype)
+    Wg = W.unflatten(-1, (-1, g))
+
+    def loss(s):
+        s = s[..., None]
+        # an all-zero group has scale 0 in fp16 (1e-12 underflows): any code gives loss 0
+        q = torch.clamp(torch.floor(((Wg / s).nan_to_num(0.0) + 8.0) + 0.5), 0.0, 15.0)
+        return (O.round_fp((q - 8.0) * s, dtype) - Wg).double().abs().pow(norm).sum(-1)
+
+    assert bool((cands == got[..., None]).any(-1).all())
+    best = torch.stack([loss(cands[..., i]) for i in range(cands.shape[-1])]).amin(0)
+    assert bool((loss(got) <= best * (1 + 1e-4)).all())
+
+
 # ------------------------------------------------------------------ compact launches
 @pytest.mark.parametrize("R,C,g,dtype,math", [(200, 512, 128, torch.bfloat16, MATH_TENSOR), (64, 384, 64, torch.float16, MATH_TENSOR),
                                               (333, 640, 32, torch.float32, MATH_TENSOR), (130, 512, 512, torch.bfloat16, MATH_FP32),
