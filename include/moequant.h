@@ -228,6 +228,9 @@ size_t mq_quantize_layer_workspace_bytes(int n_tied, int64_t R, int64_t C, int m
  * fp32; zero may be NULL, meaning the symmetric constant (maxq+1)/2.  */
 int mq_dequantize(const uint8_t* codes, int64_t R, int64_t C, const float* scale, const float* zero,
                   int64_t group, int bits, int out_dtype, void* out, void* stream);
+/* The same with scale and zero (both of scale_dtype) read in the type the caller keeps them in.  */
+int mq_dequantize_typed(const uint8_t* codes, int64_t R, int64_t C, const void* scale, const void* zero,
+                        int scale_dtype, int64_t group, int bits, int out_dtype, void* out, void* stream);
 
 /* sum over (r,c) of (A H)[r,c] * A[r,c] for A (R,C) fp32 and H (C,C) fp32, written to *out
  * (one double on the device).  Numerator (A = q - w) and denominator (A = w) of

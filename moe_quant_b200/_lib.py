@@ -61,6 +61,8 @@ SIGNATURES = {
     "mq_quantize_layer_workspace_bytes": (c_size_t, [c_int, c_int64, c_int64, c_int, c_int, c_int]),
     "mq_dequantize": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p,
                               c_void_p]),
+    "mq_dequantize_typed": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_void_p,
+                                    c_void_p]),
     "mq_quadratic_form": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int, c_int,
                                   c_void_p, c_size_t, c_void_p]),
     "mq_quadratic_form_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int, c_int]),

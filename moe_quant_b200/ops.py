@@ -273,11 +273,15 @@ def dequantize(codes: Tensor, scale: Tensor, zero: Optional[Tensor], group: int,
     R, C = codes.shape
     out = torch.empty(R, C, dtype=dtype, device=codes.device)
     codes = codes.contiguous()
-    scale = scale.to(torch.float32).contiguous()
-    zero = None if zero is None else zero.to(torch.float32).contiguous()
+    # scale and zero are read in their own type when the library knows it and they share it
+    if scale.dtype not in _lib._DTYPES or (zero is not None and zero.dtype != scale.dtype):
+        scale = scale.to(torch.float32)
+        zero = None if zero is None else zero.to(torch.float32)
+    scale = scale.contiguous()
+    zero = None if zero is None else zero.contiguous()
     with torch.cuda.device(codes.device):
-        check(lib().mq_dequantize(ptr(codes), R, C, ptr(scale), ptr(zero), group, bits, dtype_code(dtype), ptr(out),
-                                  stream_ptr(codes.device)))
+        check(lib().mq_dequantize_typed(ptr(codes), R, C, ptr(scale), ptr(zero), dtype_code(scale.dtype), group, bits,
+                                        dtype_code(dtype), ptr(out), stream_ptr(codes.device)))
     return out
 
 

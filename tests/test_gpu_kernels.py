@@ -420,6 +420,21 @@ def test_sweep_inverse_free_form_matches_reference_codes(cuda, golden, precision
     assert torch.equal(deq.cpu().float(), want.float())
 
 
+@pytest.mark.parametrize("R,C,g", [(1, 8, 8), (3, 40, 8), (5, 24, 12), (7, 1056, 1056), (33, 2048, 64), (2, 28, 4), (130, 4096, 128)])
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("held", [torch.bfloat16, torch.float16, torch.float32, torch.float64])
+def test_dequantize_every_type_and_group(cuda, R, C, g, out, held):
+    """Vector and element paths, scales held in the layer's type or another one: bit-exact."""
+    gen = torch.Generator().manual_seed(R * 7 + C + g)
+    codes = torch.randint(0, 256, (R, C), generator=gen, dtype=torch.uint8)
+    scale = (torch.rand(R, C // g, generator=gen) * 0.01 + 1e-3).to(held)
+    zero = torch.randint(0, 16, (R, C // g), generator=gen).to(held)
+    wide_s, wide_z = (t.float().repeat_interleave(g, -1) for t in (scale, zero))
+    for z, zf in ((zero, wide_z), (None, 8.0), (zero.to(torch.int32), wide_z)):
+        got = ops.dequantize(codes.to(cuda), scale.to(cuda), None if z is None else z.to(cuda), g, 4, out).cpu()
+        assert torch.equal(got, ((codes.float() - zf) * wide_s).to(out))
+
+
 # ------------------------------------------------------------------ MSE scale search
 @pytest.mark.parametrize("R,C,g,dtype", [(64, 512, 128, torch.bfloat16), (40, 256, 32, torch.float16),
                                          (24, 384, 64, torch.float32), (8, 2048, 2048, torch.bfloat16)])
