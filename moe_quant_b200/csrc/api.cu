@@ -27,9 +27,11 @@ size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split);
 int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, int64_t ldu, const float* scale,
                const float* zero, int64_t group, int64_t s_rs, int64_t s_gs, int bits, int out_dtype, uint8_t* codes,
                void* deq, const float* Worig, int64_t ldwo, int math, int split, Workspace& ws, cudaStream_t st,
-               const float* col_div, int32_t* packed);
+               const float* col_div, const float* eq, bool absmax_grid, int32_t* packed);
 int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, int split, mq_layer_flags* flags,
-                     Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled);
+                     Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled, const float* eq);
+int equilibration(const float* H, int64_t C, int64_t ldh, float* eq, cudaStream_t st);
+int copy_upper_scaled(const float* src, int64_t lds, float* dst, int64_t ldd, int64_t C, const float* eq, cudaStream_t st);
 int hessian_accum_tensor(const void* X, int x_dtype, int64_t m, int64_t C, int64_t ldx, float* H, int64_t ldh, float beta,
                          float alpha, int split, Workspace& ws, cudaStream_t st);
 size_t hessian_accum_tensor_workspace_bytes(int x_dtype, int64_t m, int64_t C, int split);
@@ -99,21 +101,10 @@ namespace mq {
 static size_t layer_fixed_bytes(int n_tied, int64_t R, int64_t C) {
   size_t b = 0;
   b += align_up((size_t)C * C * sizeof(float), 256);                        // unit factor of the damped Hessian
-  b += align_up((size_t)C * sizeof(float), 256);                            // its diagonal scaling
+  b += align_up((size_t)C * sizeof(float), 256) + align_up((size_t)(C + 1) * sizeof(float), 256);                        // its diagonal, the equilibration
   b += 2 * (size_t)n_tied * align_up((size_t)R * C * sizeof(float), 256);   // fp32 weights: original and running
   b += mq_hessian_prepare_workspace_bytes(C);
   return b;
-}
-}  // namespace mq
-
-namespace mq {
-// dst[r, c] = src[r, c] for c from the start of row r's 128-column block (ld % 4 == 0, 16-byte aligned).
-__global__ void __launch_bounds__(256) copy_upper_blocks_kernel(const float* __restrict__ src, int64_t lds,
-                                                                float* __restrict__ dst, int64_t ldd, int64_t C) {
-  const int64_t r = blockIdx.y;
-  const int64_t c_begin = (r / 128) * 128;
-  for (int64_t c = c_begin + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; c < C; c += (int64_t)gridDim.x * blockDim.x * 4)
-    *reinterpret_cast<float4*>(dst + r * ldd + c) = __ldg(reinterpret_cast<const float4*>(src + r * lds + c));
 }
 }  // namespace mq
 
@@ -155,6 +146,7 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   Workspace ws(workspace, workspace_bytes);
   float* U = ws.take<float>((size_t)C * C);
   float* diag = ws.take<float>(C);
+  float* eq = ws.take<float>(C + 1);
   float* Wf[8];
   float* Wo[8];
   for (int i = 0; i < n_tied; ++i) {
@@ -162,7 +154,7 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
     Wo[i] = ws.take<float>((size_t)R * C);
   }
   void* prep = ws.take<char>(mq_hessian_prepare_workspace_bytes(C));
-  MQ_REQUIRE(U && diag && Wf[n_tied - 1] && Wo[n_tied - 1] && prep, MQ_ERR_WORKSPACE,
+  MQ_REQUIRE(U && diag && eq && Wf[n_tied - 1] && Wo[n_tied - 1] && prep, MQ_ERR_WORKSPACE,
              "mq_quantize_layer: workspace of %zu bytes is too small", workspace_bytes);
 
   // W.clone().float()                                           src/gptq.py:149
@@ -179,14 +171,18 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   // src/gptq.py:236-242 needs (and mq_hinv_upper provides) is never computed here.
   // With tensor math only the diagonal blocks of the factor are scaled by 1/diag(T) (the sweep
   // tiles read them); the blocks above are divided where they are split into planes.
-  const bool unscaled = math == MQ_MATH_TENSOR;
   // The factorisation, the sweep tiles and the lazy updates read nothing below the diagonal
   // 128-blocks, so that half is neither copied nor zeroed.
-  copy_upper_blocks_kernel<<<dim3(8, (unsigned)C), 256, 0, st>>>(H, ldh, U, C, C);
-  MQ_LAUNCH_CHECK();
+  // At full tensor precision the copy is equilibrated by powers of two (fp16 operand pairs).  The sweep
+  // takes an equilibrated factor only where it works on such pairs itself; otherwise the factorisation
+  // gives its result back in H's units.
+  const bool pairs = math == MQ_MATH_TENSOR && split_hinv == 3 && split_sweep == 3;
+  if (pairs) MQ_TRY(equilibration(H, C, ldh, eq, st));
+  const bool unscaled = math == MQ_MATH_TENSOR && (pairs || split_hinv != 3);
+  MQ_TRY(copy_upper_scaled(H, ldh, U, C, C, pairs ? eq : nullptr, st));
   {
     Workspace sub(ws.base + ws.used, ws.size - ws.used);
-    MQ_TRY(chol_unit_factor(U, C, C, diag, sweep_math, split_hinv, flags, sub, st, true, unscaled));
+    MQ_TRY(chol_unit_factor(U, C, C, diag, sweep_math, split_hinv, flags, sub, st, true, unscaled, pairs ? eq : nullptr));
   }
   // sweep                                                       src/gptq_loop.py:141-148
   for (int i = 0; i < n_tied; ++i) {
@@ -194,7 +190,7 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
     Workspace sub(ws.base + ws.used, ws.size - ws.used);
     MQ_TRY(gptq_sweep(Wf[i], R, C, C, U, C, scale_out[i], nullptr, group, C / group, 1, bits, w_dtype, codes[i],
                       dequantized ? dequantized[i] : nullptr, Wo[i], C, sweep_math, split_sweep, sub, st, unscaled ? diag : nullptr,
-                      packed ? packed[i] : nullptr));
+                      pairs ? eq : nullptr, true, packed ? packed[i] : nullptr));
   }
   return MQ_OK;
 }

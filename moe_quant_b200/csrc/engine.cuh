@@ -43,6 +43,26 @@ __device__ __forceinline__ void split_bf16x3(float x, uint16_t& hi, uint16_t& mi
   lo = __bfloat16_as_ushort(__float2bfloat16_rn(r2));
 }
 
+// x -> hi + lo with fp16 pieces: 22 significant bits while |x| lies in [2^-3, 2^15], an absolute error of
+// 2^-25 below.  The callers scale by powers of two so that the largest values sit just under 2^14; what
+// the pair drops is then at most 2^-39 of those.  The three products hi hi, hi lo, lo hi stand in for the
+// six of three bf16 planes: half the tensor work and two thirds of the operand bytes.
+__device__ __forceinline__ void split_half2(float x, uint16_t& hi, uint16_t& lo) {
+  const __half h = __float2half_rn(x);
+  hi = __half_as_ushort(h);
+  lo = __half_as_ushort(__float2half_rn(x - __half2float(h)));
+}
+
+// 2^(14 - e) for |bound| in [2^(e-1), 2^e): scaled by it, values up to `bound` lie below 2^14.
+// 1 for zero, infinity and NaN.
+__device__ __forceinline__ float scale_below_2_14(float bound) {
+  const int b = (int)((__float_as_uint(bound) >> 23) & 0xFFu);
+  if (b == 0 || b == 255) return 1.0f;
+  int e = 14 - (b - 126);
+  e = e < -60 ? -60 : (e > 60 ? 60 : e);
+  return __uint_as_float((uint32_t)(e + 127) << 23);
+}
+
 // Tensor-core GEMM whose operands are already planes (d.A / d.B and their strides are ignored;
 // d.K is the reduction length starting at k0 of each set).  Both sets must have the same
 // number of planes.
@@ -55,6 +75,18 @@ int gemm_tensor_planes(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, 
 // divided by row_div[r] before the split.
 int make_planes_f32(const float* src, int64_t rs, int64_t cs, int rows, int K, int planes, uint16_t* dst, PlaneSet* out,
                     cudaStream_t st, bool only_k_blocks_before_rows = false, const float* row_div = nullptr);
+
+// The factor's blocks above the diagonal, transposed, as pairs of fp16 planes: destination row j, k = i holds
+//   Utilde[i][j] * t_j,  Utilde[i][j] = U[i][j] / col_div[j] * eq[j] / eq[i]   (col_div, eq optional, else 1),
+// t_j a power of two that brings the column's entries under 2^14: from the column's maximum, or, with the C
+// factors eq of an equilibration followed by the smallest of them, from the bound 2^14 / eq[C] that every entry of
+// U[i][j] / eq[i] keeps.  The damping keeps that bound useful: diag(T) is at least sqrt(rel_damp mean(diag H)),
+// so it exceeds Utilde's unit diagonal by at most sqrt(C / rel_damp), 2^10.3 for 16384 columns and 0.01, and what a
+// pair of fp16 planes drops (2^-39 of it) stays below 2^-28 of the error it multiplies.  inv_t (2 C floats)
+// receives 1 / t_j in its first half, the second is scratch.  Only k in 128-blocks in front of the row's own
+// block are written.
+int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, float* inv_t, const float* col_div, const float* eq,
+                            PlaneSet* out, cudaStream_t st);
 
 // Tensor-core GEMM on fp32 operands that are split into `split` bf16 planes on the fly.
 int gemm_tensor_f32(const GemmDesc& d, int split, Workspace ws, cudaStream_t st);

@@ -36,6 +36,10 @@ struct GemmDesc {
   // Tensor path, rank-<=128 updates: the caller runs several layers at once (MQ_MATH_COMPACT), so
   // a CTA walks a whole row of output tiles: half to a third of the CTAs, each a little longer.
   int compact = 0;
+  // Tensor path: optional per-row and per-column factors of the product (powers of two, device arrays
+  // indexed like C): C[m,n] = alpha * row_f[m] * col_f[n] * sum_k A B + beta * C[m,n].
+  const float* row_f = nullptr;
+  const float* col_f = nullptr;
 };
 
 // fp32 CUDA-core implementation; in_dtype is the element type of A and B.

@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256) trsm_rows_kernel(const float* __restrict_
                                                         float* __restrict__ rows, int64_t ldr, int64_t r_bs,
                                                         int nrows, int nb_full, int n_total,
                                                         uint16_t* __restrict__ planes, int64_t plane_stride, int n_planes,
-                                                        int plane_ld) {
+                                                        int plane_ld, int half) {
   extern __shared__ __align__(16) float smem[];
   float* TT = smem;                // [NB][TT_LD], TT[k][j] = T[j][k] for j < k, else 0
   float* dg = smem + NB * TT_LD;   // [NB] diagonal of T
@@ -347,7 +347,21 @@ __global__ void __launch_bounds__(256) trsm_rows_kernel(const float* __restrict_
         }
       }
     }
-    if (!IDENTITY && planes) {
+    if (!IDENTITY && planes && half) {
+      // the same as a pair of fp16 planes: the equilibrated factor's entries lie below 2^14
+#pragma unroll
+      for (int h = 0; h < ROWS; ++h) {
+        const int r = r0 + h;
+        if (r >= nrows) continue;
+        uint16_t hi[4], lo[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) split_half2(lane * 4 < nb ? a[h][q] : 0.0f, hi[q], lo[q]);
+        uint16_t* dst = planes + (int64_t)r * plane_ld + lane * 4;
+        *reinterpret_cast<uint2*>(dst) = make_uint2((uint32_t)hi[0] | ((uint32_t)hi[1] << 16), (uint32_t)hi[2] | ((uint32_t)hi[3] << 16));
+        *reinterpret_cast<uint2*>(dst + plane_stride) =
+            make_uint2((uint32_t)lo[0] | ((uint32_t)lo[1] << 16), (uint32_t)lo[2] | ((uint32_t)lo[3] << 16));
+      }
+    } else if (!IDENTITY && planes) {
       // the trailing update reads this panel as bf16 planes (row, k = column inside the panel)
 #pragma unroll
       for (int h = 0; h < ROWS; ++h) {
@@ -380,41 +394,91 @@ __global__ void __launch_bounds__(256) extract_diag_kernel(const float* __restri
 // upper_only = 1: what lies entirely below the diagonal is left as it is instead of being zeroed
 // (the layer path never reads it); = 2: in addition only the diagonal 128-blocks are scaled (the
 // sweep tiles read those; the blocks above are divided by whoever splits them into planes).
-__device__ __forceinline__ void scale_quad(float* __restrict__ H, int64_t ld, const float* __restrict__ diag, int64_t r,
-                                           int64_t c) {
+__device__ __forceinline__ void scale_quad(float* __restrict__ H, int64_t ld, const float* __restrict__ diag,
+                                           const float* __restrict__ eq, int64_t r, int64_t c) {
   // four columns c..c+3 of row r; what lies entirely below the diagonal is written without being read
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c + 3 >= r) {
     const float4 v = *reinterpret_cast<const float4*>(H + r * ld + c);
     const float4 d = __ldg(reinterpret_cast<const float4*>(diag + c));
-    o.x = (c + 0 > r) ? v.x / d.x : (c + 0 == r ? 1.0f : 0.0f);
-    o.y = (c + 1 > r) ? v.y / d.y : (c + 1 == r ? 1.0f : 0.0f);
-    o.z = (c + 2 > r) ? v.z / d.z : (c + 2 == r ? 1.0f : 0.0f);
-    o.w = (c + 3 > r) ? v.w / d.w : (c + 3 == r ? 1.0f : 0.0f);
+    // equilibrated: entry (r, c) of the matrix's own factor is eq[c] / eq[r] times this one's (powers of two)
+    float4 e = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (eq) {
+      const float er = 1.0f / __ldg(eq + r);
+      const float4 ec = __ldg(reinterpret_cast<const float4*>(eq + c));
+      e = make_float4(ec.x * er, ec.y * er, ec.z * er, ec.w * er);
+    }
+    o.x = (c + 0 > r) ? v.x / d.x * e.x : (c + 0 == r ? 1.0f : 0.0f);
+    o.y = (c + 1 > r) ? v.y / d.y * e.y : (c + 1 == r ? 1.0f : 0.0f);
+    o.z = (c + 2 > r) ? v.z / d.z * e.z : (c + 2 == r ? 1.0f : 0.0f);
+    o.w = (c + 3 > r) ? v.w / d.w * e.w : (c + 3 == r ? 1.0f : 0.0f);
   }
   *reinterpret_cast<float4*>(H + r * ld + c) = o;
 }
 
 __global__ void __launch_bounds__(256) scale_columns_kernel(float* __restrict__ H, int64_t C, int64_t ld,
-                                                            const float* __restrict__ diag, int upper_only) {
+                                                            const float* __restrict__ diag, const float* __restrict__ eq,
+                                                            int upper_only) {
   const int64_t r = blockIdx.y;
   if ((C & 3) == 0 && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0) {
     if (upper_only == 2) {  // launched with one block of 32 threads per row: the row's diagonal block
       const int64_t c = (r / NB) * NB + threadIdx.x * 4;
-      if (blockIdx.x == 0 && threadIdx.x < NB / 4 && c < C && c + 3 >= r) scale_quad(H, ld, diag, r, c);
+      if (blockIdx.x == 0 && threadIdx.x < NB / 4 && c < C && c + 3 >= r) scale_quad(H, ld, diag, eq, r, c);
       return;
     }
     for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; c < C; c += (int64_t)gridDim.x * blockDim.x * 4) {
       if (upper_only && c + 3 < r) continue;
-      scale_quad(H, ld, diag, r, c);
+      scale_quad(H, ld, diag, eq, r, c);
     }
     return;
   }
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < C; c += (int64_t)gridDim.x * blockDim.x) {
     if (upper_only == 2 && (c < (r / NB) * NB || c >= (r / NB + 1) * NB)) continue;
     float v = H[r * ld + c];
-    H[r * ld + c] = (c > r) ? v / diag[c] : (c == r ? 1.0f : 0.0f);
+    H[r * ld + c] = (c > r) ? v / diag[c] * (eq ? eq[c] / eq[r] : 1.0f) : (c == r ? 1.0f : 0.0f);
   }
+}
+
+// Equilibration of the matrix to be factored: eq[i] = 2^(13 - n) with H[i][i] / 4^n in [1, 4), so that the
+// diagonal of  eq H eq  lies in [2^26, 2^28) and every entry of its factor below 2^14, where a pair of fp16
+// planes holds 22 bits of all but the smallest (split_half2).  Powers of two: the factorisation does the same
+// fp32 operations, up to exponents, as on H itself.  1 where the diagonal is not a positive finite number.
+// eq[C] receives the smallest factor (positive floats order like their bits; preset by the host).
+__global__ void __launch_bounds__(256) equilibration_kernel(const float* __restrict__ H, int64_t C, int64_t ld, float* __restrict__ eq) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const float h = i < C ? H[i * ld + i] : -1.0f;
+  float v = 1.0f;
+  if (h > 0.0f && h < INFINITY) {
+    const int e = ilogbf(h);                       // floor(log2 h)
+    int n = 13 - (e >= 0 ? e / 2 : -((1 - e) / 2));
+    n = n < -60 ? -60 : (n > 60 ? 60 : n);
+    v = __uint_as_float((uint32_t)(n + 127) << 23);
+  }
+  if (i < C) eq[i] = v;
+  const int least = __reduce_min_sync(0xffffffffu, i < C ? __float_as_int(v) : 0x7f7f7f7f);
+  if ((threadIdx.x & 31) == 0) atomicMin(reinterpret_cast<int*>(eq + C), least);
+}
+
+// dst[r][c] = src[r][c] * eq[r] * eq[c] from the start of row r's diagonal 128-block on (dst may be src; eq may
+// be null: a copy).  ld % 4 == 0, 16-byte aligned.
+__global__ void __launch_bounds__(256) scaled_upper_blocks_kernel(const float* __restrict__ src, int64_t lds, float* __restrict__ dst,
+                                                                  int64_t ldd, int64_t C, const float* __restrict__ eq) {
+  const int64_t r = blockIdx.y;
+  const float er = eq ? __ldg(eq + r) : 1.0f;
+  for (int64_t c = (r / NB) * NB + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; c < C; c += (int64_t)gridDim.x * blockDim.x * 4) {
+    float4 v = *reinterpret_cast<const float4*>(src + r * lds + c);
+    if (eq) {
+      const float4 ec = __ldg(reinterpret_cast<const float4*>(eq + c));
+      v = make_float4(v.x * er * ec.x, v.y * er * ec.y, v.z * er * ec.z, v.w * er * ec.w);
+    }
+    *reinterpret_cast<float4*>(dst + r * ldd + c) = v;
+  }
+}
+
+// diag(T) of the matrix itself from that of the equilibrated one
+__global__ void __launch_bounds__(256) unscale_diag_kernel(float* __restrict__ diag, const float* __restrict__ eq, int64_t C) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < C) diag[i] = diag[i] / eq[i];
 }
 
 __global__ void __launch_bounds__(256) identity_if_failed_kernel(float* __restrict__ U, int64_t C, int64_t ld,
@@ -448,7 +512,20 @@ int configure_once() {
 }  // namespace
 
 size_t factor_workspace_bytes(int64_t C, int math, int split) {
-  return math == MQ_MATH_TENSOR ? plane_set_bytes(C, SUPER_NB, split) : 0;
+  return math == MQ_MATH_TENSOR ? plane_set_bytes(C, SUPER_NB, split) + align_up((size_t)(C + 1) * sizeof(float), 256) : 0;
+}
+
+int equilibration(const float* H, int64_t C, int64_t ldh, float* eq, cudaStream_t st) {
+  MQ_CUDA(cudaMemsetAsync(eq + C, 0x7f, sizeof(float), st));
+  equilibration_kernel<<<(unsigned)ceil_div(C, 256), 256, 0, st>>>(H, C, ldh, eq);
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
+}
+
+int copy_upper_scaled(const float* src, int64_t lds, float* dst, int64_t ldd, int64_t C, const float* eq, cudaStream_t st) {
+  scaled_upper_blocks_kernel<<<dim3(8, (unsigned)C), 256, 0, st>>>(src, lds, dst, ldd, C, eq);
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
 }
 
 size_t hinv_workspace_bytes(int64_t C, int math, int split) {
@@ -464,12 +541,27 @@ size_t hinv_workspace_bytes(int64_t C, int math, int split) {
 // unscaled: only the diagonal blocks are scaled; above them T itself is left in place and the caller
 // divides column c by diag[c] where it reads it).  diag (C floats, device) receives diag(T).  On a non-positive pivot
 // flags->not_positive is set and the result is replaced by I.
+// eq (tensor math with split 3 only): H has been equilibrated by the caller (copy_upper_scaled) with these
+// factors; unscaled then leaves the equilibrated factor above the diagonal blocks and its diagonal in diag.
+// Null: with split 3 the matrix is equilibrated here and everything is given back in H's own units.
 int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, int split, mq_layer_flags* flags,
-                     Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled) {
+                     Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled, const float* eq) {
   MQ_TRY(configure_once());
   const int compact = (math & MQ_MATH_COMPACT) ? 1 : 0;   // the panel solves and the rank-128 strips look at it
   math &= ~MQ_MATH_COMPACT;
-  Engine eng(math, split, ws, st);
+  const bool half = math == MQ_MATH_TENSOR && split == 3;   // pairs of fp16 planes, three products (split_half2)
+  MQ_REQUIRE(!eq || half, MQ_ERR_ARGUMENT, "factorisation: an equilibrated matrix needs tensor math with split 3");
+  Workspace local(ws.base ? ws.base + ws.used : nullptr, ws.base ? ws.size - ws.used : 0);
+  const bool own_units = half && !eq;
+  if (own_units) {
+    MQ_REQUIRE(!unscaled, MQ_ERR_ARGUMENT, "factorisation: an unscaled factor needs the caller's equilibration");
+    float* own = local.take<float>(C + 1);
+    MQ_REQUIRE(own, MQ_ERR_WORKSPACE, "factorisation: workspace too small");
+    MQ_TRY(equilibration(H, C, ldh, own, st));
+    MQ_TRY(copy_upper_scaled(H, ldh, H, ldh, C, own, st));
+    eq = own;
+  }
+  Engine eng(math, split, local, st);
   const int P = (int)ceil_div(C, NB);
   // Tensor path: the panel solve writes its result as bf16 planes too, and the rank-128 update
   // P P^T reads one plane set as both operands.
@@ -487,9 +579,11 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
     PlaneSet pset;
     if (tensor) {
       Workspace mine = eng.ws;
-      pset.base = mine.take<uint16_t>(plane_set_bytes(C, SUPER_NB, split) / 2);
+      const int planes = half ? 2 : split;
+      pset.base = mine.take<uint16_t>(plane_set_bytes(C, SUPER_NB, planes) / 2);
       MQ_REQUIRE(pset.base, MQ_ERR_WORKSPACE, "factorisation: workspace too small for the panel planes");
-      pset.planes = split; pset.rows_pad = (int)pad_rows(C); pset.total_rows = pset.rows_pad; pset.K_pad = SUPER_NB;
+      pset.planes = planes; pset.rows_pad = (int)pad_rows(C); pset.total_rows = pset.rows_pad; pset.K_pad = SUPER_NB;
+      pset.fp16 = half;
     }
     for (int p = P - 1; p >= 0; --p) {
       const int p_lo = (p / SUPER_PANELS) * SUPER_PANELS;      // first (lowest) panel of this super-panel
@@ -511,7 +605,7 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
         ProfScope prof(PROF_TRSM, (double)k1 * nb * nb, 0.0, st);
         MQ_CUDA(launch_chained(true, trsm_rows_kernel<false>, dim3(grid, 1), dim3(256), kTrsmSmem, st, dblk, ldh, 0, H + k1, ldh, 0,
                                (int)k1, nb, 0, tensor ? pset.base + kwin : nullptr, tensor ? pset.total_rows * (int64_t)SUPER_NB : 0,
-                               split, SUPER_NB));
+                               split, SUPER_NB, half ? 1 : 0));
       }
       MQ_LAUNCH_CHECK();
       if (!tensor) {
@@ -555,7 +649,11 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
   {
     const int mode = unscaled ? 2 : (upper_only ? 1 : 0);
     const unsigned gx = unscaled ? 1u : (unsigned)(ceil_div(C, 256) < 8 ? ceil_div(C, 256) : 8);
-    scale_columns_kernel<<<dim3(gx, (unsigned)C), unscaled ? 32 : 256, 0, st>>>(H, C, ldh, diag, mode);
+    scale_columns_kernel<<<dim3(gx, (unsigned)C), unscaled ? 32 : 256, 0, st>>>(H, C, ldh, diag, eq, mode);
+    MQ_LAUNCH_CHECK();
+  }
+  if (own_units) {
+    unscale_diag_kernel<<<(unsigned)ceil_div(C, 256), 256, 0, st>>>(diag, eq, C);
     MQ_LAUNCH_CHECK();
   }
   identity_if_failed_kernel<<<148 * 4, 256, 0, st>>>(H, C, ldh, flags, diag);
@@ -568,14 +666,14 @@ int hinv_upper(float* H, int64_t C, int64_t ldh, float* Uhat, int64_t ldu, float
   float* diag = ws.take<float>(C);
   float* scratch = ws.take<float>((size_t)C * C);
   MQ_REQUIRE(diag && scratch, MQ_ERR_WORKSPACE, "mq_hinv_upper: workspace too small");
-  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split, flags, ws, st, false, false));
+  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split, flags, ws, st, false, false, nullptr));
   if (diag_out) MQ_CUDA(cudaMemcpyAsync(diag_out, diag, C * sizeof(float), cudaMemcpyDeviceToDevice, st));
   Engine eng(math, split, ws, st);
   const int P = (int)ceil_div(C, NB);
   // ---- inverse of the unit factor: invert the diagonal blocks, then merge pairs of blocks
   MQ_CUDA(cudaMemsetAsync(Uhat, 0, (size_t)C * ldu * sizeof(float), st));
   trsm_rows_kernel<true><<<dim3(4, P), 256, kTrsmSmem, st>>>(H, ldh, (int64_t)NB * (ldh + 1), Uhat, ldu,
-                                                             (int64_t)NB * (ldu + 1), NB, NB, (int)C, nullptr, 0, 0, NB);
+                                                             (int64_t)NB * (ldu + 1), NB, NB, (int)C, nullptr, 0, 0, NB, 0);
   MQ_LAUNCH_CHECK();
   for (int64_t s = NB; s < C; s *= 2) {
     const int batch = (int)ceil_div(C - s, 2 * s);
@@ -641,7 +739,7 @@ extern "C" int mq_chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag
   float* diag = ws.take<float>(C);
   MQ_REQUIRE(diag, MQ_ERR_WORKSPACE, "mq_chol_unit_factor: workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split, flags, ws, st, false, false));
+  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split, flags, ws, st, false, false, nullptr));
   if (diag_out) MQ_CUDA(cudaMemcpyAsync(diag_out, diag, C * sizeof(float), cudaMemcpyDeviceToDevice, st));
   return MQ_OK;
 }

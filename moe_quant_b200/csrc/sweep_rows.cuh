@@ -213,7 +213,23 @@ __global__ void __launch_bounds__(THREADS, 1) sweep_rows_kernel(const SweepArgs 
           pdst[0] = (int32_t)pack_nibbles(cw[rr][0], cw[rr][1]);
           pdst[1] = (int32_t)pack_nibbles(cw[rr][2], cw[rr][3]);
         }
-        if (a.err_planes) {
+        if (a.err_planes && a.err_scale) {
+          const float rho = __ldg(a.err_scale + row);
+          uint32_t hp[CHUNK / 2], lp[CHUNK / 2];
+#pragma unroll
+          for (int t = 0; t < CHUNK; t += 2) {
+            uint16_t h0, l0, h1, l1;
+            split_half2(e[rr][t] * rho, h0, l0);
+            split_half2(e[rr][t + 1] * rho, h1, l1);
+            hp[t >> 1] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+            lp[t >> 1] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+          }
+          uint16_t* dst = a.err_planes + row * a.err_ld + j0;
+          reinterpret_cast<uint4*>(dst)[0] = make_uint4(hp[0], hp[1], hp[2], hp[3]);
+          reinterpret_cast<uint4*>(dst)[1] = make_uint4(hp[4], hp[5], hp[6], hp[7]);
+          reinterpret_cast<uint4*>(dst + a.plane_stride)[0] = make_uint4(lp[0], lp[1], lp[2], lp[3]);
+          reinterpret_cast<uint4*>(dst + a.plane_stride)[1] = make_uint4(lp[4], lp[5], lp[6], lp[7]);
+        } else if (a.err_planes) {
           uint32_t hp[CHUNK / 2], mp[CHUNK / 2], lp[CHUNK / 2];
 #pragma unroll
           for (int t = 0; t < CHUNK; t += 2) {

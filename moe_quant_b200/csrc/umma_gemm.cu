@@ -53,6 +53,9 @@ struct UmmaParams {
   uint32_t idesc;
   int mirror;  // symmetric result: every block above the diagonal is also stored transposed
   int c_tma;   // panel kernel epilogue: 0 = loads/stores by the warps, 1 = TMA store (beta == 0), 2 = TMA add (beta == 1)
+  int pairs;           // operands are pairs of fp16 planes: the leading product is summed per slab of k (see below)
+  const float* row_f;  // optional factors of the product per row / column of C
+  const float* col_f;
   int drain_slabs;  // streaming kernel: slabs of k per accumulator before it is added to C (0 = all of K)
 };
 
@@ -159,6 +162,30 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// v[i] *= alpha * row_f[row] * col_f[col + i] (the factors are powers of two: exact); M, N bound the reads.
+__device__ __forceinline__ void apply_factors(float (&v)[32], const UmmaParams& p, int row, int col) {
+  const float rf = p.alpha * ((p.row_f && row < p.M) ? __ldg(p.row_f + row) : 1.0f);
+  if (p.col_f) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = v[i] * rf * (col + i < p.N ? __ldg(p.col_f + col + i) : 1.0f);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] *= rf;
+  }
+}
+
+// One row (LEN columns) of an accumulator added to the sums in registers.
+template <int LEN>
+__device__ __forceinline__ void tmem_acc_row(uint32_t taddr, float (&sum)[LEN]) {
+#pragma unroll
+  for (int c = 0; c < LEN / 32; ++c) {
+    float v[32];
+    tmem_ld32(taddr + (uint32_t)(c * 32), v);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) sum[c * 32 + j] += v[j];
+  }
+}
+
 // Matrix descriptor of a K-major tile with the 128-byte swizzle: rows of 128 bytes,
 // groups of 8 rows 1024 bytes apart (stride byte offset), descriptor version 1.
 __device__ __forceinline__ uint64_t kmajor_sw128_desc(uint32_t smem_addr) {
@@ -230,6 +257,20 @@ __device__ __forceinline__ void issue_slab(uint32_t tmem_d, uint32_t small_off, 
       }
     }
   }
+}
+
+// One slab of fp16 pairs into a fresh accumulator: the corrections first (they lose nothing among themselves),
+// the leading products on top meet as many truncations as in an accumulator of their own.
+__device__ __forceinline__ void issue_slab_pairs(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile, uint32_t idesc) {
+  const uint64_t a0 = kmajor_sw128_desc(a_tile), b0 = kmajor_sw128_desc(b_tile);
+#pragma unroll
+  for (int kk = 0; kk < SLAB_K / 16; ++kk) {
+    const uint64_t ah = a0 + (uint64_t)((kk * 32) >> 4), bh = b0 + (uint64_t)((kk * 32) >> 4);
+    umma_bf16(tmem_d, ah, bh + (uint64_t)(PLANE_TILE_BYTES >> 4), idesc, kk > 0 ? 1u : 0u);
+    umma_bf16(tmem_d, ah + (uint64_t)(PLANE_TILE_BYTES >> 4), bh, idesc, 1u);
+  }
+#pragma unroll
+  for (int kk = 0; kk < SLAB_K / 16; ++kk) umma_bf16(tmem_d, a0 + (uint64_t)((kk * 32) >> 4), b0 + (uint64_t)((kk * 32) >> 4), idesc, 1u);
 }
 
 __device__ __forceinline__ void issue_slab_any(int planes, uint32_t tmem_d, uint32_t small_off, uint32_t a_tile, uint32_t b_tile,
@@ -633,6 +674,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_persistent_kernel(c
 // so the read-modify-write of C, the B loads and the tensor pipe overlap.
 constexpr int PANEL_MAX_RUN = 16;
 
+// 32 columns of a tile's result: leading + correction accumulator, or (pairs) the sums of the slabs.
+__device__ __forceinline__ void panel_acc_ld(uint32_t taddr, bool pairs, int n_slabs, uint32_t small_off, float (&v)[32]) {
+  tmem_ld32_sum(taddr, pairs ? (n_slabs > 1 ? (uint32_t)TILE_N : 0u) : small_off, v);
+}
 
 __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                   const __grid_constant__ CUtensorMap map_b,
@@ -676,6 +721,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
   const uint32_t small_off = p.planes > 1 ? (uint32_t)TILE_N : 0u;
   const uint32_t acc_stride = p.planes > 1 ? 2u * TILE_N : (uint32_t)TILE_N;
   const uint32_t tmem_cols = 2u * acc_stride;
+  // Pairs of fp16 planes: the products have 22 bits and the tensor core aligns them to the running sum
+  // and truncates, so each 64-wide slab of k gets an accumulator of its own (columns 0 and 128), corrections
+  // first, and the epilogue adds the two in round-to-nearest fp32.
+  const bool pairs = p.pairs != 0;
   if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), tmem_cols);
   tc_fence_before();
   __syncthreads();
@@ -728,7 +777,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
         if (lane == 0) {
           const uint32_t a_tile = smem_base + (uint32_t)(s * planes) * PLANE_TILE_BYTES;
           const uint32_t b_tile = b_base + (uint32_t)st * b_stage_bytes;
-          issue_slab_any(planes, tmem_acc + (uint32_t)acc * acc_stride, small_off, a_tile, b_tile, idesc, accumulate, accumulate_small);
+          if (pairs) issue_slab_pairs(tmem_acc + (uint32_t)acc * acc_stride + (uint32_t)(s * TILE_N), a_tile, b_tile, idesc);
+          else issue_slab_any(planes, tmem_acc + (uint32_t)acc * acc_stride, small_off, a_tile, b_tile, idesc, accumulate, accumulate_small);
           umma_commit(b_empty + 8 * st);  // the stage is free once these MMAs have read it
         }
         __syncwarp();
@@ -764,7 +814,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
 #pragma unroll 1
         for (int c = 0; c < TILE_N / 32; ++c, ++chunk) {
           float v[32];
-          tmem_ld32_sum(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_stride + (uint32_t)(c * 32), small_off, v);
+          panel_acc_ld(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_stride + (uint32_t)(c * 32), pairs, n_slabs, small_off, v);
           if (c == TILE_N / 32 - 1) {
             // the accumulator is in registers: hand its TMEM columns back to the MMA warp
             tc_fence_before();
@@ -774,11 +824,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
           if (lane == 0) bulk_wait_read_1();
           __syncwarp();
           const uint32_t dst = my_row + (uint32_t)(chunk & 1) * 4096u;
+          apply_factors(v, p, y + lane, n0 + c * 32);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((j ^ (lane & 7)) << 4)),
-                         "f"(p.alpha * v[4 * j]), "f"(p.alpha * v[4 * j + 1]), "f"(p.alpha * v[4 * j + 2]),
-                         "f"(p.alpha * v[4 * j + 3])
+                         "f"(v[4 * j]), "f"(v[4 * j + 1]), "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
                          : "memory");
           fence_async_smem();
           __syncwarp();
@@ -813,21 +863,27 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
             for (int it = 0; it < 8; ++it)
               old[c * 8 + it] = *reinterpret_cast<const float4*>(cq + (int64_t)(4 * it) * p.ldc + c * 32);
         }
+        // the row's factor is applied while a lane holds a row, the columns' after the turn
+        const float rf = p.alpha * (p.row_f ? __ldg(p.row_f + row) : 1.0f);
+        float4 cf[TILE_N / 32];
+#pragma unroll
+        for (int c = 0; c < TILE_N / 32; ++c)
+          cf[c] = p.col_f ? __ldg(reinterpret_cast<const float4*>(p.col_f + n0 + c * 32 + (lane & 7) * 4)) : make_float4(1.f, 1.f, 1.f, 1.f);
         ok = mbar_wait(acc_full + 8 * acc, (i >> 1) & 1, 15);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < TILE_N / 32; ++c) {
           float v[32];
-          tmem_ld32_sum(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_stride + (uint32_t)(c * 32), small_off, v);
+          panel_acc_ld(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_stride + (uint32_t)(c * 32), pairs, n_slabs, small_off, v);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4*>(&stage[lane * STAGE_LD + 4 * j]) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            *reinterpret_cast<float4*>(&stage[lane * STAGE_LD + 4 * j]) = make_float4(rf * v[4 * j], rf * v[4 * j + 1], rf * v[4 * j + 2], rf * v[4 * j + 3]);
           __syncwarp();
 #pragma unroll
           for (int it = 0; it < 8; ++it) {
             const float4 a4 = *reinterpret_cast<const float4*>(&stage[(4 * it + (lane >> 3)) * STAGE_LD + (lane & 7) * 4]);
-            float4 o = make_float4(p.alpha * a4.x, p.alpha * a4.y, p.alpha * a4.z, p.alpha * a4.w);
+            float4 o = make_float4(a4.x * cf[c].x, a4.y * cf[c].y, a4.z * cf[c].z, a4.w * cf[c].w);
             if (p.beta != 0.0f) {
               const float4 od = old[c * 8 + it];
               o.x = fmaf(p.beta, od.x, o.x); o.y = fmaf(p.beta, od.y, o.y);
@@ -845,13 +901,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
         for (int c = 0; c < TILE_N / 32; ++c) {
           const int col0 = n0 + c * 32;
           float v[32];
-          tmem_ld32_sum(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_stride + (uint32_t)(c * 32), small_off, v);
+          panel_acc_ld(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_stride + (uint32_t)(c * 32), pairs, n_slabs, small_off, v);
+          apply_factors(v, p, row, col0);
           if (row < p.M && col0 < p.N) {
             float* dst = dst_row + c * 32;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
               if (col0 + j < p.N) {
-                float o = p.alpha * v[j];
+                float o = v[j];
                 if (p.beta != 0.0f) o = fmaf(p.beta, dst[j], o);
                 dst[j] = o;
               }
@@ -1044,11 +1101,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_stream_kernel(const __gr
           if (lane == 0) bulk_wait_read_1();
           __syncwarp();
           const uint32_t dst = my_row + (uint32_t)(chunk & 1) * 4096u;
+          apply_factors(v, p, y + lane, n0 + c * 32);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((j ^ (lane & 7)) << 4)),
-                         "f"(p.alpha * v[4 * j]), "f"(p.alpha * v[4 * j + 1]), "f"(p.alpha * v[4 * j + 2]),
-                         "f"(p.alpha * v[4 * j + 3])
+                         "f"(v[4 * j]), "f"(v[4 * j + 1]), "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
                          : "memory");
           fence_async_smem();
           __syncwarp();
@@ -1082,6 +1139,253 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_stream_kernel(const __gr
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_acc, tmem_cols);
+  }
+}
+
+// ---------------------------------------------------------------- K > 128 with pairs of fp16 planes: CTA pairs
+// The far updates of the factorisation and of the inverse-free sweep (C += alpha A B^T, 512 of k, two fp16
+// planes per operand, three products).  Two CTAs of a cluster share one 256 x 256 output tile
+// (cta_group::2, M = 256): each keeps 128 rows of A and half of the 256 rows of B, so a slab of 64 of k costs an
+// SM 64 KB of operands for twice the output of a 128 x 128 tile.  That is what the tile size is for: with
+// 128 x 128 tiles per CTA, reading both operands fills the shared-memory bandwidth by itself (8 KB per 64
+// cycles) and the TMA's writes come on top.
+//   warp 0 of either CTA : TMA, its own rows, three stages of 64 KB; the bytes of both count on the leader's barrier
+//   warp 1 of the leader : tcgen05.mma (M 256, N 256) for both SMs, two accumulators by turns
+//   warps 4..7 / 8..11   : epilogue of the left / right 128 columns of the CTA's 128 rows (warps 2 and 3 only fill up the
+//                          warpgroup, whose registers go to the other two: 56 + 2 x 216 of 3 x 168).
+// The products of two 11-bit pieces have 22 bits; the tensor core aligns them to the running sum and
+// truncates.  So the leading sum is short: 64 of k, then the epilogue warps add it to the tile's fp32 values in
+// their registers (128 columns per thread) in round-to-nearest, and C is touched once per tile, by one add at
+// the L2.  Emptying an accumulator (commit, wait, read, an arrival at the other CTA, wait) takes about a
+// microsecond, as long as a slab's MMAs: hence two of them, and none left for the corrections.  Error of the factor of a
+// 7168-column Hessian against fp64 (2-norm, relative), three bf16 planes with one accumulator per 128 of k / this:
+// 9.0e-7 / 8.6e-7 after 4096 tokens, 5.4e-7 / 5.0e-7 after 7168, 3.8e-7 / 3.5e-7 after 14000.  All 26 deep updates
+// of a 2048 x 7168 layer: 1270 us / 855 us; of an attention block (widest layer 7168 x 16384) 18.5 ms / 10.5 ms.
+// Inside a tile the tensor pipe runs at its rate (1536 cycles per slab); what is left is the end of a tile, where
+// all SMs add 19 MB at once and the L2 takes them at about 5 TB/s.
+constexpr int PAIR_TILE = 256, PAIR_STAGES = 3, PAIR_THREADS = 384;
+constexpr uint32_t PAIR_STAGE_BYTES = 4 * PLANE_TILE_BYTES;
+constexpr size_t kPairSmem = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 8 * 4096 + 1024;
+
+__device__ __forceinline__ uint32_t leader_addr(uint32_t local) {   // the same shared-memory location in the cluster's CTA 0
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on this barrier of both CTAs once the MMAs issued so far have completed
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+// A wait that only the clock ends (a fault elsewhere does not): for copies that are under way.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+  uint64_t t0, now;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (;;) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    if (ok || now - t0 > 100000000ull) return;
+  }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+    umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                     const __grid_constant__ CUtensorMap map_c, const UmmaParams p, const int total) {
+  const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
+  const int n_tiles = (p.N + PAIR_TILE - 1) / PAIR_TILE;
+  const int my_tiles = (total - pair + n_pairs - 1) / n_pairs;   // the host launches at most one pair per tile
+  const int n_slabs = (p.K + SLAB_K - 1) / SLAB_K;
+
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  __shared__ __align__(8) uint64_t bars[2 * PAIR_STAGES + 4];
+  __shared__ uint32_t tmem_slot;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[PAIR_STAGES]);
+  // two accumulators of 256 columns, by slab & 1
+  const uint32_t acc_full = smem_u32(&bars[2 * PAIR_STAGES]), acc_empty = smem_u32(&bars[2 * PAIR_STAGES + 2]);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < PAIR_STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);    // the leader's: its producer's arrival, then the bytes of both CTAs
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full + 8 * b, 1);
+      mbar_init(acc_empty + 8 * b, 16);  // the leader's: eight epilogue warps of either CTA
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // either CTA's barriers and tensor memory exist before the other signals or writes them
+  tc_fence_after();
+  const uint32_t tmem_acc = tmem_slot;
+  chain_wait();
+  chain_release();
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 0) {
+      const uint32_t full_leader = leader_addr(full0);
+      int it = 0;
+      bool ok = true;
+      for (int i = 0; i < my_tiles && ok; ++i) {
+        TileWalk w;
+        w.seek(pair + i * n_pairs, n_tiles, p.upper_tiles_only);
+        const int a_row = w.m * PAIR_TILE + rank * TILE_M + p.a_row0;
+        const int b_row = w.n * PAIR_TILE + rank * TILE_N + p.b_row0;
+        for (int s = 0; s < n_slabs; ++s, ++it) {
+          const int st = it % PAIR_STAGES;
+          if (it >= PAIR_STAGES && !mbar_wait(empty0 + 8 * st, ((it / PAIR_STAGES) - 1) & 1, 51)) { ok = false; break; }
+          if (lane == 0) {
+            if (rank == 0) mbar_expect_tx(full0 + 8 * st, 2 * PAIR_STAGE_BYTES);
+            const uint32_t dst = smem_base + (uint32_t)st * PAIR_STAGE_BYTES;
+#pragma unroll
+            for (int pl = 0; pl < 2; ++pl) {
+              tma_load_3d_pair(dst + (uint32_t)pl * PLANE_TILE_BYTES, &map_a, full_leader + 8 * st, s * SLAB_K + p.a_k0, a_row, pl);
+              tma_load_3d_pair(dst + (uint32_t)(2 + pl) * PLANE_TILE_BYTES, &map_b, full_leader + 8 * st, s * SLAB_K + p.b_k0, b_row, pl);
+            }
+          }
+          __syncwarp();
+        }
+      }
+      if (!ok && rank == 0) {
+        // given up: the copies in flight land before this CTA's (and, behind the cluster barrier, the other's)
+        // shared memory goes away
+        for (int j = it > PAIR_STAGES ? it - PAIR_STAGES : 0; j < it; ++j) mbar_drain(full0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1);
+      }
+    } else if (warp == 1) {
+      if (rank == 0) {
+        int it = 0;
+        bool ok = true;
+        for (int i = 0; i < my_tiles && ok; ++i) {
+          for (int s = 0; s < n_slabs && ok; ++s, ++it) {
+            const int st = it % PAIR_STAGES;
+            ok = mbar_wait(full0 + 8 * st, (it / PAIR_STAGES) & 1, 52);
+            const int b = it & 1;
+            if (ok && it >= 2) ok = mbar_wait(acc_empty + 8 * b, ((it >> 1) - 1) & 1, 53);
+            if (!ok) break;
+            tc_fence_after();
+            if (lane == 0) {
+              const uint32_t a_tile = smem_base + (uint32_t)st * PAIR_STAGE_BYTES;
+              const uint64_t a0 = kmajor_sw128_desc(a_tile), b0 = kmajor_sw128_desc(a_tile + 2 * PLANE_TILE_BYTES);
+              const uint32_t acc = tmem_acc + (uint32_t)(b * PAIR_TILE);
+              // the corrections first: they lose nothing among themselves, and the leading products on top
+              // meet as many truncations as in an accumulator of their own
+#pragma unroll
+              for (int kk = 0; kk < SLAB_K / 16; ++kk) {
+                const uint64_t ah = a0 + (uint64_t)((kk * 32) >> 4), bh = b0 + (uint64_t)((kk * 32) >> 4);
+                umma_f16_pair(acc, ah, bh + (uint64_t)(PLANE_TILE_BYTES >> 4), p.idesc, kk > 0 ? 1u : 0u);
+                umma_f16_pair(acc, ah + (uint64_t)(PLANE_TILE_BYTES >> 4), bh, p.idesc, 1u);
+              }
+#pragma unroll
+              for (int kk = 0; kk < SLAB_K / 16; ++kk)
+                umma_f16_pair(acc, a0 + (uint64_t)((kk * 32) >> 4), b0 + (uint64_t)((kk * 32) >> 4), p.idesc, 1u);
+              umma_commit_pair(empty0 + 8 * st);
+              umma_commit_pair(acc_full + 8 * b);
+            }
+            __syncwarp();
+          }
+        }
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    const int h = (warp - 4) >> 2, q = warp & 3;   // half of the columns, TMEM lane quadrant
+    const uint32_t empty_leader = leader_addr(acc_empty);
+    const uint32_t t_lane = tmem_acc + ((uint32_t)(q * 32) << 16);
+    const uint32_t box = smem_base + (uint32_t)PAIR_STAGES * PAIR_STAGE_BYTES + (uint32_t)(warp - 4) * 4096u;
+    const uint32_t my_row = box + (uint32_t)lane * 128u;
+    bool ok = true;
+    int it = 0;
+#pragma unroll 1
+    for (int i = 0; i < my_tiles && ok; ++i) {
+      float acc[TILE_N];
+#pragma unroll
+      for (int j = 0; j < TILE_N; ++j) acc[j] = 0.0f;
+#pragma unroll 1
+      for (int s = 0; s < n_slabs; ++s, ++it) {
+        const int b = it & 1;
+        ok = mbar_wait(acc_full + 8 * b, (it >> 1) & 1, 54);
+        if (!ok) break;
+        tc_fence_after();
+        tmem_acc_row(t_lane + (uint32_t)(b * PAIR_TILE + h * TILE_N), acc);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * b);
+      }
+      if (!ok) break;
+      TileWalk w;
+      w.seek(pair + i * n_pairs, n_tiles, p.upper_tiles_only);
+      const int mb = 2 * w.m + rank, nb = 2 * w.n + h;          // 128-blocks
+      const int y = mb * TILE_M + q * 32, n0 = nb * TILE_N;
+      // inside a diagonal tile the 128-block below the diagonal is left alone
+      const bool keep = y < p.M && n0 < p.N && !(p.upper_tiles_only && mb > nb);
+      if (keep) {
+        const float rf = p.alpha * ((p.row_f && y + lane < p.M) ? __ldg(p.row_f + y + lane) : 1.0f);
+#pragma unroll
+        for (int c = 0; c < TILE_N / 32; ++c) {
+          const int x = n0 + c * 32;
+          if (lane == 0) bulk_wait_read_all();   // the box has left shared memory
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float4 f = make_float4(rf, rf, rf, rf);
+            if (p.col_f && x + 4 * j < p.N) {      // N % 4 == 0, col_f 16-byte aligned
+              const float4 g = __ldg(reinterpret_cast<const float4*>(p.col_f + x + 4 * j));
+              f = make_float4(rf * g.x, rf * g.y, rf * g.z, rf * g.w);
+            }
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(my_row + (uint32_t)((j ^ (lane & 7)) << 4)),
+                         "f"(f.x * acc[c * 32 + 4 * j]), "f"(f.y * acc[c * 32 + 4 * j + 1]), "f"(f.z * acc[c * 32 + 4 * j + 2]),
+                         "f"(f.w * acc[c * 32 + 4 * j + 3])
+                         : "memory");
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0 && x < p.N) {
+            tma_add_2d(&map_c, box, x, y);
+            bulk_commit();
+          }
+        }
+      }
+    }
+    if (lane == 0) bulk_wait_read_all();  // the boxes have left shared memory; the writes land before the grid completes
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // no MMA, copy or arrival of the other CTA is under way any more
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_acc) : "memory");
   }
 }
 
@@ -1202,6 +1506,88 @@ __global__ void __launch_bounds__(256) split_transposed_f32_kernel(SplitParams p
     *reinterpret_cast<uint32_t*>(dst) = (uint32_t)h0 | ((uint32_t)h1 << 16);
     if (p.planes > 1) *reinterpret_cast<uint32_t*>(dst + p.plane_stride) = (uint32_t)m0 | ((uint32_t)m1 << 16);
     if (p.planes > 2) *reinterpret_cast<uint32_t*>(dst + 2 * p.plane_stride) = (uint32_t)l0 | ((uint32_t)l1 << 16);
+  }
+}
+
+// Column maxima of the factor's blocks above the diagonal: colmax[j] = max_i |U[i][j]| over the rows in
+// front of column j's 128-block, as the bits of a non-negative float (they order like integers).  Only for a
+// factor that was not equilibrated: entries of an equilibrated one lie below 2^14.  One CTA takes 128 columns x `rows_per` rows: a warp reads 512 bytes of a row at a time, four in flight.
+__global__ void __launch_bounds__(256) factor_colmax_kernel(const float* __restrict__ U, int64_t ldu, int C, int rows_per,
+                                                            int* __restrict__ colmax) {
+  __shared__ float part[8][TILE_N];
+  const int j0 = ((int)blockIdx.x + 1) * TILE_N;   // the first block of columns has nothing above it
+  const int r_begin = (int)blockIdx.y * rows_per;
+  const int r_end = r_begin + rows_per < j0 ? r_begin + rows_per : j0;
+  if (r_begin >= r_end) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = j0 + lane * 4;
+  float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < C) {
+    for (int r = r_begin + warp; r < r_end; r += 32) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int rr = r + 8 * u;
+        v[u] = rr < r_end ? __ldg(reinterpret_cast<const float4*>(U + (int64_t)rr * ldu + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        m.x = fmaxf(m.x, fabsf(v[u].x)); m.y = fmaxf(m.y, fabsf(v[u].y));
+        m.z = fmaxf(m.z, fabsf(v[u].z)); m.w = fmaxf(m.w, fabsf(v[u].w));
+      }
+    }
+  }
+  *reinterpret_cast<float4*>(&part[warp][lane * 4]) = m;
+  __syncthreads();
+  if (threadIdx.x < TILE_N && j0 + (int)threadIdx.x < C) {
+    float x = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) x = fmaxf(x, part[w][threadIdx.x]);
+    atomicMax(colmax + j0 + threadIdx.x, __float_as_int(x));
+  }
+}
+
+// See make_factor_planes_half.  64 x 64 tiles as in split_transposed_f32_kernel.
+__global__ void __launch_bounds__(256) split_factor_half_kernel(const float* __restrict__ U, int64_t ldu, int C, int rows_pad, int K_pad,
+                                                                const float* __restrict__ col_div, const float* __restrict__ eq,
+                                                                const int* __restrict__ colmax, float* __restrict__ inv_t,
+                                                                uint16_t* __restrict__ dst, int64_t plane_stride) {
+  __shared__ float tile[64][65];  // tile[k][r]
+  const int r0 = blockIdx.y * 64, k0 = blockIdx.x * 64;
+  if (k0 >= (r0 / TILE_M) * TILE_M) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = k0 + warp + 8 * i;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = r0 + lane + 32 * h;
+      tile[warp + 8 * i][lane + 32 * h] = r < C ? __ldg(U + (int64_t)k * ldu + r) : 0.0f;   // k < r0 <= C
+    }
+  }
+  const int k = k0 + 2 * lane;
+  const float f0 = eq ? 1.0f / __ldg(eq + k) : 1.0f, f1 = eq ? 1.0f / __ldg(eq + k + 1) : 1.0f;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int rl = warp + 8 * i;
+    const int r = r0 + rl;
+    if (r >= rows_pad) continue;
+    float x0 = 0.0f, x1 = 0.0f;
+    if (r < C) {
+      const float d = col_div ? __ldg(col_div + r) : 1.0f, e = eq ? __ldg(eq + r) : 1.0f;
+      const float t = scale_below_2_14((eq ? 16384.0f / __ldg(eq + C) : __int_as_float(__ldg(colmax + r))) * e / d);
+      if (blockIdx.x == 0 && lane == 0) inv_t[r] = 1.0f / t;
+      const float m = e * t;
+      x0 = tile[2 * lane][rl] / d * f0 * m;
+      x1 = tile[2 * lane + 1][rl] / d * f1 * m;
+    }
+    uint16_t h0, l0, h1, l1;
+    split_half2(x0, h0, l0);
+    split_half2(x1, h1, l1);
+    uint16_t* o = dst + (int64_t)r * K_pad + k;
+    *reinterpret_cast<uint32_t*>(o) = (uint32_t)h0 | ((uint32_t)h1 << 16);
+    *reinterpret_cast<uint32_t*>(o + plane_stride) = (uint32_t)l0 | ((uint32_t)l1 << 16);
   }
 }
 
@@ -1351,6 +1737,7 @@ int configure_once() {
     MQ_CUDA(cudaFuncSetAttribute(umma_gemm_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
     MQ_CUDA(cudaFuncSetAttribute(umma_gemm_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
     MQ_CUDA(cudaFuncSetAttribute(umma_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    MQ_CUDA(cudaFuncSetAttribute(umma_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
     MQ_CUDA(cudaFuncSetAttribute(umma_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
     done[dev & 63] = true;
   }
@@ -1359,6 +1746,10 @@ int configure_once() {
 
 int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStream_t st) {
   MQ_TRY(configure_once());
+  // only the two kernels of the rank-<=128 and the deep updates apply row and column factors
+  MQ_REQUIRE((!d.row_f && !d.col_f) || (A.planes > 1 && d.batch == 1 && !d.a_upper && !d.b_upper && !d.n_step && !d.mirror_to_lower && d.K > 0),
+             MQ_ERR_UNSUPPORTED, "tensor engine: row and column factors need a plain update with several planes");
+  MQ_REQUIRE(!d.col_f || aligned(d.col_f, 16), MQ_ERR_ALIGNMENT, "tensor engine: column factors must be 16-byte aligned");
   CUtensorMap map_a, map_b;
   MQ_TRY(encode_map(A, &map_a));
   MQ_TRY(encode_map(B, &map_b));
@@ -1372,6 +1763,8 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
   p.a_rows_pad = A.rows_pad; p.b_rows_pad = B.rows_pad;
   p.a_row0 = (int)A.row0; p.a_k0 = A.k0; p.b_row0 = (int)B.row0; p.b_k0 = B.k0;
   p.planes = A.planes;
+  p.pairs = (A.planes == 2 && A.fp16) ? 1 : 0;
+  p.row_f = d.row_f; p.col_f = d.col_f;
   p.drain_slabs = 0;
   p.nterms = 0;
   for (int i = 0; i < A.planes; ++i)
@@ -1428,7 +1821,19 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
     const size_t staging = p.c_tma ? (size_t)4 * 2 * 4096 : (size_t)STAGE_BYTES;
     const size_t psmem = (size_t)4 * A.planes * PLANE_TILE_BYTES + 1024 + staging;  // A: two slabs, B: two stages, staging
     MQ_CUDA(launch_chained(true, umma_panel_kernel, pgrid, dim3(GEMM_THREADS), psmem, st, map_a, map_b, map_c, p, run));
-  } else if (A.planes > 1 && d.batch == 1 && !d.a_upper && !d.b_upper && !d.n_step && !d.mirror_to_lower && d.K > 2 * SLAB_K) {
+  } else if (deep_route && p.pairs) {
+    // deep update of operand pairs: C is added to at the L2
+    MQ_REQUIRE(d.beta == 1.0f && (d.ldc & 3) == 0 && (d.N & 3) == 0 && aligned(d.C, 16) && (!d.col_f || aligned(d.col_f, 16)) &&
+                   (!d.upper_tiles_only || d.M == d.N),
+               MQ_ERR_ALIGNMENT, "tensor engine: a deep update of fp16 pairs needs beta == 1 and 16-byte aligned rows of C");
+    const int m_tiles = (int)ceil_div(d.M, PAIR_TILE), n_tiles = (int)ceil_div(d.N, PAIR_TILE);
+    const long long tiles = d.upper_tiles_only ? (long long)n_tiles * (n_tiles + 1) / 2 : (long long)m_tiles * n_tiles;
+    CUtensorMap map_c;
+    MQ_TRY(encode_c_map(d.C, d.ldc, d.M, d.N, &map_c));
+    p.idesc = (1u << 4) | ((uint32_t)(PAIR_TILE >> 3) << 17) | ((uint32_t)(PAIR_TILE >> 4) << 24);   // fp16, fp32 sums, M 256, N 256
+    MQ_CUDA(launch_chained(true, umma_pair_kernel, dim3((unsigned)(2 * (tiles < 74 ? tiles : 74))), dim3(PAIR_THREADS), kPairSmem, st,
+                           map_a, map_b, map_c, p, (int)tiles));
+  } else if (deep_route) {
     // deep update with several planes: persistent streaming kernel
     const int m_tiles = (int)ceil_div(d.M, TILE_M), n_tiles = (int)ceil_div(d.N, TILE_N);
     long long tiles = (long long)m_tiles * n_tiles;
@@ -1443,6 +1848,7 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
       MQ_TRY(encode_c_map(d.C, d.ldc, d.M, d.N, &map_c));
       p.c_tma = d.beta == 0.0f ? 1 : 2;
     }
+    MQ_REQUIRE(p.c_tma || (!d.row_f && !d.col_f), MQ_ERR_ALIGNMENT, "tensor engine: row and column factors need 16-byte aligned rows of C");
     p.drain_slabs = (d.k_round > 0 && p.c_tma == 2) ? d.k_round / SLAB_K : 0;
     const size_t staging = p.c_tma ? (size_t)4 * 2 * 4096 : (size_t)STAGE_BYTES;
     const size_t ssmem = (size_t)4 * A.planes * PLANE_TILE_BYTES + 1024 + staging;   // two stages of A and B slabs, staging
@@ -1475,7 +1881,7 @@ int gemm_tensor_planes(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, 
   if (d.M <= 0 || d.N <= 0 || d.batch <= 0) return MQ_OK;
   MQ_REQUIRE(A.planes == B.planes && A.planes >= 1 && A.planes <= 3 && A.fp16 == B.fp16, MQ_ERR_ARGUMENT,
              "tensor engine: operand plane sets do not match");
-  if (d.k_round > 0 && d.K > d.k_round) {
+  if (d.k_round > 0 && d.K > d.k_round && !(A.planes == 2 && A.fp16)) {   // (pairs are summed per slab of k anyway)
     MQ_REQUIRE(d.k_round % SLAB_K == 0 && d.beta == 1.0f && d.batch == 1, MQ_ERR_ARGUMENT,
                "tensor engine: k_round needs a multiple of %d, beta == 1 and one batch", SLAB_K);
     const bool c_tma = (d.ldc & 3) == 0 && (d.N & 3) == 0 && (reinterpret_cast<uintptr_t>(d.C) & 15) == 0;
@@ -1500,6 +1906,32 @@ int make_planes_f32(const float* src, int64_t rs, int64_t cs, int rows, int K, i
                     cudaStream_t st, bool only_k_blocks_before_rows, const float* row_div) {
   Workspace ws(dst, plane_set_bytes(rows, K, planes));
   return make_planes(src, MQ_F32, rs, cs, 0, rows, K, 1, planes, 0, 0, 0, 0, ws, out, st, only_k_blocks_before_rows, row_div);
+}
+
+int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, float* inv_t, const float* col_div, const float* eq,
+                            PlaneSet* out, cudaStream_t st) {
+  PlaneSet ps;
+  ps.planes = 2;
+  ps.rows_pad = pad_to(C, TILE_M);
+  ps.K_pad = pad_to(C, SLAB_K);
+  ps.total_rows = ps.rows_pad;
+  ps.fp16 = true;
+  ps.base = dst;
+  *out = ps;
+  if (C <= TILE_M) return MQ_OK;   // no block above the diagonal
+  int* colmax = reinterpret_cast<int*>(inv_t + C);
+  ProfScope prof(PROF_SPLIT, (double)C * C * 0.5 * (4.0 + 4.0), 0.0, st);
+  if (!eq) {
+    MQ_CUDA(cudaMemsetAsync(colmax, 0, (size_t)C * sizeof(int), st));
+    const int col_blocks = (int)ceil_div(C, TILE_N) - 1;
+    const int rows_per = 128;
+    factor_colmax_kernel<<<dim3((unsigned)col_blocks, (unsigned)ceil_div(C, rows_per)), 256, 0, st>>>(U, ldu, C, rows_per, colmax);
+    MQ_LAUNCH_CHECK();
+  }
+  split_factor_half_kernel<<<dim3((unsigned)(ps.K_pad / 64), (unsigned)ceil_div(ps.rows_pad, 64)), 256, 0, st>>>(
+      U, ldu, C, ps.rows_pad, ps.K_pad, col_div, eq, colmax, inv_t, dst, ps.total_rows * (int64_t)ps.K_pad);
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
 }
 
 size_t engine_workspace_bytes(int64_t M, int64_t N, int64_t K, int math, int split) {

@@ -435,6 +435,60 @@ def test_dequantize_every_type_and_group(cuda, R, C, g, out, held):
         assert torch.equal(got, ((codes.float() - zf) * wide_s).to(out))
 
 
+# ------------------------------------------------------------------ operand pairs of the factorisation and the sweep
+@pytest.mark.parametrize("C,tokens,spread", [(8, 40, 1.0), (128, 200, 1.0), (136, 300, 1.0), (520, 700, 1.0), (640, 640, 2.0), (1032, 1500, 1.0),
+                                             (1544, 2000, 3.0)])
+@pytest.mark.parametrize("units", [1.0, 1e-12, 1e10])
+def test_factor_of_operand_pairs_against_fp64(cuda, C, tokens, spread, units):
+    """Super-panel edges (512), ragged last panels, channels whose scales spread over decades and
+    Hessians far from 1: the factor is as close to fp64 as the one of the fp32 CUDA cores, whose error is the
+    rounding of the same sums (2x: another order of additions)."""
+    gen = torch.Generator().manual_seed(C)
+    X = torch.randn(tokens, C, generator=gen, dtype=torch.float64) * torch.exp(spread * torch.randn(C, generator=gen, dtype=torch.float64))
+    H = X.T @ X * (units / tokens)
+    H.diagonal().add_(0.01 * H.diagonal().mean())
+    H32 = H.float()
+    T = torch.linalg.cholesky(H32.double().flip(0, 1)).flip(0, 1)
+    U64 = T / T.diagonal()[None, :]
+
+    def error(math):
+        U = H32.to(cuda)
+        flags, diag = ops.chol_unit_factor(U, ops.Precision(math=math))
+        assert int(flags[3]) == 0
+        e = ((U.cpu().double() - U64).norm(dim=0) / U64.norm(dim=0)).norm()
+        return float(e), float(((diag.cpu().double() - T.diagonal()) / T.diagonal()).abs().max())
+
+    got, ref = error(MATH_TENSOR), error(MATH_FP32)
+    assert got[0] <= 2 * ref[0] + 1e-6 and got[1] <= 2 * ref[1] + 1e-6
+
+
+@pytest.mark.parametrize("R,C,g,dtype", [(1, 648, 8, torch.bfloat16), (129, 1032, 24, torch.float16), (257, 1664, 128, torch.bfloat16),
+                                         (300, 776, 97 * 8, torch.float32), (40, 1280, 64, torch.bfloat16)])
+@pytest.mark.parametrize("size", [1.0, 1e-6, 1e3])
+def test_sweep_of_operand_pairs_against_fp32_math(cuda, R, C, g, dtype, size):
+    """Deep updates whose last 256 x 256 tile is ragged in rows and columns, rows of very different size,
+    a row of zeros: the codes of the fp32 CUDA cores."""
+    if dtype == torch.float16 and size < 1:
+        size = 1e-2     # the scales must be representable
+    W = synthetic.layer_weight(R, C, 5, torch.float32) * size
+    W[::3] *= 0.125
+    if R > 2:
+        W[2] = 0.0
+    W = W.to(dtype)
+    X = synthetic.activations(2 * C, C, 6, torch.bfloat16).float()
+    H = X.T @ X / C
+
+    def run(math):
+        p = ops.Precision(math=math)
+        codes, scales, _, flags = ops.quantize_layer([W.to(cuda)], H.to(cuda), g, 4, 1e-2, precision=p)
+        assert int(flags[3]) == 0
+        return codes[0].cpu(), scales[0].cpu()
+
+    (q, s), (q0, s0) = run(MATH_TENSOR), run(MATH_FP32)
+    assert torch.equal(s, s0)
+    assert O.code_agreement(q, q0) >= CODE_AGREEMENT
+
+
 # ------------------------------------------------------------------ MSE scale search
 @pytest.mark.parametrize("R,C,g,dtype", [(64, 512, 128, torch.bfloat16), (40, 256, 32, torch.float16),
                                          (24, 384, 64, torch.float32), (8, 2048, 2048, torch.bfloat16)])
