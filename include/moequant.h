@@ -49,14 +49,16 @@ typedef enum { MQ_F32 = 0, MQ_BF16 = 1, MQ_F16 = 2 } mq_dtype;
  *   MQ_MATH_TENSOR: tcgen05 tensor cores with fp32 TMEM accumulators.  bf16/fp16
  *                   operands enter exactly; fp32 operands are split into up to
  *                   three bf16 planes whose cross products are accumulated
- *                   (`split` planes: 1 -> 1 product, 2 -> 3, 3 -> 6).          */
+ *                   (`split` planes: 1 -> 1 product, 2 -> 3, 3 -> 6).  With split 3 the
+ *                   factorisation and the inverse-free sweep use pairs of fp16
+ *                   planes scaled by powers of two (3 products), at the same accuracy.  */
 typedef enum { MQ_MATH_FP32 = 0, MQ_MATH_TENSOR = 1 } mq_math;
 
 /* Flag that may be OR-ed into the `math` argument of mq_gptq_sweep and mq_quantize_layer (and of
  * their *_workspace_bytes): the caller processes several layers at once on different streams
  * (gptq.quantize_many).  The library then prefers launch shapes that occupy few SMs over the
- * lowest latency of a single layer: the sweep's tiles run one weight row per thread on R/64
- * SMs instead of sixteen lanes per row on R/8 CTAs, a CTA of a rank-128 strip update walks a whole
+ * lowest latency of a single layer: the sweep's tiles take more rows per CTA (R/44
+ * instead of R/148, at most 64), a CTA of a rank-128 strip update walks a whole
  * row of output tiles, a CTA of a panel solve takes 64 rows instead of 32.  Results are bit-identical with and without it. */
 #define MQ_MATH_COMPACT 0x100
 

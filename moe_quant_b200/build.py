@@ -40,8 +40,8 @@ def _stale(target: str, deps: list[str]) -> bool:
 
 def _includes(path: str, dirs, seen=None):
     """`path` and every file it includes with quotes, recursively (searched in `dirs`): a source
-    is recompiled when one of these is newer than its object.  The row-per-thread sweep kernels
-    take minutes to compile, so a change elsewhere should not rebuild them."""
+    is recompiled when one of these is newer than its object.  The largest sources
+    take half a minute to compile, so a change elsewhere should not rebuild them."""
     seen = seen if seen is not None else []
     if path in seen:
         return seen

@@ -2,18 +2,13 @@
 // reference's captured loop (src/gptq_loop.py:141-148) with, per 128-column tile,
 // ONE sweep kernel plus ONE GEMM.
 //
-// Sweep kernel: sixteen lanes share one weight row, lane l keeps columns 8l..8l+7 of the
-// current tile in registers (two rows per warp).  Column j is quantized as
+// Sweep kernel: a CTA takes up to 64 weight rows through the tile in sub-blocks of sixteen columns.
+// Column j is quantized as
 //   q = clamp(floor(x/s + z + 0.5), 0, maxq)   y = round_to_dtype((q - z) s)   e = y - x
 // (src/gptq_loop.py:28-40, src/quant_utils.py:30-49) and its error is applied to the columns
 // behind it, w_k += Uhat[j,k] e (src/gptq_loop.py:83-88), with one fma per (j, k) in
-// increasing j: the reference's order.  The eight columns of a lane are a chain that needs
-// no communication (the lane applies each error to its own later columns at once), so the
-// tile is sixteen such chains back to back; after a chain its eight errors are broadcast with
-// shuffles and the other lanes of the row apply them to their columns.  Rows are independent:
-// no block-wide synchronisation after the tile of Uhat is staged in shared memory.
-// (sweep_rows.cuh holds the same tile with one row per thread, for callers that run several
-// layers at once.)
+// increasing j: the reference's order.  One thread per row runs the sixteen dependent steps of a
+// sub-block; the other warps apply the errors to the rest of the tile.
 //
 // The errors of the tile (R x 128) go to a scratch matrix, as bf16 planes on the tensor path,
 // and the lazy update
@@ -26,278 +21,349 @@
 #include "engine.cuh"
 #include "profile.cuh"
 #include "sweep.cuh"
-#include "sweep_rows.cuh"
 
 namespace mq {
 
 namespace {
 
 constexpr int TILE = SWEEP_TILE;
-constexpr int TILE_THREADS = 128;                        // threads per CTA of the lane-per-chunk kernel
-// LANES lanes share one weight row and keep TILE / LANES consecutive columns each.  Sixteen lanes
-// (8 columns, 8 rows per CTA) give the shorter serial stream per warp: 4.83 against 5.03 ms per
-// 2048 x 7168 layer on one stream (with 256 threads per CTA 4.95 ms); a layer with more rows than
-// the grid holds at that shape walks its row groups in turns, and eight lanes (16 columns, 16 rows
-// per CTA) are faster again (7168 x 2048: 623 against 586 layers/s).  4 columns per lane would
-// need shuffles to form the 8-column vectors in which codes, packed words and error planes leave.
-// The tile of the factor in shared memory: row j holds LANES chunks, 4 floats of padding after
-// each, so that the lanes of a quarter-warp read their 16-byte pieces from disjoint banks.
-template <int LANES>
-struct LaneShape {
-  static constexpr int ROW_LANES = LANES;
-  static constexpr int LANE_COLS = TILE / LANES;
-  static constexpr int U_LANE_LD = LANE_COLS + 4;
-  static constexpr int U_ROW_LD = LANES * U_LANE_LD;       // 160 floats for 8 lanes, 192 for 16
-  static constexpr size_t smem = (size_t)TILE * U_ROW_LD * sizeof(float);
-};
-constexpr int MAX_SWEEP_CTAS = 2 * 148;
+constexpr int SUB = 16;                 // columns of a sub-block: one chain of quantisation steps per row
+constexpr int N_SUB = TILE / SUB;
+constexpr int SWEEP_THREADS = 256;
+constexpr int MAX_ROWS = 64;            // rows of a CTA's group
+constexpr int W_LD = TILE + 4;          // row stride of the running weights: a warp's 16-byte reads of 8 rows hit 32 banks
 // Four tiles form a super-block of 512 columns.  Behind each tile only the rest of its own
 // super-block takes the rank-128 update at once; the columns behind the super-block are updated
 // once per super-block with all 512 errors of a row in one contraction, so a tile of W is read
 // and written once per 512 instead of once per 128 swept columns.
 constexpr int SUPER = 4 * TILE;
 
-// One 128 x 128 tile of the factor (top-left element at `src`) -> shared memory in the chunked
-// row layout, strict upper triangle only.  stage: issue the copies (asynchronous 16-byte copies,
-// all in flight at once; a copy with source size 0 writes zeros: everything below the diagonal
-// and past nb); trim: wait for them and zero the entries on and below the diagonal inside each
-// row's diagonal quad.  Every thread of the CTA must call both.
-template <int LANES>
-__device__ __forceinline__ void stage_factor_tile(float* ublk, const float* __restrict__ src, int64_t ldu, int nb) {
-  constexpr int LANE_COLS = LaneShape<LANES>::LANE_COLS, U_LANE_LD = LaneShape<LANES>::U_LANE_LD, U_ROW_LD = LaneShape<LANES>::U_ROW_LD;
+constexpr size_t sweep_smem_bytes(int rows, bool uniform) {
+  return (size_t)(TILE * TILE + rows * W_LD + rows * (uniform ? N_SUB : 2 * SUB) * 4) * sizeof(float);
+}
+
+// One 128 x 128 tile of the factor (top-left element at `src`) -> shared memory, row-major, by
+// asynchronous 16-byte copies, all in flight at once.  Quads that lie below the diagonal are not
+// copied and not read; everything past nb becomes zero (a copy with source size 0).
+__device__ __forceinline__ void stage_factor_tile(float* us, const float* __restrict__ src, int64_t ldu, int nb) {
   for (int idx = threadIdx.x; idx < TILE * TILE / 4; idx += blockDim.x) {
     const int j = idx >> 5, k4 = (idx & 31) * 4;
-    const bool keep = j < nb && k4 < nb && k4 + 3 > j;
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&ublk[j * U_ROW_LD + (k4 / LANE_COLS) * U_LANE_LD + (k4 % LANE_COLS)]);
+    if (k4 + 3 <= j) continue;
+    const bool keep = j < nb && k4 < nb;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&us[j * TILE + k4]);
     const float* g = keep ? src + (int64_t)j * ldu + k4 : src;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(g), "r"(keep ? 16 : 0) : "memory");
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-template <int LANES>
-__device__ __forceinline__ void trim_factor_tile(float* ublk, int nb) {
-  constexpr int LANE_COLS = LaneShape<LANES>::LANE_COLS, U_LANE_LD = LaneShape<LANES>::U_LANE_LD, U_ROW_LD = LaneShape<LANES>::U_ROW_LD;
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-  for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-    const int k4 = j & ~3;
-    float* q = &ublk[j * U_ROW_LD + (k4 / LANE_COLS) * U_LANE_LD + (k4 % LANE_COLS)];
-    for (int k = 0; k <= (j & 3); ++k) q[k] = 0.0f;
-  }
-  __syncthreads();
-}
-
-// UNIFORM: the columns of a lane lie in one quantization group (group % LANE_COLS == 0).
-template <int DT, bool UNIFORM, int LANES>
-__global__ void __launch_bounds__(TILE_THREADS) sweep_tile_kernel(const SweepArgs a) {
-  constexpr int ROW_LANES = LANES, LANE_COLS = LaneShape<LANES>::LANE_COLS;
-  constexpr int U_LANE_LD = LaneShape<LANES>::U_LANE_LD, U_ROW_LD = LaneShape<LANES>::U_ROW_LD;
-  constexpr int ROWS_PER_CTA = TILE_THREADS / ROW_LANES;
+// One 128-column tile of the sweep for up to MAX_ROWS rows per CTA, in eight sub-blocks of sixteen columns.
+// Thread r < rows takes row r through sub-block c:
+//   chain:  the sixteen columns in order, in registers: quantize column j, add e_j U[j, k] to the columns k behind
+//           it inside the sub-block.  The only serial dependence is quantize(j) -> one FMA -> quantize(j + 1),
+//           about fifteen operations;
+//   next:   the sixteen errors go to the sixteen columns of sub-block c + 1, which it then holds.
+// Meanwhile the other warps add the errors of sub-block c - 1 to the columns from sub-block c + 1 on: a lane
+// keeps the 16 x 4 entries of the factor for its four columns in registers and walks the rows.  One barrier
+// per sub-block hands the errors over and orders the two: before `next` touches sub-block c + 1 the other
+// warps have added everything up to c - 1 there.  Every element so takes the errors in increasing column order
+// with one FMA each, as a column-at-a-time recurrence does.
+// What bounds a tile is the chain, 128 steps whatever the number of rows: 4.4 us at 65 cycles per step.  (With
+// sixteen or eight lanes per row and the row's tile in their registers, the owner of a chunk ran its chain while
+// the others waited, and both the chain and the rest were one serial instruction stream: 19 us for 2048 rows,
+// 36 us for 7168; one row per thread for everything, 30 us.  Now 16.5 and 20 us, and 15.7 instead of 20.3 us
+// with a scale per column; a step of the chain takes 84 cycles, handing a sub-block over 800 to 1100.)
+// UNIFORM: the columns of a sub-block lie in one quantization group (group % 16 == 0).
+// INVERSE_FREE (a.Worig given): U is the unit factor Utilde = Uhat^-1 and what is propagated is minus the
+// total change of the column, -(y - w_original), instead of the error against the running value;
+// x_j = w_j - sum_{i<j} (y_i - w_i) Utilde[i,j] is the same number as the reference's running weight
+// (E Uhat = Y - W  <=>  E = (Y - W) Utilde).
+template <int DT, bool UNIFORM, bool INVERSE_FREE>
+__global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const SweepArgs a, const int group_rows) {
   using T = typename StorageOf<DT>::type;
-  extern __shared__ __align__(16) float ublk[];  // [TILE][U_ROW_LD], strict upper triangle of the tile, 0 elsewhere
-  const int nb = a.nb, i1 = a.i1;
+  extern __shared__ __align__(16) float sweep_smem[];
+  float* us = sweep_smem;                            // [TILE][TILE], strict upper triangle
+  float* ws = sweep_smem + TILE * TILE;              // [group_rows][W_LD]: running weights, replaced by the errors as they become known
+  // the grid of every row (scale, its reciprocal, zero point): UNIFORM [N_SUB][group_rows], one per sub-block;
+  // otherwise [2][SUB][group_rows], the columns of two sub-blocks by turns
+  float4* gs = reinterpret_cast<float4*>(ws + group_rows * W_LD);
+  const int nb = a.nb, i1 = a.i1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // The factor is constant during the sweep: its tile is staged before this grid waits for the
   // rank-128 update that precedes it in the stream (only W depends on that update).
-  stage_factor_tile<LANES>(ublk, a.U + (int64_t)i1 * a.ldu + i1, a.ldu, nb);
+  stage_factor_tile(us, a.U + (int64_t)i1 * a.ldu + i1, a.ldu, nb);
   chain_wait();
   chain_release();
-  trim_factor_tile<LANES>(ublk, nb);
-
-  const int sub = threadIdx.x & (ROW_LANES - 1);   // this lane's chunk of the row
-  const int c_local = sub * LANE_COLS;
-  const int c0 = i1 + c_local;
   const float maxq = a.maxq;
-  // Inverse-free form (Worig != nullptr): U is the unit factor Utilde = Uhat^-1 and what is
-  // propagated is minus the total change of the column, -(y - w_original), instead of the
-  // error against the running value; x_j = w_j - sum_{i<j} (y_i - w_i) Utilde[i,j] is the same
-  // number as the reference's running weight (E Uhat = Y - W  <=>  E = (Y - W) Utilde).
-  const bool inverse_free = a.Worig != nullptr;
-  const int n_owner = (nb + LANE_COLS - 1) / LANE_COLS;
-  const int row_groups = (a.R + ROWS_PER_CTA - 1) / ROWS_PER_CTA;
+  const bool wide_codes = (a.C & 15) == 0 && (reinterpret_cast<uintptr_t>(a.codes) & 15) == 0;
+  const uint32_t group = (uint32_t)a.group;
 
-  // the CTA walks row groups together (the shuffles below are warp-wide); rows past R carry zeros
-  for (int rg = blockIdx.x; rg < row_groups; rg += gridDim.x) {
-    const int r = rg * ROWS_PER_CTA + (threadIdx.x / ROW_LANES);
-    const bool valid = r < a.R;
-    float w[LANE_COLS], wo[LANE_COLS];
-#pragma unroll
-    for (int qd = 0; qd < LANE_COLS / 4; ++qd) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f), vo = v;
-      if (valid && c_local + 4 * qd < nb) {
-        v = *reinterpret_cast<const float4*>(a.W + (int64_t)r * a.ldw + c0 + 4 * qd);
-        if (inverse_free) vo = *reinterpret_cast<const float4*>(a.Worig + (int64_t)r * a.ldwo + c0 + 4 * qd);
-      }
-      w[4 * qd] = v.x; w[4 * qd + 1] = v.y; w[4 * qd + 2] = v.z; w[4 * qd + 3] = v.w;
-      wo[4 * qd] = vo.x; wo[4 * qd + 1] = vo.y; wo[4 * qd + 2] = vo.z; wo[4 * qd + 3] = vo.w;
+  for (int row0 = blockIdx.x * group_rows; row0 < a.R; row0 += gridDim.x * group_rows) {
+    const int rows = a.R - row0 < group_rows ? a.R - row0 : group_rows;
+    const int chain_warps = (rows + 31) >> 5;
+    for (int idx = tid; idx < rows * (TILE / 4); idx += SWEEP_THREADS) {
+      const int r = idx >> 5, k4 = (idx & 31) * 4;
+      const bool keep = k4 < nb;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&ws[r * W_LD + k4]);
+      const float* g = a.W + (int64_t)(row0 + r) * a.ldw + i1 + (keep ? k4 : 0);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(g), "r"(keep ? 16 : 0) : "memory");
     }
-    // grid of the lane's columns; x / s goes through the reciprocal and one correction step (the
-    // final stage of a correctly rounded division): a few FMAs on the serial chain instead of
-    // the full division sequence
-    constexpr int NS = UNIFORM ? 1 : LANE_COLS;
-    float sc[NS], zr[NS], rs[NS];
-#pragma unroll
-    for (int t = 0; t < NS; ++t) {
-      sc[t] = 1.0f;
-      zr[t] = a.zero_default;
-      if (valid && c_local + t < nb) {
-        const int64_t off = (int64_t)r * a.s_rs + (int64_t)((c0 + t) / a.group) * a.s_gs;
-        sc[t] = __ldg(a.scale + off);
-        if (a.zero) zr[t] = __ldg(a.zero + off);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    auto grid_of = [&](int r, int j) {   // column j of the tile
+      float s = 1.0f, z = a.zero_default;
+      if (j < nb) {
+        const int64_t off = (int64_t)(row0 + r) * a.s_rs + (int64_t)((uint32_t)(i1 + j) / group) * a.s_gs;
+        s = __ldg(a.scale + off);
+        if (a.zero) z = __ldg(a.zero + off);
       }
-      rs[t] = 1.0f / sc[t];
+      return make_float4(s, 1.0f / s, z, 0.0f);
+    };
+    auto fill_columns = [&](int c, int from, int step) {   // !UNIFORM: the sixteen columns of sub-block c
+      for (int idx = from; idx < rows * SUB; idx += step)
+        gs[((c & 1) * SUB + (idx & (SUB - 1))) * group_rows + idx / SUB] = grid_of(idx / SUB, c * SUB + (idx & (SUB - 1)));
+    };
+    if constexpr (UNIFORM) {
+      for (int idx = tid; idx < rows * N_SUB; idx += SWEEP_THREADS) gs[(idx & 7) * group_rows + (idx >> 3)] = grid_of(idx >> 3, (idx & 7) * SUB);
+    } else {
+      fill_columns(0, tid, SWEEP_THREADS);
     }
-    // what this lane produces when its turn comes: the errors of its columns and their
-    // codes, two to a float (q0 + 256 q1 is exact for codes below 256)
-    float e[LANE_COLS], qacc[LANE_COLS / 2];
-#pragma unroll
-    for (int t = 0; t < LANE_COLS; ++t) e[t] = 0.0f;
-#pragma unroll
-    for (int h = 0; h < LANE_COLS / 2; ++h) qacc[h] = 0.0f;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
 
+    if (warp < chain_warps) {
+      // ---- chains.  Lanes past the last row repeat it and store nothing.
+      const bool valid = tid < rows;
+      const int r = valid ? tid : rows - 1;
+      const int64_t row = row0 + r;
+      float* wrow = ws + r * W_LD;
+      const float* worow = INVERSE_FREE ? a.Worig + row * a.ldwo + i1 : nullptr;
+      float w[SUB], wo[SUB];
+      auto fetch_original = [&](int j0) {
+#pragma unroll
+        for (int qd = 0; qd < SUB / 4; ++qd) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (INVERSE_FREE && j0 + 4 * qd < nb) v = __ldg(reinterpret_cast<const float4*>(worow + j0 + 4 * qd));
+          wo[4 * qd] = v.x; wo[4 * qd + 1] = v.y; wo[4 * qd + 2] = v.z; wo[4 * qd + 3] = v.w;
+        }
+      };
+      fetch_original(0);
+#pragma unroll
+      for (int qd = 0; qd < SUB / 4; ++qd) {
+        const float4 v = *reinterpret_cast<const float4*>(wrow + 4 * qd);
+        w[4 * qd] = v.x; w[4 * qd + 1] = v.y; w[4 * qd + 2] = v.z; w[4 * qd + 3] = v.w;
+      }
 #pragma unroll 1
-    for (int lo = 0; lo < n_owner; ++lo) {
-      if (sub == lo) {
-        // Chain of this lane's columns against its diagonal LANE_COLS x LANE_COLS block of the factor
-        // (the lanes of the warp that own chunk `lo` of their rows run it; the others wait).
-        // A step applies the error to the whole quad rows behind it: entries on and below the
-        // diagonal are zero in the staged tile and the columns they touch are finished.
-        const float* ud = &ublk[(lo * LANE_COLS) * U_ROW_LD + lo * U_LANE_LD];
+      for (int c = 0; c < N_SUB; ++c) {
+        const int j0 = c * SUB;
+        constexpr int NS = UNIFORM ? 1 : SUB;
+        float sc[NS], zr[NS], rs[NS];
+        if constexpr (UNIFORM) {
+          const float4 g = gs[c * group_rows + r];
+          sc[0] = g.x; rs[0] = g.y; zr[0] = g.z;
+        } else {
 #pragma unroll
-        for (int t = 0; t < LANE_COLS; ++t) {
+          for (int t = 0; t < SUB; ++t) {
+            const float4 g = gs[((c & 1) * SUB + t) * group_rows + r];
+            sc[t] = g.x; rs[t] = g.y; zr[t] = g.z;
+          }
+        }
+        float e[SUB];
+        uint32_t cw[SUB / 4];
+        const float* ud = us + j0 * TILE + j0;   // the sub-block's own 16 x 16 block of the factor
+#pragma unroll
+        for (int t = 0; t < SUB; ++t) {
           const float s_t = sc[UNIFORM ? 0 : t], z_t = zr[UNIFORM ? 0 : t], r_t = rs[UNIFORM ? 0 : t];
+          float4 ur[SUB / 4];
+#pragma unroll
+          for (int qd = t >> 2; qd < SUB / 4; ++qd) {
+            if (qd == (t >> 2) && (t & 3) == 3) continue;
+            ur[qd] = *reinterpret_cast<const float4*>(ud + t * TILE + 4 * qd);
+          }
           const float x = w[t];
+          // x / s through the reciprocal and one residual correction (Markstein 1990): two FMAs on the chain
           float d = x * r_t;
           d = fmaf(fmaf(-s_t, d, x), r_t, d);
-          const float q = fminf(fmaxf(floorf((d + z_t) + 0.5f), 0.0f), maxq);
+          // clamp first, then floor (the bounds are whole numbers, so the order does not matter): adding 2^23
+          // with rounding towards minus infinity leaves the whole part, and the code in the low bits
+          const float v = fminf(fmaxf((d + z_t) + 0.5f, 0.0f), maxq);
+          const float big = __fadd_rd(v, 8388608.0f);
+          const float q = big - 8388608.0f;
           const float y = round_through<DT>((q - z_t) * s_t);
-          const float et = inverse_free ? (wo[t] - y) : (y - x);
+          const float et = INVERSE_FREE ? (wo[t] - y) : (y - x);
           e[t] = et;
-          qacc[t >> 1] = (t & 1) ? fmaf(q, 256.0f, qacc[t >> 1]) : q;
+          const uint32_t code = __float_as_uint(big) & 0xFFu;
+          if ((t & 3) == 0) cw[t >> 2] = code;
+          else cw[t >> 2] |= code << (8 * (t & 3));
+          // the rest of t's own quad one by one, whole quads after it
+          if ((t & 3) != 3) {
+            const float4 u = ur[t >> 2];
+            if ((t & 3) < 1) w[(t & ~3) + 1] = fmaf(u.y, et, w[(t & ~3) + 1]);
+            if ((t & 3) < 2) w[(t & ~3) + 2] = fmaf(u.z, et, w[(t & ~3) + 2]);
+            w[(t & ~3) + 3] = fmaf(u.w, et, w[(t & ~3) + 3]);
+          }
           const float2 e2 = make_float2(et, et);
 #pragma unroll
-          for (int qd = (t + 1) >> 2; qd < LANE_COLS / 4; ++qd) {
-            const float4 u = *reinterpret_cast<const float4*>(&ud[t * U_ROW_LD + 4 * qd]);
+          for (int qd = (t >> 2) + 1; qd < SUB / 4; ++qd) {
+            const float4 u = ur[qd];
+            // packed fp32 FMA: two columns per instruction, each half an ordinary fma.rn
             const float2 p01 = __ffma2_rn(make_float2(u.x, u.y), e2, make_float2(w[4 * qd], w[4 * qd + 1]));
             const float2 p23 = __ffma2_rn(make_float2(u.z, u.w), e2, make_float2(w[4 * qd + 2], w[4 * qd + 3]));
             w[4 * qd] = p01.x; w[4 * qd + 1] = p01.y; w[4 * qd + 2] = p23.x; w[4 * qd + 3] = p23.y;
           }
         }
-      }
-      __syncwarp();
-      // The errors of lane lo reach the other lanes of the row, which apply them to their
-      // own columns in the same order, with the same FMAs, as a one-column-at-a-time recurrence.
-      // (For the lanes in front of lo the staged factor holds zeros; lane lo's own values are
-      // not needed any more.)
+        if (c + 1 < N_SUB) fetch_original(j0 + SUB);
+        if (valid) {
 #pragma unroll
-      for (int t = 0; t < LANE_COLS; ++t) {
-        const float eb = __shfl_sync(0xffffffffu, e[t], lo, ROW_LANES);
-        const float4* up = reinterpret_cast<const float4*>(&ublk[(lo * LANE_COLS + t) * U_ROW_LD + sub * U_LANE_LD]);
-        const float2 eb2 = make_float2(eb, eb);
-#pragma unroll
-        for (int qd = 0; qd < LANE_COLS / 4; ++qd) {
-          // packed fp32 FMA: two columns per instruction, each half an ordinary fma.rn
-          const float4 u = up[qd];
-          const float2 p01 = __ffma2_rn(make_float2(u.x, u.y), eb2, make_float2(w[4 * qd], w[4 * qd + 1]));
-          const float2 p23 = __ffma2_rn(make_float2(u.z, u.w), eb2, make_float2(w[4 * qd + 2], w[4 * qd + 3]));
-          w[4 * qd] = p01.x; w[4 * qd + 1] = p01.y; w[4 * qd + 2] = p23.x; w[4 * qd + 3] = p23.y;
+          for (int qd = 0; qd < SUB / 4; ++qd)
+            *reinterpret_cast<float4*>(wrow + j0 + 4 * qd) = make_float4(e[4 * qd], e[4 * qd + 1], e[4 * qd + 2], e[4 * qd + 3]);
         }
-      }
-    }
-
-    // ---- every lane writes what its columns produced
-    if (valid) {
+        __syncthreads();
+        if (c + 1 < N_SUB) {
+          // ---- next: this row's errors on the columns of the following sub-block
 #pragma unroll
-      for (int qd = 0; qd < LANE_COLS / 4; ++qd) {
-        if (c_local + 4 * qd >= nb) continue;
-        const uint32_t q4 = (uint32_t)qacc[2 * qd] | ((uint32_t)qacc[2 * qd + 1] << 16);   // four codes, one per byte, first column lowest
-        *reinterpret_cast<uint32_t*>(a.codes + (int64_t)r * a.C + c0 + 4 * qd) = q4;
-        if (a.deq) {
-          T* dq = static_cast<T*>(a.deq) + (int64_t)r * a.C + c0 + 4 * qd;
+          for (int qd = 0; qd < SUB / 4; ++qd) {
+            const float4 v = *reinterpret_cast<const float4*>(wrow + j0 + SUB + 4 * qd);
+            w[4 * qd] = v.x; w[4 * qd + 1] = v.y; w[4 * qd + 2] = v.z; w[4 * qd + 3] = v.w;
+          }
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const float qf = (float)((q4 >> (8 * t)) & 0xFFu);
-            dq[t] = from_float<T>((qf - zr[UNIFORM ? 0 : 4 * qd + t]) * sc[UNIFORM ? 0 : 4 * qd + t]);
+          for (int t = 0; t < SUB; ++t) {
+            const float2 e2 = make_float2(e[t], e[t]);
+#pragma unroll
+            for (int qd = 0; qd < SUB / 4; ++qd) {
+              const float4 u = *reinterpret_cast<const float4*>(ud + t * TILE + SUB + 4 * qd);
+              const float2 p01 = __ffma2_rn(make_float2(u.x, u.y), e2, make_float2(w[4 * qd], w[4 * qd + 1]));
+              const float2 p23 = __ffma2_rn(make_float2(u.z, u.w), e2, make_float2(w[4 * qd + 2], w[4 * qd + 3]));
+              w[4 * qd] = p01.x; w[4 * qd + 1] = p01.y; w[4 * qd + 2] = p23.x; w[4 * qd + 3] = p23.y;
+            }
+          }
+        }
+        // codes (and packed words) leave; a narrow last tile ends on a multiple of eight columns
+        if (valid) {
+          uint8_t* cdst = a.codes + row * a.C + i1 + j0;
+          if (wide_codes && j0 + SUB <= nb) {
+            *reinterpret_cast<uint4*>(cdst) = make_uint4(cw[0], cw[1], cw[2], cw[3]);
+          } else {
+#pragma unroll
+            for (int qd = 0; qd < SUB / 4; ++qd)
+              if (j0 + 4 * qd < nb) *reinterpret_cast<uint32_t*>(cdst + 4 * qd) = cw[qd];
+          }
+          if (a.packed) {
+#pragma unroll
+            for (int h = 0; h < SUB / 8; ++h)
+              if (j0 + 8 * h < nb) a.packed[row * (a.C >> 3) + ((i1 + j0 + 8 * h) >> 3)] = (int32_t)pack_nibbles(cw[2 * h], cw[2 * h + 1]);
+          }
+          if (a.deq) {
+            T* dq = static_cast<T*>(a.deq) + row * a.C + i1 + j0;
+#pragma unroll
+            for (int t = 0; t < SUB; ++t)
+              if (j0 + t < nb)
+                dq[t] = from_float<T>(((float)((cw[t >> 2] >> (8 * (t & 3))) & 0xFFu) - zr[UNIFORM ? 0 : t]) * sc[UNIFORM ? 0 : t]);
           }
         }
       }
-      if (a.packed) {
-        // the compressed-tensors word of columns 8k..8k+7 (column 8k+i at bits 4i..4i+3), written
-        // here so that no separate packing pass has to read the codes back
+    } else {
+      // ---- the errors of sub-block c on the columns from sub-block c + 2 on.  `quads` column quads; the lanes of
+      // a warp divide into rows of `span` lanes, so that few lanes idle as the region shrinks
+      const int first = warp - chain_warps, helpers = SWEEP_THREADS / 32 - chain_warps;
+#pragma unroll 1
+      for (int c = 0; c < N_SUB; ++c) {
+        const int j0 = c * SUB;
+        const int quads = (TILE - 2 * SUB - j0) / 4;
+        const int span = quads > 16 ? 32 : quads > 8 ? 16 : quads > 4 ? 8 : 4;
+        const int quad = lane & (span - 1);
+        const bool mine = quad < quads;
+        const int k = j0 + 2 * SUB + 4 * quad;
+        float4 u[SUB];
+        if (mine) {
 #pragma unroll
-        for (int h = 0; h < LANE_COLS / 8; ++h) {
-          if (c_local + 8 * h >= nb) continue;
-          const uint32_t lo4 = (uint32_t)qacc[4 * h] | ((uint32_t)qacc[4 * h + 1] << 16);
-          const uint32_t hi4 = (uint32_t)qacc[4 * h + 2] | ((uint32_t)qacc[4 * h + 3] << 16);
-          a.packed[(int64_t)r * (a.C >> 3) + ((c0 + 8 * h) >> 3)] = (int32_t)pack_nibbles(lo4, hi4);
+          for (int t = 0; t < SUB; ++t) u[t] = *reinterpret_cast<const float4*>(us + (j0 + t) * TILE + k);
         }
-      }
-      // columns past nb of a narrow last tile hold zeros so that the GEMM may read all 128
-      if (a.err_planes && a.err_scale) {
-        const float rho = __ldg(a.err_scale + r);
-        uint32_t hp[LANE_COLS / 2], lp[LANE_COLS / 2];
+        if (!UNIFORM && c + 1 < N_SUB) fill_columns(c + 1, tid - 32 * chain_warps, SWEEP_THREADS - 32 * chain_warps);
+        __syncthreads();
+        if (mine) {
+          const int per_warp = 32 / span;
+          for (int r = first * per_warp + lane / span; r < rows; r += helpers * per_warp) {
+            float* wr = ws + r * W_LD;
+            float4 v = *reinterpret_cast<const float4*>(wr + k);
 #pragma unroll
-        for (int t = 0; t < LANE_COLS; t += 2) {
-          uint16_t h0, l0, h1, l1;
-          split_half2(e[t] * rho, h0, l0);
-          split_half2(e[t + 1] * rho, h1, l1);
-          hp[t >> 1] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-          lp[t >> 1] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+            for (int t4 = 0; t4 < SUB / 4; ++t4) {
+              const float4 e4 = *reinterpret_cast<const float4*>(wr + j0 + 4 * t4);
+              const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+              for (int t = 0; t < 4; ++t) {
+                const float4 uu = u[4 * t4 + t];
+                const float2 e2 = make_float2(ev[t], ev[t]);
+                const float2 p01 = __ffma2_rn(make_float2(uu.x, uu.y), e2, make_float2(v.x, v.y));
+                const float2 p23 = __ffma2_rn(make_float2(uu.z, uu.w), e2, make_float2(v.z, v.w));
+                v = make_float4(p01.x, p01.y, p23.x, p23.y);
+              }
+            }
+            *reinterpret_cast<float4*>(wr + k) = v;
+          }
         }
-        uint16_t* dst = a.err_planes + (int64_t)r * a.err_ld + c_local;
-#pragma unroll
-        for (int v = 0; v < LANE_COLS / 8; ++v) {
-          reinterpret_cast<uint4*>(dst)[v] = make_uint4(hp[4 * v], hp[4 * v + 1], hp[4 * v + 2], hp[4 * v + 3]);
-          reinterpret_cast<uint4*>(dst + a.plane_stride)[v] = make_uint4(lp[4 * v], lp[4 * v + 1], lp[4 * v + 2], lp[4 * v + 3]);
-        }
-      } else if (a.err_planes) {
-        // the tensor-core update reads the errors as bf16 planes: write them in that form directly
-        uint32_t hp[LANE_COLS / 2], mp[LANE_COLS / 2], lp[LANE_COLS / 2];
-#pragma unroll
-        for (int t = 0; t < LANE_COLS; t += 2) {
-          uint16_t h0, m0, l0, h1, m1, l1;
-          split_bf16x3(e[t], h0, m0, l0);
-          split_bf16x3(e[t + 1], h1, m1, l1);
-          hp[t >> 1] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-          mp[t >> 1] = (uint32_t)m0 | ((uint32_t)m1 << 16);
-          lp[t >> 1] = (uint32_t)l0 | ((uint32_t)l1 << 16);
-        }
-        uint16_t* dst = a.err_planes + (int64_t)r * a.err_ld + c_local;
-#pragma unroll
-        for (int v = 0; v < LANE_COLS / 8; ++v) {
-          reinterpret_cast<uint4*>(dst)[v] = make_uint4(hp[4 * v], hp[4 * v + 1], hp[4 * v + 2], hp[4 * v + 3]);
-          if (a.n_planes > 1)
-            reinterpret_cast<uint4*>(dst + a.plane_stride)[v] = make_uint4(mp[4 * v], mp[4 * v + 1], mp[4 * v + 2], mp[4 * v + 3]);
-          if (a.n_planes > 2)
-            reinterpret_cast<uint4*>(dst + 2 * a.plane_stride)[v] = make_uint4(lp[4 * v], lp[4 * v + 1], lp[4 * v + 2], lp[4 * v + 3]);
-        }
-      } else {
-        float4* dst = reinterpret_cast<float4*>(a.err + (int64_t)r * a.err_ld + c_local);
-#pragma unroll
-        for (int qd = 0; qd < LANE_COLS / 4; ++qd) dst[qd] = make_float4(e[4 * qd], e[4 * qd + 1], e[4 * qd + 2], e[4 * qd + 3]);
       }
     }
+    __syncthreads();
+
+    // ---- the errors of the tile (columns past nb are zero: the update may read all 128)
+    for (int idx = tid; idx < rows * (TILE / 8); idx += SWEEP_THREADS) {
+      const int r = idx >> 4, k = (idx & 15) * 8;
+      const float4 lo4 = *reinterpret_cast<const float4*>(ws + r * W_LD + k), hi4 = *reinterpret_cast<const float4*>(ws + r * W_LD + k + 4);
+      const float e[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+      const int64_t gr = row0 + r;
+      if (!a.err_planes) {
+        float4* dst = reinterpret_cast<float4*>(a.err + gr * a.err_ld + k);
+        dst[0] = lo4;
+        dst[1] = hi4;
+        continue;
+      }
+      uint32_t p0[4], p1[4], p2[4];
+      if (a.err_scale) {
+        const float rho = __ldg(a.err_scale + gr);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          uint16_t h0, l0, h1, l1;
+          split_half2(e[2 * t] * rho, h0, l0);
+          split_half2(e[2 * t + 1] * rho, h1, l1);
+          p0[t] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+          p1[t] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          uint16_t h0, m0, l0, h1, m1, l1;
+          split_bf16x3(e[2 * t], h0, m0, l0);
+          split_bf16x3(e[2 * t + 1], h1, m1, l1);
+          p0[t] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+          p1[t] = (uint32_t)m0 | ((uint32_t)m1 << 16);
+          p2[t] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+        }
+      }
+      uint16_t* dst = a.err_planes + gr * a.err_ld + k;
+      *reinterpret_cast<uint4*>(dst) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
+      if (a.n_planes > 1) *reinterpret_cast<uint4*>(dst + a.plane_stride) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+      if (a.n_planes > 2) *reinterpret_cast<uint4*>(dst + 2 * a.plane_stride) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+    }
+    __syncthreads();   // the next group's weights replace the errors
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");   // a CTA without rows leaves no copy behind
 }
 
 template <int DT>
-int launch_sweep_tile(bool chained, bool uniform, int lanes, int grid, cudaStream_t st, const SweepArgs& args) {
-  if (lanes == 16) {
-    if (uniform) MQ_CUDA(launch_chained(chained, sweep_tile_kernel<DT, true, 16>, dim3(grid), dim3(TILE_THREADS), LaneShape<16>::smem, st, args));
-    else MQ_CUDA(launch_chained(chained, sweep_tile_kernel<DT, false, 16>, dim3(grid), dim3(TILE_THREADS), LaneShape<16>::smem, st, args));
-  } else {
-    if (uniform) MQ_CUDA(launch_chained(chained, sweep_tile_kernel<DT, true, 8>, dim3(grid), dim3(TILE_THREADS), LaneShape<8>::smem, st, args));
-    else MQ_CUDA(launch_chained(chained, sweep_tile_kernel<DT, false, 8>, dim3(grid), dim3(TILE_THREADS), LaneShape<8>::smem, st, args));
-  }
+int launch_sweep_tile(bool chained, bool uniform, int grid, int rows, cudaStream_t st, const SweepArgs& args) {
+  const bool free = args.Worig != nullptr;
+  auto* kernel = uniform ? (free ? sweep_tile_kernel<DT, true, true> : sweep_tile_kernel<DT, true, false>)
+                         : (free ? sweep_tile_kernel<DT, false, true> : sweep_tile_kernel<DT, false, false>);
+  MQ_CUDA(launch_chained(chained, kernel, dim3(grid), dim3(SWEEP_THREADS), sweep_smem_bytes(rows, uniform), st, args, rows));
   return MQ_OK;
 }
 
 template <int DT>
 int configure_dtype() {
-  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, true, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LaneShape<8>::smem));
-  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LaneShape<8>::smem));
-  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, true, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LaneShape<16>::smem));
-  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, false, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LaneShape<16>::smem));
+  constexpr int bytes = (int)sweep_smem_bytes(MAX_ROWS, false);
+  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   return MQ_OK;
 }
 
@@ -420,20 +486,18 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   sa.Worig = Worig; sa.ldwo = ldwo;
   sa.err_planes = nullptr;
   sa.plane_stride = tensor ? err_set.total_rows * (int64_t)SUPER : 0;
-  sa.n_planes = split;
+  sa.n_planes = half ? 2 : split;
   sa.err_scale = half ? row_f + R : nullptr;
   sa.err_ld = tensor ? SUPER : TILE;
   sa.bits = bits;
-  // sixteen lanes per row while the grid holds every row group at once, eight beyond that
-  const int lanes = ceil_div(R, TILE_THREADS / 16) <= MAX_SWEEP_CTAS ? 16 : 8;
-  const bool uniform = group % (TILE / lanes) == 0;
-  // every CTA stages the tile of the factor once and then walks row groups: no more CTAs than
-  // two per SM, so that a tall layer does not stage the same tile thousands of times
-  const int64_t row_groups = ceil_div(R, TILE_THREADS / lanes);
-  const int grid = (int)(row_groups < MAX_SWEEP_CTAS ? row_groups : MAX_SWEEP_CTAS);
-  // compact launches: full tiles whose groups are 32, 64 or a multiple of 128 columns wide run one
-  // row per thread (a third slower per tile, on an eighth of the SMs)
-  const int gpt = !compact ? 0 : group % TILE == 0 ? 1 : group == 64 ? 2 : group == 32 ? 4 : 0;
+  const bool uniform = group % SUB == 0;
+  // Rows per CTA: the chain costs the same for 1 row and for 64, so a tile of 2048 rows takes 16.5 us on 148 SMs,
+  // 17.4 on 74 and 19.0 on 48.  Alone, one CTA per SM; a caller with several layers in flight gives each
+  // few SMs.  Fewer than eight rows per CTA gain nothing.
+  int rows = (int)ceil_div(R, compact ? 44 : 148);
+  rows = rows < 8 ? 8 : (rows > MAX_ROWS ? MAX_ROWS : rows);
+  const int64_t row_groups = ceil_div(R, rows);
+  const int grid = (int)(row_groups < 148 ? row_groups : 148);
 
   for (int64_t i1 = 0; i1 < C; i1 += TILE) {
     const int nb = (int)((C - i1) < TILE ? (C - i1) : TILE);
@@ -445,18 +509,10 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       ProfScope prof(PROF_SWEEP_TILE, (double)R * nb * (4.0 + 1.0 + 4.0) + 2.0 * nb * nb, (double)R * nb * (nb - 1), st);
       sa.i1 = (int)i1; sa.nb = nb;
       if (tensor) sa.err_planes = err_set.base + (i1 % SUPER);
-      if (gpt && nb == TILE) {
-        switch (out_dtype) {
-          case MQ_F32: MQ_TRY(launch_sweep_rows<MQ_F32>(chained, gpt, (int)R, st, sa)); break;
-          case MQ_BF16: MQ_TRY(launch_sweep_rows<MQ_BF16>(chained, gpt, (int)R, st, sa)); break;
-          default: MQ_TRY(launch_sweep_rows<MQ_F16>(chained, gpt, (int)R, st, sa));
-        }
-      } else {
-        switch (out_dtype) {
-          case MQ_F32: MQ_TRY(launch_sweep_tile<MQ_F32>(chained, uniform, lanes, grid, st, sa)); break;
-          case MQ_BF16: MQ_TRY(launch_sweep_tile<MQ_BF16>(chained, uniform, lanes, grid, st, sa)); break;
-          default: MQ_TRY(launch_sweep_tile<MQ_F16>(chained, uniform, lanes, grid, st, sa));
-        }
+      switch (out_dtype) {
+        case MQ_F32: MQ_TRY(launch_sweep_tile<MQ_F32>(chained, uniform, grid, rows, st, sa)); break;
+        case MQ_BF16: MQ_TRY(launch_sweep_tile<MQ_BF16>(chained, uniform, grid, rows, st, sa)); break;
+        default: MQ_TRY(launch_sweep_tile<MQ_F16>(chained, uniform, grid, rows, st, sa));
       }
     }
     MQ_LAUNCH_CHECK();

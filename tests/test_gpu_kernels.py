@@ -592,3 +592,27 @@ def test_compact_sweep_is_bit_identical(cuda, R, C, g, dtype, math):
         p = ops.Precision(math=math, compact=compact)
         res.append(ops.gptq_sweep(W.float().clone(), U, scale, zero, g, C // g, 1, 4, dtype, True, p))
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1].float(), res[1][1].float())
+
+
+# ------------------------------------------------------------------ row groups of the sweep tile
+@pytest.mark.parametrize("R", [1, 7, 8, 9, 33, 1184, 1185, 4737, 9473])
+@pytest.mark.parametrize("C,g", [(24, 24), (136, 8), (256, 32)])
+def test_sweep_tile_row_groups(cuda, R, C, g):
+    """One chain warp or two, groups that are not full, more groups than CTAs, a last tile of 8 columns,
+    scales per sub-block and per column.  Rows are independent: every row's codes equal those of the
+    same row swept in another grouping (the compact one, and alone)."""
+    gen = torch.Generator().manual_seed(R + C)
+    base = 0.02 * torch.randn(64, C, generator=gen)
+    W = base[torch.arange(R) % 64].contiguous()
+    U = torch.triu(0.2 * torch.randn(C, C, generator=gen), 1) + torch.eye(C)
+
+    def sweep(w, precision):
+        s = ops.absmax_scales(w, g, 4, torch.bfloat16)
+        codes, deq = ops.gptq_sweep(w.clone(), U.to(cuda), s, None, g, C // g, 1, 4, torch.bfloat16, True, precision, W_original=w)
+        assert torch.equal(deq, ops.dequantize(codes, s, None, g, 4, torch.bfloat16))
+        return codes.cpu()
+
+    got = sweep(W.to(cuda), ops.Precision())
+    want = sweep(base[: min(R, 64)].to(cuda), ops.Precision())
+    assert torch.equal(got, want[torch.arange(R) % 64])
+    assert torch.equal(got, sweep(W.to(cuda), ops.Precision(compact=True)))
