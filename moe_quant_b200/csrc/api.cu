@@ -18,7 +18,10 @@ void set_error(const char* fmt, ...) {
 }
 
 // defined in the other translation units
-int launch_to_fp32(const void* src, int dtype, float* dst, int64_t n, cudaStream_t st);
+int weights_in(const void* src, int dtype, int64_t R, int64_t C, float* run, float* orig, const float* H, int64_t ldh, int* nonzero,
+               int64_t group, int bits, float* scale, cudaStream_t st);
+int prepare_layer(const void* Wsrc, int dtype, int64_t R, int64_t C, float* run, float* orig, float* H, int64_t ldh, int64_t group, int bits,
+                  float rel_damp, float* scale, float* eq, mq_layer_flags* flags, void* prep, cudaStream_t st);
 size_t hinv_workspace_bytes(int64_t C, int math, int split);
 size_t factor_workspace_bytes(int64_t C, int math, int split);
 int hinv_upper(float* H, int64_t C, int64_t ldh, float* Uhat, int64_t ldu, float* diag_out, int math, int split, mq_layer_flags* flags,
@@ -30,7 +33,6 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
                const float* col_div, const float* eq, bool absmax_grid, int32_t* packed);
 int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, int split, mq_layer_flags* flags,
                      Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled, const float* eq);
-int equilibration(const float* H, int64_t C, int64_t ldh, float* eq, cudaStream_t st);
 int copy_upper_scaled(const float* src, int64_t lds, float* dst, int64_t ldd, int64_t C, const float* eq, cudaStream_t st);
 int hessian_accum_tensor(const void* X, int x_dtype, int64_t m, int64_t C, int64_t ldx, float* H, int64_t ldh, float beta,
                          float alpha, int split, Workspace& ws, cudaStream_t st);
@@ -157,14 +159,17 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   MQ_REQUIRE(U && diag && eq && Wf[n_tied - 1] && Wo[n_tied - 1] && prep, MQ_ERR_WORKSPACE,
              "mq_quantize_layer: workspace of %zu bytes is too small", workspace_bytes);
 
-  // W.clone().float()                                           src/gptq.py:149
-  for (int i = 0; i < n_tied; ++i) MQ_TRY(launch_to_fp32(Wsrc[i], w_dtype, Wf[i], R * C, st));
-  // pre-step + masking + damping, driven by the first layer's weight: the handle that owns H.
-  // A tied handle meets an H that is already regularised and changes neither H nor its own
-  // weight (src/gptq.py:129-136, 227).                          src/gptq.py:140-152, 224-234
-  MQ_TRY(mq_hessian_prepare(H, C, ldh, Wf[0], R, C, rel_damp, flags, prep, mq_hessian_prepare_workspace_bytes(C), st));
-  // grid                                                        src/quant_utils.py:75-101
-  for (int i = 0; i < n_tied; ++i) MQ_TRY(mq_absmax_scales(Wf[i], R, C, C, group, bits, w_dtype, scale_out[i], st));
+  // At full tensor precision the factorisation works on a copy equilibrated by powers of two (fp16 operand
+  // pairs).  The sweep takes an equilibrated factor only where it works on such pairs itself; otherwise the
+  // factorisation gives its result back in H's units.
+  const bool pairs = math == MQ_MATH_TENSOR && split_hinv == 3 && split_sweep == 3;
+  const bool unscaled = math == MQ_MATH_TENSOR && (pairs || split_hinv != 3);
+  // W.clone().float(), pre-step, masking and damping, grid; driven by the first layer's weight: the handle that
+  // owns H.  A tied handle meets an H that is already regularised and changes neither H nor its own
+  // weight (src/gptq.py:129-136, 227).       src/gptq.py:140-152, 224-234, src/quant_utils.py:75-101
+  MQ_TRY(prepare_layer(Wsrc[0], w_dtype, R, C, Wf[0], Wo[0], H, ldh, group, bits, rel_damp, scale_out[0], pairs ? eq : nullptr, flags, prep, st));
+  for (int i = 1; i < n_tied; ++i)
+    MQ_TRY(weights_in(Wsrc[i], w_dtype, R, C, Wf[i], Wo[i], nullptr, 0, nullptr, group, bits, scale_out[i], st));
   // Factor a copy (the caller's H keeps the damped Hessian, which the reference leaves in
   // handle.H, quant.py:314-316).  Only the unit factor Utilde = T diag(T)^-1 of H = T T^T is
   // built: the sweep below runs in its inverse-free form, so the triangular inverse that
@@ -173,12 +178,6 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   // tiles read them); the blocks above are divided where they are split into planes.
   // The factorisation, the sweep tiles and the lazy updates read nothing below the diagonal
   // 128-blocks, so that half is neither copied nor zeroed.
-  // At full tensor precision the copy is equilibrated by powers of two (fp16 operand pairs).  The sweep
-  // takes an equilibrated factor only where it works on such pairs itself; otherwise the factorisation
-  // gives its result back in H's units.
-  const bool pairs = math == MQ_MATH_TENSOR && split_hinv == 3 && split_sweep == 3;
-  if (pairs) MQ_TRY(equilibration(H, C, ldh, eq, st));
-  const bool unscaled = math == MQ_MATH_TENSOR && (pairs || split_hinv != 3);
   MQ_TRY(copy_upper_scaled(H, ldh, U, C, C, pairs ? eq : nullptr, st));
   {
     Workspace sub(ws.base + ws.used, ws.size - ws.used);
@@ -186,7 +185,6 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   }
   // sweep                                                       src/gptq_loop.py:141-148
   for (int i = 0; i < n_tied; ++i) {
-    MQ_CUDA(cudaMemcpyAsync(Wo[i], Wf[i], (size_t)R * C * sizeof(float), cudaMemcpyDeviceToDevice, st));
     Workspace sub(ws.base + ws.used, ws.size - ws.used);
     MQ_TRY(gptq_sweep(Wf[i], R, C, C, U, C, scale_out[i], nullptr, group, C / group, 1, bits, w_dtype, codes[i],
                       dequantized ? dequantized[i] : nullptr, Wo[i], C, sweep_math, split_sweep, sub, st, unscaled ? diag : nullptr,

@@ -63,6 +63,18 @@ __device__ __forceinline__ float scale_below_2_14(float bound) {
   return __uint_as_float((uint32_t)(e + 127) << 23);
 }
 
+// Equilibration of a matrix to be factored: the power of two 2^(13 - n) with h / 4^n in [1, 4) for the diagonal
+// entry h, so that the diagonal of  eq H eq  lies in [2^26, 2^28) and every entry of its triangular factor
+// below 2^14, where a pair of fp16 planes holds 22 bits of all but the smallest.  Powers of two: the factorisation
+// does the same fp32 operations, up to exponents, as on H itself.  1 where h is not a positive finite number.
+__device__ __forceinline__ float equilibrating_power(float h) {
+  if (!(h > 0.0f && h < INFINITY)) return 1.0f;
+  const int e = ilogbf(h);   // floor(log2 h)
+  int n = 13 - (e >= 0 ? e / 2 : -((1 - e) / 2));
+  n = n < -60 ? -60 : (n > 60 ? 60 : n);
+  return __uint_as_float((uint32_t)(n + 127) << 23);
+}
+
 // Tensor-core GEMM whose operands are already planes (d.A / d.B and their strides are ignored;
 // d.K is the reduction length starting at k0 of each set).  Both sets must have the same
 // number of planes.

@@ -391,16 +391,15 @@ __global__ void __launch_bounds__(256) extract_diag_kernel(const float* __restri
 }
 
 // T -> T diag(T)^-1 on the upper triangle (unit diagonal), zeros below it.
-// upper_only = 1: what lies entirely below the diagonal is left as it is instead of being zeroed
-// (the layer path never reads it); = 2: in addition only the diagonal 128-blocks are scaled (the
-// sweep tiles read those; the blocks above are divided by whoever splits them into planes).
+// upper_only: what lies entirely below the diagonal is left as it is instead of being zeroed
+// (the layer path never reads it).
 __device__ __forceinline__ void scale_quad(float* __restrict__ H, int64_t ld, const float* __restrict__ diag,
                                            const float* __restrict__ eq, int64_t r, int64_t c) {
   // four columns c..c+3 of row r; what lies entirely below the diagonal is written without being read
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c + 3 >= r) {
     const float4 v = *reinterpret_cast<const float4*>(H + r * ld + c);
-    const float4 d = __ldg(reinterpret_cast<const float4*>(diag + c));
+    const float4 d = *reinterpret_cast<const float4*>(diag + c);
     // equilibrated: entry (r, c) of the matrix's own factor is eq[c] / eq[r] times this one's (powers of two)
     float4 e = make_float4(1.f, 1.f, 1.f, 1.f);
     if (eq) {
@@ -416,16 +415,30 @@ __device__ __forceinline__ void scale_quad(float* __restrict__ H, int64_t ld, co
   *reinterpret_cast<float4*>(H + r * ld + c) = o;
 }
 
+// The end of an unscaled factorisation, one CTA per diagonal 128-block: diag(T) to `diag`, the block divided by it
+// (the sweep tiles read the diagonal blocks; the blocks above are divided by whoever splits them into planes).
+__global__ void __launch_bounds__(1024) finish_diag_blocks_kernel(float* __restrict__ H, int64_t C, int64_t ld, float* __restrict__ diag,
+                                                                 const float* __restrict__ eq) {
+  __shared__ __align__(16) float d[NB];
+  const int64_t k0 = (int64_t)blockIdx.x * NB;
+  const int nb = C - k0 < NB ? (int)(C - k0) : NB;
+  const int t = threadIdx.x;
+  if (t < nb) {
+    d[t] = H[(k0 + t) * ld + k0 + t];
+    diag[k0 + t] = d[t];
+  }
+  __syncthreads();
+  for (int idx = t; idx < nb * (NB / 4); idx += blockDim.x) {
+    const int r = idx >> 5, c = (idx & 31) * 4;
+    if (c < nb && c + 3 >= r) scale_quad(H, ld, d - k0, eq, k0 + r, k0 + c);   // C % 8 == 0: quads are whole
+  }
+}
+
 __global__ void __launch_bounds__(256) scale_columns_kernel(float* __restrict__ H, int64_t C, int64_t ld,
                                                             const float* __restrict__ diag, const float* __restrict__ eq,
                                                             int upper_only) {
   const int64_t r = blockIdx.y;
   if ((C & 3) == 0 && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0) {
-    if (upper_only == 2) {  // launched with one block of 32 threads per row: the row's diagonal block
-      const int64_t c = (r / NB) * NB + threadIdx.x * 4;
-      if (blockIdx.x == 0 && threadIdx.x < NB / 4 && c < C && c + 3 >= r) scale_quad(H, ld, diag, eq, r, c);
-      return;
-    }
     for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; c < C; c += (int64_t)gridDim.x * blockDim.x * 4) {
       if (upper_only && c + 3 < r) continue;
       scale_quad(H, ld, diag, eq, r, c);
@@ -433,27 +446,16 @@ __global__ void __launch_bounds__(256) scale_columns_kernel(float* __restrict__ 
     return;
   }
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < C; c += (int64_t)gridDim.x * blockDim.x) {
-    if (upper_only == 2 && (c < (r / NB) * NB || c >= (r / NB + 1) * NB)) continue;
     float v = H[r * ld + c];
     H[r * ld + c] = (c > r) ? v / diag[c] * (eq ? eq[c] / eq[r] : 1.0f) : (c == r ? 1.0f : 0.0f);
   }
 }
 
-// Equilibration of the matrix to be factored: eq[i] = 2^(13 - n) with H[i][i] / 4^n in [1, 4), so that the
-// diagonal of  eq H eq  lies in [2^26, 2^28) and every entry of its factor below 2^14, where a pair of fp16
-// planes holds 22 bits of all but the smallest (split_half2).  Powers of two: the factorisation does the same
-// fp32 operations, up to exponents, as on H itself.  1 where the diagonal is not a positive finite number.
-// eq[C] receives the smallest factor (positive floats order like their bits; preset by the host).
+// The equilibration of H (equilibrating_power) for callers that hand over H alone; eq[C] receives the smallest
+// factor (positive floats order like their bits; preset by the host).
 __global__ void __launch_bounds__(256) equilibration_kernel(const float* __restrict__ H, int64_t C, int64_t ld, float* __restrict__ eq) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const float h = i < C ? H[i * ld + i] : -1.0f;
-  float v = 1.0f;
-  if (h > 0.0f && h < INFINITY) {
-    const int e = ilogbf(h);                       // floor(log2 h)
-    int n = 13 - (e >= 0 ? e / 2 : -((1 - e) / 2));
-    n = n < -60 ? -60 : (n > 60 ? 60 : n);
-    v = __uint_as_float((uint32_t)(n + 127) << 23);
-  }
+  const float v = i < C ? equilibrating_power(H[i * ld + i]) : 1.0f;
   if (i < C) eq[i] = v;
   const int least = __reduce_min_sync(0xffffffffu, i < C ? __float_as_int(v) : 0x7f7f7f7f);
   if ((threadIdx.x & 31) == 0) atomicMin(reinterpret_cast<int*>(eq + C), least);
@@ -515,7 +517,7 @@ size_t factor_workspace_bytes(int64_t C, int math, int split) {
   return math == MQ_MATH_TENSOR ? plane_set_bytes(C, SUPER_NB, split) + align_up((size_t)(C + 1) * sizeof(float), 256) : 0;
 }
 
-int equilibration(const float* H, int64_t C, int64_t ldh, float* eq, cudaStream_t st) {
+static int equilibration(const float* H, int64_t C, int64_t ldh, float* eq, cudaStream_t st) {
   MQ_CUDA(cudaMemsetAsync(eq + C, 0x7f, sizeof(float), st));
   equilibration_kernel<<<(unsigned)ceil_div(C, 256), 256, 0, st>>>(H, C, ldh, eq);
   MQ_LAUNCH_CHECK();
@@ -644,12 +646,14 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
     }
   }
   // ---- T -> unit-diagonal factor
-  extract_diag_kernel<<<(unsigned)ceil_div(C, 256), 256, 0, st>>>(H, C, ldh, diag);
-  MQ_LAUNCH_CHECK();
-  {
-    const int mode = unscaled ? 2 : (upper_only ? 1 : 0);
-    const unsigned gx = unscaled ? 1u : (unsigned)(ceil_div(C, 256) < 8 ? ceil_div(C, 256) : 8);
-    scale_columns_kernel<<<dim3(gx, (unsigned)C), unscaled ? 32 : 256, 0, st>>>(H, C, ldh, diag, eq, mode);
+  if (unscaled) {
+    finish_diag_blocks_kernel<<<(unsigned)P, 1024, 0, st>>>(H, C, ldh, diag, eq);
+    MQ_LAUNCH_CHECK();
+  } else {
+    extract_diag_kernel<<<(unsigned)ceil_div(C, 256), 256, 0, st>>>(H, C, ldh, diag);
+    MQ_LAUNCH_CHECK();
+    const unsigned gx = (unsigned)(ceil_div(C, 256) < 8 ? ceil_div(C, 256) : 8);
+    scale_columns_kernel<<<dim3(gx, (unsigned)C), 256, 0, st>>>(H, C, ldh, diag, eq, upper_only ? 1 : 0);
     MQ_LAUNCH_CHECK();
   }
   if (own_units) {

@@ -2,9 +2,11 @@
 // and the symmetric absmax grid.  All of it is one or two passes over H / W, i.e.
 // HBM-bound, and everything stays on the device: no host round trip for the
 // `.any().item()` of the reference (src/gptq.py:141).
-#include "common.cuh"
+#include "engine.cuh"
 
 namespace mq {
+
+int launch_to_fp32(const void* src, int dtype, float* dst, int64_t n, cudaStream_t st);
 
 // ---------------------------------------------------------------- NaN guard
 __global__ void __launch_bounds__(256) nan_scan_kernel(const float* __restrict__ H, int64_t C, int64_t ldh,
@@ -31,11 +33,14 @@ __global__ void __launch_bounds__(256) nan_scan_kernel(const float* __restrict__
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicExch(&flags->nan_hessian, 1);
 }
 
+// Also clears the column flags (may be null) for the pass over the weights that follows.
 __global__ void __launch_bounds__(256) identity_if_nan_kernel(float* __restrict__ H, int64_t C, int64_t ldh,
-                                                              const mq_layer_flags* flags) {
-  if (flags->nan_hessian == 0) return;
+                                                              const mq_layer_flags* flags, int* __restrict__ nonzero) {
   int64_t n = C * C;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  if (nonzero)
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < C; i += stride) nonzero[i] = 0;
+  if (flags->nan_hessian == 0) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     int64_t r = i / C, c = i - r * C;
     H[r * ldh + c] = (r == c) ? 1.0f : 0.0f;
@@ -56,36 +61,90 @@ __global__ void __launch_bounds__(256) column_nonzero_kernel(const float* __rest
   if (nz) nonzero[c] = 1;
 }
 
-// One block: lists the masked channels (diag(H)==0, or an all-zero weight column).
-// list[0] = count, list[1..] = channel indices (order is irrelevant).
-__global__ void __launch_bounds__(1024) build_mask_kernel(const float* __restrict__ H, int64_t C, int64_t ldh,
-                                                          const int* __restrict__ nonzero, int* __restrict__ list,
-                                                          mq_layer_flags* flags) {
-  __shared__ int n_masked, n_dead, n_zero;
-  if (threadIdx.x == 0) n_masked = n_dead = n_zero = 0;
+// One block, everything that happens on the diagonal: lists the masked channels (diag(H)==0, or an all-zero weight
+// column; list[0] = count, list[1..] = channel indices in any order), sets their diagonal to 1, adds
+// rel_damp * mean(diag H) and, where eq is given, computes the equilibration of the damped diagonal
+// (equilibrating_power); eq[C] is the smallest factor.
+// The diagonal is read once, DIAG_KEEP values per thread in flight: with a pass per purpose (list, damping,
+// equilibration) the three took 12 + 16 + 3 us at 7168 channels, all of it memory latency.
+constexpr int DIAG_THREADS_PREP = 1024, DIAG_KEEP = 8;
+
+__global__ void __launch_bounds__(DIAG_THREADS_PREP) diagonal_kernel(float* __restrict__ H, int64_t C, int64_t ldh,
+                                                                     const int* __restrict__ nonzero, int* __restrict__ list,
+                                                                     float rel_damp, float* __restrict__ eq, mq_layer_flags* flags) {
+  __shared__ int n_masked, n_dead, n_zero, least;
+  __shared__ float partial[32];
+  __shared__ float damp_s;
+  if (threadIdx.x == 0) { n_masked = n_dead = n_zero = 0; least = 0x7f7f7f7f; }
   __syncthreads();
-  for (int64_t c = threadIdx.x; c < C; c += blockDim.x) {
-    bool dead = H[c * ldh + c] == 0.0f;
-    // The reference zeroes W[:, dead] before looking for all-zero columns, so a dead
-    // channel is always also a zero column (src/gptq.py:145-152, 224).
-    bool zero_col = dead || (nonzero != nullptr && nonzero[c] == 0);
-    if (dead) atomicAdd(&n_dead, 1);
-    if (zero_col) {
-      atomicAdd(&n_zero, 1);
-      int slot = atomicAdd(&n_masked, 1);
-      list[1 + slot] = (int)c;
+  float acc = 0.0f, kept[DIAG_KEEP];
+  for (int64_t c0 = threadIdx.x; c0 < C; c0 += (int64_t)DIAG_KEEP * DIAG_THREADS_PREP) {
+    float h[DIAG_KEEP];
+    int nz[DIAG_KEEP];
+#pragma unroll
+    for (int u = 0; u < DIAG_KEEP; ++u) {
+      const int64_t c = c0 + (int64_t)u * DIAG_THREADS_PREP;
+      h[u] = c < C ? H[c * ldh + c] : 0.0f;
+      nz[u] = (c < C && nonzero != nullptr) ? nonzero[c] : 1;
+    }
+#pragma unroll
+    for (int u = 0; u < DIAG_KEEP; ++u) {
+      const int64_t c = c0 + (int64_t)u * DIAG_THREADS_PREP;
+      if (c >= C) continue;
+      // The reference zeroes W[:, dead] before looking for all-zero columns, so a dead
+      // channel is always also a zero column (src/gptq.py:145-152, 224).
+      const bool dead = h[u] == 0.0f;
+      if (dead) atomicAdd(&n_dead, 1);
+      if (dead || nz[u] == 0) {
+        atomicAdd(&n_zero, 1);
+        list[1 + atomicAdd(&n_masked, 1)] = (int)c;
+        h[u] = 1.0f;
+      }
+      acc += h[u];
+      if (c0 == threadIdx.x) kept[u] = h[u];
+      else H[c * ldh + c] = h[u];                  // beyond the kept ones: written now, read again below
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    float v = threadIdx.x < (blockDim.x >> 5) ? partial[threadIdx.x] : 0.0f;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) {
+      damp_s = rel_damp * (v / (float)C);
+      list[0] = n_masked;
+      flags->dead_channels = n_dead;
+      flags->zero_columns = n_zero;
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    list[0] = n_masked;
-    flags->dead_channels = n_dead;
-    flags->zero_columns = n_zero;
+  const float damp = damp_s;
+  int mine = 0x7f7f7f7f;
+  auto finish = [&](int64_t c, float h) {
+    h += damp;
+    H[c * ldh + c] = h;
+    if (eq) {
+      const float e = equilibrating_power(h);
+      eq[c] = e;
+      mine = min(mine, __float_as_int(e));         // positive floats order like their bits
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < DIAG_KEEP; ++u) {
+    const int64_t c = threadIdx.x + (int64_t)u * DIAG_THREADS_PREP;
+    if (c < C) finish(c, kept[u]);
+  }
+  for (int64_t c = threadIdx.x + (int64_t)DIAG_KEEP * DIAG_THREADS_PREP; c < C; c += DIAG_THREADS_PREP) finish(c, H[c * ldh + c]);
+  if (eq) {
+    atomicMin(&least, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) eq[C] = __int_as_float(least);
   }
 }
 
-// Rows and columns of the masked channels become those of the identity; their weight
-// column becomes zero.
+// Rows and columns of the masked channels become those of the identity (the diagonal is
+// diagonal_kernel's); their weight column becomes zero.
 __global__ void __launch_bounds__(256) apply_mask_kernel(float* __restrict__ H, int64_t C, int64_t ldh,
                                                          float* __restrict__ W, int64_t R, int64_t ldw,
                                                          const int* __restrict__ list) {
@@ -96,33 +155,14 @@ __global__ void __launch_bounds__(256) apply_mask_kernel(float* __restrict__ H, 
   for (int k = 0; k < n_masked; ++k) {
     int64_t c = list[1 + k];
     for (int64_t i = tid; i < C; i += stride) {
-      float v = (i == c) ? 1.0f : 0.0f;
-      H[c * ldh + i] = v;
-      H[i * ldh + c] = v;
+      if (i == c) continue;
+      H[c * ldh + i] = 0.0f;
+      H[i * ldh + c] = 0.0f;
     }
     if (W != nullptr) {
       for (int64_t r = tid; r < R; r += stride) W[r * ldw + c] = 0.0f;
     }
   }
-}
-
-// One block: H[i,i] += rel_damp * mean(diag H).
-__global__ void __launch_bounds__(1024) damp_kernel(float* __restrict__ H, int64_t C, int64_t ldh, float rel_damp) {
-  __shared__ float partial[32];
-  __shared__ float damp_s;
-  float acc = 0.0f;
-  for (int64_t c = threadIdx.x; c < C; c += blockDim.x) acc += H[c * ldh + c];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float v = threadIdx.x < (blockDim.x >> 5) ? partial[threadIdx.x] : 0.0f;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) damp_s = rel_damp * (v / (float)C);
-  }
-  __syncthreads();
-  float damp = damp_s;
-  for (int64_t c = threadIdx.x; c < C; c += blockDim.x) H[c * ldh + c] += damp;
 }
 
 // ---------------------------------------------------------------- absmax grid
@@ -292,6 +332,112 @@ void launch_mse_scales(int grid, cudaStream_t st, const float* W, int64_t R, int
   else mse_scales_kernel<DT, 0><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
 }
 
+// ---------------------------------------------------------------- the weights' way in
+// One pass over the layer's weights: two fp32 copies (original and running), columns of dead channels (diag(H)==0,
+// hdiag given) zeroed, flags of the columns that hold a non-zero, and the absmax scales of groups of 32,
+// 64 or 128 columns (GROUP_LANES = lanes of 4 columns per group; 0: none).  A warp takes 128 columns of
+// eight rows, four rows in flight.  As separate passes (conversion, column flags, absmax, copy) the same took
+// 14 + 16 + 27 + 20 us for 2048 x 7168; the scales of 64-wide groups, half of whose warps' lanes idled, 49.
+template <typename S, int GROUP_LANES>
+__global__ void __launch_bounds__(256) weights_in_kernel(const S* __restrict__ src, int64_t R, int64_t C, float* __restrict__ run,
+                                                         float* __restrict__ orig, const float* __restrict__ H, int64_t ldh,
+                                                         int* __restrict__ nonzero, float two_over_maxq, int out_dtype,
+                                                         float* __restrict__ scale) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t c = (int64_t)blockIdx.x * 128 + lane * 4;
+  const bool in = c < C;   // C % 8 == 0: a lane is in or out as a whole; one that is out only takes part in the shuffles
+  bool dead[4] = {false, false, false, false};
+  if (H != nullptr && in) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dead[q] = __ldg(H + (c + q) * (ldh + 1)) == 0.0f;
+  }
+  bool nz[4] = {false, false, false, false};
+  const int64_t r_end = ((int64_t)blockIdx.y + 1) * 64 < R ? ((int64_t)blockIdx.y + 1) * 64 : R;
+  for (int64_t r0 = (int64_t)blockIdx.y * 64 + warp * 8; r0 < r_end && r0 < (int64_t)blockIdx.y * 64 + warp * 8 + 8; r0 += 4) {
+    float v[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const S* p = src + (r0 + u) * C + c;
+      const bool ok = in && r0 + u < r_end;
+      if constexpr (sizeof(S) == 4) {
+        const float4 x = ok ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w;
+      } else {
+        union { uint2 w; S t[4]; } x;
+        x.w = ok ? __ldg(reinterpret_cast<const uint2*>(p)) : make_uint2(0u, 0u);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[u][q] = to_float(x.t[q]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t r = r0 + u;
+      float m = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        nz[q] |= v[u][q] != 0.0f;
+        if (dead[q]) v[u][q] = 0.0f;
+        m = fmaxf(m, fabsf(v[u][q]));
+      }
+      if (r >= r_end) break;   // uniform in the warp
+      if (in) {
+        const float4 o = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+        *reinterpret_cast<float4*>(run + r * C + c) = o;
+        *reinterpret_cast<float4*>(orig + r * C + c) = o;
+      }
+      if constexpr (GROUP_LANES > 0) {
+#pragma unroll
+        for (int o = GROUP_LANES / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (in && (lane & (GROUP_LANES - 1)) == 0) {
+          const float s = __fadd_rn(__fmul_rn(two_over_maxq, m), 1e-12f);   // as in absmax_scales_kernel
+          scale[r * (C / (4 * GROUP_LANES)) + c / (4 * GROUP_LANES)] =
+              out_dtype == MQ_BF16 ? round_through<MQ_BF16>(s) : out_dtype == MQ_F16 ? round_through<MQ_F16>(s) : s;
+        }
+      }
+    }
+  }
+  if (nonzero != nullptr && in) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (nz[q]) nonzero[c + q] = 1;
+  }
+}
+
+template <typename S>
+static int launch_weights_in(const void* src, int dtype, int64_t R, int64_t C, float* run, float* orig, const float* H, int64_t ldh,
+                             int* nonzero, int64_t group, int bits, float* scale, cudaStream_t st) {
+  const dim3 grid((unsigned)ceil_div(C, 128), (unsigned)ceil_div(R, 64));
+  const float f = 2.0f / (float)((1 << bits) - 1);
+  const S* p = static_cast<const S*>(src);
+  switch (group) {
+    case 32: weights_in_kernel<S, 8><<<grid, 256, 0, st>>>(p, R, C, run, orig, H, ldh, nonzero, f, dtype, scale); break;
+    case 64: weights_in_kernel<S, 16><<<grid, 256, 0, st>>>(p, R, C, run, orig, H, ldh, nonzero, f, dtype, scale); break;
+    case 128: weights_in_kernel<S, 32><<<grid, 256, 0, st>>>(p, R, C, run, orig, H, ldh, nonzero, f, dtype, scale); break;
+    default: weights_in_kernel<S, 0><<<grid, 256, 0, st>>>(p, R, C, run, orig, H, ldh, nonzero, f, dtype, scale);
+  }
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
+}
+
+// The layer's weights -> both fp32 copies and the scales.  H, nonzero: see weights_in_kernel (null for a tied layer).
+int weights_in(const void* src, int dtype, int64_t R, int64_t C, float* run, float* orig, const float* H, int64_t ldh, int* nonzero,
+               int64_t group, int bits, float* scale, cudaStream_t st) {
+  // a weight view that starts off a 4-element boundary goes through an aligned copy of itself
+  const bool vec = aligned(src, dtype == MQ_F32 ? 16 : 8);
+  if (!vec) {
+    MQ_TRY(launch_to_fp32(src, dtype, orig, R * C, st));
+    MQ_TRY(launch_weights_in<float>(orig, dtype, R, C, run, orig, H, ldh, nonzero, group, bits, scale, st));
+  } else {
+    switch (dtype) {
+      case MQ_F32: MQ_TRY(launch_weights_in<float>(src, dtype, R, C, run, orig, H, ldh, nonzero, group, bits, scale, st)); break;
+      case MQ_BF16: MQ_TRY(launch_weights_in<__nv_bfloat16>(src, dtype, R, C, run, orig, H, ldh, nonzero, group, bits, scale, st)); break;
+      default: MQ_TRY(launch_weights_in<__half>(src, dtype, R, C, run, orig, H, ldh, nonzero, group, bits, scale, st));
+    }
+  }
+  if (group != 32 && group != 64 && group != 128) MQ_TRY(mq_absmax_scales(run, R, C, C, group, bits, dtype, scale, st));
+  return MQ_OK;
+}
+
 // ---------------------------------------------------------------- fp32 working copy
 template <typename T>
 __global__ void __launch_bounds__(256) to_fp32_kernel(const T* __restrict__ src, float* __restrict__ dst, int64_t n) {
@@ -322,6 +468,44 @@ int launch_to_fp32(const void* src, int dtype, float* dst, int64_t n, cudaStream
 
 }  // namespace mq
 
+namespace mq {
+
+// Flags cleared, NaN guard, column flags (may be null) cleared.
+int scan_hessian(float* H, int64_t C, int64_t ldh, int* nonzero, mq_layer_flags* flags, cudaStream_t st) {
+  MQ_CUDA(cudaMemsetAsync(flags, 0, sizeof(mq_layer_flags), st));
+  const unsigned gx = (unsigned)ceil_div(C / 4, 256);
+  unsigned gy = (unsigned)(148 * 8 / gx);
+  if (gy < 1) gy = 1;
+  if ((int64_t)gy > C) gy = (unsigned)C;
+  nan_scan_kernel<<<dim3(gx, gy), 256, 0, st>>>(H, C, ldh, flags);
+  MQ_LAUNCH_CHECK();
+  identity_if_nan_kernel<<<148 * 4, 256, 0, st>>>(H, C, ldh, flags, nonzero);
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
+}
+
+int mask_and_damp(float* H, int64_t C, int64_t ldh, float* W, int64_t R, int64_t ldw, const int* nonzero, int* list, float rel_damp,
+                  float* eq, mq_layer_flags* flags, cudaStream_t st) {
+  diagonal_kernel<<<1, DIAG_THREADS_PREP, 0, st>>>(H, C, ldh, nonzero, list, rel_damp, eq, flags);
+  MQ_LAUNCH_CHECK();
+  apply_mask_kernel<<<148, 256, 0, st>>>(H, C, ldh, W, R, ldw, list);
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
+}
+
+// The whole preparation of a layer: H masked and damped, eq (may be null) its equilibration, the weights as two
+// fp32 copies and the scales.
+int prepare_layer(const void* Wsrc, int dtype, int64_t R, int64_t C, float* run, float* orig, float* H, int64_t ldh, int64_t group, int bits,
+                  float rel_damp, float* scale, float* eq, mq_layer_flags* flags, void* prep, cudaStream_t st) {
+  int* nonzero = static_cast<int*>(prep);
+  int* list = nonzero + align_up((size_t)C * sizeof(int), 256) / sizeof(int);
+  MQ_TRY(scan_hessian(H, C, ldh, nonzero, flags, st));
+  MQ_TRY(weights_in(Wsrc, dtype, R, C, run, orig, H, ldh, nonzero, group, bits, scale, st));
+  return mask_and_damp(H, C, ldh, nullptr, R, C, nonzero, list, rel_damp, eq, flags, st);
+}
+
+}  // namespace mq
+
 extern "C" size_t mq_hessian_prepare_workspace_bytes(int64_t C) {
   if (C < 0) return 0;
   // nonzero[C] + list[1 + C], each rounded up to 256 bytes
@@ -342,31 +526,14 @@ extern "C" int mq_hessian_prepare(float* H, int64_t C, int64_t ldh, float* W, in
   MQ_REQUIRE(nonzero && list, MQ_ERR_WORKSPACE, "mq_hessian_prepare: workspace of %zu bytes is too small", workspace_bytes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-  MQ_CUDA(cudaMemsetAsync(flags, 0, sizeof(mq_layer_flags), st));
-  {
-    const unsigned gx = (unsigned)ceil_div(C / 4, 256);
-    unsigned gy = (unsigned)(148 * 8 / gx);
-    if (gy < 1) gy = 1;
-    if ((int64_t)gy > C) gy = (unsigned)C;
-    nan_scan_kernel<<<dim3(gx, gy), 256, 0, st>>>(H, C, ldh, flags);
-  }
-  MQ_LAUNCH_CHECK();
-  identity_if_nan_kernel<<<148 * 4, 256, 0, st>>>(H, C, ldh, flags);
-  MQ_LAUNCH_CHECK();
+  MQ_TRY(scan_hessian(H, C, ldh, W ? nonzero : nullptr, flags, st));
   if (W) {
-    MQ_CUDA(cudaMemsetAsync(nonzero, 0, C * sizeof(int), st));
     const int rows_per_block = 64;
     dim3 grid((unsigned)ceil_div(C, 256), (unsigned)ceil_div(R, rows_per_block));
     column_nonzero_kernel<<<grid, 256, 0, st>>>(W, R, C, ldw, rows_per_block, nonzero);
     MQ_LAUNCH_CHECK();
   }
-  build_mask_kernel<<<1, 1024, 0, st>>>(H, C, ldh, W ? nonzero : nullptr, list, flags);
-  MQ_LAUNCH_CHECK();
-  apply_mask_kernel<<<148, 256, 0, st>>>(H, C, ldh, W, R, ldw, list);
-  MQ_LAUNCH_CHECK();
-  damp_kernel<<<1, 1024, 0, st>>>(H, C, ldh, rel_damp);
-  MQ_LAUNCH_CHECK();
-  return MQ_OK;
+  return mask_and_damp(H, C, ldh, W, R, ldw, W ? nonzero : nullptr, list, rel_damp, nullptr, flags, st);
 }
 
 extern "C" int mq_absmax_scales(const float* W, int64_t R, int64_t C, int64_t ldw, int64_t group, int bits,

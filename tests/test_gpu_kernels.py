@@ -616,3 +616,38 @@ def test_sweep_tile_row_groups(cuda, R, C, g):
     want = sweep(base[: min(R, 64)].to(cuda), ops.Precision())
     assert torch.equal(got, want[torch.arange(R) % 64])
     assert torch.equal(got, sweep(W.to(cuda), ops.Precision(compact=True)))
+
+
+# ------------------------------------------------------------------ the weights' way in, the diagonal pass
+@pytest.mark.parametrize("R,C,g", [(1, 8, 8), (65, 136, 8), (7, 160, 32), (64, 192, 64), (130, 1152, 128), (3, 9216, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_layer_preparation_against_oracle(cuda, R, C, g, dtype, offset):
+    """Dead channels, all-zero columns, ragged column blocks, more channels than one pass over the diagonal
+    keeps, weights that start off a vector boundary: scales, damped Hessian and flags."""
+    gen = torch.Generator().manual_seed(R + C)
+    W = (0.02 * torch.randn(R, C, generator=gen)).to(dtype)
+    W[:, 3] = 0.0
+    H = torch.diag(torch.rand(C, generator=gen) + 0.5)
+    H[0, 5] = H[5, 0] = 0.1
+    H[3, 4] = H[4, 3] = 0.2
+    H[6] = 0.0
+    H[:, 6] = 0.0
+    store = torch.empty(offset + R * C, dtype=dtype, device=cuda)
+    w = store[offset:].view(R, C)
+    w.copy_(W)
+    Hd = H.to(cuda)
+    _, scales, _, flags = ops.quantize_layer([w], Hd, g, 4, 1e-2)
+    Wm = W.float().clone()
+    Wm[:, 6] = 0.0
+    s0, _, _ = O.symmetric_grid(Wm, g, 4, dtype)
+    assert torch.equal(scales[0].cpu(), s0.float().reshape(R, C // g))
+    zero_cols = int((Wm == 0).all(0).sum())
+    assert flags.tolist()[:3] == [0, 1, zero_cols] and int(flags[3]) == 0
+    want = H.clone()
+    for c in torch.nonzero((Wm == 0).all(0)).flatten().tolist():
+        want[c] = 0.0
+        want[:, c] = 0.0
+        want[c, c] = 1.0
+    want.diagonal().add_(1e-2 * want.diagonal().double().mean().float())
+    torch.testing.assert_close(Hd.cpu(), want, rtol=2e-6, atol=0)   # the mean's sum in another order
