@@ -242,6 +242,10 @@ int mq_quadratic_form(const float* A, int64_t R, int64_t C, int64_t lda, const f
                       double* out, int math, int split, void* workspace, size_t workspace_bytes,
                       void* stream);
 size_t mq_quadratic_form_workspace_bytes(int64_t R, int64_t C, int math, int split);
+/* Both forms of the metric at once, at full tensor precision: out[0] for q - w, out[1] for w.  */
+int mq_error_forms(const float* q, int64_t ldq, const float* w, int64_t ldw, int64_t R, int64_t C, const float* H,
+                   int64_t ldh, double* out, void* workspace, size_t workspace_bytes, void* stream);
+size_t mq_error_forms_workspace_bytes(int64_t R, int64_t C);
 
 /* ------------------------------------------------------------------ a11
  * compressed-tensors int4 -> int32 packing of pack_weight / pack_to_int32

@@ -66,6 +66,9 @@ SIGNATURES = {
     "mq_quadratic_form": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int, c_int,
                                   c_void_p, c_size_t, c_void_p]),
     "mq_quadratic_form_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int, c_int]),
+    "mq_error_forms": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_size_t,
+                               c_void_p]),
+    "mq_error_forms_workspace_bytes": (c_size_t, [c_int64, c_int64]),
     "mq_pack_int4": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_void_p]),
 }
 

@@ -59,7 +59,7 @@ __device__ __forceinline__ float scale_below_2_14(float bound) {
   const int b = (int)((__float_as_uint(bound) >> 23) & 0xFFu);
   if (b == 0 || b == 255) return 1.0f;
   int e = 14 - (b - 126);
-  e = e < -60 ? -60 : (e > 60 ? 60 : e);
+  e = e < -100 ? -100 : (e > 100 ? 100 : e);
   return __uint_as_float((uint32_t)(e + 127) << 23);
 }
 

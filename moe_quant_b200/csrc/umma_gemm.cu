@@ -40,6 +40,15 @@ constexpr int GEMM_THREADS = 192;
 constexpr int STAGE_LD = 36;                        // floats per row of an epilogue staging tile
 constexpr int STAGE_BYTES = 4 * 32 * STAGE_LD * 4;  // four epilogue warps
 
+// Sum of (A S)[r, n] A[r, n] over a tile instead of the tile itself.  Rows [0, rows) of the operand are x0 - x1 (x0
+// if x1 is null), those of the second form, which starts at row `second`, are x1; out[0], out[1] take the sums.
+struct DotForm {
+  const float* x0; int64_t ld0;
+  const float* x1; int64_t ld1;
+  int rows, second;
+  double* out;
+};
+
 struct UmmaParams {
   float* C;
   int64_t ldc, c_bs;
@@ -56,6 +65,7 @@ struct UmmaParams {
   int pairs;           // operands are pairs of fp16 planes: the leading product is summed per slab of k (see below)
   const float* row_f;  // optional factors of the product per row / column of C
   const float* col_f;
+  DotForm dot;         // pair kernel, DOT form
   int drain_slabs;  // streaming kernel: slabs of k per accumulator before it is added to C (0 = all of K)
 };
 
@@ -1212,13 +1222,30 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
   }
 }
 
+// DOT: nothing is stored; B is upper triangular (rows past a tile's last column hold nothing: k stops there), tiles are
+// taken from the right, longest first, and the epilogue sums the tile's products with A in fp64.
+__device__ __forceinline__ void pair_tile(TileWalk& w, int idx, int n_tiles, int m_tiles, bool dot, int upper) {
+  if (dot) {
+    w.n = n_tiles - 1 - idx / m_tiles;
+    w.m = idx % m_tiles;
+  } else {
+    w.seek(idx, n_tiles, upper);
+  }
+}
+
+template <bool DOT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const __grid_constant__ CUtensorMap map_c, const UmmaParams p, const int total) {
   const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
   const int n_tiles = (p.N + PAIR_TILE - 1) / PAIR_TILE;
   const int my_tiles = (total - pair + n_pairs - 1) / n_pairs;   // the host launches at most one pair per tile
-  const int n_slabs = (p.K + SLAB_K - 1) / SLAB_K;
+  const int m_tiles = (p.M + PAIR_TILE - 1) / PAIR_TILE;
+  const int all_slabs = (p.K + SLAB_K - 1) / SLAB_K;
+  auto slabs_of = [&](const TileWalk& w) {
+    const int last = (w.n + 1) * (PAIR_TILE / SLAB_K);
+    return DOT && last < all_slabs ? last : all_slabs;
+  };
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -1259,7 +1286,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
       bool ok = true;
       for (int i = 0; i < my_tiles && ok; ++i) {
         TileWalk w;
-        w.seek(pair + i * n_pairs, n_tiles, p.upper_tiles_only);
+        pair_tile(w, pair + i * n_pairs, n_tiles, m_tiles, DOT, p.upper_tiles_only);
+        const int n_slabs = slabs_of(w);
         const int a_row = w.m * PAIR_TILE + rank * TILE_M + p.a_row0;
         const int b_row = w.n * PAIR_TILE + rank * TILE_N + p.b_row0;
         for (int s = 0; s < n_slabs; ++s, ++it) {
@@ -1287,6 +1315,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
         int it = 0;
         bool ok = true;
         for (int i = 0; i < my_tiles && ok; ++i) {
+          TileWalk w;
+          pair_tile(w, pair + i * n_pairs, n_tiles, m_tiles, DOT, p.upper_tiles_only);
+          const int n_slabs = slabs_of(w);
           for (int s = 0; s < n_slabs && ok; ++s, ++it) {
             const int st = it % PAIR_STAGES;
             ok = mbar_wait(full0 + 8 * st, (it / PAIR_STAGES) & 1, 52);
@@ -1326,8 +1357,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     const uint32_t my_row = box + (uint32_t)lane * 128u;
     bool ok = true;
     int it = 0;
+    double total0 = 0.0, total1 = 0.0;
 #pragma unroll 1
     for (int i = 0; i < my_tiles && ok; ++i) {
+      TileWalk w;
+      pair_tile(w, pair + i * n_pairs, n_tiles, m_tiles, DOT, p.upper_tiles_only);
+      const int n_slabs = slabs_of(w);
       float acc[TILE_N];
 #pragma unroll
       for (int j = 0; j < TILE_N; ++j) acc[j] = 0.0f;
@@ -1343,10 +1378,47 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
         if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * b);
       }
       if (!ok) break;
-      TileWalk w;
-      w.seek(pair + i * n_pairs, n_tiles, p.upper_tiles_only);
       const int mb = 2 * w.m + rank, nb = 2 * w.n + h;          // 128-blocks
       const int y = mb * TILE_M + q * 32, n0 = nb * TILE_N;
+      if constexpr (DOT) {
+        // this lane's row of A against its 128 sums, 32 columns at a time: the block of A is read along its rows
+        // (a load is one 128-byte segment) and turned through a swizzled tile of this warp
+        const bool two = y >= p.dot.second;                  // forms begin at whole tiles: uniform in the warp
+        const int r_first = two ? y - p.dot.second : y;
+        const float* a0 = two ? p.dot.x1 + (int64_t)r_first * p.dot.ld1 : p.dot.x0 + (int64_t)r_first * p.dot.ld0;
+        const int64_t ld0 = two ? p.dot.ld1 : p.dot.ld0;
+        const float* a1 = (two || p.dot.x1 == nullptr) ? nullptr : p.dot.x1 + (int64_t)r_first * p.dot.ld1;
+        float* boxf = reinterpret_cast<float*>(smem_raw + (box - smem_u32(smem_raw)));
+        double sum = 0.0;
+#pragma unroll
+        for (int c = 0; c < TILE_N / 32; ++c) {
+          const int x = n0 + c * 32;
+          const bool col_in = x + lane < p.N;
+#pragma unroll 8
+          for (int r = 0; r < 32; ++r) {
+            const bool in = col_in && r_first + r < p.dot.rows;
+            float v = in ? __ldg(a0 + (int64_t)r * ld0 + x + lane) : 0.0f;
+            if (a1 && in) v -= __ldg(a1 + (int64_t)r * p.dot.ld1 + x + lane);
+            boxf[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)] = v;
+          }
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(boxf + lane * 32 + ((j ^ (lane & 7)) << 2));
+            const float av[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+              if (x + 4 * j + t < p.N) sum += (double)acc[c * 32 + 4 * j + t] * (double)__ldg(p.col_f + x + 4 * j + t) * (double)av[t];
+          }
+          __syncwarp();
+        }
+        if (r_first + lane < p.dot.rows) {
+          const double f = (double)__ldg(p.row_f + y + lane);
+          if (two) total1 += sum * f;
+          else total0 += sum * f;
+        }
+        continue;
+      }
       // inside a diagonal tile the 128-block below the diagonal is left alone
       const bool keep = y < p.M && n0 < p.N && !(p.upper_tiles_only && mb > nb);
       if (keep) {
@@ -1375,6 +1447,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             bulk_commit();
           }
         }
+      }
+    }
+    if constexpr (DOT) {
+      for (int o = 16; o > 0; o >>= 1) {
+        total0 += __shfl_xor_sync(0xffffffffu, total0, o);
+        total1 += __shfl_xor_sync(0xffffffffu, total1, o);
+      }
+      if (lane == 0) {
+        atomicAdd(p.dot.out, total0);
+        if (p.dot.x1) atomicAdd(p.dot.out + 1, total1);
       }
     }
     if (lane == 0) bulk_wait_read_all();  // the boxes have left shared memory; the writes land before the grid completes
@@ -1591,6 +1673,129 @@ __global__ void __launch_bounds__(256) split_factor_half_kernel(const float* __r
   }
 }
 
+// ---- operands of a quadratic form  sum_r a_r H a_r^T  (pair kernel, DOT form).  Only the symmetric part of H counts, so B is
+// the upper triangle S[i][j] = H[i][j] + H[j][i] (i < j), H[i][i]: half the contraction, any square H.
+// bound[j] >= max_i |S[i][j]|: upper[j] = max over i <= j of |H[i][j]|, lower[j] = max over i < j of |H[j][i]|, as the bits
+// of non-negative floats.  A CTA takes 64 rows x 128 columns, a warp 8 rows with four in flight.
+__global__ void __launch_bounds__(256) form_bound_kernel(const float* __restrict__ H, int64_t ldh, int C, int* __restrict__ upper,
+                                                         int* __restrict__ lower) {
+  __shared__ float part[8][TILE_N];
+  const int c0 = (int)blockIdx.x * TILE_N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r0 = (int)blockIdx.y * 64 + warp * 8;
+  float m[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    float v[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = r0 + half * 4 + u, c = c0 + lane + 32 * q;
+        v[u][q] = r < C && c < C ? fabsf(__ldg(H + (int64_t)r * ldh + c)) : 0.0f;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = r0 + half * 4 + u;
+      float low = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (c0 + lane + 32 * q >= r) m[q] = fmaxf(m[q], v[u][q]);
+        else low = fmaxf(low, v[u][q]);
+      }
+      if (c0 < r) {   // uniform in the warp
+        for (int o = 16; o > 0; o >>= 1) low = fmaxf(low, __shfl_xor_sync(0xffffffffu, low, o));
+        if (lane == 0 && r < C) atomicMax(lower + r, __float_as_int(low));
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) part[warp][lane + 32 * q] = m[q];
+  __syncthreads();
+  if (threadIdx.x < TILE_N && c0 + (int)threadIdx.x < C) {
+    float x = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) x = fmaxf(x, part[w][threadIdx.x]);
+    if (x > 0.0f) atomicMax(upper + c0 + threadIdx.x, __float_as_int(x));
+  }
+}
+
+// S -> fp16 pairs, destination row j, k = i, scaled by a power of two per j (inv_t[j] = its inverse); zero for
+// k > j up to the end of the row's 256-block, not written beyond.  64 x 64 tiles, the upper one read through a transposing tile.
+__global__ void __launch_bounds__(256) split_form_kernel(const float* __restrict__ H, int64_t ldh, int C, int rows_pad, int K_pad,
+                                                         const int* __restrict__ upper, const int* __restrict__ lower,
+                                                         float* __restrict__ inv_t, uint16_t* __restrict__ dst, int64_t plane_stride) {
+  __shared__ float tile[64][65];  // tile[k][r] = H[k][r]
+  const int r0 = blockIdx.y * 64, k0 = blockIdx.x * 64;
+  if (k0 >= (r0 / PAIR_TILE + 1) * PAIR_TILE) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = k0 + warp + 8 * i;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = r0 + lane + 32 * h;
+      tile[warp + 8 * i][lane + 32 * h] = (k <= r && r < C) ? __ldg(H + (int64_t)k * ldh + r) : 0.0f;
+    }
+  }
+  __syncthreads();
+  const int k = k0 + 2 * lane;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int rl = warp + 8 * i, r = r0 + rl;
+    if (r >= rows_pad || k >= K_pad) continue;
+    float x0 = 0.0f, x1 = 0.0f;
+    if (r < C) {
+      const float t = scale_below_2_14(__int_as_float(__ldg(upper + r)) + __int_as_float(__ldg(lower + r)));
+      if (blockIdx.x == 0 && lane == 0) inv_t[r] = 1.0f / t;
+      if (k < r) x0 = (tile[2 * lane][rl] + __ldg(H + (int64_t)r * ldh + k)) * t;
+      else if (k == r) x0 = tile[2 * lane][rl] * t;
+      if (k + 1 < r) x1 = (tile[2 * lane + 1][rl] + __ldg(H + (int64_t)r * ldh + k + 1)) * t;
+      else if (k + 1 == r) x1 = tile[2 * lane + 1][rl] * t;
+    }
+    uint16_t h0, l0, h1, l1;
+    split_half2(x0, h0, l0);
+    split_half2(x1, h1, l1);
+    uint16_t* o = dst + (int64_t)r * K_pad + k;
+    *reinterpret_cast<uint32_t*>(o) = (uint32_t)h0 | ((uint32_t)h1 << 16);
+    *reinterpret_cast<uint32_t*>(o + plane_stride) = (uint32_t)l0 | ((uint32_t)l1 << 16);
+  }
+}
+
+// The forms' rows -> fp16 pairs scaled by a power of two per row (row_f = its inverse); zero rows behind each form up
+// to a whole tile.  One CTA per row, which is read twice (the second time from the cache).
+__global__ void __launch_bounds__(256) split_rows_kernel(DotForm f, int C, int K_pad, float* __restrict__ row_f,
+                                                         uint16_t* __restrict__ dst, int64_t plane_stride) {
+  __shared__ float part[8];
+  const int row = blockIdx.x, t = threadIdx.x;
+  const bool two = row >= f.second;
+  const int r = two ? row - f.second : row;
+  const bool in = r < f.rows;
+  const float* a0 = in ? (two ? f.x1 + (int64_t)r * f.ld1 : f.x0 + (int64_t)r * f.ld0) : nullptr;
+  const float* a1 = (!in || two || f.x1 == nullptr) ? nullptr : f.x1 + (int64_t)r * f.ld1;
+  auto value = [&](int c) { return a1 ? __ldg(a0 + c) - __ldg(a1 + c) : __ldg(a0 + c); };
+  float m = 0.0f;
+  if (in) {
+#pragma unroll 8
+    for (int c = t; c < C; c += 256) m = fmaxf(m, fabsf(value(c)));
+  }
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((t & 31) == 0) part[t >> 5] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) m = fmaxf(m, part[w]);
+  const float scale = scale_below_2_14(m);
+  if (t == 0) row_f[row] = 1.0f / scale;
+  uint16_t* o = dst + (int64_t)row * K_pad;
+#pragma unroll 4
+  for (int k = 2 * t; k < K_pad; k += 512) {
+    uint16_t h0, l0, h1, l1;
+    split_half2(in && k < C ? value(k) * scale : 0.0f, h0, l0);
+    split_half2(in && k + 1 < C ? value(k + 1) * scale : 0.0f, h1, l1);
+    *reinterpret_cast<uint32_t*>(o + k) = (uint32_t)h0 | ((uint32_t)h1 << 16);
+    *reinterpret_cast<uint32_t*>(o + k + plane_stride) = (uint32_t)l0 | ((uint32_t)l1 << 16);
+  }
+}
+
 // 16-bit activations whose row index is the contiguous one (X stored tokens x channels, wanted as
 // channels x tokens): a plain transposing copy of one plane, 64 x 64 tiles, 128-byte rows on both
 // the global reads and the global writes.  Zero outside (rows, K) up to (rows_pad, K_pad).
@@ -1737,7 +1942,8 @@ int configure_once() {
     MQ_CUDA(cudaFuncSetAttribute(umma_gemm_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
     MQ_CUDA(cudaFuncSetAttribute(umma_gemm_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
     MQ_CUDA(cudaFuncSetAttribute(umma_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-    MQ_CUDA(cudaFuncSetAttribute(umma_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
+    MQ_CUDA(cudaFuncSetAttribute(umma_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
+    MQ_CUDA(cudaFuncSetAttribute(umma_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
     MQ_CUDA(cudaFuncSetAttribute(umma_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
     done[dev & 63] = true;
   }
@@ -1753,7 +1959,7 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
   CUtensorMap map_a, map_b;
   MQ_TRY(encode_map(A, &map_a));
   MQ_TRY(encode_map(B, &map_b));
-  UmmaParams p;
+  UmmaParams p = {};
   p.C = d.C; p.ldc = d.ldc; p.c_bs = d.c_bs;
   p.M = d.M; p.N = d.N; p.K = d.K;
   p.alpha = d.alpha; p.beta = d.beta;
@@ -1831,7 +2037,7 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
     CUtensorMap map_c;
     MQ_TRY(encode_c_map(d.C, d.ldc, d.M, d.N, &map_c));
     p.idesc = (1u << 4) | ((uint32_t)(PAIR_TILE >> 3) << 17) | ((uint32_t)(PAIR_TILE >> 4) << 24);   // fp16, fp32 sums, M 256, N 256
-    MQ_CUDA(launch_chained(true, umma_pair_kernel, dim3((unsigned)(2 * (tiles < 74 ? tiles : 74))), dim3(PAIR_THREADS), kPairSmem, st,
+    MQ_CUDA(launch_chained(true, umma_pair_kernel<false>, dim3((unsigned)(2 * (tiles < 74 ? tiles : 74))), dim3(PAIR_THREADS), kPairSmem, st,
                            map_a, map_b, map_c, p, (int)tiles));
   } else if (deep_route) {
     // deep update with several planes: persistent streaming kernel
@@ -1930,6 +2136,62 @@ int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, f
   }
   split_factor_half_kernel<<<dim3((unsigned)(ps.K_pad / 64), (unsigned)ceil_div(ps.rows_pad, 64)), 256, 0, st>>>(
       U, ldu, C, ps.rows_pad, ps.K_pad, col_div, eq, colmax, inv_t, dst, ps.total_rows * (int64_t)ps.K_pad);
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
+}
+
+size_t quadratic_forms_workspace_bytes(int64_t R, int64_t C, int forms) {
+  const int64_t rows = (int64_t)forms * pad_to((int)R, PAIR_TILE);
+  return plane_set_bytes(rows, C, 2) + plane_set_bytes(C, C, 2) + align_up((size_t)rows * sizeof(float), 256) +
+         align_up((size_t)C * 3 * sizeof(float), 256);
+}
+
+// out[0] = sum (X0 - X1) H (X0 - X1)^T, out[1] = sum X1 H X1^T over the rows (R x C fp32 each); X1 null: out[0] = sum X0 H X0^T.
+int quadratic_forms(const float* X0, int64_t ld0, const float* X1, int64_t ld1, int64_t R, int64_t C, const float* H, int64_t ldh, double* out,
+                    Workspace& ws, cudaStream_t st) {
+  MQ_TRY(configure_once());
+  const int forms = X1 ? 2 : 1;
+  DotForm f;
+  f.x0 = X0; f.ld0 = ld0; f.x1 = X1; f.ld1 = ld1;
+  f.rows = (int)R; f.second = pad_to((int)R, PAIR_TILE);
+  f.out = out;
+  PlaneSet A, Bp;
+  A.planes = Bp.planes = 2;
+  A.fp16 = Bp.fp16 = true;
+  A.K_pad = Bp.K_pad = pad_to((int)C, SLAB_K);
+  A.rows_pad = forms * f.second; A.total_rows = A.rows_pad;
+  Bp.rows_pad = pad_to((int)C, TILE_N); Bp.total_rows = Bp.rows_pad;
+  A.base = ws.take<uint16_t>((size_t)2 * A.total_rows * A.K_pad);
+  Bp.base = ws.take<uint16_t>((size_t)2 * Bp.total_rows * Bp.K_pad);
+  float* row_f = ws.take<float>((size_t)A.total_rows);
+  float* col_f = ws.take<float>((size_t)C * 3);
+  MQ_REQUIRE(A.base && Bp.base && row_f && col_f, MQ_ERR_WORKSPACE, "quadratic form: workspace too small");
+  int* upper = reinterpret_cast<int*>(col_f + C);
+  int* lower = upper + C;
+  MQ_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * forms, st));
+  MQ_CUDA(cudaMemsetAsync(upper, 0, sizeof(int) * 2 * (size_t)C, st));
+  form_bound_kernel<<<dim3((unsigned)ceil_div(C, TILE_N), (unsigned)ceil_div(C, 64)), 256, 0, st>>>(H, ldh, (int)C, upper, lower);
+  MQ_LAUNCH_CHECK();
+  split_form_kernel<<<dim3((unsigned)(Bp.K_pad / 64), (unsigned)(Bp.rows_pad / 64)), 256, 0, st>>>(
+      H, ldh, (int)C, Bp.rows_pad, Bp.K_pad, upper, lower, col_f, Bp.base, Bp.total_rows * (int64_t)Bp.K_pad);
+  MQ_LAUNCH_CHECK();
+  split_rows_kernel<<<(unsigned)A.total_rows, 256, 0, st>>>(f, (int)C, A.K_pad, row_f, A.base,
+                                                                         A.total_rows * (int64_t)A.K_pad);
+  MQ_LAUNCH_CHECK();
+  CUtensorMap map_a, map_b;
+  MQ_TRY(encode_map(A, &map_a));
+  MQ_TRY(encode_map(Bp, &map_b));
+  UmmaParams p = {};
+  p.M = (int)A.total_rows; p.N = (int)C; p.K = (int)C;
+  p.alpha = 1.0f;
+  p.planes = 2; p.pairs = 1;
+  p.row_f = row_f; p.col_f = col_f;
+  p.dot = f;
+  p.idesc = (1u << 4) | ((uint32_t)(PAIR_TILE >> 3) << 17) | ((uint32_t)(PAIR_TILE >> 4) << 24);
+  const long long tiles = (long long)(A.total_rows / PAIR_TILE) * ceil_div(C, PAIR_TILE);
+  ProfScope prof(PROF_UMMA_DEEP, (double)forms * R * C * (C + 1), 3.0 * forms * R * C * (C + 1), st);
+  MQ_CUDA(launch_chained(false, umma_pair_kernel<true>, dim3((unsigned)(2 * (tiles < 74 ? tiles : 74))), dim3(PAIR_THREADS), kPairSmem, st,
+                         map_a, map_b, map_a, p, (int)tiles));
   MQ_LAUNCH_CHECK();
   return MQ_OK;
 }

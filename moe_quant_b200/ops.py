@@ -304,6 +304,24 @@ def quadratic_form(A: Tensor, H: Tensor, precision: Optional[Precision] = None) 
     return out
 
 
+def error_forms(q: Tensor, w: Tensor, H: Tensor) -> Tensor:
+    """(sum((d @ H) * d) with d = q - w, sum((w @ H) * w)) as a float64 tensor on the device, from one contraction.
+    q, w (R, C) fp32, H (C, C) fp32; full tensor precision."""
+    for t, n in ((q, "q"), (w, "w"), (H, "H")):
+        require_cuda(t, n)
+    if any(t.dtype != torch.float32 or t.dim() != 2 for t in (q, w, H)) or q.shape != w.shape or H.shape != (q.shape[1], q.shape[1]):
+        raise MoeQuantError("error_forms: q and w must be (R, C) fp32 and H (C, C) fp32")
+    q, w, H = (t if t.stride(1) == 1 else t.contiguous() for t in (q, w, H))
+    R, C = q.shape
+    out = torch.empty(2, dtype=torch.float64, device=q.device)
+    L = lib()
+    ws = _lib.workspace(q.device, L.mq_error_forms_workspace_bytes(R, C))
+    with torch.cuda.device(q.device):
+        check(L.mq_error_forms(ptr(q), q.stride(0), ptr(w), w.stride(0), R, C, ptr(H), H.stride(0), ptr(out), ptr(ws), ws.numel(),
+                               stream_ptr(q.device)))
+    return out
+
+
 def pack_int4(codes: Tensor, zero_i8: Optional[Tensor] = None, group: int = 0) -> Tensor:
     """(R, C) uint8 codes -> (R, ceil(C/8)) int32 words in the compressed-tensors layout."""
     require_cuda(codes, "codes")

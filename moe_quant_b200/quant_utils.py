@@ -67,10 +67,15 @@ def get_relative_mse_error(q: Tensor, w: Tensor, H: Optional[Tensor] = None) -> 
     """mean((q-w) H o (q-w)) / (mean(w H o w) + 1e-6) (src/quant_utils.py:259-264).  Both
     quadratic forms run on the engine (`mq_quadratic_form`); the result is an fp32 scalar on the
     device like the reference's."""
+    n = float(w.numel())
+    p = ops.DEFAULT_PRECISION
+    if (H is not None and q.dtype == w.dtype == torch.float32 and q.dim() == 2 and q.shape == w.shape and w.numel() > 0
+            and p.math == ops.MATH_TENSOR and p.split_hinv == 3):
+        num, den = (ops.error_forms(q, w, H.float()) / n).unbind()
+        return (num / (den + 1e-6)).float()
     delta = (q - w).float()
     if H is None:
         return delta.pow(2).mean() / w.pow(2).mean()
-    n = float(w.numel())
     num = ops.quadratic_form(delta, H.float()) / n
     den = ops.quadratic_form(w.float(), H.float()) / n
     return (num / (den + 1e-6)).float()

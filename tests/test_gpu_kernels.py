@@ -651,3 +651,30 @@ def test_layer_preparation_against_oracle(cuda, R, C, g, dtype, offset):
         want[c, c] = 1.0
     want.diagonal().add_(1e-2 * want.diagonal().double().mean().float())
     torch.testing.assert_close(Hd.cpu(), want, rtol=2e-6, atol=0)   # the mean's sum in another order
+
+
+# ------------------------------------------------------------------ quadratic forms
+@pytest.mark.parametrize("R,C", [(1, 1), (3, 13), (255, 64), (257, 200), (40, 257), (300, 1031), (512, 768)])
+@pytest.mark.parametrize("kind", ["hessian", "unsymmetric", "spread", "tiny"])
+def test_quadratic_forms_against_fp64(cuda, R, C, kind):
+    """Ragged tiles in rows, columns and k; any square H, not only symmetric ones; scales over many decades; row
+    strides.  Error: three of four half products of 22-bit pairs, 2^-22 each, sums of 64 of k in the
+    tensor core (four truncations at 2^-23): below 2^-20 of the sum of absolute products."""
+    gen = torch.Generator().manual_seed(R * 1000 + C)
+    X = torch.randn(2 * C + 3, C, generator=gen, dtype=torch.float64)
+    if kind == "spread":
+        X *= torch.exp(3.0 * torch.randn(C, generator=gen, dtype=torch.float64))
+    H = (X.T @ X / X.shape[0]).float()
+    if kind == "unsymmetric":
+        H = torch.randn(C, C, generator=gen)
+    q, w = torch.randn(R, C, generator=gen), torch.randn(R, C, generator=gen)
+    if kind == "tiny":
+        q, w, H = q * 1e-9, w * 1e-12, H * 1e-20
+    wide = torch.empty(R, C + 5, device=cuda)
+    wide[:, :C] = q.to(cuda)
+    got = ops.error_forms(wide[:, :C], w.to(cuda), H.to(cuda)).cpu()
+    one = ops.quadratic_form(w.to(cuda), H.to(cuda)).cpu()
+    for a, g in (((q - w), got[0]), (w, got[1]), (w, one)):
+        a, h = a.double(), H.double()
+        want, size = float(((a @ h) * a).sum()), float(((a.abs() @ h.abs()) * a.abs()).sum())
+        assert abs(float(g) - want) <= 2.0 ** -20 * size
