@@ -130,9 +130,6 @@ class GPTQ:
     @torch.no_grad()
     def update(self, input: Tensor) -> None:
         """H <- n/(n+m) H + 2/(n+m) X^T X (src/gptq.py:74-105)."""
-        if self.H is None:
-            self.H = torch.zeros((self.d_col, self.d_col), device=input.device, dtype=torch.float32)
-            self._was_reset = False
         if isinstance(self.layer, nn.Linear):
             x = input.reshape(-1, input.shape[-1])
         else:
@@ -142,6 +139,19 @@ class GPTQ:
         if x.dtype not in (torch.float32, torch.bfloat16, torch.float16):
             x = x.float()
         m = x.shape[0]
+        if self.H is None:
+            self._was_reset = False
+            # the first batch writes the whole matrix (beta = 0 reads nothing)
+            first = torch.empty if m > 0 and self.num_samples == 0 else torch.zeros
+            self.H = first((self.d_col, self.d_col), device=input.device, dtype=torch.float32)
+            if first is torch.empty:
+                try:
+                    ops.hessian_accum(self.H, x, 0.0, 2.0 / m, self.precision)
+                except Exception:
+                    self.H.zero_()
+                    raise
+                self.num_samples = m
+                return
         if m == 0:
             return
         beta = self.num_samples / (self.num_samples + m)
