@@ -322,11 +322,13 @@ class GPTQ:
             ops.mse_scales(Wf, scale, g, bits, self.W_dtype)
         perm = torch.argsort(self.H.diag(), descending=True)
         Hp = self.H[perm][:, perm].contiguous()
-        U, flags, _ = ops.hinv_upper(Hp, self.precision)
+        # the inverse-free sweep, as in the default order: the triangular inverse is not needed
+        flags, _ = ops.chol_unit_factor(Hp, self.precision)
         self._absorb_flags(flags)
         Wp = Wf[:, perm].contiguous()
         sp = scale.repeat_interleave(g, dim=-1)[:, perm].contiguous()
-        codes_p, _ = ops.gptq_sweep(Wp, U, sp, None, 1, self.d_col, 1, bits, self.W_dtype, precision=self.precision)
+        codes_p, _ = ops.gptq_sweep(Wp.clone(), Hp, sp, None, 1, self.d_col, 1, bits, self.W_dtype, precision=self.precision,
+                                    W_original=Wp)
         codes = torch.empty_like(codes_p)
         codes[:, perm] = codes_p
         return codes, scale
