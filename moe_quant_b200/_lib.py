@@ -150,7 +150,27 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the raw handle of the current stream, without building a Stream object for it
+    return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
+
+
+class _Nothing:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NOTHING = _Nothing()
+
+
+def on_device(device: torch.device):
+    """torch.cuda.device(device), or nothing where that device is the current one already: the calls of a small
+    layer are bound by the host, and the guard alone cost a tenth of them."""
+    if device.index is None or device.index == torch.cuda.current_device():
+        return _NOTHING
+    return torch.cuda.device(device)
 
 
 _workspaces: dict = {}
@@ -164,7 +184,7 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     layer would otherwise pin gigabytes on every stream it ever ran on).  The caching allocator
     keeps the old block alive until the stream's queued work has used it."""
     index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (index, torch.cuda.current_stream(device).cuda_stream)
+    key = (index, stream_ptr(device))
     buf = _workspaces.get(key)
     oversized = buf is not None and buf.numel() > (1 << 30) and 4 * max(int(nbytes), 1) < buf.numel()
     if buf is None or buf.numel() < nbytes or oversized:

@@ -71,7 +71,7 @@ def hessian_accum(H: Tensor, x: Tensor, beta: float, alpha: float, precision: Op
     L = lib()
     nbytes = L.mq_hessian_accum_workspace_bytes(code, m, C, p.math, p.split_hessian)
     ws = _lib.workspace(H.device, nbytes)
-    with torch.cuda.device(H.device):
+    with _lib.on_device(H.device):
         check(L.mq_hessian_accum(ptr(x) if m else None, code, m, C, x.stride(0) if m else C, ptr(H), H.stride(0),
                                  beta, alpha, p.math, p.split_hessian, ptr(ws), ws.numel(), stream_ptr(H.device)))
 
@@ -92,7 +92,7 @@ def gemm(A: Tensor, B: Tensor, C: Tensor, alpha: float = 1.0, beta: float = 0.0,
     sp = p.split_hinv if split is None else split
     L = lib()
     ws = _lib.workspace(C.device, L.mq_gemm_workspace_bytes(M, N, K, p.math, sp))
-    with torch.cuda.device(C.device):
+    with _lib.on_device(C.device):
         check(L.mq_gemm(ptr(A), A.stride(0), A.stride(1), ptr(B), B.stride(0), B.stride(1), ptr(C), C.stride(0), M, N, K,
                         alpha, beta, int(upper_tiles_only), p.math, sp, ptr(ws), ws.numel(), stream_ptr(C.device)))
 
@@ -110,7 +110,7 @@ def hessian_prepare(H: Tensor, W: Optional[Tensor], rel_damp: float) -> Tensor:
         require_cuda(W, "W")
         if W.dtype != torch.float32 or W.stride(1) != 1:
             raise MoeQuantError("W must be the fp32 working copy with unit column stride")
-    with torch.cuda.device(H.device):
+    with _lib.on_device(H.device):
         check(L.mq_hessian_prepare(ptr(H), C, H.stride(0), ptr(W), 0 if W is None else W.shape[0],
                                    0 if W is None else W.stride(0), rel_damp, ptr(flags), ptr(ws), ws.numel(),
                                    stream_ptr(H.device)))
@@ -124,7 +124,7 @@ def hessian_prepare_noalloc(H: Tensor, W: Optional[Tensor], rel_damp: float, fla
     not overlap on the GPU: they share the array."""
     require_cuda(H, "H")
     require_cuda(flags, "flags")
-    with torch.cuda.device(H.device):
+    with _lib.on_device(H.device):
         check(lib().mq_hessian_prepare_noalloc(ptr(H), H.shape[0], H.stride(0), ptr(W), 0 if W is None else W.shape[0],
                                                0 if W is None else W.stride(0), rel_damp, ptr(flags),
                                                stream_ptr(H.device)))
@@ -144,7 +144,7 @@ def hinv_upper(H: Tensor, precision: Optional[Precision] = None, flags: Optional
         flags = _flags_tensor(H.device)
     nbytes = L.mq_hinv_upper_workspace_bytes(C, p.math, p.split_hinv)
     ws = _lib.workspace(H.device, nbytes)
-    with torch.cuda.device(H.device):
+    with _lib.on_device(H.device):
         check(L.mq_hinv_upper(ptr(H), C, H.stride(0), ptr(U), C, ptr(diag), p.math, p.split_hinv, ptr(flags), ptr(ws),
                               ws.numel(), stream_ptr(H.device)))
     return U, flags, diag
@@ -157,7 +157,7 @@ def absmax_scales(W: Tensor, group: int, bits: int, dtype: torch.dtype) -> Tenso
         raise MoeQuantError("W must be fp32 with unit column stride")
     R, C = W.shape
     out = torch.empty(R, C // group, dtype=torch.float32, device=W.device)
-    with torch.cuda.device(W.device):
+    with _lib.on_device(W.device):
         check(lib().mq_absmax_scales(ptr(W), R, C, W.stride(0), group, bits, dtype_code(dtype), ptr(out),
                                      stream_ptr(W.device)))
     return out
@@ -172,7 +172,7 @@ def mse_scales(W: Tensor, scale: Tensor, group: int, bits: int, dtype: torch.dty
         raise MoeQuantError("W must be fp32 with unit column stride, scale contiguous fp32")
     R, C = W.shape
     shrink = torch.linspace(1, max_shrink, n_grid, dtype=torch.float32, device=W.device)   # src/quant_utils.py:219
-    with torch.cuda.device(W.device):
+    with _lib.on_device(W.device):
         check(lib().mq_mse_scales(ptr(W), R, C, W.stride(0), group, bits, dtype_code(dtype), ptr(shrink), n_grid, norm,
                                   ptr(scale), stream_ptr(W.device)))
     return scale
@@ -189,7 +189,7 @@ def chol_unit_factor(H: Tensor, precision: Optional[Precision] = None, flags: Op
         flags = _flags_tensor(H.device)
     nbytes = L.mq_chol_unit_factor_workspace_bytes(C, p.math, p.split_hinv)
     ws = _lib.workspace(H.device, nbytes)
-    with torch.cuda.device(H.device):
+    with _lib.on_device(H.device):
         check(L.mq_chol_unit_factor(ptr(H), C, H.stride(0), ptr(diag), p.math, p.split_hinv, ptr(flags), ptr(ws),
                                     ws.numel(), stream_ptr(H.device)))
     return flags, diag
@@ -215,7 +215,7 @@ def gptq_sweep(W: Tensor, Uhat: Tensor, scale: Tensor, zero: Optional[Tensor], g
     deq = torch.empty(R, C, dtype=dtype, device=W.device) if want_dequantized else None
     nbytes = L.mq_gptq_sweep_workspace_bytes(R, C, p.math, p.split_sweep)
     ws = _lib.workspace(W.device, nbytes)
-    with torch.cuda.device(W.device):
+    with _lib.on_device(W.device):
         check(L.mq_gptq_sweep(ptr(W), R, C, W.stride(0), ptr(Uhat), Uhat.stride(0), ptr(scale), ptr(zero), group,
                               row_stride, group_stride, bits, dtype_code(dtype), ptr(codes), ptr(packed_out), ptr(deq),
                               ptr(W_original), 0 if W_original is None else W_original.stride(0), p.sweep_math,
@@ -258,7 +258,7 @@ def quantize_layer(weights: Sequence[Tensor], H: Tensor, group: int, bits: int, 
     s_arr = arr(*[t.data_ptr() for t in scales])
     d_arr = arr(*[t.data_ptr() for t in deqs]) if deqs is not None else None
     p_arr = arr(*[t.data_ptr() for t in packed]) if packed is not None else None
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         check(L.mq_quantize_layer(w_arr, dtype_code(dtype), n, R, C, ptr(H), H.stride(0), group, bits, rel_damp, c_arr,
                                   p_arr, s_arr, d_arr, ptr(flags), p.sweep_math, p.split_hinv, p.split_sweep, ptr(ws), ws.numel(),
                                   stream_ptr(dev)))
@@ -279,7 +279,7 @@ def dequantize(codes: Tensor, scale: Tensor, zero: Optional[Tensor], group: int,
         zero = None if zero is None else zero.to(torch.float32)
     scale = scale.contiguous()
     zero = None if zero is None else zero.contiguous()
-    with torch.cuda.device(codes.device):
+    with _lib.on_device(codes.device):
         check(lib().mq_dequantize_typed(ptr(codes), R, C, ptr(scale), ptr(zero), dtype_code(scale.dtype), group, bits,
                                         dtype_code(dtype), ptr(out), stream_ptr(codes.device)))
     return out
@@ -298,7 +298,7 @@ def quadratic_form(A: Tensor, H: Tensor, precision: Optional[Precision] = None) 
     out = torch.empty((), dtype=torch.float64, device=A.device)
     L = lib()
     ws = _lib.workspace(A.device, L.mq_quadratic_form_workspace_bytes(R, C, p.math, p.split_hinv))
-    with torch.cuda.device(A.device):
+    with _lib.on_device(A.device):
         check(L.mq_quadratic_form(ptr(A), R, C, A.stride(0), ptr(H), H.stride(0), ptr(out), p.math, p.split_hinv,
                                   ptr(ws), ws.numel(), stream_ptr(A.device)))
     return out
@@ -311,12 +311,12 @@ def error_forms(q: Tensor, w: Tensor, H: Tensor) -> Tensor:
         require_cuda(t, n)
     if any(t.dtype != torch.float32 or t.dim() != 2 for t in (q, w, H)) or q.shape != w.shape or H.shape != (q.shape[1], q.shape[1]):
         raise MoeQuantError("error_forms: q and w must be (R, C) fp32 and H (C, C) fp32")
-    q, w, H = (t if t.stride(1) == 1 else t.contiguous() for t in (q, w, H))
+    q, w, H = (t if t.stride(1) == 1 and t.stride(0) >= t.shape[1] else t.contiguous() for t in (q, w, H))
     R, C = q.shape
     out = torch.empty(2, dtype=torch.float64, device=q.device)
     L = lib()
     ws = _lib.workspace(q.device, L.mq_error_forms_workspace_bytes(R, C))
-    with torch.cuda.device(q.device):
+    with _lib.on_device(q.device):
         check(L.mq_error_forms(ptr(q), q.stride(0), ptr(w), w.stride(0), R, C, ptr(H), H.stride(0), ptr(out), ptr(ws), ws.numel(),
                                stream_ptr(q.device)))
     return out
@@ -332,6 +332,6 @@ def pack_int4(codes: Tensor, zero_i8: Optional[Tensor] = None, group: int = 0) -
     out = torch.empty(R, (C + 7) // 8, dtype=torch.int32, device=codes.device)
     if zero_i8 is not None:
         zero_i8 = zero_i8.to(torch.int8).contiguous()
-    with torch.cuda.device(codes.device):
+    with _lib.on_device(codes.device):
         check(lib().mq_pack_int4(ptr(codes), R, C, ptr(zero_i8), group, ptr(out), stream_ptr(codes.device)))
     return out
