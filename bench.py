@@ -47,7 +47,8 @@ sys.path.insert(0, ROOT)
 R, C, TOKENS, GROUP, BITS = 2048, 7168, 4096, 128, 4
 WORKLOAD = "deepseek_v3_routed_expert_gate_proj_2048x7168_bf16_g128 (one rank's expert shard, Hessian resident)"
 METRIC = "GPTQ layers/sec (2048x7168, 4b g128)"
-# DRAM traffic of one 128 x 128 output tile of a 512-deep three-plane update (ncu, profiles/)
+# DRAM traffic of one 128 x 128 output tile of a 512-deep update (ncu of the three-plane kernel, profiles/: the C tile in
+# and out, which the operand format does not change, is all but a few KB of it)
 DEEP_DRAM_BYTES_PER_TILE = 103.0e3
 CONFIG = {"workload": WORKLOAD, "rows": R, "cols": C, "bits": BITS, "group_size": GROUP, "rel_damp": 1e-2,
           "weight_dtype": "bf16", "calibration_tokens_mean": TOKENS}
@@ -419,7 +420,7 @@ def headline(cx):
 
         def tensor_line(kind, v):
             secs = v["ms"] / 1e3
-            products = 1.0 if kind == "simt_gemm" else 6.0     # bf16 products per fp32 product with three planes
+            products = 1.0 if kind == "simt_gemm" else 3.0     # fp16 products per fp32 product with pairs of planes
             achieved = v["work"] * products / secs / 1e12
             return {"kernel": kind, "bound": "tensor", "achieved": achieved, "peak": peaks["tensor_sustained"],
                     "unit": "TFLOP/s", "frac": achieved / peaks["tensor_sustained"],
@@ -429,7 +430,7 @@ def headline(cx):
 
         if top in ("umma_gemm", "umma_deep", "simt_gemm"):
             roofline = tensor_line(top, v)
-            products = 1.0 if top == "simt_gemm" else 6.0
+            products = 1.0 if top == "simt_gemm" else 3.0
             out_tiles = v["work2"] / v["launches"] / (2.0 * 128 * 128 * products)   # output tiles x k per launch
             if top == "umma_deep":
                 # DRAM bytes per 128 x 128 output tile of a 512-deep update, from an ncu capture of the
@@ -444,8 +445,8 @@ def headline(cx):
                                               "rank-128 update), not measured in this run")
             else:
                 roofline["traffic"] = None
-            roofline["note"] = ("algorithmic work of the split-bf16 GEMM: 2MNK on the kept tiles x 6 bf16 tensor products per "
-                                "fp32 product (3 planes); fp32_equivalent_tflops counts each fp32 product once; timed on one "
+            roofline["note"] = ("algorithmic work of the GEMM on pairs of fp16 planes: 2MNK on the kept tiles x 3 fp16 tensor products "
+                                "per fp32 product; fp32_equivalent_tflops counts each fp32 product once; timed on one "
                                 "stream with full grids; chosen as the member of the tensor-GEMM family with the most work")
             roofline["peak_source"] = peaks["source"] + " (sustained bf16)"
             roofline["others"] = [tensor_line(k, kv) for k, kv in family.items() if k != top]
