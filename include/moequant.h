@@ -234,6 +234,12 @@ int mq_dequantize(const uint8_t* codes, int64_t R, int64_t C, const float* scale
 int mq_dequantize_typed(const uint8_t* codes, int64_t R, int64_t C, const void* scale, const void* zero,
                         int scale_dtype, int64_t group, int bits, int out_dtype, void* out, void* stream);
 
+/* out[r, j] = src[rows[r], cols[j] / group] for r < R, j < C_out (rows may be NULL: r); elements of 1 or 4 bytes, src with
+ * row stride ld and C_in columns, out (R, C_out) contiguous.  The activation order (src/gptq.py:180-187) reads H, W and the
+ * scales through its permutation and brings the codes back through the inverse.  Indices are not checked.  */
+int mq_permute_columns(const void* src, int elem_bytes, int64_t ld, const int32_t* rows, const int32_t* cols,
+                       int64_t group, int64_t R, int64_t C_in, int64_t C_out, void* out, void* stream);
+
 /* sum over (r,c) of (A H)[r,c] * A[r,c] for A (R,C) fp32 and H (C,C) fp32, written to *out
  * (one double on the device).  Numerator (A = q - w) and denominator (A = w) of
  * get_relative_mse_error (src/quant_utils.py:259-264), the metric quant.py:314-316 logs

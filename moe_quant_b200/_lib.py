@@ -69,6 +69,7 @@ SIGNATURES = {
     "mq_error_forms": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_size_t,
                                c_void_p]),
     "mq_error_forms_workspace_bytes": (c_size_t, [c_int64, c_int64]),
+    "mq_permute_columns": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_void_p, c_void_p]),
     "mq_pack_int4": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_void_p]),
 }
 

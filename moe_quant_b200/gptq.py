@@ -321,16 +321,18 @@ class GPTQ:
         if self._mse_search():
             ops.mse_scales(Wf, scale, g, bits, self.W_dtype)
         perm = torch.argsort(self.H.diag(), descending=True)
-        Hp = self.H[perm][:, perm].contiguous()
+        cols = perm.to(torch.int32)
+        Hp = ops.permute_columns(self.H, cols, rows=cols)
         # the inverse-free sweep, as in the default order: the triangular inverse is not needed
         flags, _ = ops.chol_unit_factor(Hp, self.precision)
         self._absorb_flags(flags)
-        Wp = Wf[:, perm].contiguous()
-        sp = scale.repeat_interleave(g, dim=-1)[:, perm].contiguous()
+        Wp = ops.permute_columns(Wf, cols)
+        sp = ops.permute_columns(scale, cols, group=g)
         codes_p, _ = ops.gptq_sweep(Wp.clone(), Hp, sp, None, 1, self.d_col, 1, bits, self.W_dtype, precision=self.precision,
                                     W_original=Wp)
-        codes = torch.empty_like(codes_p)
-        codes[:, perm] = codes_p
+        back = torch.empty_like(cols)
+        back[perm] = torch.arange(self.d_col, dtype=torch.int32, device=cols.device)
+        codes = ops.permute_columns(codes_p, back)
         return codes, scale
 
     def quantize(self, bits: int | float) -> Tuple[Tensor, Tensor, Tensor]:

@@ -322,6 +322,24 @@ def error_forms(q: Tensor, w: Tensor, H: Tensor) -> Tensor:
     return out
 
 
+def permute_columns(src: Tensor, cols: Tensor, rows: Optional[Tensor] = None, group: int = 1) -> Tensor:
+    """out[r, j] = src[rows[r], cols[j] // group] for a 2-D fp32 or uint8 tensor; cols and rows are int32 index vectors
+    on its device (rows None: every row in place).  The indices must be in range."""
+    for t, n in ((src, "src"), (cols, "cols")) + (() if rows is None else ((rows, "rows"),)):
+        require_cuda(t, n)
+    if src.dim() != 2 or src.dtype not in (torch.float32, torch.uint8) or cols.dtype != torch.int32 or cols.dim() != 1 or (
+            rows is not None and (rows.dtype != torch.int32 or rows.dim() != 1)):
+        raise MoeQuantError("permute_columns: src must be a 2-D fp32 or uint8 tensor, indices int32 vectors")
+    src = src if src.stride(1) == 1 and src.stride(0) >= src.shape[1] else src.contiguous()
+    cols, rows = cols.contiguous(), None if rows is None else rows.contiguous()
+    R = src.shape[0] if rows is None else rows.numel()
+    out = torch.empty(R, cols.numel(), dtype=src.dtype, device=src.device)
+    with _lib.on_device(src.device):
+        check(lib().mq_permute_columns(ptr(src), src.element_size(), src.stride(0), ptr(rows), ptr(cols), group, R, src.shape[1],
+                                       cols.numel(), ptr(out), stream_ptr(src.device)))
+    return out
+
+
 def pack_int4(codes: Tensor, zero_i8: Optional[Tensor] = None, group: int = 0) -> Tensor:
     """(R, C) uint8 codes -> (R, ceil(C/8)) int32 words in the compressed-tensors layout."""
     require_cuda(codes, "codes")

@@ -678,3 +678,20 @@ def test_quadratic_forms_against_fp64(cuda, R, C, kind):
         a, h = a.double(), H.double()
         want, size = float(((a @ h) * a).sum()), float(((a.abs() @ h.abs()) * a.abs()).sum())
         assert abs(float(g) - want) <= 2.0 ** -20 * size
+
+
+# ------------------------------------------------------------------ column permutation
+@pytest.mark.parametrize("R,C", [(1, 1), (3, 7), (130, 1032), (1300, 64), (2, 24577)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.uint8])
+def test_permute_columns(cuda, R, C, dtype):
+    """Rows that fit the staging and rows that do not, ragged widths, row strides, a row index, groups."""
+    gen = torch.Generator().manual_seed(R + C)
+    src = torch.randint(0, 255, (R, C + 3), generator=gen).to(dtype)[:, :C]
+    cols, rows = torch.randperm(C, generator=gen), torch.randint(0, R, (R + 2,), generator=gen)
+    dev = torch.empty(R, C + 3, dtype=dtype, device=cuda)[:, :C]
+    dev.copy_(src)
+    c32, r32 = cols.int().to(cuda), rows.int().to(cuda)
+    assert torch.equal(ops.permute_columns(dev, c32).cpu(), src[:, cols])
+    assert torch.equal(ops.permute_columns(dev, c32, rows=r32).cpu(), src[rows][:, cols])
+    few = src[:, : (C + 7) // 8].contiguous()
+    assert torch.equal(ops.permute_columns(few.to(cuda), c32, group=8).cpu(), few.repeat_interleave(8, -1)[:, cols])
