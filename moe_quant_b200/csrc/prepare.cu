@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256) absmax_scales_kernel(const float* __restr
 //    alone reach the best loss so far cannot win.  The terms of the segment's largest and smallest
 //    element, which the shrunk grids clip, are computed for 32 candidates at a time (one candidate
 //    per lane); two thirds of the 100 candidates of a 128-wide group fall to them.  Wide groups
-//    also compare the partial sum every eight elements per lane.
+//    (mse_scales_wide_kernel) compare the partial sum every eight elements per lane instead.
 //  * the elements of a 32-, 64- or 128-wide group stay in registers over all candidates.
 //  * x / s goes through the reciprocal of s, which the whole warp shares, and one residual correction
 //    (Markstein 1990); scales so small or large that the residual could underflow keep the division.
@@ -235,7 +235,7 @@ __device__ __forceinline__ float mse_term(float x, float s, float rs, bool plain
   return __expf(__logf(fabsf(y - x)) * norm);
 }
 
-// EPL: elements per lane of a group of 32 * EPL columns, held in registers; 0: any group size.
+// EPL: elements per lane of a group of 32 * EPL columns, held in registers; 0: any group below 256 columns.
 template <int DT, int EPL>
 __global__ void __launch_bounds__(256) mse_scales_kernel(const float* __restrict__ W, int64_t R, int64_t C, int64_t ldw,
                                                          int64_t group, float maxq, float zero,
@@ -294,23 +294,12 @@ __global__ void __launch_bounds__(256) mse_scales_kernel(const float* __restrict
         const float s = __shfl_sync(0xffffffffu, s_lane, j), rs = __shfl_sync(0xffffffffu, rs_lane, j);
         const bool plain = s > 1e-18f && s < 1e18f;
         float loss = 0.0f;
-        bool beaten = false;
         if constexpr (EPL > 0) {
 #pragma unroll
           for (int e = 0; e < EPL; ++e) loss += mse_term<DT>(xr[e], s, rs, plain, zero, maxq, norm);
         } else {
-          int n = 0;
-          for (int64_t k0 = 0; k0 < group; k0 += 32) {
-            if (k0 + lane < group) loss += mse_term<DT>(__ldg(x + k0 + lane), s, rs, plain, zero, maxq, norm);
-            if (best_i >= 0 && (++n & 7) == 0 && k0 + 32 < group) {
-              float part = loss;
-              for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-              beaten = part >= best;   // the same tree as below, over smaller numbers: never above the final sum
-              if (beaten) break;
-            }
-          }
+          for (int64_t k = lane; k < group; k += 32) loss += mse_term<DT>(__ldg(x + k), s, rs, plain, zero, maxq, norm);
         }
-        if (beaten) continue;
         for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
         if (best_i < 0 || loss < best) {
           best = loss;
@@ -323,13 +312,78 @@ __global__ void __launch_bounds__(256) mse_scales_kernel(const float* __restrict
   }
 }
 
+// Groups of 256 columns and more: a CTA per (row, group), its warps share out the candidates.  A layer with one group
+// per row has few segments, and a warp per segment left the chip idle over a serial stream (796 x 4040, one group per
+// row: the whole call 4870 us, 3120 us here).  19860 x 632 is level: 2470 us by warps, 2560 us by CTAs.  Every warp takes candidate 0 first, so that all start from the same best; a
+// candidate's loss is summed by one warp in the order of the kernel above.  Of equal losses the first candidate wins.
+template <int DT>
+__global__ void __launch_bounds__(256) mse_scales_wide_kernel(const float* __restrict__ W, int64_t R, int64_t C, int64_t ldw, int64_t group,
+                                                              float maxq, float zero, const float* __restrict__ p, int p_size, float norm,
+                                                              float* __restrict__ scale) {
+  __shared__ int shared_best;          // bits of the smallest loss so far: non-negative floats order like them
+  __shared__ float w_best[8];
+  __shared__ int w_index[8];
+  const int64_t G = C / group, n_seg = R * G;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t seg = blockIdx.x; seg < n_seg; seg += gridDim.x) {
+    const int64_t r = seg / G, gi = seg - r * G;
+    const float* x = W + r * ldw + gi * group;
+    const float s0 = scale[seg];
+    if (threadIdx.x == 0) shared_best = 0x7f800000;
+    __syncthreads();
+    float best = 0.0f;
+    int best_i = 0;
+    // i = 0 for every warp, then warp + 1, warp + 9, ...
+    for (int i = 0; i < p_size; i = i == 0 ? warp + 1 : i + 8) {
+      const float s = round_through<DT>(__fmul_rn(s0, __ldg(p + i)));
+      const float rs = 1.0f / s;
+      const bool plain = s > 1e-18f && s < 1e18f;
+      float loss = 0.0f;
+      bool beaten = false;
+      for (int64_t k0 = 0; k0 < group; k0 += 256) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int64_t k = k0 + u * 32 + lane;
+          if (k < group) loss += mse_term<DT>(__ldg(x + k), s, rs, plain, zero, maxq, norm);
+        }
+        if (i > 0 && k0 + 256 < group) {
+          float part = loss;
+          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+          // another warp's best may belong to a later candidate: only a larger loss is out for certain
+          beaten = part >= best || part > __int_as_float(*reinterpret_cast<volatile int*>(&shared_best));
+          beaten = __any_sync(0xffffffffu, beaten);
+          if (beaten) break;
+        }
+      }
+      if (beaten) continue;
+      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+      if (i == 0 || loss < best) {
+        best = loss;
+        best_i = i;
+        if (lane == 0 && loss >= 0.0f) atomicMin(&shared_best, __float_as_int(loss));
+      }
+    }
+    if (lane == 0) { w_best[warp] = best; w_index[warp] = best_i; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 0; w < 8; ++w)
+        if (w_best[w] < best || (w_best[w] == best && w_index[w] < best_i)) { best = w_best[w]; best_i = w_index[w]; }
+      scale[seg] = round_through<DT>(__fmul_rn(s0, __ldg(p + best_i)));
+    }
+    __syncthreads();
+  }
+}
+
 template <int DT>
 void launch_mse_scales(int grid, cudaStream_t st, const float* W, int64_t R, int64_t C, int64_t ldw, int64_t group, float maxq, float zero,
                        const float* p, int p_size, float norm, float* scale) {
   if (group == 128) mse_scales_kernel<DT, 4><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
   else if (group == 64) mse_scales_kernel<DT, 2><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
   else if (group == 32) mse_scales_kernel<DT, 1><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
-  else mse_scales_kernel<DT, 0><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
+  else if (group >= 256) {
+    const int64_t n_seg = R * (C / group);
+    mse_scales_wide_kernel<DT><<<(unsigned)(n_seg < 148 * 8 ? n_seg : 148 * 8), 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
+  } else mse_scales_kernel<DT, 0><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
 }
 
 // ---------------------------------------------------------------- the weights' way in
