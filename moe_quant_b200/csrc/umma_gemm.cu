@@ -1189,6 +1189,11 @@ __device__ __forceinline__ uint32_t leader_addr(uint32_t local) {   // the same 
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local));
   return r;
 }
+__device__ __forceinline__ void set_in_cta(int* local, int rank, int v) {   // *local of the cluster's CTA `rank`
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(r), "r"(v) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -1213,7 +1218,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
-// A wait that only the clock ends (a fault elsewhere does not): for copies that are under way.
+// A wait that only the clock ends (a fault elsewhere does not): for what is still under way after a wait was given up.
 __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
   uint64_t t0, now;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
@@ -1258,6 +1263,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   __shared__ __align__(8) uint64_t bars[2 * PAIR_STAGES + 4];
   __shared__ uint32_t tmem_slot;
+  // for the end of the kernel: a wait of either CTA was given up, slabs multiplied (both set in both CTAs), slabs
+  // whose copies either producer has issued (the leader's)
+  __shared__ int given_up, n_multiplied, n_copied[2];
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[PAIR_STAGES]);
   // two accumulators of 256 columns, by slab & 1
   const uint32_t acc_full = smem_u32(&bars[2 * PAIR_STAGES]), acc_empty = smem_u32(&bars[2 * PAIR_STAGES + 2]);
@@ -1271,8 +1279,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
       mbar_init(acc_full + 8 * b, 1);
       mbar_init(acc_empty + 8 * b, 16);  // the leader's: eight epilogue warps of either CTA
     }
+    given_up = n_multiplied = n_copied[0] = n_copied[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  auto give_up = [&]() {
+    set_in_cta(&given_up, 0, 1);
+    set_in_cta(&given_up, 1, 1);
+  };
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -1312,10 +1325,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           __syncwarp();
         }
       }
-      if (!ok && rank == 0) {
-        // given up: the copies in flight land before this CTA's (and, behind the cluster barrier, the other's)
-        // shared memory goes away
-        for (int j = it > PAIR_STAGES ? it - PAIR_STAGES : 0; j < it; ++j) mbar_drain(full0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1);
+      // the last use of every stage: its MMAs have read it (so its copies had landed) and their commit has
+      // arrived in this CTA
+      for (int j = it > PAIR_STAGES ? it - PAIR_STAGES : 0; j < it && ok; ++j)
+        ok = mbar_wait(empty0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1, 55);
+      if (lane == 0) {
+        set_in_cta(&n_copied[rank], 0, it);
+        if (!ok) give_up();
       }
     } else if (warp == 1) {
       if (rank == 0) {
@@ -1352,6 +1368,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             }
             __syncwarp();
           }
+        }
+        if (lane == 0) {
+          set_in_cta(&n_multiplied, 0, it);
+          set_in_cta(&n_multiplied, 1, it);
+          if (!ok) give_up();
         }
       }
     }
@@ -1466,12 +1487,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
         if (p.dot.x1) atomicAdd(p.dot.out + 1, total1);
       }
     }
-    if (lane == 0) bulk_wait_read_all();  // the boxes have left shared memory; the writes land before the grid completes
+    if (lane == 0) {
+      bulk_wait_read_all();  // the boxes have left shared memory; the writes land before the grid completes
+      if (!ok) give_up();
+    }
     __syncwarp();
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync();   // no MMA, copy or arrival of the other CTA is under way any more
+  cluster_sync();   // neither CTA issues a copy, an MMA or an arrival any more
+  // With every wait satisfied nothing is under way either: the producers have seen the last commits on `empty`, the
+  // epilogue warps all of those on `acc_full`, and the barrier orders the arrivals on the leader's `acc_empty`.
+  // After a wait that was given up what is under way comes to its end first: the MMAs through their commits, of which the
+  // last use of every barrier is known, the copies through the leader's `full` (a stage that one producer alone
+  // has filled never completes; the copy lands long before that wait runs out).
+  if (given_up) {   // the same in both CTAs
+    if (warp == 0) {
+      const int n = n_multiplied;
+      for (int j = n > PAIR_STAGES ? n - PAIR_STAGES : 0; j < n; ++j) mbar_drain(empty0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1);
+      for (int j = n > 2 ? n - 2 : 0; j < n; ++j) mbar_drain(acc_full + 8 * (j & 1), (j >> 1) & 1);
+      if (rank == 0) {
+        const int c = n_copied[0] > n_copied[1] ? n_copied[0] : n_copied[1];
+        for (int j = c > PAIR_STAGES ? c - PAIR_STAGES : 0; j < c; ++j) mbar_drain(full0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1);
+      }
+    }
+    __syncthreads();
+    cluster_sync();   // the other CTA's copies signal the leader's barriers
+  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_acc) : "memory");

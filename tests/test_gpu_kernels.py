@@ -681,6 +681,26 @@ def test_quadratic_forms_against_fp64(cuda, R, C, kind):
         assert abs(float(g) - want) <= 2.0 ** -20 * size
 
 
+@pytest.mark.parametrize("R,widths", [(1, (1, 64, 65, 150, 200, 257, 330, 400, 450)), (300, (40, 128, 250, 320, 513)), (300, (5000,))])
+def test_quadratic_forms_back_to_back(cuda, R, widths):
+    """One to eight slabs of k, one tile per CTA pair and several: whatever use of the ring is the last one, the pair leaves
+    with its commits and copies received, and the launch that follows on the same SMs finds its barriers its own (no wait
+    expires, which is checked after every test, and every result of the series is right)."""
+    gen = torch.Generator().manual_seed(R + len(widths))
+    cases = []
+    for C in widths:
+        X = torch.randn(C + 3, C, generator=gen)
+        cases.append((torch.randn(R, C, generator=gen), torch.randn(R, C, generator=gen), X.T @ X / C))
+    dev = [tuple(t.to(cuda) for t in c) for c in cases]
+    got = [[ops.error_forms(*c) for c in dev] for _ in range(6)]
+    for i, (q, w, H) in enumerate(cases):
+        for a, k in ((q - w, 0), (w, 1)):
+            a, h = a.double(), H.double()
+            want, size = float(((a @ h) * a).sum()), float(((a.abs() @ h.abs()) * a.abs()).sum())
+            for series in got:      # bound: as in test_quadratic_forms_against_fp64
+                assert abs(float(series[i][k]) - want) <= 2.0 ** -20 * size
+
+
 # ------------------------------------------------------------------ column permutation
 @pytest.mark.parametrize("R,C", [(1, 1), (3, 7), (130, 1032), (1300, 64), (2, 24577)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.uint8])

@@ -1,0 +1,153 @@
+"""The barriers of the CTA-pair kernel (csrc/umma_gemm.cu, umma_pair_kernel) as a model on the CPU: two producers, one MMA
+issuer, one epilogue per CTA and an engine that lands copies, runs MMAs and delivers commits on its own, under random
+schedules.  When the CTAs leave, no copy, MMA, commit or arrival may be under way, whether every wait was satisfied or
+one was given up: it would write into shared memory that belongs to the next CTA.
+"""
+import random
+
+import pytest
+
+STAGES = 3
+
+
+class Barrier:
+    def __init__(self, need):
+        self.need, self.pending, self.bytes, self.phase = need, need, 0, 0
+
+    def _turn(self):
+        if self.pending == 0 and self.bytes == 0:
+            self.phase, self.pending = self.phase + 1, self.need
+
+    def arrive(self, expect=0):
+        assert self.pending > 0
+        self.pending, self.bytes = self.pending - 1, self.bytes + expect
+        self._turn()
+
+    def land(self):
+        self.bytes -= 1
+        self._turn()
+
+    def done(self, parity):
+        return (self.phase & 1) != parity
+
+
+def last_uses(count, slots):
+    return range(max(0, count - slots), count)
+
+
+def under_way_at_exit(slabs, seed, tail, fault_at=None):
+    rnd = random.Random(seed)
+    full = [Barrier(1) for _ in range(STAGES)]
+    empty = [[Barrier(1) for _ in range(STAGES)] for _ in range(2)]
+    acc_full = [[Barrier(1) for _ in range(2)] for _ in range(2)]
+    acc_empty = [Barrier(2) for _ in range(2)]
+    engine, remote, mmas = [], [], []
+    end = {"given_up": False, "multiplied": 0, "copied": [0, 0]}
+    fault = [False]
+
+    def wait(bar, parity):
+        while not bar.done(parity):
+            if fault[0]:
+                return False
+            yield
+        return True
+
+    def drain(bar, parity):
+        for _ in range(4000):
+            if bar.done(parity):
+                return
+            yield
+
+    def producer(rank):
+        ok, it = True, 0
+        while it < slabs:
+            s = it % STAGES
+            if it >= STAGES:
+                ok = yield from wait(empty[rank][s], (it // STAGES - 1) & 1)
+                if not ok:
+                    break
+            if rank == 0:
+                full[s].arrive(expect=2)
+            engine.append(full[s].land)
+            it += 1
+            yield
+        if tail:
+            for j in last_uses(it, STAGES):
+                ok = ok and (yield from wait(empty[rank][j % STAGES], (j // STAGES) & 1))
+        end["copied"][rank] = it
+        end["given_up"] |= not ok
+
+    def issuer():
+        ok, it = True, 0
+        while it < slabs:
+            ok = yield from wait(full[it % STAGES], (it // STAGES) & 1)
+            if ok and it >= 2:
+                ok = yield from wait(acc_empty[it & 1], ((it >> 1) - 1) & 1)
+            if not ok:
+                break
+            mmas.append(it)
+            it += 1
+            yield
+        end["multiplied"] = it
+        end["given_up"] |= not ok
+
+    def epilogue(rank):
+        ok = True
+        for it in range(slabs):
+            ok = yield from wait(acc_full[rank][it & 1], (it >> 1) & 1)
+            if not ok:
+                break
+            if rank == 0:
+                acc_empty[it & 1].arrive()
+            else:
+                remote.append(acc_empty[it & 1].arrive)
+            yield
+        end["given_up"] |= not ok
+
+    def last_words(rank):
+        n = end["multiplied"]
+        for j in last_uses(n, STAGES):
+            yield from drain(empty[rank][j % STAGES], (j // STAGES) & 1)
+        for j in last_uses(n, 2):
+            yield from drain(acc_full[rank][j & 1], (j >> 1) & 1)
+        if rank == 0:
+            for j in last_uses(max(end["copied"]), STAGES):
+                yield from drain(full[j % STAGES], (j // STAGES) & 1)
+
+    def play(actors, step=0):
+        while actors:
+            step += 1
+            assert step < 400000, "a wait never ends"
+            if step == fault_at:
+                fault[0] = True
+            k = rnd.random()
+            if engine and k < 0.25:
+                engine.pop(rnd.randrange(len(engine)))()
+            elif mmas and k < 0.45:
+                j = mmas.pop(0)
+                for rank in range(2):
+                    engine.extend([empty[rank][j % STAGES].arrive, acc_full[rank][j & 1].arrive])
+            elif remote and k < 0.6:
+                remote.pop(rnd.randrange(len(remote)))()
+            else:
+                a = rnd.choice(actors)
+                if next(a, "end") == "end":
+                    actors.remove(a)
+
+    play([producer(0), producer(1), issuer(), epilogue(0), epilogue(1)])
+    while remote:               # the cluster barrier orders what threads did before it, not what the engine does
+        remote.pop()()
+    if tail and end["given_up"]:
+        play([last_words(0), last_words(1)])
+    return len(engine) + len(mmas)
+
+
+@pytest.mark.parametrize("slabs", [1, 2, 3, 4, 5, 6, 7, 13])
+@pytest.mark.parametrize("gives_up", [False, True])
+def test_nothing_is_under_way_when_the_pair_leaves(slabs, gives_up):
+    def runs(tail):
+        for seed in range(150):
+            yield under_way_at_exit(slabs, seed, tail, random.Random(seed).randrange(1, 60 * slabs) if gives_up else None)
+
+    assert not any(runs(True))
+    assert any(runs(False))     # without the waits at the end some schedule does leave something
