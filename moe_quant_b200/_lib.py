@@ -146,6 +146,12 @@ def require_cuda(t: torch.Tensor, what: str) -> None:
         raise MoeQuantError(f"{what} must live on a CUDA device (got {t.device}); this engine has no CPU path")
 
 
+def require_one_device(what: str, *tensors: torch.Tensor) -> None:
+    """The kernel runs on the first tensor's device and stream: a pointer of another GPU is not its to read."""
+    if any(t.device != tensors[0].device for t in tensors[1:]):
+        raise MoeQuantError(f"{what}: expected all tensors on one device, got {', '.join(str(t.device) for t in tensors)}")
+
+
 def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 

@@ -12,7 +12,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from ._lib import MATH_COMPACT, MATH_FP32, MATH_TENSOR, MoeQuantError, check, dtype_code, lib, ptr, require_cuda, stream_ptr
+from ._lib import MATH_COMPACT, MATH_FP32, MATH_TENSOR, MoeQuantError, check, dtype_code, lib, ptr, require_cuda, require_one_device, stream_ptr
 
 
 @dataclass
@@ -292,6 +292,7 @@ def quadratic_form(A: Tensor, H: Tensor, precision: Optional[Precision] = None) 
     require_cuda(H, "H")
     if A.dtype != torch.float32 or H.dtype != torch.float32 or A.dim() != 2 or H.shape != (A.shape[1], A.shape[1]):
         raise MoeQuantError("quadratic_form: A must be (R, C) fp32 and H (C, C) fp32")
+    require_one_device("quadratic_form", A, H)
     A = A if A.stride(1) == 1 else A.contiguous()
     H = H if H.stride(1) == 1 else H.contiguous()
     R, C = A.shape
@@ -311,6 +312,7 @@ def error_forms(q: Tensor, w: Tensor, H: Tensor) -> Tensor:
         require_cuda(t, n)
     if any(t.dtype != torch.float32 or t.dim() != 2 for t in (q, w, H)) or q.shape != w.shape or H.shape != (q.shape[1], q.shape[1]):
         raise MoeQuantError("error_forms: q and w must be (R, C) fp32 and H (C, C) fp32")
+    require_one_device("error_forms", q, w, H)
     q, w, H = (t if t.stride(1) == 1 and t.stride(0) >= t.shape[1] else t.contiguous() for t in (q, w, H))
     R, C = q.shape
     out = torch.empty(2, dtype=torch.float64, device=q.device)

@@ -1,9 +1,11 @@
 """Bookkeeping of the GPTQ handle that needs no device (src/gptq.py:22-136)."""
+import math
+
 import pytest
 import torch
 import torch.nn as nn
 
-from moe_quant_b200 import GPTQ, QuantizationOrder, model_utils
+from moe_quant_b200 import GPTQ, QuantizationOrder, model_utils, ops, quant_utils
 from moe_quant_b200._lib import MoeQuantError
 
 
@@ -50,6 +52,46 @@ def test_update_on_cpu_raises():
     h = GPTQ(_layer(), 8, True)
     with pytest.raises(MoeQuantError):
         h.update(torch.zeros(4, 16, dtype=torch.bfloat16))
+
+
+class _On:
+    """What the checks in front of a launch look at, on a GPU that need not be there."""
+    is_cuda, dtype = True, torch.float32
+
+    def __init__(self, index, *shape, dtype=torch.float32):
+        self.device, self.shape, self.dtype = torch.device("cuda", index), shape, dtype
+
+    def dim(self):
+        return len(self.shape)
+
+    def numel(self):
+        return math.prod(self.shape)
+
+    def stride(self, d):
+        return math.prod(self.shape[d + 1:])
+
+    def float(self):
+        return self
+
+
+@pytest.fixture
+def no_launch(monkeypatch):
+    def reached(*a, **k):
+        raise AssertionError("went on to the library")
+    for name in ("lib", "check"):
+        monkeypatch.setattr(ops, name, reached)
+    monkeypatch.setattr(torch, "empty", reached)
+
+
+@pytest.mark.parametrize("devices", [(0, 1, 0), (1, 0, 0), (0, 0, 1)])
+def test_error_metric_refuses_tensors_of_several_gpus(no_launch, devices):
+    q, w, H = _On(devices[0], 4, 8), _On(devices[1], 4, 8), _On(devices[2], 8, 8)
+    for call in (lambda: quant_utils.get_relative_mse_error(q, w, H), lambda: ops.error_forms(q, w, H)):
+        with pytest.raises(MoeQuantError, match="one device"):
+            call()
+    if devices[0] != devices[2]:
+        with pytest.raises(MoeQuantError, match="one device"):
+            ops.quadratic_form(q, H)
 
 
 def test_asymmetric_is_refused():
