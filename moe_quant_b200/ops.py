@@ -332,6 +332,7 @@ def permute_columns(src: Tensor, cols: Tensor, rows: Optional[Tensor] = None, gr
     if src.dim() != 2 or src.dtype not in (torch.float32, torch.uint8) or cols.dtype != torch.int32 or cols.dim() != 1 or (
             rows is not None and (rows.dtype != torch.int32 or rows.dim() != 1)):
         raise MoeQuantError("permute_columns: src must be a 2-D fp32 or uint8 tensor, indices int32 vectors")
+    require_one_device("permute_columns", *(t for t in (src, cols, rows) if t is not None))
     src = src if src.stride(1) == 1 and src.stride(0) >= src.shape[1] else src.contiguous()
     cols, rows = cols.contiguous(), None if rows is None else rows.contiguous()
     R = src.shape[0] if rows is None else rows.numel()

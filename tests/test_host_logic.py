@@ -73,6 +73,8 @@ class _On:
     def float(self):
         return self
 
+    contiguous = float
+
 
 @pytest.fixture
 def no_launch(monkeypatch):
@@ -92,6 +94,14 @@ def test_error_metric_refuses_tensors_of_several_gpus(no_launch, devices):
     if devices[0] != devices[2]:
         with pytest.raises(MoeQuantError, match="one device"):
             ops.quadratic_form(q, H)
+
+
+@pytest.mark.parametrize("devices", [(0, 1, 0), (1, 0, 0), (0, 0, 1), (0, 1, None)])
+def test_permutation_refuses_indices_of_another_gpu(no_launch, devices):
+    src, cols, rows = (None if d is None else _On(d, *shape, dtype=dtype) for d, shape, dtype in
+                       zip(devices, [(4, 8), (8,), (4,)], [torch.float32, torch.int32, torch.int32]))
+    with pytest.raises(MoeQuantError, match="one device"):
+        ops.permute_columns(src, cols, rows=rows)
 
 
 def test_asymmetric_is_refused():
