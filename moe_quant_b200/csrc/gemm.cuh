@@ -38,8 +38,11 @@ struct GemmDesc {
   int compact = 0;
   // Tensor path: optional per-row and per-column factors of the product (powers of two, device arrays
   // indexed like C): C[m,n] = alpha * row_f[m] * col_f[n] * sum_k A B + beta * C[m,n].
+  // Pairs of fp16 planes with K > 128: row_f holds one set per 128 of k, row_f_step floats apart; each is applied to
+  // its part of the sum.
   const float* row_f = nullptr;
   const float* col_f = nullptr;
+  int64_t row_f_step = 0;
 };
 
 // fp32 CUDA-core implementation; in_dtype is the element type of A and B.

@@ -317,8 +317,17 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
         continue;
       }
       uint32_t p0[4], p1[4], p2[4];
-      if (a.err_scale) {
-        const float rho = __ldg(a.err_scale + gr);
+      if (a.row_f) {
+        // The largest error of the row's 128 comes just under 2^14, so that a pair holds 22 bits of every error down to 2^-17 of
+        // it; the sixteen lanes of a row agree on it.  (One power of two per row of the matrix cost a row whose groups differ
+        // by 2^20 the last bits of its small groups: 13 to 16 times the error of three bf16 planes there.)
+        float m = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) m = fmaxf(m, fabsf(e[t]));
+        const unsigned half_warp = 0xffffu << (lane & 16);
+        for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(half_warp, m, o));
+        const float rho = scale_below_2_14(m);
+        if ((lane & 15) == 0) a.row_f[gr] = 1.0f / rho;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           uint16_t h0, l0, h1, l1;
@@ -382,43 +391,10 @@ int configure_once() {
 
 }  // namespace
 
-// Bounds the errors of a row in the inverse-free form: e = w_original - y, |y| <= max over the row's groups of
-// |q - z| s with q on the grid.  row_f[r] = 1 / rho, row_f[R + r] = rho, the power of two that brings the
-// bound just under 2^14.  W null: the grid is the absmax grid of the weights, whose largest weight is that
-// of the grid up to the rounding of the scale.  One warp per row.
-__global__ void __launch_bounds__(256) error_scale_kernel(const float* __restrict__ W, int64_t ldw, int64_t R, int64_t C,
-                                                          const float* __restrict__ scale, const float* __restrict__ zero, int64_t G,
-                                                          int64_t s_rs, int64_t s_gs, float maxq, float zero_default,
-                                                          float* __restrict__ row_f) {
-  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (r >= R) return;
-  float y = 0.0f, w = 0.0f;
-  for (int64_t g = lane; g < G; g += 32) {
-    const int64_t off = r * s_rs + g * s_gs;
-    const float s = fabsf(__ldg(scale + off)), z = zero ? __ldg(zero + off) : zero_default;
-    y = fmaxf(y, s * fmaxf(fabsf(z), fabsf(maxq - z)));
-  }
-  for (int64_t c = lane * 4; W != nullptr && c < C; c += 128) {   // C % 4 == 0, rows 16-byte aligned
-    const float4 v = __ldg(reinterpret_cast<const float4*>(W + r * ldw + c));
-    w = fmaxf(w, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    y = fmaxf(y, __shfl_xor_sync(0xffffffffu, y, o));
-    w = fmaxf(w, __shfl_xor_sync(0xffffffffu, w, o));
-  }
-  if (lane == 0) {
-    // (a scale of 0 is an underflow of the layer's type: weights below 2^-20)
-    const float rho = scale_below_2_14(W ? y + w : (y > 0.0f ? 2.0f * y : 0x1p-20f));
-    row_f[r] = 1.0f / rho;
-    row_f[R + r] = rho;
-  }
-}
-
 size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split) {
   math &= ~MQ_MATH_COMPACT;
   if (math == MQ_MATH_TENSOR)
-    return plane_set_bytes(R, SUPER, split) + plane_set_bytes(C, C, split) + align_up((size_t)R * 2 * sizeof(float), 256) +
+    return plane_set_bytes(R, SUPER, split) + plane_set_bytes(C, C, split) + align_up((size_t)R * (SUPER / TILE) * sizeof(float), 256) +
            align_up((size_t)C * 2 * sizeof(float), 256);
   return align_up((size_t)R * TILE * sizeof(float), 256);
 }
@@ -426,7 +402,7 @@ size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split) {
 int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, int64_t ldu, const float* scale,
                const float* zero, int64_t group, int64_t s_rs, int64_t s_gs, int bits, int out_dtype, uint8_t* codes,
                void* deq, const float* Worig, int64_t ldwo, int math, int split, Workspace& ws, cudaStream_t st,
-               const float* col_div, const float* eq, bool absmax_grid, int32_t* packed) {
+               const float* col_div, const float* eq, int32_t* packed) {
   // col_div (tensor math only): above its diagonal 128-blocks Uhat holds the factor before its
   // columns were divided by col_div; the plane split divides where it reads it.  The diagonal
   // blocks, which the tiles read, are already scaled.  eq (with col_div): what lies above is the factor
@@ -443,11 +419,9 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   // and the sweep kernel writes its errors as planes itself.  No per-tile conversion passes.
   //
   // Inverse-free form at full precision (split 3): the operands are pairs of fp16 planes, three
-  // products instead of six (split_half2).  The errors are bounded there (|w_original - y|, y on the
-  // grid), so a power of two per row brings them into fp16's range, and one per column does so for
-  // the factor; the GEMM's epilogue takes both back exactly.  (absmax_grid: the scales are the absmax grid
-  // of Worig, so that the bound needs no pass over the weights.)  The other form propagates y - x with an
-  // unbounded running value x and keeps three bf16 planes.
+  // products instead of six (split_half2).  A power of two per row and tile brings the errors into fp16's
+  // range, and one per column does so for the factor; the GEMM's epilogue takes both back exactly.  The
+  // other form, which propagates y - x against the inverse, keeps three bf16 planes.
   const bool half = tensor && split == 3 && Worig != nullptr;
   MQ_REQUIRE(!eq || half || !tensor, MQ_ERR_ARGUMENT, "mq_gptq_sweep: an equilibrated factor needs the inverse-free form");
   PlaneSet err_set, u_set;
@@ -455,15 +429,12 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   if (half) {
     uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, SUPER, 2) / 2);
     uint16_t* up = ws.take<uint16_t>(plane_set_bytes(C, C, 2) / 2);
-    row_f = ws.take<float>((size_t)R * 2);
+    row_f = ws.take<float>((size_t)R * (SUPER / TILE));
     col_f = ws.take<float>((size_t)C * 2);
     MQ_REQUIRE(ep && up && row_f && col_f, MQ_ERR_WORKSPACE, "mq_gptq_sweep: workspace too small for the operand planes");
     err_set.base = ep; err_set.planes = 2; err_set.rows_pad = (int)pad_rows(R); err_set.total_rows = err_set.rows_pad;
     err_set.K_pad = SUPER; err_set.fp16 = true;
     MQ_TRY(make_factor_planes_half(Uhat, ldu, (int)C, up, col_f, col_div, eq, &u_set, st));
-    error_scale_kernel<<<(unsigned)ceil_div(R, 8), 256, 0, st>>>(absmax_grid ? nullptr : Worig, ldwo, R, C, scale, zero, C / group, s_rs, s_gs,
-                                                                 (float)((1 << bits) - 1), 0.5f * (float)(1 << bits), row_f);
-    MQ_LAUNCH_CHECK();
   } else if (tensor) {
     MQ_REQUIRE(split >= 1 && split <= 3, MQ_ERR_ARGUMENT, "mq_gptq_sweep: split must be 1, 2 or 3 (got %d)", split);
     uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, SUPER, split) / 2);
@@ -487,7 +458,6 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   sa.err_planes = nullptr;
   sa.plane_stride = tensor ? err_set.total_rows * (int64_t)SUPER : 0;
   sa.n_planes = half ? 2 : split;
-  sa.err_scale = half ? row_f + R : nullptr;
   sa.err_ld = tensor ? SUPER : TILE;
   sa.bits = bits;
   const bool uniform = group % SUB == 0;
@@ -509,6 +479,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       ProfScope prof(PROF_SWEEP_TILE, (double)R * nb * (4.0 + 1.0 + 4.0) + 2.0 * nb * nb, (double)R * nb * (nb - 1), st);
       sa.i1 = (int)i1; sa.nb = nb;
       if (tensor) sa.err_planes = err_set.base + (i1 % SUPER);
+      sa.row_f = half ? row_f + (i1 % SUPER) / TILE * R : nullptr;
       switch (out_dtype) {
         case MQ_F32: MQ_TRY(launch_sweep_tile<MQ_F32>(chained, uniform, grid, rows, st, sa)); break;
         case MQ_BF16: MQ_TRY(launch_sweep_tile<MQ_BF16>(chained, uniform, grid, rows, st, sa)); break;
@@ -537,7 +508,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       g.M = (int)R; g.N = (int)(s1 - i2); g.K = nb;
       g.alpha = 1.0f; g.beta = 1.0f;
       g.compact = compact ? 1 : 0;
-      g.row_f = row_f; g.col_f = col_f ? col_f + i2 : nullptr;
+      g.row_f = sa.row_f; g.col_f = col_f ? col_f + i2 : nullptr;
       PlaneSet a = err_set, b = u_set;
       a.k0 = (int)(i1 - s0);
       b.row0 = i2; b.k0 = (int)i1;
@@ -548,7 +519,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       g.C = W + s1; g.ldc = ldw;
       g.M = (int)R; g.N = (int)(C - s1); g.K = (int)(s1 - s0);
       g.alpha = 1.0f; g.beta = 1.0f;
-      g.row_f = row_f; g.col_f = col_f ? col_f + s1 : nullptr;
+      g.row_f = row_f; g.row_f_step = R; g.col_f = col_f ? col_f + s1 : nullptr;
       PlaneSet b = u_set;
       b.row0 = s1; b.k0 = (int)s0;
       MQ_TRY(gemm_tensor_planes(g, err_set, b, st));
@@ -590,5 +561,5 @@ extern "C" int mq_gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const 
   MQ_REQUIRE(!packed || (bits == 4 && !zero && aligned(packed, 4)), MQ_ERR_UNSUPPORTED,
              "mq_gptq_sweep: packed words need bits == 4, the symmetric zero point and a 4-byte aligned buffer");
   return gptq_sweep(W, R, C, ldw, Uhat, ldu, scale, zero, group, row_stride, group_stride, bits, out_dtype, codes,
-                    dequantized, W_original, ldwo, math, split, ws, static_cast<cudaStream_t>(stream), nullptr, nullptr, false, packed);
+                    dequantized, W_original, ldwo, math, split, ws, static_cast<cudaStream_t>(stream), nullptr, nullptr, packed);
 }

@@ -70,6 +70,7 @@ struct UmmaParams {
   int pairs;           // operands are pairs of fp16 planes: the leading product is summed per slab of k (see below)
   const float* row_f;  // optional factors of the product per row / column of C
   const float* col_f;
+  int64_t row_f_step;  // pair kernel: row_f of the k-th 128 of k lies at row_f + k * row_f_step
   DotForm dot;         // pair kernel, DOT form
   int drain_slabs;  // streaming kernel: slabs of k per accumulator before it is added to C (0 = all of K)
 };
@@ -178,8 +179,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 }
 
 // v[i] *= alpha * row_f[row] * col_f[col + i] (the factors are powers of two: exact); M, N bound the reads.
+// row_f is read at the L2: the kernel in front, which this one may overlap up to its chain_wait, has just written it.
 __device__ __forceinline__ void apply_factors(float (&v)[32], const UmmaParams& p, int row, int col) {
-  const float rf = p.alpha * ((p.row_f && row < p.M) ? __ldg(p.row_f + row) : 1.0f);
+  const float rf = p.alpha * ((p.row_f && row < p.M) ? __ldcg(p.row_f + row) : 1.0f);
   if (p.col_f) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = v[i] * rf * (col + i < p.N ? __ldg(p.col_f + col + i) : 1.0f);
@@ -189,15 +191,15 @@ __device__ __forceinline__ void apply_factors(float (&v)[32], const UmmaParams& 
   }
 }
 
-// One row (LEN columns) of an accumulator added to the sums in registers.
+// One row (LEN columns) of an accumulator times f (a power of two: exact) added to the sums in registers.
 template <int LEN>
-__device__ __forceinline__ void tmem_acc_row(uint32_t taddr, float (&sum)[LEN]) {
+__device__ __forceinline__ void tmem_acc_row(uint32_t taddr, float f, float (&sum)[LEN]) {
 #pragma unroll
   for (int c = 0; c < LEN / 32; ++c) {
     float v[32];
     tmem_ld32(taddr + (uint32_t)(c * 32), v);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) sum[c * 32 + j] += v[j];
+    for (int j = 0; j < 32; ++j) sum[c * 32 + j] = fmaf(f, v[j], sum[c * 32 + j]);
   }
 }
 
@@ -881,7 +883,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
               old[c * 8 + it] = *reinterpret_cast<const float4*>(cq + (int64_t)(4 * it) * p.ldc + c * 32);
         }
         // the row's factor is applied while a lane holds a row, the columns' after the turn
-        const float rf = p.alpha * (p.row_f ? __ldg(p.row_f + row) : 1.0f);
+        const float rf = p.alpha * (p.row_f ? __ldcg(p.row_f + row) : 1.0f);
         float4 cf[TILE_N / 32];
 #pragma unroll
         for (int c = 0; c < TILE_N / 32; ++c)
@@ -1394,13 +1396,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
       float acc[TILE_N];
 #pragma unroll
       for (int j = 0; j < TILE_N; ++j) acc[j] = 0.0f;
+      // the row's factor, one per 128 of k (the sweep's tiles scale their errors each by its own power of two)
+      const int my_m = (2 * w.m + rank) * TILE_M + q * 32 + lane;
+      const float* row_f = (!DOT && p.row_f && my_m < p.M) ? p.row_f + my_m : nullptr;
+      float rf = 1.0f;
 #pragma unroll 1
       for (int s = 0; s < n_slabs; ++s, ++it) {
         const int b = it & 1;
+        if (row_f && (s & 1) == 0) rf = __ldcg(row_f + (s >> 1) * p.row_f_step);
         ok = mbar_wait(acc_full + 8 * b, (it >> 1) & 1, 54);
         if (!ok) break;
         tc_fence_after();
-        tmem_acc_row(t_lane + (uint32_t)(b * PAIR_TILE + h * TILE_N), acc);
+        tmem_acc_row(t_lane + (uint32_t)(b * PAIR_TILE + h * TILE_N), rf, acc);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * b);
@@ -1450,7 +1457,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
       // inside a diagonal tile the 128-block below the diagonal is left alone
       const bool keep = y < p.M && n0 < p.N && !(p.upper_tiles_only && mb > nb);
       if (keep) {
-        const float rf = p.alpha * ((p.row_f && y + lane < p.M) ? __ldg(p.row_f + y + lane) : 1.0f);
 #pragma unroll
         for (int c = 0; c < TILE_N / 32; ++c) {
           const int x = n0 + c * 32;
@@ -1458,10 +1464,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           __syncwarp();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            float4 f = make_float4(rf, rf, rf, rf);
+            float4 f = make_float4(p.alpha, p.alpha, p.alpha, p.alpha);
             if (p.col_f && x + 4 * j < p.N) {      // N % 4 == 0, col_f 16-byte aligned
               const float4 g = __ldg(reinterpret_cast<const float4*>(p.col_f + x + 4 * j));
-              f = make_float4(rf * g.x, rf * g.y, rf * g.z, rf * g.w);
+              f = make_float4(p.alpha * g.x, p.alpha * g.y, p.alpha * g.z, p.alpha * g.w);
             }
             asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(my_row + (uint32_t)((j ^ (lane & 7)) << 4)),
                          "f"(f.x * acc[c * 32 + 4 * j]), "f"(f.y * acc[c * 32 + 4 * j + 1]), "f"(f.z * acc[c * 32 + 4 * j + 2]),
@@ -2019,7 +2025,7 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
   p.a_row0 = (int)A.row0; p.a_k0 = A.k0; p.b_row0 = (int)B.row0; p.b_k0 = B.k0;
   p.planes = A.planes;
   p.pairs = (A.planes == 2 && A.fp16) ? 1 : 0;
-  p.row_f = d.row_f; p.col_f = d.col_f;
+  p.row_f = d.row_f; p.col_f = d.col_f; p.row_f_step = d.row_f_step;
   p.drain_slabs = 0;
   p.nterms = 0;
   for (int i = 0; i < A.planes; ++i)

@@ -489,6 +489,59 @@ def test_sweep_of_operand_pairs_against_fp32_math(cuda, R, C, g, dtype, size):
     assert O.code_agreement(q, q0) >= CODE_AGREEMENT
 
 
+@pytest.mark.parametrize("C,g", [(136, 8), (648, 8), (1280, 32), (1664, 128)])
+@pytest.mark.parametrize("kind", ["plain", "small_first", "big_first", "by_group"])
+def test_sweep_running_values_against_fp64(cuda, C, g, kind):
+    """What every column has received from the tiles in front of it, against fp64 sums over the same errors, for rows whose
+    groups differ by up to 2^28.  Bound per element: products of pairs 2^-22 (lo lo left out) + 2 * 2^-23, the tensor
+    core's truncations four times 2^-23 of a part of the sum: 2^-20 of the sum of absolute products; and one fp32
+    rounding of the running value per update."""
+    R = 40
+    W = synthetic.layer_weight(R, C, 5, torch.float32)
+    gen = torch.Generator().manual_seed(C + g)
+    if kind == "small_first":
+        W[:, : C // 2] *= 2.0 ** -28
+    elif kind == "big_first":
+        W[:, C // 2 :] *= 2.0 ** -28
+    elif kind == "by_group":
+        W *= torch.exp2(-torch.randint(0, 21, (R, C // g), generator=gen).float()).repeat_interleave(g, -1)
+    X = synthetic.activations(2 * C, C, 6, torch.bfloat16).double()
+    H = X.T @ X / C
+    H.diagonal().add_(0.01 * H.diagonal().mean())
+    T = torch.linalg.cholesky(H.flip(0, 1)).flip(0, 1)
+    U = (T / T.diagonal()[None, :]).float().contiguous()
+    w, run = W.to(cuda), W.to(cuda)
+    scale = ops.absmax_scales(w, g, 4, torch.float32)
+    _, deq = ops.gptq_sweep(run, U.to(cuda), scale, None, g, C // g, 1, 4, torch.float32, True, ops.Precision(), W_original=w)
+    E, U64 = (W - deq.cpu()).double(), U.double()
+    for j in range(128, C, 128):
+        e, u = E[:, :j], U64[:j, j : j + 128]
+        size = e.abs() @ u.abs()
+        want = W[:, j : j + 128].double() + e @ u
+        got = run[:, j : j + 128].cpu().double()
+        bound = 2.0 ** -20 * size + (C // 128 + 3) * 2.0 ** -24 * (W[:, j : j + 128].abs().double() + size)
+        assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("rel_damp", [0.0, 1e-6, 1e-2])
+@pytest.mark.parametrize("spread", [1.0, 2.5])
+@pytest.mark.parametrize("C", [520, 1544])
+def test_layer_with_little_damping_against_fp32_math(cuda, rel_damp, spread, C):
+    """Channels over e^+-7 and a damping that does not lift the small ones: the factor's columns are scaled from one bound
+    over the whole matrix, and the codes are still those of the fp32 CUDA cores."""
+    gen = torch.Generator().manual_seed(C)
+    X = torch.randn(2 * C, C, generator=gen, dtype=torch.float64) * torch.exp(spread * torch.randn(C, generator=gen, dtype=torch.float64))
+    H = (X.T @ X / C).float()
+    W = synthetic.layer_weight(200, C, 5, torch.bfloat16)
+
+    def run(math):
+        codes, _, _, flags = ops.quantize_layer([W.to(cuda)], H.to(cuda), 8, 4, rel_damp, precision=ops.Precision(math=math))
+        assert int(flags[3]) == 0
+        return codes[0].cpu()
+
+    assert O.code_agreement(run(MATH_TENSOR), run(MATH_FP32)) >= CODE_AGREEMENT
+
+
 # ------------------------------------------------------------------ MSE scale search
 @pytest.mark.parametrize("R,C,g,dtype", [(64, 512, 128, torch.bfloat16), (40, 256, 32, torch.float16),
                                          (24, 384, 64, torch.float32), (8, 2048, 2048, torch.bfloat16)])
