@@ -50,8 +50,8 @@ typedef enum { MQ_F32 = 0, MQ_BF16 = 1, MQ_F16 = 2 } mq_dtype;
  *                   operands enter exactly; fp32 operands are split into up to
  *                   three bf16 planes whose cross products are accumulated
  *                   (`split` planes: 1 -> 1 product, 2 -> 3, 3 -> 6).  With split 3 the
- *                   factorisation and the inverse-free sweep use pairs of fp16
- *                   planes scaled by powers of two (3 products), at the same accuracy.  */
+ *                   factorisation and the inverse-free sweep of more than 512 columns use
+ *                   pairs of fp16 planes scaled by powers of two (3 products).  */
 typedef enum { MQ_MATH_FP32 = 0, MQ_MATH_TENSOR = 1 } mq_math;
 
 /* Flag that may be OR-ed into the `math` argument of mq_gptq_sweep and mq_quantize_layer (and of

@@ -162,8 +162,8 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   // At full tensor precision the factorisation works on a copy equilibrated by powers of two (fp16 operand
   // pairs).  The sweep takes an equilibrated factor only where it works on such pairs itself; otherwise the
   // factorisation gives its result back in H's units.
-  const bool pairs = math == MQ_MATH_TENSOR && split_hinv == 3 && split_sweep == 3;
-  const bool unscaled = math == MQ_MATH_TENSOR && (pairs || split_hinv != 3);
+  const bool pairs = uses_pairs(C, math, split_hinv) && uses_pairs(C, math, split_sweep);
+  const bool unscaled = math == MQ_MATH_TENSOR && (pairs || !uses_pairs(C, math, split_hinv));
   // W.clone().float(), pre-step, masking and damping, grid; driven by the first layer's weight: the handle that
   // owns H.  A tied handle meets an H that is already regularised and changes neither H nor its own
   // weight (src/gptq.py:129-136, 227).       src/gptq.py:140-152, 224-234, src/quant_utils.py:75-101

@@ -75,6 +75,16 @@ __device__ __forceinline__ float equilibrating_power(float h) {
   return __uint_as_float((uint32_t)(n + 127) << 23);
 }
 
+// Whether a factorisation or an inverse-free sweep at full precision (split 3) works on pairs of fp16 planes (three
+// products) instead of three bf16 planes (six).  Up to 512 columns there is no deep update, which is what pairs are for and
+// where sums of 64 of k win back the bits that the operands lose: error of a layer's running values against fp64, pairs in units of
+// three planes (mean of 12 seeds): 1.012 to 1.022 at 256 to 512 columns, 0.96 at 648, 0.90 from 2048 on.  Nor are they faster
+// there: 2048 x 256 takes 135.5 us with pairs and 131.9 with three planes, 32768 x 512 551 and 531.
+constexpr int64_t PAIRS_FROM_COLUMNS = 512;
+inline bool uses_pairs(int64_t C, int math, int split) {
+  return (math & ~MQ_MATH_COMPACT) == MQ_MATH_TENSOR && split == 3 && C > PAIRS_FROM_COLUMNS;
+}
+
 // Tensor-core GEMM whose operands are already planes (d.A / d.B and their strides are ignored;
 // d.K is the reduction length starting at k0 of each set).  Both sets must have the same
 // number of planes.

@@ -543,16 +543,16 @@ size_t hinv_workspace_bytes(int64_t C, int math, int split) {
 // unscaled: only the diagonal blocks are scaled; above them T itself is left in place and the caller
 // divides column c by diag[c] where it reads it).  diag (C floats, device) receives diag(T).  On a non-positive pivot
 // flags->not_positive is set and the result is replaced by I.
-// eq (tensor math with split 3 only): H has been equilibrated by the caller (copy_upper_scaled) with these
+// eq (uses_pairs only): H has been equilibrated by the caller (copy_upper_scaled) with these
 // factors; unscaled then leaves the equilibrated factor above the diagonal blocks and its diagonal in diag.
-// Null: with split 3 the matrix is equilibrated here and everything is given back in H's own units.
+// Null: where pairs are used the matrix is equilibrated here and everything is given back in H's own units.
 int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, int split, mq_layer_flags* flags,
                      Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled, const float* eq) {
   MQ_TRY(configure_once());
   const int compact = (math & MQ_MATH_COMPACT) ? 1 : 0;   // the panel solves and the rank-128 strips look at it
   math &= ~MQ_MATH_COMPACT;
-  const bool half = math == MQ_MATH_TENSOR && split == 3;   // pairs of fp16 planes, three products (split_half2)
-  MQ_REQUIRE(!eq || half, MQ_ERR_ARGUMENT, "factorisation: an equilibrated matrix needs tensor math with split 3");
+  const bool half = uses_pairs(C, math, split);   // pairs of fp16 planes, three products (split_half2)
+  MQ_REQUIRE(!eq || half, MQ_ERR_ARGUMENT, "factorisation: an equilibrated matrix needs pairs of planes");
   Workspace local(ws.base ? ws.base + ws.used : nullptr, ws.base ? ws.size - ws.used : 0);
   const bool own_units = half && !eq;
   if (own_units) {

@@ -418,11 +418,11 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   // update of tile i1 then reads the window k in [i1, i1+128), rows n >= i2 of those planes,
   // and the sweep kernel writes its errors as planes itself.  No per-tile conversion passes.
   //
-  // Inverse-free form at full precision (split 3): the operands are pairs of fp16 planes, three
+  // Inverse-free form at full precision (uses_pairs): the operands are pairs of fp16 planes, three
   // products instead of six (split_half2).  A power of two per row and tile brings the errors into fp16's
   // range, and one per column does so for the factor; the GEMM's epilogue takes both back exactly.  The
   // other form, which propagates y - x against the inverse, keeps three bf16 planes.
-  const bool half = tensor && split == 3 && Worig != nullptr;
+  const bool half = uses_pairs(C, math, split) && Worig != nullptr;
   MQ_REQUIRE(!eq || half || !tensor, MQ_ERR_ARGUMENT, "mq_gptq_sweep: an equilibrated factor needs the inverse-free form");
   PlaneSet err_set, u_set;
   float *row_f = nullptr, *col_f = nullptr;

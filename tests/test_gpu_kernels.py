@@ -523,6 +523,27 @@ def test_sweep_running_values_against_fp64(cuda, C, g, kind):
         assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
 
 
+@pytest.mark.parametrize("C", [136, 384, 512])
+def test_narrow_sweep_keeps_whole_operands(cuda, C):
+    """One product per column: up to 512 columns an error and an entry of the factor enter an update with all of their 24
+    bits, so a single product is off by its own rounding and what three planes leave out, below 2^-23 together."""
+    gen = torch.Generator().manual_seed(C)
+    R = 64
+    W = 0.02 * torch.randn(R, C, generator=gen)
+    W[:, 128:] = 0.0
+    U = torch.eye(C)
+    rows = torch.randint(0, 128, (C - 128,), generator=gen)
+    U[rows, torch.arange(128, C)] = 0.5 * torch.randn(C - 128, generator=gen)
+    w, run = W.to(cuda), W.to(cuda)
+    scale = ops.absmax_scales(w[:, :128].contiguous(), 8, 4, torch.bfloat16)
+    scale = torch.cat([scale, torch.ones(R, (C - 128) // 8, device=cuda)], 1).contiguous()
+    # inside the first tile the factor is the identity, so its errors are those of plain rounding (to bf16: exact in fp32)
+    _, deq = ops.gptq_sweep(run, U.to(cuda), scale, None, 8, C // 8, 1, 4, torch.bfloat16, True, ops.Precision(), W_original=w)
+    e = (W - deq.cpu().float())[:, rows].double()
+    want = e * U[rows, torch.arange(128, C)].double()
+    assert bool(((run.cpu()[:, 128:].double() - want).abs() <= 2.0 ** -23 * want.abs()).all())
+
+
 @pytest.mark.parametrize("rel_damp", [0.0, 1e-6, 1e-2])
 @pytest.mark.parametrize("spread", [1.0, 2.5])
 @pytest.mark.parametrize("C", [520, 1544])
