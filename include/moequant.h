@@ -51,7 +51,9 @@ typedef enum { MQ_F32 = 0, MQ_BF16 = 1, MQ_F16 = 2 } mq_dtype;
  *                   three bf16 planes whose cross products are accumulated
  *                   (`split` planes: 1 -> 1 product, 2 -> 3, 3 -> 6).  With split 3 the
  *                   factorisation and the inverse-free sweep of more than 512 columns use
- *                   pairs of fp16 planes scaled by powers of two (3 products).  */
+ *                   pairs of fp16 planes scaled by powers of two (3 products); split 4, which only
+ *                   these take, adds the product of the low pieces: for Hessians of fewer tokens than
+ *                   half the columns, where the factorisation's sums cancel.  mq_hinv_upper always adds it.  */
 typedef enum { MQ_MATH_FP32 = 0, MQ_MATH_TENSOR = 1 } mq_math;
 
 /* Flag that may be OR-ed into the `math` argument of mq_gptq_sweep and mq_quantize_layer (and of

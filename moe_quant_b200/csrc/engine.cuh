@@ -75,15 +75,20 @@ __device__ __forceinline__ float equilibrating_power(float h) {
   return __uint_as_float((uint32_t)(n + 127) << 23);
 }
 
-// Whether a factorisation or an inverse-free sweep at full precision (split 3) works on pairs of fp16 planes (three
-// products) instead of three bf16 planes (six).  Up to 512 columns there is no deep update, which is what pairs are for and
+// The `split` of a factorisation or a sweep: 1 and 2 keep that many bf16 planes; 3 and 4 are full precision, and work on pairs
+// of fp16 planes (3 with three products, 4 with all four) or on three bf16 planes (six products).
+// Pairs from 513 columns on: below there is no deep update, which is what pairs are for and
 // where sums of 64 of k win back the bits that the operands lose: error of a layer's running values against fp64, pairs in units of
 // three planes (mean of 12 seeds): 1.012 to 1.022 at 256 to 512 columns, 0.96 at 648, 0.90 from 2048 on.  Nor are they faster
 // there: 2048 x 256 takes 135.5 us with pairs and 131.9 with three planes, 32768 x 512 551 and 531.
+// The low pieces' product shows where the factorisation's sums cancel.  Tokens for 0.17 / 0.35 / 0.7 of the columns, the same error
+// with three products: 1.07 / 1.00 / 0.93 at 4096 columns, 1.08 / 1.05 / 0.97 at 1024; with all four 0.99 / 0.95 / 0.90 and
+// 1.01 / 0.99 / 0.95.  It costs 2048 x 7168 1.9 % (3889 -> 3962 us), 7168 x 16384 3.9 %.
 constexpr int64_t PAIRS_FROM_COLUMNS = 512;
 inline bool uses_pairs(int64_t C, int math, int split) {
-  return (math & ~MQ_MATH_COMPACT) == MQ_MATH_TENSOR && split == 3 && C > PAIRS_FROM_COLUMNS;
+  return (math & ~MQ_MATH_COMPACT) == MQ_MATH_TENSOR && (split == 3 || split == 4) && C > PAIRS_FROM_COLUMNS;
 }
+inline int plane_count(int split) { return split == 4 ? 3 : split; }
 
 // Tensor-core GEMM whose operands are already planes (d.A / d.B and their strides are ignored;
 // d.K is the reduction length starting at k0 of each set).  Both sets must have the same

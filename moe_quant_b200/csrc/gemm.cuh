@@ -43,6 +43,8 @@ struct GemmDesc {
   const float* row_f = nullptr;
   const float* col_f = nullptr;
   int64_t row_f_step = 0;
+  // Pairs of fp16 planes: the product of the two low pieces as well (four products instead of three).
+  int all_products = 0;
 };
 
 // fp32 CUDA-core implementation; in_dtype is the element type of A and B.

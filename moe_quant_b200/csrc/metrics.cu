@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256) dot_reduce_kernel(const float* __restrict
 extern "C" size_t mq_quadratic_form_workspace_bytes(int64_t R, int64_t C, int math, int split) {
   using namespace mq;
   if (R <= 0 || C <= 0) return 0;
+  split = plane_count(split);
   if (math == MQ_MATH_TENSOR && split == 3) return quadratic_forms_workspace_bytes(R, C, 1);
   return align_up((size_t)R * C * sizeof(float), 256) + engine_workspace_bytes(R, C, C, math, split);
 }
@@ -55,6 +56,7 @@ extern "C" int mq_quadratic_form(const float* A, int64_t R, int64_t C, int64_t l
   MQ_REQUIRE(math == MQ_MATH_FP32 || math == MQ_MATH_TENSOR, MQ_ERR_ARGUMENT, "mq_quadratic_form: bad math %d", math);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Workspace ws(workspace, workspace_bytes);
+  split = plane_count(split);
   if (math == MQ_MATH_TENSOR && split == 3) return quadratic_forms(A, lda, nullptr, 0, R, C, H, ldh, out, ws, st);
   float* T = ws.take<float>((size_t)R * C);
   MQ_REQUIRE(T, MQ_ERR_WORKSPACE, "mq_quadratic_form: workspace of %zu bytes is too small", workspace_bytes);

@@ -393,6 +393,7 @@ int configure_once() {
 
 size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split) {
   math &= ~MQ_MATH_COMPACT;
+  split = plane_count(split);
   if (math == MQ_MATH_TENSOR)
     return plane_set_bytes(R, SUPER, split) + plane_set_bytes(C, C, split) + align_up((size_t)R * (SUPER / TILE) * sizeof(float), 256) +
            align_up((size_t)C * 2 * sizeof(float), 256);
@@ -413,6 +414,9 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   const bool tensor = math == MQ_MATH_TENSOR;
   float* err = tensor ? nullptr : ws.take<float>((size_t)R * TILE);
   MQ_REQUIRE(tensor || err, MQ_ERR_WORKSPACE, "mq_gptq_sweep: workspace too small");
+  MQ_REQUIRE(!tensor || (split >= 1 && split <= 4), MQ_ERR_ARGUMENT, "mq_gptq_sweep: split must be 1, 2, 3 or 4 (got %d)", split);
+  const int all_products = split == 4 ? 1 : 0;   // of pairs
+  split = plane_count(split);
   Engine eng(math, split, ws, st);
   // Tensor path: the factor is cut into transposed planes once (row n, k -> U[k][n]); the lazy
   // update of tile i1 then reads the window k in [i1, i1+128), rows n >= i2 of those planes,
@@ -436,7 +440,6 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
     err_set.K_pad = SUPER; err_set.fp16 = true;
     MQ_TRY(make_factor_planes_half(Uhat, ldu, (int)C, up, col_f, col_div, eq, &u_set, st));
   } else if (tensor) {
-    MQ_REQUIRE(split >= 1 && split <= 3, MQ_ERR_ARGUMENT, "mq_gptq_sweep: split must be 1, 2 or 3 (got %d)", split);
     uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, SUPER, split) / 2);
     uint16_t* up = ws.take<uint16_t>(plane_set_bytes(C, C, split) / 2);
     MQ_REQUIRE(ep && up, MQ_ERR_WORKSPACE, "mq_gptq_sweep: workspace too small for the operand planes");
@@ -508,6 +511,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       g.M = (int)R; g.N = (int)(s1 - i2); g.K = nb;
       g.alpha = 1.0f; g.beta = 1.0f;
       g.compact = compact ? 1 : 0;
+      g.all_products = all_products;
       g.row_f = sa.row_f; g.col_f = col_f ? col_f + i2 : nullptr;
       PlaneSet a = err_set, b = u_set;
       a.k0 = (int)(i1 - s0);
@@ -519,6 +523,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       g.C = W + s1; g.ldc = ldw;
       g.M = (int)R; g.N = (int)(C - s1); g.K = (int)(s1 - s0);
       g.alpha = 1.0f; g.beta = 1.0f;
+      g.all_products = all_products;
       g.row_f = row_f; g.row_f_step = R; g.col_f = col_f ? col_f + s1 : nullptr;
       PlaneSet b = u_set;
       b.row0 = s1; b.k0 = (int)s0;

@@ -68,6 +68,7 @@ struct UmmaParams {
   int mirror;  // symmetric result: every block above the diagonal is also stored transposed
   int c_tma;   // panel kernel epilogue: 0 = loads/stores by the warps, 1 = TMA store (beta == 0), 2 = TMA add (beta == 1)
   int pairs;           // operands are pairs of fp16 planes: the leading product is summed per slab of k (see below)
+  int all_products;    // pairs: lo lo as well
   const float* row_f;  // optional factors of the product per row / column of C
   const float* col_f;
   int64_t row_f_step;  // pair kernel: row_f of the k-th 128 of k lies at row_f + k * row_f_step
@@ -276,15 +277,21 @@ __device__ __forceinline__ void issue_slab(uint32_t tmem_d, uint32_t small_off, 
   }
 }
 
-// One slab of fp16 pairs into a fresh accumulator: the corrections first (they lose nothing among themselves),
-// the leading products on top meet as many truncations as in an accumulator of their own.
-__device__ __forceinline__ void issue_slab_pairs(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile, uint32_t idesc) {
+// One slab of fp16 pairs into a fresh accumulator: lo lo first where it is asked for, then the corrections (they lose
+// nothing among themselves); the leading products on top meet as many truncations as in an accumulator of their own.
+__device__ __forceinline__ void issue_slab_pairs(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile, uint32_t idesc, uint32_t all_products) {
   const uint64_t a0 = kmajor_sw128_desc(a_tile), b0 = kmajor_sw128_desc(b_tile);
+  constexpr uint64_t LO = PLANE_TILE_BYTES >> 4;
+  if (all_products) {
+#pragma unroll
+    for (int kk = 0; kk < SLAB_K / 16; ++kk)
+      umma_bf16(tmem_d, a0 + LO + (uint64_t)((kk * 32) >> 4), b0 + LO + (uint64_t)((kk * 32) >> 4), idesc, kk > 0 ? 1u : 0u);
+  }
 #pragma unroll
   for (int kk = 0; kk < SLAB_K / 16; ++kk) {
     const uint64_t ah = a0 + (uint64_t)((kk * 32) >> 4), bh = b0 + (uint64_t)((kk * 32) >> 4);
-    umma_bf16(tmem_d, ah, bh + (uint64_t)(PLANE_TILE_BYTES >> 4), idesc, kk > 0 ? 1u : 0u);
-    umma_bf16(tmem_d, ah + (uint64_t)(PLANE_TILE_BYTES >> 4), bh, idesc, 1u);
+    umma_bf16(tmem_d, ah, bh + LO, idesc, kk > 0 ? 1u : all_products);
+    umma_bf16(tmem_d, ah + LO, bh, idesc, 1u);
   }
 #pragma unroll
   for (int kk = 0; kk < SLAB_K / 16; ++kk) umma_bf16(tmem_d, a0 + (uint64_t)((kk * 32) >> 4), b0 + (uint64_t)((kk * 32) >> 4), idesc, 1u);
@@ -796,7 +803,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_panel_kernel(const __gri
         if (lane == 0) {
           const uint32_t a_tile = smem_base + (uint32_t)(s * planes) * PLANE_TILE_BYTES;
           const uint32_t b_tile = b_base + (uint32_t)st * b_stage_bytes;
-          if (pairs) issue_slab_pairs(tmem_acc + (uint32_t)acc * acc_stride + (uint32_t)(s * TILE_N), a_tile, b_tile, idesc);
+          if (pairs) issue_slab_pairs(tmem_acc + (uint32_t)acc * acc_stride + (uint32_t)(s * TILE_N), a_tile, b_tile, idesc, (uint32_t)p.all_products);
           else issue_slab_any(planes, tmem_acc + (uint32_t)acc * acc_stride, small_off, a_tile, b_tile, idesc, accumulate, accumulate_small);
           umma_commit(b_empty + 8 * st);  // the stage is free once these MMAs have read it
         }
@@ -1354,13 +1361,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
               const uint32_t a_tile = smem_base + (uint32_t)st * PAIR_STAGE_BYTES;
               const uint64_t a0 = kmajor_sw128_desc(a_tile), b0 = kmajor_sw128_desc(a_tile + 2 * PLANE_TILE_BYTES);
               const uint32_t acc = tmem_acc + (uint32_t)(b * PAIR_TILE);
-              // the corrections first: they lose nothing among themselves, and the leading products on top
-              // meet as many truncations as in an accumulator of their own
+              // in the order of issue_slab_pairs
+              constexpr uint64_t LO = PLANE_TILE_BYTES >> 4;
+              const uint32_t all_products = (uint32_t)p.all_products;
+              if (all_products) {
+#pragma unroll
+                for (int kk = 0; kk < SLAB_K / 16; ++kk)
+                  umma_f16_pair(acc, a0 + LO + (uint64_t)((kk * 32) >> 4), b0 + LO + (uint64_t)((kk * 32) >> 4), p.idesc, kk > 0 ? 1u : 0u);
+              }
 #pragma unroll
               for (int kk = 0; kk < SLAB_K / 16; ++kk) {
                 const uint64_t ah = a0 + (uint64_t)((kk * 32) >> 4), bh = b0 + (uint64_t)((kk * 32) >> 4);
-                umma_f16_pair(acc, ah, bh + (uint64_t)(PLANE_TILE_BYTES >> 4), p.idesc, kk > 0 ? 1u : 0u);
-                umma_f16_pair(acc, ah + (uint64_t)(PLANE_TILE_BYTES >> 4), bh, p.idesc, 1u);
+                umma_f16_pair(acc, ah, bh + LO, p.idesc, kk > 0 ? 1u : all_products);
+                umma_f16_pair(acc, ah + LO, bh, p.idesc, 1u);
               }
 #pragma unroll
               for (int kk = 0; kk < SLAB_K / 16; ++kk)
@@ -2025,6 +2038,7 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
   p.a_row0 = (int)A.row0; p.a_k0 = A.k0; p.b_row0 = (int)B.row0; p.b_k0 = B.k0;
   p.planes = A.planes;
   p.pairs = (A.planes == 2 && A.fp16) ? 1 : 0;
+  p.all_products = (p.pairs && d.all_products) ? 1 : 0;
   p.row_f = d.row_f; p.col_f = d.col_f; p.row_f_step = d.row_f_step;
   p.drain_slabs = 0;
   p.nterms = 0;

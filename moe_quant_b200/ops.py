@@ -22,7 +22,9 @@ class Precision:
     math: MATH_TENSOR (tcgen05, fp32 accumulation in TMEM) or MATH_FP32 (CUDA cores).
     split_*: number of bf16 planes an fp32 operand is cut into on the tensor path
     (1, 2 or 3 planes -> 1, 3 or 6 products).  bf16/fp16 activations always enter the
-    Hessian exactly with one product.
+    Hessian exactly with one product.  The factorisation and the sweep of more than 512 columns take pairs
+    of fp16 planes for 3, with three products; 4 adds the product of the low pieces, which a Hessian
+    of few tokens needs (a handle asks for it by itself).
     compact: several layers are in flight on different streams (quantize_many sets it): the sweep
     uses launch shapes that occupy few SMs (MQ_MATH_COMPACT); the results do not change.
     """
@@ -89,7 +91,7 @@ def gemm(A: Tensor, B: Tensor, C: Tensor, alpha: float = 1.0, beta: float = 0.0,
     K2, N = B.shape
     if K2 != K or C.shape != (M, N) or C.stride(1) != 1:
         raise MoeQuantError("gemm: shape mismatch")
-    sp = p.split_hinv if split is None else split
+    sp = min(p.split_hinv, 3) if split is None else split
     L = lib()
     ws = _lib.workspace(C.device, L.mq_gemm_workspace_bytes(M, N, K, p.math, sp))
     with _lib.on_device(C.device):

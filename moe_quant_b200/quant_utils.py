@@ -70,7 +70,7 @@ def get_relative_mse_error(q: Tensor, w: Tensor, H: Optional[Tensor] = None) -> 
     n = float(w.numel())
     p = ops.DEFAULT_PRECISION
     if (H is not None and q.dtype == w.dtype == torch.float32 and q.dim() == 2 and q.shape == w.shape and w.numel() > 0
-            and p.math == ops.MATH_TENSOR and p.split_hinv == 3):
+            and p.math == ops.MATH_TENSOR and p.split_hinv >= 3):
         num, den = (ops.error_forms(q, w, H.float()) / n).unbind()
         return (num / (den + 1e-6)).float()
     delta = (q - w).float()

@@ -491,7 +491,8 @@ def test_sweep_of_operand_pairs_against_fp32_math(cuda, R, C, g, dtype, size):
 
 @pytest.mark.parametrize("C,g", [(136, 8), (648, 8), (1280, 32), (1664, 128)])
 @pytest.mark.parametrize("kind", ["plain", "small_first", "big_first", "by_group"])
-def test_sweep_running_values_against_fp64(cuda, C, g, kind):
+@pytest.mark.parametrize("split", [3, 4])
+def test_sweep_running_values_against_fp64(cuda, C, g, kind, split):
     """What every column has received from the tiles in front of it, against fp64 sums over the same errors, for rows whose
     groups differ by up to 2^28.  Bound per element: products of pairs 2^-22 (lo lo left out) + 2 * 2^-23, the tensor
     core's truncations four times 2^-23 of a part of the sum: 2^-20 of the sum of absolute products; and one fp32
@@ -512,7 +513,7 @@ def test_sweep_running_values_against_fp64(cuda, C, g, kind):
     U = (T / T.diagonal()[None, :]).float().contiguous()
     w, run = W.to(cuda), W.to(cuda)
     scale = ops.absmax_scales(w, g, 4, torch.float32)
-    _, deq = ops.gptq_sweep(run, U.to(cuda), scale, None, g, C // g, 1, 4, torch.float32, True, ops.Precision(), W_original=w)
+    _, deq = ops.gptq_sweep(run, U.to(cuda), scale, None, g, C // g, 1, 4, torch.float32, True, ops.Precision(split_sweep=split), W_original=w)
     E, U64 = (W - deq.cpu()).double(), U.double()
     for j in range(128, C, 128):
         e, u = E[:, :j], U64[:j, j : j + 128]
@@ -521,6 +522,36 @@ def test_sweep_running_values_against_fp64(cuda, C, g, kind):
         got = run[:, j : j + 128].cpu().double()
         bound = 2.0 ** -20 * size + (C // 128 + 3) * 2.0 ** -24 * (W[:, j : j + 128].abs().double() + size)
         assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("C,tokens", [(648, 110), (1024, 174), (1544, 260)])
+def test_all_products_where_the_sums_cancel(cuda, C, tokens):
+    """A Hessian of few tokens: the product of the low pieces takes error off the factor (its 2^-22 per product is most of
+    what a pair loses; the mean of eight seeds differs by several per cent), and the explicit inverse has it by itself.
+    Up to 512 columns there are no pairs and the two are the same bits."""
+    def errors(split, seed):
+        gen = torch.Generator().manual_seed(seed)
+        X = torch.randn(tokens, C, generator=gen, dtype=torch.float64) * torch.exp(torch.randn(C, generator=gen, dtype=torch.float64))
+        H = X.T @ X * (2.0 / tokens)
+        H.diagonal().add_(0.01 * H.diagonal().mean())
+        H = H.float()
+        T = torch.linalg.cholesky(H.double().flip(0, 1)).flip(0, 1)
+        U64 = T / T.diagonal()[None, :]
+        U = H.to(cuda)
+        flags, _ = ops.chol_unit_factor(U, ops.Precision(split_hinv=split))
+        assert int(flags[3]) == 0
+        return float((U.cpu().double() - U64).norm() / torch.triu(U64, 1).norm())
+
+    three, four = (sum(errors(split, seed) for seed in range(8)) for split in (3, 4))
+    assert four < 0.99 * three
+
+    X = torch.randn(2 * C, C, generator=torch.Generator().manual_seed(C))
+    H = (X.T @ X / C).to(cuda)
+    assert torch.equal(ops.hinv_upper(H.clone(), ops.Precision(split_hinv=3))[0], ops.hinv_upper(H.clone(), ops.Precision(split_hinv=4))[0])
+    narrow = [H[:512, :512].clone() for _ in range(2)]
+    for U, split in zip(narrow, (3, 4)):
+        ops.chol_unit_factor(U, ops.Precision(split_hinv=split))
+    assert torch.equal(*narrow)
 
 
 @pytest.mark.parametrize("C", [136, 384, 512])

@@ -104,6 +104,23 @@ def test_permutation_refuses_indices_of_another_gpu(no_launch, devices):
         ops.permute_columns(src, cols, rows=rows)
 
 
+def test_few_tokens_ask_for_all_products():
+    """Below half as many tokens as columns; a tied handle goes by the handle that owns the Hessian; what the caller chose
+    otherwise stays."""
+    gate = GPTQ(_layer(C=1024), 8, True)
+    up = GPTQ(_layer(C=1024), 8, True, tied_gptq_handle=gate)
+    for tokens, split in ((0, 4), (511, 4), (512, 3), (5000, 3)):
+        gate.num_samples = tokens
+        assert gate._layer_precision().split_hinv == up._layer_precision().split_hinv == split
+        assert gate._layer_precision().split_sweep == 3
+    gate.num_samples = 10
+    for p in (ops.Precision(split_hinv=2), ops.Precision(math=ops.MATH_FP32)):
+        gate.precision = p
+        assert gate._layer_precision() == p
+    gate.precision = ops.Precision(compact=True)
+    assert gate._layer_precision() == ops.Precision(split_hinv=4, compact=True)
+
+
 def test_asymmetric_is_refused():
     h = GPTQ(_layer(), 8, False)
     h.H = torch.eye(16)
