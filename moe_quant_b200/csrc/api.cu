@@ -30,7 +30,7 @@ size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split);
 int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, int64_t ldu, const float* scale,
                const float* zero, int64_t group, int64_t s_rs, int64_t s_gs, int bits, int out_dtype, uint8_t* codes,
                void* deq, const float* Worig, int64_t ldwo, int math, int split, Workspace& ws, cudaStream_t st,
-               const float* col_div, const float* eq, int32_t* packed);
+               const float* col_div, const float* eq, bool eq_bounds, int32_t* packed);
 int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, int split, mq_layer_flags* flags,
                      Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled, const float* eq);
 int copy_upper_scaled(const float* src, int64_t lds, float* dst, int64_t ldd, int64_t C, const float* eq, cudaStream_t st);
@@ -188,7 +188,7 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
     Workspace sub(ws.base + ws.used, ws.size - ws.used);
     MQ_TRY(gptq_sweep(Wf[i], R, C, C, U, C, scale_out[i], nullptr, group, C / group, 1, bits, w_dtype, codes[i],
                       dequantized ? dequantized[i] : nullptr, Wo[i], C, sweep_math, split_sweep, sub, st, unscaled ? diag : nullptr,
-                      pairs ? eq : nullptr, packed ? packed[i] : nullptr));
+                      pairs ? eq : nullptr, equilibration_bounds_factor(C, rel_damp), packed ? packed[i] : nullptr));
   }
   return MQ_OK;
 }

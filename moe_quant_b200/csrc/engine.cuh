@@ -105,15 +105,19 @@ int make_planes_f32(const float* src, int64_t rs, int64_t cs, int rows, int K, i
 
 // The factor's blocks above the diagonal, transposed, as pairs of fp16 planes: destination row j, k = i holds
 //   Utilde[i][j] * t_j,  Utilde[i][j] = U[i][j] / col_div[j] * eq[j] / eq[i]   (col_div, eq optional, else 1),
-// t_j a power of two that brings the column's entries under 2^14: from the column's maximum, or, with the C
-// factors eq of an equilibration followed by the smallest of them, from the bound 2^14 / eq[C] that every entry of
-// U[i][j] / eq[i] keeps.  The damping keeps that bound useful: diag(T) is at least sqrt(rel_damp mean(diag H)),
-// so it exceeds Utilde's unit diagonal by at most sqrt(C / rel_damp), 2^10.3 for 16384 columns and 0.01, and what a
-// pair of fp16 planes drops (2^-39 of it) stays below 2^-28 of the error it multiplies.  inv_t (2 C floats)
+// t_j a power of two that brings the column's entries under 2^14: from the column's maximum (a pass of its own), or, where
+// eq_bounds says that this is near enough, with the C factors eq of an equilibration followed by the smallest of them, from the
+// bound 2^14 / eq[C] that every entry of U[i][j] / eq[i] keeps.  inv_t (2 C floats)
 // receives 1 / t_j in its first half, the second is scratch.  Only k in 128-blocks in front of the row's own
 // block are written.
 int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, float* inv_t, const float* col_div, const float* eq,
-                            PlaneSet* out, cudaStream_t st);
+                            bool eq_bounds, PlaneSet* out, cudaStream_t st);
+
+// Whether that bound is near enough, by the damping: diag(T) is at least sqrt(rel_damp mean(diag H)), so the bound exceeds Utilde's unit
+// diagonal by at most 2 sqrt(C / rel_damp), 2^11.5 here, and what a pair of fp16 planes drops (2^-39 of it) stays below
+// 2^-27 of the error it multiplies.  With less damping a column of small channels, in front of one that is 2^24 times as large,
+// kept ten bits and less of its entries.
+inline bool equilibration_bounds_factor(int64_t C, float rel_damp) { return (float)C <= 0x1p21f * rel_damp; }
 
 // Tensor-core GEMM on fp32 operands that are split into `split` bf16 planes on the fly.
 int gemm_tensor_f32(const GemmDesc& d, int split, Workspace ws, cudaStream_t st);

@@ -403,11 +403,12 @@ size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split) {
 int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, int64_t ldu, const float* scale,
                const float* zero, int64_t group, int64_t s_rs, int64_t s_gs, int bits, int out_dtype, uint8_t* codes,
                void* deq, const float* Worig, int64_t ldwo, int math, int split, Workspace& ws, cudaStream_t st,
-               const float* col_div, const float* eq, int32_t* packed) {
+               const float* col_div, const float* eq, bool eq_bounds, int32_t* packed) {
   // col_div (tensor math only): above its diagonal 128-blocks Uhat holds the factor before its
   // columns were divided by col_div; the plane split divides where it reads it.  The diagonal
   // blocks, which the tiles read, are already scaled.  eq (with col_div): what lies above is the factor
-  // of the equilibrated matrix, entry (i, j) times eq[j] / eq[i] is the one of the matrix itself.
+  // of the equilibrated matrix, entry (i, j) times eq[j] / eq[i] is the one of the matrix itself; eq_bounds: see
+  // make_factor_planes_half.
   MQ_TRY(configure_once());
   const bool compact = (math & MQ_MATH_COMPACT) != 0;
   math &= ~MQ_MATH_COMPACT;
@@ -438,7 +439,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
     MQ_REQUIRE(ep && up && row_f && col_f, MQ_ERR_WORKSPACE, "mq_gptq_sweep: workspace too small for the operand planes");
     err_set.base = ep; err_set.planes = 2; err_set.rows_pad = (int)pad_rows(R); err_set.total_rows = err_set.rows_pad;
     err_set.K_pad = SUPER; err_set.fp16 = true;
-    MQ_TRY(make_factor_planes_half(Uhat, ldu, (int)C, up, col_f, col_div, eq, &u_set, st));
+    MQ_TRY(make_factor_planes_half(Uhat, ldu, (int)C, up, col_f, col_div, eq, eq_bounds, &u_set, st));
   } else if (tensor) {
     uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, SUPER, split) / 2);
     uint16_t* up = ws.take<uint16_t>(plane_set_bytes(C, C, split) / 2);
@@ -566,5 +567,5 @@ extern "C" int mq_gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const 
   MQ_REQUIRE(!packed || (bits == 4 && !zero && aligned(packed, 4)), MQ_ERR_UNSUPPORTED,
              "mq_gptq_sweep: packed words need bits == 4, the symmetric zero point and a 4-byte aligned buffer");
   return gptq_sweep(W, R, C, ldw, Uhat, ldu, scale, zero, group, row_stride, group_stride, bits, out_dtype, codes,
-                    dequantized, W_original, ldwo, math, split, ws, static_cast<cudaStream_t>(stream), nullptr, nullptr, packed);
+                    dequantized, W_original, ldwo, math, split, ws, static_cast<cudaStream_t>(stream), nullptr, nullptr, false, packed);
 }

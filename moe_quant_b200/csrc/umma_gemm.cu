@@ -1660,10 +1660,10 @@ __global__ void __launch_bounds__(256) split_transposed_f32_kernel(SplitParams p
 }
 
 // Column maxima of the factor's blocks above the diagonal: colmax[j] = max_i |U[i][j]| over the rows in
-// front of column j's 128-block, as the bits of a non-negative float (they order like integers).  Only for a
-// factor that was not equilibrated: entries of an equilibrated one lie below 2^14.  One CTA takes 128 columns x `rows_per` rows: a warp reads 512 bytes of a row at a time, four in flight.
+// front of column j's 128-block, as the bits of a non-negative float (they order like integers); with eq of |U[i][j]| / eq[i].
+// One CTA takes 128 columns x `rows_per` rows: a warp reads 512 bytes of a row at a time, four in flight.
 __global__ void __launch_bounds__(256) factor_colmax_kernel(const float* __restrict__ U, int64_t ldu, int C, int rows_per,
-                                                            int* __restrict__ colmax) {
+                                                            const float* __restrict__ eq, int* __restrict__ colmax) {
   __shared__ float part[8][TILE_N];
   const int j0 = ((int)blockIdx.x + 1) * TILE_N;   // the first block of columns has nothing above it
   const int r_begin = (int)blockIdx.y * rows_per;
@@ -1675,15 +1675,17 @@ __global__ void __launch_bounds__(256) factor_colmax_kernel(const float* __restr
   if (c < C) {
     for (int r = r_begin + warp; r < r_end; r += 32) {
       float4 v[4];
+      float f[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int rr = r + 8 * u;
         v[u] = rr < r_end ? __ldg(reinterpret_cast<const float4*>(U + (int64_t)rr * ldu + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        f[u] = eq && rr < r_end ? 1.0f / __ldg(eq + rr) : 1.0f;
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        m.x = fmaxf(m.x, fabsf(v[u].x)); m.y = fmaxf(m.y, fabsf(v[u].y));
-        m.z = fmaxf(m.z, fabsf(v[u].z)); m.w = fmaxf(m.w, fabsf(v[u].w));
+        m.x = fmaxf(m.x, f[u] * fabsf(v[u].x)); m.y = fmaxf(m.y, f[u] * fabsf(v[u].y));
+        m.z = fmaxf(m.z, f[u] * fabsf(v[u].z)); m.w = fmaxf(m.w, f[u] * fabsf(v[u].w));
       }
     }
   }
@@ -1697,7 +1699,7 @@ __global__ void __launch_bounds__(256) factor_colmax_kernel(const float* __restr
   }
 }
 
-// See make_factor_planes_half.  64 x 64 tiles as in split_transposed_f32_kernel.
+// See make_factor_planes_half (colmax null: the bound from eq).  64 x 64 tiles as in split_transposed_f32_kernel.
 __global__ void __launch_bounds__(256) split_factor_half_kernel(const float* __restrict__ U, int64_t ldu, int C, int rows_pad, int K_pad,
                                                                 const float* __restrict__ col_div, const float* __restrict__ eq,
                                                                 const int* __restrict__ colmax, float* __restrict__ inv_t,
@@ -1726,11 +1728,10 @@ __global__ void __launch_bounds__(256) split_factor_half_kernel(const float* __r
     float x0 = 0.0f, x1 = 0.0f;
     if (r < C) {
       const float d = col_div ? __ldg(col_div + r) : 1.0f, e = eq ? __ldg(eq + r) : 1.0f;
-      const float t = scale_below_2_14((eq ? 16384.0f / __ldg(eq + C) : __int_as_float(__ldg(colmax + r))) * e / d);
+      const float t = scale_below_2_14((colmax ? __int_as_float(__ldg(colmax + r)) : 16384.0f / __ldg(eq + C)) * e / d);
       if (blockIdx.x == 0 && lane == 0) inv_t[r] = 1.0f / t;
-      const float m = e * t;
-      x0 = tile[2 * lane][rl] / d * f0 * m;
-      x1 = tile[2 * lane + 1][rl] / d * f1 * m;
+      x0 = tile[2 * lane][rl] / d * f0 * e * t;   // (e t may leave fp32's range, the entry times e does not)
+      x1 = tile[2 * lane + 1][rl] / d * f1 * e * t;
     }
     uint16_t h0, l0, h1, l1;
     split_half2(x0, h0, l0);
@@ -2184,7 +2185,7 @@ int make_planes_f32(const float* src, int64_t rs, int64_t cs, int rows, int K, i
 }
 
 int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, float* inv_t, const float* col_div, const float* eq,
-                            PlaneSet* out, cudaStream_t st) {
+                            bool eq_bounds, PlaneSet* out, cudaStream_t st) {
   PlaneSet ps;
   ps.planes = 2;
   ps.rows_pad = pad_to(C, TILE_M);
@@ -2194,13 +2195,13 @@ int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, f
   ps.base = dst;
   *out = ps;
   if (C <= TILE_M) return MQ_OK;   // no block above the diagonal
-  int* colmax = reinterpret_cast<int*>(inv_t + C);
+  int* colmax = eq && eq_bounds ? nullptr : reinterpret_cast<int*>(inv_t + C);
   ProfScope prof(PROF_SPLIT, (double)C * C * 0.5 * (4.0 + 4.0), 0.0, st);
-  if (!eq) {
+  if (colmax) {
     MQ_CUDA(cudaMemsetAsync(colmax, 0, (size_t)C * sizeof(int), st));
     const int col_blocks = (int)ceil_div(C, TILE_N) - 1;
     const int rows_per = 128;
-    factor_colmax_kernel<<<dim3((unsigned)col_blocks, (unsigned)ceil_div(C, rows_per)), 256, 0, st>>>(U, ldu, C, rows_per, colmax);
+    factor_colmax_kernel<<<dim3((unsigned)col_blocks, (unsigned)ceil_div(C, rows_per)), 256, 0, st>>>(U, ldu, C, rows_per, eq, colmax);
     MQ_LAUNCH_CHECK();
   }
   split_factor_half_kernel<<<dim3((unsigned)(ps.K_pad / 64), (unsigned)ceil_div(ps.rows_pad, 64)), 256, 0, st>>>(

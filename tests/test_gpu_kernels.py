@@ -594,6 +594,29 @@ def test_layer_with_little_damping_against_fp32_math(cuda, rel_damp, spread, C):
     assert O.code_agreement(run(MATH_TENSOR), run(MATH_FP32)) >= CODE_AGREEMENT
 
 
+@pytest.mark.parametrize("C", [520, 1544])
+@pytest.mark.parametrize("large", ["first", "last"])
+@pytest.mark.parametrize("tied", [1, 2])
+def test_undamped_layer_with_a_few_large_channels(cuda, C, large, tied):
+    """Small channels that depend on each other, column j on column j - 128, beside independent ones 2^32 as large: a bound
+    over the whole matrix says nothing about the columns of the small ones, which are scaled by their own maxima."""
+    gen = torch.Generator().manual_seed(C)
+    n = 256 if C == 520 else 1024
+    T = torch.eye(n, dtype=torch.float64)
+    j = torch.arange(128, n)
+    T[j - 128, j] = 0.5 + 0.5 * torch.rand(n - 128, generator=gen, dtype=torch.float64)
+    big = 2.0 ** 64 * torch.eye(C - n, dtype=torch.float64)
+    H = torch.block_diag(*((big, T @ T.T) if large == "first" else (T @ T.T, big))).float()
+    W = [synthetic.layer_weight(200, C, 5 + i, torch.bfloat16).to(cuda) for i in range(tied)]
+
+    def run(math):
+        codes, _, _, flags = ops.quantize_layer(W, H.to(cuda), 8, 4, 0.0, precision=ops.Precision(math=math))
+        assert int(flags[3]) == 0
+        return torch.cat(codes).cpu()
+
+    assert O.code_agreement(run(MATH_TENSOR), run(MATH_FP32)) >= CODE_AGREEMENT
+
+
 # ------------------------------------------------------------------ MSE scale search
 @pytest.mark.parametrize("R,C,g,dtype", [(64, 512, 128, torch.bfloat16), (40, 256, 32, torch.float16),
                                          (24, 384, 64, torch.float32), (8, 2048, 2048, torch.bfloat16)])
