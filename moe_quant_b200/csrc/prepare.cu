@@ -212,12 +212,12 @@ __global__ void __launch_bounds__(256) absmax_scales_kernel(const float* __restr
 //  * every term is non-negative and fp32 addition is monotone, so a candidate whose largest terms
 //    alone reach the best loss so far cannot win.  The terms of the segment's largest and smallest
 //    element, which the shrunk grids clip, are computed for 32 candidates at a time (one candidate
-//    per lane); two thirds of the 100 candidates of a 128-wide group fall to them.  Wide groups
-//    (mse_scales_wide_kernel) compare the partial sum every eight elements per lane instead.
+//    per lane); two thirds of the 100 candidates of a 128-wide group fall to them.  mse_scales_wide_kernel
+//    compares the partial sum every eight elements per lane instead.
 //  * the elements of a 32-, 64- or 128-wide group stay in registers over all candidates.
 //  * x / s goes through the reciprocal of s, which the whole warp shares, and one residual correction
 //    (Markstein 1990); scales so small or large that the residual could underflow keep the division.
-// 7168 x 2048 bf16, groups of 128, 100 candidates: 2826 us before, about 715 us now (4394 -> 2283 us for the whole quantize call).
+// 7168 x 2048 bf16, groups of 128, 100 candidates: 2826 us before, about 715 us now (4394 -> 1951 us for the whole quantize call).
 template <int DT>
 __device__ __forceinline__ float mse_term(float x, float s, float rs, bool plain, float zero, float maxq, float norm) {
   float d;
@@ -235,7 +235,7 @@ __device__ __forceinline__ float mse_term(float x, float s, float rs, bool plain
   return __expf(__logf(fabsf(y - x)) * norm);
 }
 
-// EPL: elements per lane of a group of 32 * EPL columns, held in registers; 0: any group below 256 columns.
+// EPL: elements per lane of a group of 32 * EPL columns, held in registers; 0: any group.
 template <int DT, int EPL>
 __global__ void __launch_bounds__(256) mse_scales_kernel(const float* __restrict__ W, int64_t R, int64_t C, int64_t ldw,
                                                          int64_t group, float maxq, float zero,
@@ -312,10 +312,9 @@ __global__ void __launch_bounds__(256) mse_scales_kernel(const float* __restrict
   }
 }
 
-// Groups of 256 columns and more: a CTA per (row, group), its warps share out the candidates.  A layer with one group
-// per row has few segments, and a warp per segment left the chip idle over a serial stream (796 x 4040, one group per
-// row: the whole call 4870 us, 3120 us here).  19860 x 632 is level: 2470 us by warps, 2560 us by CTAs.  Every warp takes candidate 0 first, so that all start from the same best; a
-// candidate's loss is summed by one warp in the order of the kernel above.  Of equal losses the first candidate wins.
+// A CTA per (row, group), its warps share out the candidates (mse_by_ctas: few or very wide groups).  Every warp takes candidate 0
+// first, so that all start from the same best; a candidate's loss is summed by one warp in the order of the kernel above.  Of
+// equal losses the first candidate wins.
 template <int DT>
 __global__ void __launch_bounds__(256) mse_scales_wide_kernel(const float* __restrict__ W, int64_t R, int64_t C, int64_t ldw, int64_t group,
                                                               float maxq, float zero, const float* __restrict__ p, int p_size, float norm,
@@ -374,14 +373,26 @@ __global__ void __launch_bounds__(256) mse_scales_wide_kernel(const float* __res
   }
 }
 
+// A warp per segment needs about 0.28 us per column of the group however few there are, and its 64 warps per SM then finish
+// together; the bound of the two extreme elements drops most candidates of a narrow group.  A CTA per segment shortens the
+// serial stream, and its partial sums drop candidates of a wide group, where two elements say little.  The search alone, bf16, us by
+// warps / by CTAs:
+//   group  256:  1792 segments   86 / 109   4736  107 /  236    57344   900 / 2589
+//   group  512:   896           141 /  99   2368  146 /  183    28672  1035 / 1891
+//   group 1024:  1184           289 / 163   2960  357 /  356    14336  1214 / 1610
+//   group 1536:  4096           755 / 685  16384 2192 / 2728
+//   group 2048:  3072           852 / 655   7168 1710 / 1556    16384  3210 / 3604
+//   group 4096:   500          1457 / 321   8192 5338 / 3689    16384 10328 / 7162
+// The line lies at 1300 segments, and from 684 columns on at a number that grows with the square of the width.
+inline bool mse_by_ctas(int64_t n_seg, int64_t group) { return group >= 256 && (n_seg < 1300 || n_seg < group * group / 360); }
+
 template <int DT>
 void launch_mse_scales(int grid, cudaStream_t st, const float* W, int64_t R, int64_t C, int64_t ldw, int64_t group, float maxq, float zero,
                        const float* p, int p_size, float norm, float* scale) {
   if (group == 128) mse_scales_kernel<DT, 4><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
   else if (group == 64) mse_scales_kernel<DT, 2><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
   else if (group == 32) mse_scales_kernel<DT, 1><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
-  else if (group >= 256) {
-    const int64_t n_seg = R * (C / group);
+  else if (const int64_t n_seg = R * (C / group); mse_by_ctas(n_seg, group)) {
     mse_scales_wide_kernel<DT><<<(unsigned)(n_seg < 148 * 8 ? n_seg : 148 * 8), 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
   } else mse_scales_kernel<DT, 0><<<grid, 256, 0, st>>>(W, R, C, ldw, group, maxq, zero, p, p_size, norm, scale);
 }

@@ -646,6 +646,7 @@ def test_mse_scales_match_oracle(cuda, R, C, g, dtype):
 @pytest.mark.parametrize("R,C,g,factor,dtype", [
     (16, 384, 384, 1.0, torch.bfloat16),      # wide groups: partial sums are compared on the way
     (5, 1536, 256, 1.0, torch.float32), (1300, 264, 264, 1.0, torch.bfloat16), (7, 248, 248, 1.0, torch.float16),
+    (1299, 264, 264, 1.0, torch.float16), (1340, 688, 688, 1.0, torch.bfloat16), (1313, 688, 688, 1.0, torch.float32),   # either side of the line
     (9, 1056, 1056, 1e-6, torch.float32),     # a last trip of the lanes that is not full
     (16, 96, 24, 1.0, torch.float16),         # fewer elements than lanes
     (12, 256, 32, 1e-10, torch.bfloat16),
