@@ -53,13 +53,13 @@ __device__ __forceinline__ void split_half2(float x, uint16_t& hi, uint16_t& lo)
   lo = __half_as_ushort(__float2half_rn(x - __half2float(h)));
 }
 
-// 2^(14 - e) for |bound| in [2^(e-1), 2^e): scaled by it, values up to `bound` lie below 2^14.
-// 1 for zero, infinity and NaN.
+// 2^(14 - e) for |bound| in [2^(e-1), 2^e): scaled by it, values up to `bound` lie below 2^14 (2^126 at most, so that the inverse
+// is a normal number too).  1 for zero, infinity and NaN.
 __device__ __forceinline__ float scale_below_2_14(float bound) {
   const int b = (int)((__float_as_uint(bound) >> 23) & 0xFFu);
   if (b == 0 || b == 255) return 1.0f;
-  int e = 14 - (b - 126);
-  e = e < -100 ? -100 : (e > 100 ? 100 : e);
+  int e = 14 - (b - 126);   // -114 ..
+  e = e > 126 ? 126 : e;
   return __uint_as_float((uint32_t)(e + 127) << 23);
 }
 

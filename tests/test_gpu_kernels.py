@@ -785,7 +785,7 @@ def test_layer_preparation_against_oracle(cuda, R, C, g, dtype, offset):
 
 # ------------------------------------------------------------------ quadratic forms
 @pytest.mark.parametrize("R,C", [(1, 1), (3, 13), (255, 64), (257, 200), (40, 257), (300, 1031), (512, 768)])
-@pytest.mark.parametrize("kind", ["hessian", "unsymmetric", "spread", "tiny"])
+@pytest.mark.parametrize("kind", ["hessian", "unsymmetric", "spread", "tiny", "huge"])
 def test_quadratic_forms_against_fp64(cuda, R, C, kind):
     """Ragged tiles in rows, columns and k; any square H, not only symmetric ones; scales over many decades; row
     strides.  Error: three of four half products of 22-bit pairs, 2^-22 each, sums of 64 of k in the
@@ -800,6 +800,8 @@ def test_quadratic_forms_against_fp64(cuda, R, C, kind):
     q, w = torch.randn(R, C, generator=gen), torch.randn(R, C, generator=gen)
     if kind == "tiny":
         q, w, H = q * 1e-9, w * 1e-12, H * 1e-20
+    if kind == "huge":
+        q, w, H = q * 1e-2, w * 1e-2, H * 2.0 ** 117
     wide = torch.empty(R, C + 5, device=cuda)
     wide[:, :C] = q.to(cuda)
     got = ops.error_forms(wide[:, :C], w.to(cuda), H.to(cuda)).cpu()
