@@ -154,6 +154,24 @@ def test_hessian_accum_activation_views(cuda, dtype, pad, offset):
     assert torch.equal(Hc, Hc.t())
 
 
+@pytest.mark.parametrize("C", [8, 129, 250, 256, 1000, 1031])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_hessian_accum_first_batch_reads_nothing(cuda, precision, C, dtype):
+    """With beta = 0 every element of both triangles is written and none is read: a handle's first batch goes into memory as the
+    allocator gives it.  Every route: rows read in place, the transposed copy, planes of fp32, the CUDA cores."""
+    for m in (1, 37, 333):
+        for offset in (0, 1):
+            gen = torch.Generator().manual_seed(100 * m + offset)
+            big = torch.randn(m, C + 8, generator=gen).to(dtype)
+            H = torch.full((C, C), float("nan"), device=cuda)
+            ops.hessian_accum(H, big.to(cuda)[:, offset : offset + C], 0.0, 2.0 / m, precision)
+            x = big[:, offset : offset + C].double()
+            want = (2.0 / m) * (x.t() @ x)
+            got = H.cpu()
+            assert float((got.double() - want).abs().max() / want.abs().max()) < 5e-6
+            assert torch.equal(got, got.t())
+
+
 # ------------------------------------------------------------------ prepare
 def test_prepare_golden(cuda, golden):
     H = golden.t("H_final").clone().to(cuda)
