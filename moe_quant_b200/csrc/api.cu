@@ -26,7 +26,7 @@ size_t hinv_workspace_bytes(int64_t C, int math, int split);
 size_t factor_workspace_bytes(int64_t C, int math, int split);
 int hinv_upper(float* H, int64_t C, int64_t ldh, float* Uhat, int64_t ldu, float* diag_out, int math, int split, mq_layer_flags* flags,
                Workspace& ws, cudaStream_t st);
-size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split);
+size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split, bool inverse_free);
 int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, int64_t ldu, const float* scale,
                const float* zero, int64_t group, int64_t s_rs, int64_t s_gs, int bits, int out_dtype, uint8_t* codes,
                void* deq, const float* Worig, int64_t ldwo, int math, int split, Workspace& ws, cudaStream_t st,
@@ -116,7 +116,7 @@ extern "C" size_t mq_quantize_layer_workspace_bytes(int n_tied, int64_t R, int64
   if (n_tied <= 0 || R <= 0 || C <= 0) return 0;
   math &= ~MQ_MATH_COMPACT;
   size_t a = factor_workspace_bytes(C, math, split_hinv);            // factorisation: the planes of a super-panel
-  size_t b = sweep_workspace_bytes(R, C, math, split_sweep);
+  size_t b = sweep_workspace_bytes(R, C, math, split_sweep, true);
   return layer_fixed_bytes(n_tied, R, C) + (a > b ? a : b);
 }
 

@@ -391,13 +391,13 @@ int configure_once() {
 
 }  // namespace
 
-size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split) {
-  math &= ~MQ_MATH_COMPACT;
-  split = plane_count(split);
-  if (math == MQ_MATH_TENSOR)
-    return plane_set_bytes(R, SUPER, split) + plane_set_bytes(C, C, split) + align_up((size_t)R * (SUPER / TILE) * sizeof(float), 256) +
+// inverse_free: the sweep has the original weights and works on pairs of planes where uses_pairs says so.
+size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split, bool inverse_free) {
+  if ((math & ~MQ_MATH_COMPACT) != MQ_MATH_TENSOR) return align_up((size_t)R * TILE * sizeof(float), 256);
+  if (inverse_free && uses_pairs(C, math, split))
+    return plane_set_bytes(R, SUPER, 2) + plane_set_bytes(C, C, 2) + align_up((size_t)R * (SUPER / TILE) * sizeof(float), 256) +
            align_up((size_t)C * 2 * sizeof(float), 256);
-  return align_up((size_t)R * TILE * sizeof(float), 256);
+  return plane_set_bytes(R, SUPER, plane_count(split)) + plane_set_bytes(C, C, plane_count(split));
 }
 
 int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, int64_t ldu, const float* scale,
@@ -463,7 +463,6 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   sa.plane_stride = tensor ? err_set.total_rows * (int64_t)SUPER : 0;
   sa.n_planes = half ? 2 : split;
   sa.err_ld = tensor ? SUPER : TILE;
-  sa.bits = bits;
   const bool uniform = group % SUB == 0;
   // Rows per CTA: the chain costs the same for 1 row and for 64, so a tile of 2048 rows takes 16.5 us on 148 SMs,
   // 17.4 on 74 and 19.0 on 48.  Alone, one CTA per SM; a caller with several layers in flight gives each
@@ -538,7 +537,8 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
 
 extern "C" size_t mq_gptq_sweep_workspace_bytes(int64_t R, int64_t C, int math, int split) {
   if (R <= 0 || C <= 0) return 0;
-  return mq::sweep_workspace_bytes(R, C, math, split);
+  const size_t with_original = mq::sweep_workspace_bytes(R, C, math, split, true), without = mq::sweep_workspace_bytes(R, C, math, split, false);
+  return with_original > without ? with_original : without;
 }
 
 extern "C" int mq_gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, int64_t ldu,

@@ -28,7 +28,6 @@ struct SweepArgs {
   const float* Worig; int64_t ldwo;
   uint16_t* err_planes; int64_t plane_stride; int n_planes;
   int err_ld;   // row stride of err / err_planes (both already point at this tile's k window)
-  int bits;
   // not null: the errors are written as two fp16 planes, each row scaled by a power of two of its own for this tile,
   // whose inverse goes to row_f[row]
   float* row_f;

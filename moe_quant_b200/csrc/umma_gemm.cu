@@ -1127,11 +1127,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_stream_kernel(const __gr
           if (lane == 0) bulk_wait_read_1();
           __syncwarp();
           const uint32_t dst = my_row + (uint32_t)(chunk & 1) * 4096u;
-          apply_factors(v, p, y + lane, n0 + c * 32);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((j ^ (lane & 7)) << 4)),
-                         "f"(v[4 * j]), "f"(v[4 * j + 1]), "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
+                         "f"(p.alpha * v[4 * j]), "f"(p.alpha * v[4 * j + 1]), "f"(p.alpha * v[4 * j + 2]),
+                         "f"(p.alpha * v[4 * j + 3])
                          : "memory");
           fence_async_smem();
           __syncwarp();
@@ -2021,9 +2021,9 @@ int configure_once() {
 
 int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStream_t st) {
   MQ_TRY(configure_once());
-  // only the two kernels of the rank-<=128 and the deep updates apply row and column factors
-  MQ_REQUIRE((!d.row_f && !d.col_f) || (A.planes > 1 && d.batch == 1 && !d.a_upper && !d.b_upper && !d.n_step && !d.mirror_to_lower && d.K > 0),
-             MQ_ERR_UNSUPPORTED, "tensor engine: row and column factors need a plain update with several planes");
+  // only the updates of operand pairs (panel and pair kernel) apply row and column factors
+  MQ_REQUIRE((!d.row_f && !d.col_f) || (A.planes == 2 && A.fp16 && d.batch == 1 && !d.a_upper && !d.b_upper && !d.n_step && !d.mirror_to_lower && d.K > 0),
+             MQ_ERR_UNSUPPORTED, "tensor engine: row and column factors need a plain update of operand pairs");
   MQ_REQUIRE(!d.col_f || aligned(d.col_f, 16), MQ_ERR_ALIGNMENT, "tensor engine: column factors must be 16-byte aligned");
   CUtensorMap map_a, map_b;
   MQ_TRY(encode_map(A, &map_a));
@@ -2124,7 +2124,6 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
       MQ_TRY(encode_c_map(d.C, d.ldc, d.M, d.N, &map_c));
       p.c_tma = d.beta == 0.0f ? 1 : 2;
     }
-    MQ_REQUIRE(p.c_tma || (!d.row_f && !d.col_f), MQ_ERR_ALIGNMENT, "tensor engine: row and column factors need 16-byte aligned rows of C");
     p.drain_slabs = (d.k_round > 0 && p.c_tma == 2) ? d.k_round / SLAB_K : 0;
     const size_t staging = p.c_tma ? (size_t)4 * 2 * 4096 : (size_t)STAGE_BYTES;
     const size_t ssmem = (size_t)4 * A.planes * PLANE_TILE_BYTES + 1024 + staging;   // two stages of A and B slabs, staging
