@@ -76,6 +76,7 @@ class GPTQ:
         self._hessian_ready = False   # True once H has been masked and damped
         self._uhat: Optional[Tensor] = None
         self._was_reset = False
+        self._hessian_tokens = 0      # tokens behind H where num_samples does not say: after a reduction or a reset
 
     @staticmethod
     def _validate_layer(layer) -> None:
@@ -158,6 +159,7 @@ class GPTQ:
         alpha = 2.0 / (self.num_samples + m)
         ops.hessian_accum(self.H, x, beta, alpha, self.precision)
         self.num_samples += m
+        self._hessian_tokens = 0
 
     @property
     def tokens_collected(self) -> int:
@@ -178,6 +180,8 @@ class GPTQ:
         elif self.num_tied_handles == 0:
             self._drop_hessian()
         self._was_reset = True
+        if self.H is not None:
+            self._hessian_tokens = max(self._hessian_tokens, self.num_samples)   # tied handles may still quantize with it
         self.num_samples = 0
         self.pre_step_completed = False
 
@@ -185,6 +189,7 @@ class GPTQ:
         self.H = None
         self._uhat = None
         self._hessian_ready = False
+        self._hessian_tokens = 0
 
     # ------------------------------------------------------------------ pre-step
     @torch.no_grad()
@@ -212,6 +217,7 @@ class GPTQ:
         if total > 0:
             self.H.mul_(self.num_samples / total)
             dist.all_reduce(self.H, op=dist.ReduceOp.SUM)
+            self._hessian_tokens = int(total)
 
     # ------------------------------------------------------------------ quantize
     def _group(self) -> int:
@@ -256,10 +262,12 @@ class GPTQ:
     def _layer_precision(self) -> ops.Precision:
         """The handle's precision; from fewer tokens than half the columns the factorisation takes all four products of
         its operand pairs (its sums cancel there: with three, the layer's error against fp64 is up to 1.08 of that of
-        three bf16 planes, with four 1.01; above half the columns three do: 0.97 and less)."""
+        three bf16 planes, with four 1.01; above half the columns three do: 0.97 and less).  What counts are the tokens of
+        all ranks behind the Hessian; the identity that stands in for no token at all has nothing to cancel."""
         p = ops.DEFAULT_PRECISION if self.precision is None else self.precision
         owner = self if self.tied_gptq_handle is None else self.tied_gptq_handle
-        if p.math == ops.MATH_TENSOR and p.split_hinv == 3 and 2 * owner.num_samples < self.d_col:
+        tokens = max(owner.num_samples, owner._hessian_tokens)
+        if p.math == ops.MATH_TENSOR and p.split_hinv == 3 and 2 * tokens < self.d_col and not owner.issue_zero_samples:
             return dataclasses.replace(p, split_hinv=4)
         return p
 

@@ -5,7 +5,7 @@ import pytest
 import torch
 import torch.nn as nn
 
-from moe_quant_b200 import GPTQ, QuantizationOrder, model_utils, ops, quant_utils
+from moe_quant_b200 import GPTQ, QuantizationOrder, gptq, model_utils, ops, quant_utils
 from moe_quant_b200._lib import MoeQuantError
 
 
@@ -119,6 +119,38 @@ def test_few_tokens_ask_for_all_products():
         assert gate._layer_precision() == p
     gate.precision = ops.Precision(compact=True)
     assert gate._layer_precision() == ops.Precision(split_hinv=4, compact=True)
+
+
+def test_few_tokens_are_counted_over_all_ranks(monkeypatch):
+    """A rank that holds a third of the tokens decides by all of them, as a single process with the same tokens would."""
+    h = GPTQ(_layer(C=1024), 8, True, is_distributed=True)
+    h.H, h.num_samples = torch.eye(1024), 200
+    assert h._layer_precision().split_hinv == 4
+    monkeypatch.setattr(gptq.dist_utils, "is_dist_available_and_initialized", lambda: True)
+    monkeypatch.setattr(gptq.dist, "all_reduce", lambda t, op=None: t.mul_(3))
+    h.quantization_pre_step()
+    assert h.tokens_collected == 200 and h._layer_precision().split_hinv == 3
+    torch.testing.assert_close(h.H, torch.eye(1024))
+    h.reset()
+    assert h._hessian_tokens == 0
+
+
+def test_few_tokens_after_the_owner_was_reset():
+    """gate_proj quantized and reset before up_proj: the Hessian is still that of its tokens; a new batch starts afresh."""
+    gate = GPTQ(_layer(C=1024), 8, True)
+    up = GPTQ(_layer(C=1024), 8, True, tied_gptq_handle=gate)
+    gate.H, gate.num_samples = torch.eye(1024), 5000
+    gate.reset()
+    assert gate.H is not None and gate.tokens_collected == 0
+    assert up._layer_precision().split_hinv == 3
+    up.reset()
+    assert gate.H is None and gate._layer_precision().split_hinv == 4
+
+
+def test_no_token_at_all_has_nothing_to_cancel():
+    h = GPTQ(_layer(C=1024), 8, True)
+    h.quantization_pre_step()
+    assert h.issue_zero_samples and h._layer_precision().split_hinv == 3
 
 
 def test_asymmetric_is_refused():
