@@ -148,7 +148,7 @@ class GPTQ:
             if first is torch.empty:
                 try:
                     ops.hessian_accum(self.H, x, 0.0, 2.0 / m, self.precision)
-                except Exception:
+                except BaseException:      # an interrupt too: the memory is as the allocator gave it
                     self.H.zero_()
                     raise
                 self.num_samples = m

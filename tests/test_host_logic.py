@@ -54,6 +54,18 @@ def test_update_on_cpu_raises():
         h.update(torch.zeros(4, 16, dtype=torch.bfloat16))
 
 
+@pytest.mark.parametrize("error", [MoeQuantError, KeyboardInterrupt])
+def test_failed_first_batch_leaves_an_empty_hessian(monkeypatch, error):
+    def fail(H, *a):
+        H.fill_(float("nan"))
+        raise error("stop")
+    monkeypatch.setattr(ops, "hessian_accum", fail)
+    h = GPTQ(_layer(), 8, True)
+    with pytest.raises(error):
+        h.update(torch.zeros(4, 16, dtype=torch.bfloat16))
+    assert torch.equal(h.H, torch.zeros(16, 16)) and h.tokens_collected == 0
+
+
 class _On:
     """What the checks in front of a launch look at, on a GPU that need not be there."""
     is_cuda, dtype = True, torch.float32
