@@ -47,9 +47,10 @@ sys.path.insert(0, ROOT)
 R, C, TOKENS, GROUP, BITS = 2048, 7168, 4096, 128, 4
 WORKLOAD = "deepseek_v3_routed_expert_gate_proj_2048x7168_bf16_g128 (one rank's expert shard, Hessian resident)"
 METRIC = "GPTQ layers/sec (2048x7168, 4b g128)"
-# DRAM traffic of one 128 x 128 output tile of a 512-deep update (ncu of the three-plane kernel, profiles/: the C tile in
-# and out, which the operand format does not change, is all but a few KB of it)
-DEEP_DRAM_BYTES_PER_TILE = 103.0e3
+# DRAM traffic of one 128 x 128 output tile of a 512-deep update: 104 MB read and 33 MB written over the 1378 tiles on and above
+# the diagonal of a 6656 x 6656 one (ncu, profiles/umma_pair_kernel_far_update.md).  C in and out alone is 128 KB: part of the
+# matrix stays in the L2
+DEEP_DRAM_BYTES_PER_TILE = 99.4e3
 CONFIG = {"workload": WORKLOAD, "rows": R, "cols": C, "bits": BITS, "group_size": GROUP, "rel_damp": 1e-2,
           "weight_dtype": "bf16", "calibration_tokens_mean": TOKENS}
 
@@ -433,20 +434,14 @@ def headline(cx):
             products = 1.0 if top == "simt_gemm" else 3.0
             out_tiles = v["work2"] / v["launches"] / (2.0 * 128 * 128 * products)   # output tiles x k per launch
             if top == "umma_deep":
-                # DRAM bytes per 128 x 128 output tile of a 512-deep update, from an ncu capture of the
-                # 6656 x 6656 x 512 upper-triangle update (profiles/): the C tile once in, once out, and
-                # the operand slabs that miss the L2
                 roofline["traffic"] = DEEP_DRAM_BYTES_PER_TILE * out_tiles / 512.0
                 roofline["traffic_source"] = ("scaled by output tiles from an ncu capture of one 512-deep update "
-                                              "(profiles/umma_stream_kernel_far_update.md), not measured in this run")
-            elif top == "umma_gemm":
-                roofline["traffic"] = 95.0e3 * out_tiles / 128.0
-                roofline["traffic_source"] = ("scaled from an ncu capture (95 KB of DRAM traffic per 128x128 tile of a "
-                                              "rank-128 update), not measured in this run")
+                                              "(profiles/umma_pair_kernel_far_update.md), not measured in this run")
             else:
                 roofline["traffic"] = None
             roofline["note"] = ("algorithmic work of the GEMM on pairs of fp16 planes: 2MNK on the kept tiles x 3 fp16 tensor products "
-                                "per fp32 product; fp32_equivalent_tflops counts each fp32 product once; timed on one "
+                                "per fp32 product (the factorisation of fewer tokens than half the columns issues a fourth, not counted); "
+                                "fp32_equivalent_tflops counts each fp32 product once; timed on one "
                                 "stream with full grids; chosen as the member of the tensor-GEMM family with the most work")
             roofline["peak_source"] = peaks["source"] + " (sustained bf16)"
             roofline["others"] = [tensor_line(k, kv) for k, kv in family.items() if k != top]
@@ -589,7 +584,8 @@ def headline(cx):
                    "single_stream_layers_per_s_per_gpu": steps_aux / (ms_single / 1e3),
                    "tied_gate_up_layers_per_s_per_gpu": tied_layers_per_s,
                    "e2e_step": "one layer of a gate_proj/up_proj pair: X uploaded once per expert, one factorisation per pair",
-                   "math": "tcgen05 split-bf16 x3 planes (6 products), fp32 TMEM accumulation"})
+                   "math": "tcgen05 on pairs of fp16 planes (3 products, 4 below half as many tokens as columns), 64 of k per TMEM accumulator, "
+                           "fp32 sums"})
     return {
         "metric": METRIC, "value": value, "unit": "layers/s", "n_gpus": world, "steps": steps, "warmup": cx.warmup,
         "ms_per_step": ms_med / steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

@@ -1,5 +1,5 @@
 // Picks the arithmetic for a dense contraction: fp32 CUDA cores or tcgen05
-// tensor cores on split-bf16 planes.  One Engine lives for the duration of one
+// tensor cores on 16-bit planes.  One Engine lives for the duration of one
 // C-ABI call and carves its scratch out of that call's workspace.
 #pragma once
 

@@ -1,6 +1,6 @@
 // Dense-contraction interface shared by the Hessian, the factorisation and the
 // lazy block update.  Two implementations sit behind it: fp32 FMAs on the CUDA
-// cores (gemm_simt.cu) and tcgen05 tensor cores on bf16 planes (umma_gemm.cu).
+// cores (gemm_simt.cu) and tcgen05 tensor cores on 16-bit planes (umma_gemm.cu).
 #pragma once
 
 #include "common.cuh"

@@ -568,7 +568,7 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
   }
   Engine eng(math, split, local, st);
   const int P = (int)ceil_div(C, NB);
-  // Tensor path: the panel solve writes its result as bf16 planes too, and the rank-128 update
+  // Tensor path: the panel solve writes its result as planes too, and the rank-128 update
   // P P^T reads one plane set as both operands.
   const bool tensor = math == MQ_MATH_TENSOR;
   {

@@ -8,7 +8,9 @@
 // against the upper triangle of H + H^T (the form sees only the symmetric part), three products, k up to the
 // diagonal, and the sum taken in the epilogue.  2048 x 7168: 1984 us of contractions (two, six products, all of
 // k), planes of H twice and a pass over each product became one of 603 us: the whole call, dequantization included,
-// 2740 -> 926 us, and its error against fp64 3.3e-7 -> 1.4e-8.
+// 2740 -> 926 us.  Relative error of a form against fp64 (mean of four seeds, both forms alike): with one accumulator over
+// all of k 0.9e-6 at 1024 columns, 7e-6 at 7168, 1.6e-5 at 16384 (the tensor core truncates, always towards zero); with sums of
+// 64 of k added in fp32 and the rest in fp64 3e-8 to 4e-8 throughout.
 #include "engine.cuh"
 
 namespace mq {

@@ -10,8 +10,8 @@
 // increasing j: the reference's order.  One thread per row runs the sixteen dependent steps of a
 // sub-block; the other warps apply the errors to the rest of the tile.
 //
-// The errors of the tile (R x 128) go to a scratch matrix, as bf16 planes on the tensor path,
-// and the lazy update
+// The errors of the tile (R x 128) go to a scratch matrix, on the tensor path as operand planes (pairs
+// of fp16 planes in the inverse-free form of more than 512 columns, bf16 planes otherwise), and the lazy update
 //   W[:, later] += E Uhat[tile, later]             (src/gptq_loop.py:148)
 // is a GEMM: on the tensor path in two levels (the rest of the tile's 512-column super-block at
 // once, everything behind the super-block once per super-block with all 512 errors of a row
@@ -68,11 +68,12 @@ __device__ __forceinline__ void stage_factor_tile(float* us, const float* __rest
 // per sub-block hands the errors over and orders the two: before `next` touches sub-block c + 1 the other
 // warps have added everything up to c - 1 there.  Every element so takes the errors in increasing column order
 // with one FMA each, as a column-at-a-time recurrence does.
-// What bounds a tile is the chain, 128 steps whatever the number of rows: 4.4 us at 65 cycles per step.  (With
+// What bounds a tile is the chain, 128 steps of 84 cycles whatever the number of rows (5.6 us), and handing the
+// sub-blocks over, 800 to 1100 cycles each (3.7 us).  (With
 // sixteen or eight lanes per row and the row's tile in their registers, the owner of a chunk ran its chain while
 // the others waited, and both the chain and the rest were one serial instruction stream: 19 us for 2048 rows,
 // 36 us for 7168; one row per thread for everything, 30 us.  Now 16.5 and 20 us, and 15.7 instead of 20.3 us
-// with a scale per column; a step of the chain takes 84 cycles, handing a sub-block over 800 to 1100.)
+// with a scale per column.)
 // UNIFORM: the columns of a sub-block lie in one quantization group (group % 16 == 0).
 // INVERSE_FREE (a.Worig given): U is the unit factor Utilde = Uhat^-1 and what is propagated is minus the
 // total change of the column, -(y - w_original), instead of the error against the running value;
@@ -466,7 +467,8 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   const bool uniform = group % SUB == 0;
   // Rows per CTA: the chain costs the same for 1 row and for 64, so a tile of 2048 rows takes 16.5 us on 148 SMs,
   // 17.4 on 74 and 19.0 on 48.  Alone, one CTA per SM; a caller with several layers in flight gives each
-  // few SMs.  Fewer than eight rows per CTA gain nothing.
+  // few SMs: eight streams, ms per layer with R / 148, R / 74, R / 44 and R / 22 rows per CTA (64 at most): 2048 x 7168 2.14, 1.79, 1.69
+  // and 1.65, 7168 x 2048 0.528, 0.470, 0.470 and 0.474, 4096 x 4096 1.10, 0.94, 0.89 and 0.91.  Fewer than eight rows per CTA gain nothing.
   int rows = (int)ceil_div(R, compact ? 44 : 148);
   rows = rows < 8 ? 8 : (rows > MAX_ROWS ? MAX_ROWS : rows);
   const int64_t row_groups = ceil_div(R, rows);
