@@ -4,7 +4,7 @@ raw pointers plus the current CUDA stream.  No arithmetic happens here.
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import Optional, Sequence, Tuple
 
 import ctypes
@@ -181,8 +181,11 @@ def mse_scales(W: Tensor, scale: Tensor, group: int, bits: int, dtype: torch.dty
 
 
 def chol_unit_factor(H: Tensor, precision: Optional[Precision] = None, flags: Optional[Tensor] = None):
-    """In place: damped H -> Utilde = T diag(T)^-1 (unit upper), H = T T^T.  Returns (flags, diag(T))."""
+    """In place: damped H -> Utilde = T diag(T)^-1 (unit upper), H = T T^T.  Returns (flags, diag(T)).
+    Without a precision of the caller's, all four products of the operand pairs are taken."""
     p = _prec(precision)
+    if precision is None and p.split_hinv == 3:
+        p = replace(p, split_hinv=4)   # the factor itself is the result: no sweep averages its error (as in mq_hinv_upper)
     require_cuda(H, "H")
     C = H.shape[0]
     L = lib()

@@ -572,6 +572,18 @@ def test_all_products_where_the_sums_cancel(cuda, C, tokens):
     assert torch.equal(*narrow)
 
 
+@pytest.mark.parametrize("C,tokens", [(520, 88), (1032, 1032)])
+def test_factor_takes_all_products_unless_told(cuda, C, tokens):
+    X = torch.randn(tokens, C, generator=torch.Generator().manual_seed(C))
+    H = X.T @ X / tokens
+    H.diagonal().add_(0.01 * H.diagonal().mean())
+    own, four, three = (H.to(cuda) for _ in range(3))
+    ops.chol_unit_factor(own)
+    ops.chol_unit_factor(four, ops.Precision(split_hinv=4))
+    ops.chol_unit_factor(three, ops.Precision(split_hinv=3))
+    assert torch.equal(own, four) and not torch.equal(own, three)
+
+
 @pytest.mark.parametrize("C", [136, 384, 512])
 def test_narrow_sweep_keeps_whole_operands(cuda, C):
     """One product per column: up to 512 columns an error and an entry of the factor enter an update with all of their 24
