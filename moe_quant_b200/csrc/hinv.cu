@@ -11,9 +11,9 @@
 //
 // Blocked right-looking factorisation with 128-wide panels processed from the last
 // panel to the first:
-//   1. chol_diag_rev_kernel  : the 128x128 diagonal block, one CTA, register tiled;
-//   2. trsm_rows_kernel      : the panel above it, one warp per row, substitution
-//                              against the diagonal block staged in shared memory;
+//   1. the 128x128 diagonal block, one CTA, and
+//   2. the panel above it, substitution against that block: both in one launch (factor_panel_kernel) when the
+//                              layer has the GPU to itself, else chol_diag_rev_kernel and trsm_rows_kernel;
 //   3. GEMMs (GemmDesc)      : trailing update of the upper triangle; on the tensor path in two
 //                              levels (the rest of the panel's 512-column super-panel at once,
 //                              everything in front of the super-panel once per super-panel with
@@ -24,6 +24,7 @@
 // log2(C/128) levels of two batched GEMMs each.
 #include "gemm.cuh"
 #include "engine.cuh"
+#include "mbarrier.cuh"
 #include "profile.cuh"
 
 namespace mq {
@@ -35,77 +36,108 @@ constexpr int SUPER_PANELS = 4;               // panels whose far update is appl
 constexpr int SUPER_NB = SUPER_PANELS * NB;   // 512
 
 // ------------------------------------------------------------------ diagonal block
-// D (nb x nb, upper triangle valid) -> T_d upper with D = T_d T_d^T, one CTA of 512 threads.
-// The block lives in shared memory.  The 128 pivots are taken 8 at a time (a "leaf", columns
-// 8kt..8kt+7, kt = 15 first).  One warp's instruction stream runs at a fraction of an instruction
-// per cycle here (every step depends on the one before), so a leaf is arranged to put as few
-// instructions as possible in any one stream:
-//   a. thread r < 8kt + 8 takes ROW r of the column strip: it factors its own copy of the 8x8
-//      leaf in registers (the same arithmetic in every thread, no communication inside the chain
-//      of 8 pivots) and solves its own row against it; the row's eight results are final: they go
-//      to global memory at once and, transposed, to the panel buffer;
-//   b. every element on or above the diagonal tiles in front of the strip takes its rank-8 update
-//      from the panel buffer.  The region shrinks with every leaf, so its 4x4 micro-tiles are dealt
-//      out to all 512 threads anew each time (with the tiles in registers of fixed owners, four
-//      fifths of the lanes idled through this phase, which the FMA pipe of the one SM bounds).
-constexpr int PAN_LD = NB + 4;
-constexpr int DIAG_THREADS = 512;
-constexpr int DIAG_LD = NB + 4;   // row stride of the block in shared memory (16-byte aligned rows)
-constexpr size_t kDiagSmem = (size_t)NB * DIAG_LD * sizeof(float);
+// D (nb x nb, upper triangle valid) -> T_d upper with D = T_d T_d^T, by one CTA, eight pivots at a time (a "leaf", columns
+// 8kt..8kt+7, the last one first).  What bounds it is the chain of 128 pivots, so everything else is kept out of its way:
+//   chain (2 warps)   : thread t holds rows t and t + 64 of the leaf's column strip in registers.  It factors its own copy of the
+//                       8x8 leaf (the same arithmetic in every thread, no communication inside the chain of 8 pivots) and
+//                       solves its rows against it; their results are final.  Then it brings its rows of the NEXT leaf's
+//                       strip up to date itself and goes on;
+//   helpers (4 warps) : meanwhile take the rank-8 update of the columns in front of the next leaf.  A thread keeps one 8x8
+//                       tile in registers from the load to the end and hands it over when its columns come next.  Tiles are
+//                       dealt out by columns, so whole warps retire;
+//   writer (1 warp)   : takes finished strips to global memory, 32 columns (128-byte rows) at a time.
+// One barrier per leaf orders the first two: chain(kt) runs beside update(kt + 1).  Every element takes its updates in the
+// order of the leaves with one FMA per column.
+// What counts beside the chain is the 128 bytes a cycle at which shared memory answers, broadcasts included: two rows per chain thread and
+// 8x8 tiles halve what is read (with one row and 4x4 tiles a leaf took 1780 cycles).  Now a leaf takes 1300: 460 to 540 for the
+// pivots, 200 to put the strip down, 350 for the next strip, 100 to 240 to exchange the leaf; the block 15.0 us (21.4 with all threads
+// updating the block in shared memory between two barriers per leaf, and no look-ahead).
+constexpr int PAN_HALF = 80;                // rows of a strip column in shared memory: quads of rows 8i.. first, of rows 8i + 4.. from here on,
+constexpr int PAN_LD = PAN_HALF + NB / 2;   // so that neither a row per lane nor eight rows per lane meet bank conflicts
+constexpr int DIAG_LD = NB + 4;             // row stride of the finished block in shared memory
+constexpr int CHAIN_THREADS = NB / 2;
+constexpr int HELP_THREADS = 128;           // 14 * 15 / 2 = 105 tiles in front of the last two leaves
+constexpr int DIAG_THREADS = CHAIN_THREADS + HELP_THREADS + 32;
+constexpr int DIAG_SMEM_FLOATS = NB * DIAG_LD + 4 * 8 * PAN_LD + 64;
+constexpr size_t kDiagSmem = (size_t)DIAG_SMEM_FLOATS * sizeof(float) + (NB / 8) * sizeof(uint64_t);
 
-__global__ void __launch_bounds__(DIAG_THREADS) chol_diag_rev_kernel(float* __restrict__ blk, int64_t ld, int nb,
-                                                                     int k_global, mq_layer_flags* flags) {
-  extern __shared__ __align__(16) float Ms[];         // [NB][DIAG_LD]: the block, tiles on and above the diagonal
-  __shared__ __align__(16) float pan[8][PAN_LD];      // pan[kk][row]: column 8kt+kk of the solved strip
-  chain_wait();
-  chain_release();
-  const int t = threadIdx.x;
-  // A whole, 16-byte aligned block moves as float4; rows and columns past nb read as the identity.
-  const bool vec = nb == NB && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(blk) & 15) == 0;
-  for (int idx = t; idx < NB * NB / 4; idx += DIAG_THREADS) {
-    const int r = idx >> 5, c4 = (idx & 31) * 4;
-    if ((c4 >> 3) < (r >> 3)) continue;               // tiles below the diagonal are never read
-    float4 v;
-    if (vec) {
-      v = *reinterpret_cast<const float4*>(blk + (int64_t)r * ld + c4);
-    } else {
-      float e[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) e[q] = (r < nb && c4 + q < nb) ? blk[(int64_t)r * ld + c4 + q] : (r == c4 + q ? 1.0f : 0.0f);
-      v = make_float4(e[0], e[1], e[2], e[3]);
-    }
-    *reinterpret_cast<float4*>(&Ms[r * DIAG_LD + c4]) = v;
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ int pan_pos(int row) { return ((row >> 2) & 1) * PAN_HALF + (row >> 3) * 4 + (row & 3); }
+
+// The memory of a CTA that factors a block.  Finished leaves stay in T, and ready[leaf] tells whoever takes them on.
+struct DiagShared {
+  float* T;         // [NB][DIAG_LD]: the finished strips
+  float* pan;       // [2][8][PAN_LD]: the strip just solved, by kt & 1
+  float* next;      // [2][8][PAN_LD]: what the helpers hand over, by strip & 1
+  float* leaf;      // [8][8]
+  uint64_t* ready;  // [NB / 8] barriers
+  __device__ __forceinline__ explicit DiagShared(float* smem)
+      : T(smem), pan(T + NB * DIAG_LD), next(pan + 2 * 8 * PAN_LD), leaf(next + 2 * 8 * PAN_LD), ready(reinterpret_cast<uint64_t*>(leaf + 64)) {}
+  __device__ __forceinline__ void init() const {   // one thread, before the CTA's first barrier
+    for (int k = 0; k < NB / 8; ++k) mbar_init(smem_u32(ready + k), CHAIN_THREADS / 32);
   }
-  __syncthreads();
-  for (int kt = 15; kt >= 0; --kt) {
-    // ---- a. one row of the strip per thread
-    const int row = t;
-    if (row < kt * 8 + 8) {
-      float L[8][8];   // L[i][j] = leaf element (row 8kt+i, column 8kt+j), upper triangle
+};
+
+// Called by the first DIAG_THREADS threads of a CTA after DiagShared::init.  diag receives the block's diagonal.
+__device__ __forceinline__ void factor_diag_block(const DiagShared sh, float* __restrict__ blk, int64_t ld, int nb, int k_global,
+                                                  float* __restrict__ diag, mq_layer_flags* flags, int* fault) {
+  const int t = threadIdx.x;
+  const int kt0 = ((nb + 7) >> 3) - 1;                // the last leaf; rows and columns past nb read as the identity
+  // A whole, 16-byte aligned block moves as float4.
+  const bool vec = nb == NB && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(blk) & 15) == 0;
+  auto load4 = [&](int r, int c) {
+    if (vec) return *reinterpret_cast<const float4*>(blk + (int64_t)r * ld + c);
+    float e[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 lo = *reinterpret_cast<const float4*>(&Ms[(kt * 8 + i) * DIAG_LD + kt * 8]);
-        const float4 hi = *reinterpret_cast<const float4*>(&Ms[(kt * 8 + i) * DIAG_LD + kt * 8 + 4]);
-        L[i][0] = lo.x; L[i][1] = lo.y; L[i][2] = lo.z; L[i][3] = lo.w;
+    for (int q = 0; q < 4; ++q) e[q] = (r < nb && c + q < nb) ? blk[(int64_t)r * ld + c + q] : (r == c + q ? 1.0f : 0.0f);
+    return make_float4(e[0], e[1], e[2], e[3]);
+  };
+  if (t < CHAIN_THREADS) {
+    float x[2][8], y[2][8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int row = t + 64 * h;
+        const float4 v = row < 8 * kt0 + 8 ? load4(row, 8 * kt0 + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 u = row < 8 * kt0 ? load4(row, 8 * kt0 - 8 + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[h][4 * q] = v.x; x[h][4 * q + 1] = v.y; x[h][4 * q + 2] = v.z; x[h][4 * q + 3] = v.w;
+        y[h][4 * q] = u.x; y[h][4 * q + 1] = u.y; y[h][4 * q + 2] = u.z; y[h][4 * q + 3] = u.w;
+      }
+    const int p0 = pan_pos(t), p1 = pan_pos(t + 64);
+#pragma unroll 1
+    for (int kt = kt0;; --kt) {
+      const int li = ((t - 8 * kt) & 63) < 8 ? (t & 7) : -1;   // row of the leaf that this thread holds, as its row number lh
+      const int lh = kt >> 3;
+      if (li >= 0) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          *reinterpret_cast<float4*>(sh.leaf + li * 8 + 4 * q) =
+              lh ? make_float4(x[1][4 * q], x[1][4 * q + 1], x[1][4 * q + 2], x[1][4 * q + 3])
+                 : make_float4(x[0][4 * q], x[0][4 * q + 1], x[0][4 * q + 2], x[0][4 * q + 3]);
+      }
+      bar_sync(1, CHAIN_THREADS);
+      float L[8][8];   // L[i][j] = leaf element (row 8kt+i, column 8kt+j), i <= j
+#pragma unroll
+      for (int i = 7; i >= 0; --i) {
+        const float4 hi = *reinterpret_cast<const float4*>(sh.leaf + i * 8 + 4);
         L[i][4] = hi.x; L[i][5] = hi.y; L[i][6] = hi.z; L[i][7] = hi.w;
       }
-      float x[8];
-      {
-        const float4 lo = *reinterpret_cast<const float4*>(&Ms[row * DIAG_LD + kt * 8]);
-        const float4 hi = *reinterpret_cast<const float4*>(&Ms[row * DIAG_LD + kt * 8 + 4]);
-        x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w; x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+#pragma unroll
+      for (int i = 3; i >= 0; --i) {
+        const float4 lo = *reinterpret_cast<const float4*>(sh.leaf + i * 8);
+        L[i][0] = lo.x; L[i][1] = lo.y; L[i][2] = lo.z; L[i][3] = lo.w;
       }
       // The 8 pivots are one straight line of code (no branch), so that the scheduler can put
       // the row arithmetic of pivot kk into the latency of pivot kk-1's rsqrt chain.  The rows
-      // of the leaf itself run the row arithmetic too; that copy is discarded below.
+      // of the leaf itself, and those below it, run the row arithmetic too.  A pivot that is not positive
+      // turns what follows into NaN; it is reported, and the whole factor is replaced.
       int fail = 0;
 #pragma unroll
       for (int kk = 7; kk >= 0; --kk) {
-        float d = L[kk][kk];
-        const bool bad = !(d > 0.0f);  // also catches NaN
-        fail = (bad && fail == 0) ? kk + 1 : fail;
-        d = bad ? 1.0f : d;
-        float r;                       // d is a positive, normal pivot (or 1): the hardware approximation, refined below
+        const float d = L[kk][kk];
+        fail = (!(d > 0.0f) && fail == 0) ? kk + 1 : fail;   // also catches NaN
+        float r;                       // d is a positive, normal pivot: the hardware approximation, refined below
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
         r = r * fmaf(-0.5f * d * r, r, 1.5f);  // one Newton step: r = 1/sqrt(d) to about 1 ulp
         L[kk][kk] = d * r;
@@ -117,87 +149,165 @@ __global__ void __launch_bounds__(DIAG_THREADS) chol_diag_rev_kernel(float* __re
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             if (i <= j && j < kk) L[i][j] = fmaf(-L[i][kk], L[j][kk], L[i][j]);
-        // this row above the leaf: p_kk = x_kk / T[kk][kk]; x_j -= p_kk T[j][kk]  (j < kk)
-        const float pv = x[kk] * r;
-        x[kk] = pv;
+        // these rows above the leaf: p_kk = x_kk / T[kk][kk]; x_j -= p_kk T[j][kk]  (j < kk)
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (j < kk) x[j] = fmaf(-pv, L[j][kk], x[j]);
-      }
-      const int li = row - kt * 8;   // >= 0: a row of the leaf, which gets the factor instead
-      if (li >= 0) {
-        if (li == 0 && fail != 0 && kt * 8 + fail - 1 < nb) atomicCAS(&flags->not_positive, 0, k_global + kt * 8 + fail);
+        for (int h = 0; h < 2; ++h) {
+          const float pv = x[h][kk] * r;
+          x[h][kk] = pv;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          float v = 0.0f;
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (i == li && i <= kk) v = L[i][kk];
-          x[kk] = v;
+          for (int j = 0; j < 8; ++j)
+            if (j < kk) x[h][j] = fmaf(-pv, L[j][kk], x[h][j]);
         }
       }
+      if (t == 0 && fail != 0 && kt * 8 + fail - 1 < nb) atomicCAS(&flags->not_positive, 0, k_global + kt * 8 + fail);
+      // A row of the leaf has gone through the same operations as its copy in L: it is the factor from its diagonal on.
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) pan[kk][row] = x[kk];
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int kk = 0; kk < 7; ++kk)
+          if (t + 64 * h > 8 * kt + kk) x[h][kk] = 0.0f;
+      float* pb = sh.pan + (kt & 1) * 8 * PAN_LD;
+      const bool in0 = t < 8 * kt + 8, in1 = t + 64 < 8 * kt + 8;
+      if (in0) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) pb[kk * PAN_LD + p0] = x[0][kk];
+      }
+      if (in1) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) pb[kk * PAN_LD + p1] = x[1][kk];
+      }
+      if (kt > 0) bar_sync(2, CHAIN_THREADS + HELP_THREADS);
       // the strip is final
-      if (vec) {
-        *reinterpret_cast<float4*>(blk + (int64_t)row * ld + kt * 8) = make_float4(x[0], x[1], x[2], x[3]);
-        *reinterpret_cast<float4*>(blk + (int64_t)row * ld + kt * 8 + 4) = make_float4(x[4], x[5], x[6], x[7]);
-      } else if (row < nb) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          if (kt * 8 + kk < nb) blk[(int64_t)row * ld + kt * 8 + kk] = x[kk];
-      }
-    } else if (row < NB) {
-      // below the leaf: zeros
-      if (vec) {
-        *reinterpret_cast<float4*>(blk + (int64_t)row * ld + kt * 8) = make_float4(0.f, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(blk + (int64_t)row * ld + kt * 8 + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-      } else if (row < nb) {
+      for (int h = 0; h < 2; ++h)
+        if (h ? in1 : in0) {
+          float* dst = sh.T + (t + 64 * h) * DIAG_LD + 8 * kt;
+          *reinterpret_cast<float4*>(dst) = make_float4(x[h][0], x[h][1], x[h][2], x[h][3]);
+          *reinterpret_cast<float4*>(dst + 4) = make_float4(x[h][4], x[h][5], x[h][6], x[h][7]);
+        }
+      __syncwarp();
+      if ((t & 31) == 0) mbar_arrive(smem_u32(sh.ready + kt));
+      if (kt == 0) break;
+      // the next strip: what the helpers have done to it, then this leaf
+      if (kt < kt0) {
+        const float* nx = sh.next + ((kt - 1) & 1) * 8 * PAN_LD;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          if (kt * 8 + kk < nb) blk[(int64_t)row * ld + kt * 8 + kk] = 0.0f;
+        for (int j = 0; j < 8; ++j) {
+          y[0][j] = nx[j * PAN_LD + p0];
+          y[1][j] = nx[j * PAN_LD + p1];
+        }
       }
-    }
-    __syncthreads();
-    // ---- b. rank-8 update of what lies in front of the strip: rows and columns below 8kt, 4x4
-    // micro-tiles on and above the diagonal 8x8 tiles.  n micro-rows (even); rows i and n-1-i
-    // together hold n + 1 micro-tiles on or right of the diagonal, which makes the triangle a
-    // rectangle of n/2 x (n + 1) items.  (A micro-tile left of the diagonal micro-tile of its
-    // row but inside a diagonal 8x8 tile is never read: it is skipped with the rest.)
-    const int n = 2 * kt;
-    const int items = (n >> 1) * (n + 1);
-    for (int m = t; m < items; m += DIAG_THREADS) {
-      const int i = m / (n + 1), jj = m - i * (n + 1);
-      int mi, mj;
-      if (jj < n - i) { mi = i; mj = i + jj; }
-      else { mi = n - 1 - i; mj = mi + (jj - (n - i)); }
-      const int r0 = 4 * mi, c0 = 4 * mj;
-      float c[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const float4 v = *reinterpret_cast<const float4*>(&Ms[(r0 + a) * DIAG_LD + c0]);
-        c[a][0] = v.x; c[a][1] = v.y; c[a][2] = v.z; c[a][3] = v.w;
-      }
+      const int pn = pan_pos(8 * kt - 8);   // rows 8kt-8.. of the strip: the next leaf's columns
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
-        const float4 pi4 = *reinterpret_cast<const float4*>(&pan[kk][r0]);
-        const float4 pj4 = *reinterpret_cast<const float4*>(&pan[kk][c0]);
-        const float pi[4] = {pi4.x, pi4.y, pi4.z, pi4.w};
-        // two columns per instruction (packed fp32 FMA: each half is an ordinary fma.rn)
+        const float4 lo = *reinterpret_cast<const float4*>(&pb[kk * PAN_LD + pn]);
+        const float4 hi = *reinterpret_cast<const float4*>(&pb[kk * PAN_LD + pn + PAN_HALF]);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const float2 npi = make_float2(-pi[a], -pi[a]);
-          const float2 q01 = __ffma2_rn(npi, make_float2(pj4.x, pj4.y), make_float2(c[a][0], c[a][1]));
-          const float2 q23 = __ffma2_rn(npi, make_float2(pj4.z, pj4.w), make_float2(c[a][2], c[a][3]));
-          c[a][0] = q01.x; c[a][1] = q01.y; c[a][2] = q23.x; c[a][3] = q23.y;
+        for (int h = 0; h < 2; ++h) {
+          const float2 n = make_float2(-x[h][kk], -x[h][kk]);
+          // two columns per instruction (packed fp32 FMA: each half is an ordinary fma.rn)
+          const float2 q0 = __ffma2_rn(n, make_float2(lo.x, lo.y), make_float2(y[h][0], y[h][1]));
+          const float2 q1 = __ffma2_rn(n, make_float2(lo.z, lo.w), make_float2(y[h][2], y[h][3]));
+          const float2 q2 = __ffma2_rn(n, make_float2(hi.x, hi.y), make_float2(y[h][4], y[h][5]));
+          const float2 q3 = __ffma2_rn(n, make_float2(hi.z, hi.w), make_float2(y[h][6], y[h][7]));
+          y[h][0] = q0.x; y[h][1] = q0.y; y[h][2] = q1.x; y[h][3] = q1.y;
+          y[h][4] = q2.x; y[h][5] = q2.y; y[h][6] = q3.x; y[h][7] = q3.y;
         }
       }
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
-        *reinterpret_cast<float4*>(&Ms[(r0 + a) * DIAG_LD + c0]) = make_float4(c[a][0], c[a][1], c[a][2], c[a][3]);
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) x[h][kk] = y[h][kk];
     }
-    __syncthreads();
+    // the diagonal (T is complete; its rows are other threads')
+    bar_sync(1, CHAIN_THREADS);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (t + 64 * h < nb) diag[t + 64 * h] = sh.T[(t + 64 * h) * (DIAG_LD + 1)];
+  } else if (t < CHAIN_THREADS + HELP_THREADS) {
+    // tile (mi, mj), mi <= mj, in the order of the columns
+    const int id = t - CHAIN_THREADS;
+    int mj = (int)((sqrtf(8.0f * id + 1.0f) - 1.0f) * 0.5f);
+    if ((mj + 1) * (mj + 2) / 2 <= id) ++mj;
+    if (mj * (mj + 1) / 2 > id) --mj;
+    const int mi = id - mj * (mj + 1) / 2;
+    const bool mine = mj < kt0 - 1;     // the last two strips belong to the chain from the start
+    float c[8][8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const float4 v = mine ? load4(8 * mi + a, 8 * mj + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        c[a][4 * q] = v.x; c[a][4 * q + 1] = v.y; c[a][4 * q + 2] = v.z; c[a][4 * q + 3] = v.w;
+      }
+#pragma unroll 1
+    for (int kt = kt0; kt > 0; --kt) {
+      bar_sync(2, CHAIN_THREADS + HELP_THREADS);
+      if (!mine || mj >= kt - 1) continue;          // columns in front of the next strip
+      const float* pb = sh.pan + (kt & 1) * 8 * PAN_LD;
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        const float4 i0 = *reinterpret_cast<const float4*>(pb + kk * PAN_LD + 4 * mi);
+        const float4 i1 = *reinterpret_cast<const float4*>(pb + kk * PAN_LD + PAN_HALF + 4 * mi);
+        const float4 j0 = *reinterpret_cast<const float4*>(pb + kk * PAN_LD + 4 * mj);
+        const float4 j1 = *reinterpret_cast<const float4*>(pb + kk * PAN_LD + PAN_HALF + 4 * mj);
+        const float pi[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
+        const float2 pj[4] = {make_float2(j0.x, j0.y), make_float2(j0.z, j0.w), make_float2(j1.x, j1.y), make_float2(j1.z, j1.w)};
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+          const float2 n = make_float2(-pi[a], -pi[a]);
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const float2 q = __ffma2_rn(n, pj[b], make_float2(c[a][2 * b], c[a][2 * b + 1]));
+            c[a][2 * b] = q.x; c[a][2 * b + 1] = q.y;
+          }
+        }
+      }
+      if (mj == kt - 2) {
+        float* nx = sh.next + (mj & 1) * 8 * PAN_LD;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          *reinterpret_cast<float4*>(nx + j * PAN_LD + 4 * mi) = make_float4(c[0][j], c[1][j], c[2][j], c[3][j]);
+          *reinterpret_cast<float4*>(nx + j * PAN_LD + PAN_HALF + 4 * mi) = make_float4(c[4][j], c[5][j], c[6][j], c[7][j]);
+        }
+      }
+    }
+  } else {
+    // finished columns, 32 at a time: eight lanes a row
+    const int lane = t & 31;
+    for (int kt = kt0; kt >= 0; --kt) {
+      if (!mbar_wait(smem_u32(sh.ready + kt), 0, fault, 63)) return;
+      if (kt & 3) continue;
+      const int c = 8 * kt + (lane & 7) * 4;
+      if (c >= nb) continue;
+      for (int r = lane >> 3; r < nb; r += 4) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);      // below the diagonal tiles
+        if ((r >> 3) <= (c >> 3)) v = *reinterpret_cast<const float4*>(sh.T + r * DIAG_LD + c);
+        if (vec) {
+          *reinterpret_cast<float4*>(blk + (int64_t)r * ld + c) = v;
+        } else {
+          const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (c + q < nb) blk[(int64_t)r * ld + c + q] = e[q];
+        }
+      }
+    }
   }
+}
+
+__global__ void __launch_bounds__(DIAG_THREADS, 1) chol_diag_rev_kernel(float* __restrict__ blk, int64_t ld, int nb, int k_global,
+                                                                     float* __restrict__ diag, mq_layer_flags* flags, int* fault) {
+  extern __shared__ __align__(16) float smem[];
+  const DiagShared sh(smem);
+  if (threadIdx.x == 0) {
+    sh.init();
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  chain_wait();
+  chain_release();
+  factor_diag_block(sh, blk, ld, nb, k_global, diag, flags, fault);
 }
 
 // ------------------------------------------------------------------ substitution
@@ -208,6 +318,31 @@ __global__ void __launch_bounds__(DIAG_THREADS) chol_diag_rev_kernel(float* __re
 // IDENTITY: the right-hand side is I and the result is stored transposed, which
 // yields T^-1 (upper triangular) in `rows`.
 constexpr int TT_LD = NB + 4;
+
+// a / d through the reciprocal and one correction step (the last stage of a correctly rounded division)
+__device__ __forceinline__ float quotient(float a, float d, float rd) {
+  const float q = a * rd;
+  return fmaf(fmaf(-d, q, a), rd, q);
+}
+
+// Four neighbouring entries of a solved row as operand planes: a pair of fp16 planes (the equilibrated factor's entries lie
+// below 2^14) or up to three bf16 planes.
+__device__ __forceinline__ void store_planes(const float (&a)[4], uint16_t* dst, int64_t plane_stride, int n_planes, int half) {
+  uint16_t p0[4], p1[4], p2[4];
+  if (half) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) split_half2(a[q], p0[q], p1[q]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) split_bf16x3(a[q], p0[q], p1[q], p2[q]);
+  }
+  auto put = [&](uint16_t* to, const uint16_t (&v)[4]) {
+    *reinterpret_cast<uint2*>(to) = make_uint2((uint32_t)v[0] | ((uint32_t)v[1] << 16), (uint32_t)v[2] | ((uint32_t)v[3] << 16));
+  };
+  put(dst, p0);
+  if (half || n_planes > 1) put(dst + plane_stride, p1);
+  if (!half && n_planes > 2) put(dst + 2 * plane_stride, p2);
+}
 
 template <bool IDENTITY>
 __global__ void __launch_bounds__(256) trsm_rows_kernel(const float* __restrict__ tblk, int64_t ldt, int64_t t_bs,
@@ -326,12 +461,7 @@ __global__ void __launch_bounds__(256) trsm_rows_kernel(const float* __restrict_
 #pragma unroll
       for (int h = 0; h < ROWS; ++h)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          // a / d through the reciprocal and one correction step (the last stage of a correctly
-          // rounded division)
-          float pq = a[h][q] * rr[q];
-          a[h][q] = fmaf(fmaf(-dd[q], pq, a[h][q]), rr[q], pq);
-        }
+        for (int q = 0; q < 4; ++q) a[h][q] = quotient(a[h][q], dd[q], rr[q]);
     }
     if (lane * 4 < nb) {
 #pragma unroll
@@ -347,49 +477,213 @@ __global__ void __launch_bounds__(256) trsm_rows_kernel(const float* __restrict_
         }
       }
     }
-    if (!IDENTITY && planes && half) {
-      // the same as a pair of fp16 planes: the equilibrated factor's entries lie below 2^14
+    if (!IDENTITY && planes) {
+      // the updates read this panel as operand planes (row, k = column inside the panel)
 #pragma unroll
       for (int h = 0; h < ROWS; ++h) {
         const int r = r0 + h;
         if (r >= nrows) continue;
-        uint16_t hi[4], lo[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) split_half2(lane * 4 < nb ? a[h][q] : 0.0f, hi[q], lo[q]);
-        uint16_t* dst = planes + (int64_t)r * plane_ld + lane * 4;
-        *reinterpret_cast<uint2*>(dst) = make_uint2((uint32_t)hi[0] | ((uint32_t)hi[1] << 16), (uint32_t)hi[2] | ((uint32_t)hi[3] << 16));
-        *reinterpret_cast<uint2*>(dst + plane_stride) =
-            make_uint2((uint32_t)lo[0] | ((uint32_t)lo[1] << 16), (uint32_t)lo[2] | ((uint32_t)lo[3] << 16));
-      }
-    } else if (!IDENTITY && planes) {
-      // the trailing update reads this panel as bf16 planes (row, k = column inside the panel)
-#pragma unroll
-      for (int h = 0; h < ROWS; ++h) {
-        const int r = r0 + h;
-        if (r >= nrows) continue;
-        uint16_t hi[4], mi[4], lo[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) split_bf16x3(lane * 4 < nb ? a[h][q] : 0.0f, hi[q], mi[q], lo[q]);
-        uint16_t* dst = planes + (int64_t)r * plane_ld + lane * 4;   // `planes` already points at this panel's k window
-        *reinterpret_cast<uint2*>(dst) = make_uint2((uint32_t)hi[0] | ((uint32_t)hi[1] << 16), (uint32_t)hi[2] | ((uint32_t)hi[3] << 16));
-        if (n_planes > 1)
-          *reinterpret_cast<uint2*>(dst + plane_stride) =
-              make_uint2((uint32_t)mi[0] | ((uint32_t)mi[1] << 16), (uint32_t)mi[2] | ((uint32_t)mi[3] << 16));
-        if (n_planes > 2)
-          *reinterpret_cast<uint2*>(dst + 2 * plane_stride) =
-              make_uint2((uint32_t)lo[0] | ((uint32_t)lo[1] << 16), (uint32_t)lo[2] | ((uint32_t)lo[3] << 16));
+        if (lane * 4 >= nb) a[h][0] = a[h][1] = a[h][2] = a[h][3] = 0.0f;
+        store_planes(a[h], planes + (int64_t)r * plane_ld + lane * 4, plane_stride, n_planes, half);   // `planes` points at this panel's k window
       }
     }
   }
 }
 
-// ------------------------------------------------------------------ small passes
-__global__ void __launch_bounds__(256) extract_diag_kernel(const float* __restrict__ H, int64_t C, int64_t ld,
-                                                           float* __restrict__ diag) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < C) diag[i] = H[i * ld + i];
+// ------------------------------------------------------------------ one panel in one launch
+// The diagonal block and the solve of the rows above it, for a caller whose layer has the GPU to itself.  The block is a chain
+// on one SM, and the solve takes its columns in the order in which the block produces them, the last ones first: so one CTA
+// factors the block and passes every strip of eight columns on as it becomes final, and the others follow it strip by strip,
+// each with its rows in registers (a warp has RPW rows, a lane four columns of them).  When the block is done the solve is one strip
+// behind it.
+// Which CTA factors is settled by a ticket, so that it is one that runs: the others wait for it, it waits for nobody.  Waits are bounded.
+// The arithmetic is that of trsm_rows_kernel, column by column: a_j -= a_k (T[j,k] / T[k,k]), the quotients at the end.
+// A panel takes 21 us with 32 rows per CTA, 25.7 with 64 (4705 rows and more), where the two launches took 15 + 12.9 and the gap between
+// them: 2048 x 7168 4242 -> 3693 us, 7168 x 2048 1154 -> 1025.  One warp that fetches the strips is not enough (46 us a panel: a strip is under way
+// for 2 to 3 us, poll and load, and a new one is there every 0.7).  With several layers in flight the solving CTAs would hold
+// their SMs while they wait, so compact launches keep the two kernels.
+constexpr int PANEL_WARPS = 8;                             // of a solving CTA
+constexpr int FETCH_WARPS = 4;                             // the strips' way takes longer than the next strip: several fetch, by turns
+constexpr int PANEL_THREADS = (PANEL_WARPS + FETCH_WARPS) * 32;
+constexpr int STRIP_WORDS = (NB / 8) * NB * 8;             // one block on its way: [leaf][column pair][row][column]
+constexpr size_t kPanelSmem = 120 * 1024;                  // more than half of an SM: the block's CTA shares its SM with none
+static_assert(PANEL_THREADS >= DIAG_THREADS + 32, "the block's CTA has a warp to spare that passes the strips on");
+static_assert(kPanelSmem >= kDiagSmem && kPanelSmem >= (size_t)(NB * (NB + 4) + 2 * NB) * sizeof(float), "either role fits");
+
+struct PanelArgs {
+  float* blk;          // the diagonal block
+  float* rows;         // the rows above it (nrows x nb)
+  int64_t ld;
+  int nb, nrows, k_global;
+  float* diag;         // of the block
+  mq_layer_flags* flags;
+  uint16_t* planes;    // the result as operand planes (this panel's k window)
+  int64_t plane_stride;
+  int n_planes, plane_ld, half;
+  int* ticket;         // zero before the launch
+  uint64_t* strips;    // STRIP_WORDS; no word carries `tag` before the launch
+  uint32_t tag;
+  int* fault;
+};
+
+// Strips of the block on their way to other CTAs: 64-bit words of value and tag, each written and read whole, so that a word whose
+// tag is right carries its value with it and neither side needs a fence.
+__device__ __forceinline__ void store_tagged(uint64_t* dst, float a, float b, uint32_t tag) {
+  const uint64_t t = (uint64_t)tag << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(dst), "l"(t | __float_as_uint(a)), "l"(t | __float_as_uint(b)) : "memory");
+}
+__device__ __forceinline__ void load_tagged(const uint64_t* src, uint64_t& a, uint64_t& b) {
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(src) : "memory");
+}
+// columns 8 kt + 2 q and the next of a row
+__device__ __forceinline__ uint64_t* strip_words(uint64_t* strips, int kt, int q, int row) { return strips + ((int64_t)(kt * 4 + q) * NB + row) * 2; }
+
+// one warp of the block's CTA
+__device__ __forceinline__ void publish_strips(const DiagShared sh, const PanelArgs& p, int lane) {
+  for (int kt = ((p.nb + 7) >> 3) - 1; kt >= 0; --kt) {
+    if (!mbar_wait(smem_u32(sh.ready + kt), 0, p.fault, 64)) return;
+    for (int row = lane; row < 8 * kt + 8; row += 32) {
+      const float4 lo = *reinterpret_cast<const float4*>(sh.T + row * DIAG_LD + 8 * kt), hi = *reinterpret_cast<const float4*>(sh.T + row * DIAG_LD + 8 * kt + 4);
+      store_tagged(strip_words(p.strips, kt, 0, row), lo.x, lo.y, p.tag);
+      store_tagged(strip_words(p.strips, kt, 1, row), lo.z, lo.w, p.tag);
+      store_tagged(strip_words(p.strips, kt, 2, row), hi.x, hi.y, p.tag);
+      store_tagged(strip_words(p.strips, kt, 3, row), hi.z, hi.w, p.tag);
+    }
+  }
 }
 
+// One of the warps of a solving CTA that bring strips from global memory to TT, dg and rdg; full[kt] says that strip kt is there.
+__device__ __forceinline__ void fetch_strips(const PanelArgs& p, float* TT, float* dg, float* rdg, uint32_t full0, int which, int lane) {
+#pragma unroll 1
+  for (int kt = ((p.nb + 7) >> 3) - 1 - which; kt >= 0; kt -= FETCH_WARPS) {
+    uint64_t v[4][8];
+    WaitLimit limit;
+    const uint64_t none = (uint64_t)p.tag << 32;
+    for (uint32_t it = 0;; ++it) {
+      // one word (of those passed on last) until it is there, then all of them
+      uint64_t a = none, b = none;
+      if (lane == 0) load_tagged(strip_words(p.strips, kt, 3, 8 * kt + 7), a, b);
+      bool ok = __shfl_sync(0xffffffffu, (uint32_t)(a >> 32), 0) == p.tag;
+      if (ok) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            v[i][2 * q] = v[i][2 * q + 1] = none;
+            if (lane + 32 * i < 8 * kt + 8) load_tagged(strip_words(p.strips, kt, q, lane + 32 * i), v[i][2 * q], v[i][2 * q + 1]);
+          }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) ok = ok && (uint32_t)(v[i][q] >> 32) == p.tag;
+        if (__all_sync(0xffffffffu, ok)) break;
+      }
+      int gone = 0;
+      if ((it & 255u) == 255u && lane == 0) gone = limit.expired(p.fault, 61);
+      if (__shfl_sync(0xffffffffu, gone, 0)) return;   // the solving warps give up by themselves
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int kk = lane + 32 * i - 8 * kt;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q == kk) {
+          const float d = __uint_as_float((uint32_t)v[i][q]);
+          dg[8 * kt + kk] = d;
+          rdg[8 * kt + kk] = 1.0f / d;
+        }
+    }
+    __syncwarp();
+    const float4 r0 = *reinterpret_cast<const float4*>(rdg + 8 * kt), r1 = *reinterpret_cast<const float4*>(rdg + 8 * kt + 4);
+    const float rd[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = lane + 32 * i;
+      if (row >= 8 * kt + 8) continue;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) TT[(8 * kt + q) * TT_LD + row] = row < 8 * kt + q ? __uint_as_float((uint32_t)v[i][q]) * rd[q] : 0.0f;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(full0 + 8 * kt);
+  }
+}
+
+template <int RPW>
+__global__ void __launch_bounds__(PANEL_THREADS, 1) factor_panel_kernel(const PanelArgs p) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ __align__(8) uint64_t full[NB / 8];
+  __shared__ int role;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const DiagShared sh(smem);
+  if (t == 0) {
+    role = atomicAdd(p.ticket, 1);
+    for (int k = 0; k < NB / 8; ++k) mbar_init(smem_u32(&full[k]), 1);
+    sh.init();
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  chain_wait();
+  chain_release();
+  if (role == 0) {
+    if (t < DIAG_THREADS) factor_diag_block(sh, p.blk, p.ld, p.nb, p.k_global, p.diag, p.flags, p.fault);
+    else if (warp == DIAG_THREADS / 32) publish_strips(sh, p, lane);
+    return;
+  }
+  float* TT = smem;                // [NB][TT_LD], TT[k][j] = T[j][k] / T[k][k] for j < k, else 0 (up to the end of k's leaf)
+  float* dg = smem + NB * TT_LD;   // [NB] diagonal of T
+  float* rdg = dg + NB;            // [NB] its reciprocal
+  if (warp >= PANEL_WARPS) {
+    fetch_strips(p, TT, dg, rdg, smem_u32(&full[0]), warp - PANEL_WARPS, lane);
+    return;
+  }
+  const int kt0 = ((p.nb + 7) >> 3) - 1;
+  // ---- the rows
+  const int groups = (int)gridDim.x - 1;
+  for (int r0 = ((role - 1) * PANEL_WARPS + warp) * RPW; r0 < p.nrows; r0 += groups * PANEL_WARPS * RPW) {
+    float a[RPW][4];
+#pragma unroll
+    for (int h = 0; h < RPW; ++h) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r0 + h < p.nrows && lane * 4 < p.nb) v = *reinterpret_cast<const float4*>(p.rows + (int64_t)(r0 + h) * p.ld + lane * 4);
+      a[h][0] = v.x; a[h][1] = v.y; a[h][2] = v.z; a[h][3] = v.w;
+    }
+#pragma unroll 1
+    for (int kt = kt0; kt >= 0; --kt) {
+      if (!mbar_wait(smem_u32(&full[kt]), 0, p.fault, 62)) return;
+#pragma unroll
+      for (int kk = 7; kk >= 0; --kk) {
+        float4 tt = make_float4(0.f, 0.f, 0.f, 0.f);     // columns behind the leaf are done
+        if (lane < 2 * kt + 2) tt = *reinterpret_cast<const float4*>(&TT[(8 * kt + kk) * TT_LD + lane * 4]);
+#pragma unroll
+        for (int h = 0; h < RPW; ++h) {
+          const float ak = __shfl_sync(0xffffffffu, a[h][kk & 3], 2 * kt + (kk >> 2));
+          // packed fp32 FMA: two columns per instruction, each half an ordinary fma.rn
+          const float2 nak = make_float2(-ak, -ak);
+          const float2 lo = __ffma2_rn(nak, make_float2(tt.x, tt.y), make_float2(a[h][0], a[h][1]));
+          const float2 hi = __ffma2_rn(nak, make_float2(tt.z, tt.w), make_float2(a[h][2], a[h][3]));
+          a[h][0] = lo.x; a[h][1] = lo.y; a[h][2] = hi.x; a[h][3] = hi.y;
+        }
+      }
+    }
+    const bool in = lane * 4 < p.nb;
+    float4 d4 = make_float4(1.f, 1.f, 1.f, 1.f), r4 = d4;
+    if (in) {
+      d4 = *reinterpret_cast<const float4*>(&dg[lane * 4]);
+      r4 = *reinterpret_cast<const float4*>(&rdg[lane * 4]);
+    }
+    const float dd[4] = {d4.x, d4.y, d4.z, d4.w}, rr[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+    for (int h = 0; h < RPW; ++h) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[h][q] = quotient(a[h][q], dd[q], rr[q]);
+      if (r0 + h >= p.nrows) continue;
+      if (in) *reinterpret_cast<float4*>(p.rows + (int64_t)(r0 + h) * p.ld + lane * 4) = make_float4(a[h][0], a[h][1], a[h][2], a[h][3]);
+      store_planes(a[h], p.planes + (int64_t)(r0 + h) * p.plane_ld + lane * 4, p.plane_stride, p.n_planes, p.half);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ small passes
 // T -> T diag(T)^-1 on the upper triangle (unit diagonal), zeros below it.
 // upper_only: what lies entirely below the diagonal is left as it is instead of being zeroed
 // (the layer path never reads it).
@@ -415,18 +709,15 @@ __device__ __forceinline__ void scale_quad(float* __restrict__ H, int64_t ld, co
   *reinterpret_cast<float4*>(H + r * ld + c) = o;
 }
 
-// The end of an unscaled factorisation, one CTA per diagonal 128-block: diag(T) to `diag`, the block divided by it
+// The end of an unscaled factorisation, one CTA per diagonal 128-block: the block divided by diag(T)
 // (the sweep tiles read the diagonal blocks; the blocks above are divided by whoever splits them into planes).
-__global__ void __launch_bounds__(1024) finish_diag_blocks_kernel(float* __restrict__ H, int64_t C, int64_t ld, float* __restrict__ diag,
-                                                                 const float* __restrict__ eq) {
+__global__ void __launch_bounds__(1024) finish_diag_blocks_kernel(float* __restrict__ H, int64_t C, int64_t ld,
+                                                                 const float* __restrict__ diag, const float* __restrict__ eq) {
   __shared__ __align__(16) float d[NB];
   const int64_t k0 = (int64_t)blockIdx.x * NB;
   const int nb = C - k0 < NB ? (int)(C - k0) : NB;
   const int t = threadIdx.x;
-  if (t < nb) {
-    d[t] = H[(k0 + t) * ld + k0 + t];
-    diag[k0 + t] = d[t];
-  }
+  if (t < nb) d[t] = diag[k0 + t];
   __syncthreads();
   for (int idx = t; idx < nb * (NB / 4); idx += blockDim.x) {
     const int r = idx >> 5, c = (idx & 31) * 4;
@@ -504,6 +795,9 @@ int configure_once() {
   MQ_CUDA(cudaGetDevice(&dev));
   if (!done[dev & 63]) {
     MQ_CUDA(cudaFuncSetAttribute(chol_diag_rev_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem));
+    MQ_CUDA(cudaFuncSetAttribute(factor_panel_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem));
+    MQ_CUDA(cudaFuncSetAttribute(factor_panel_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem));
+    MQ_CUDA(cudaFuncSetAttribute(factor_panel_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem));
     MQ_CUDA(cudaFuncSetAttribute(trsm_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
     MQ_CUDA(cudaFuncSetAttribute(trsm_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
     done[dev & 63] = true;
@@ -513,8 +807,39 @@ int configure_once() {
 
 }  // namespace
 
+// what the CTAs of factor_panel_kernel tell one another: the strips of the block in flight, a ticket per panel
+static size_t panel_sync_bytes(int64_t C) {
+  return align_up(STRIP_WORDS * sizeof(uint64_t) + (size_t)ceil_div(C, NB) * sizeof(int), 256);
+}
+
 size_t factor_workspace_bytes(int64_t C, int math, int split) {
-  return math == MQ_MATH_TENSOR ? plane_set_bytes(C, SUPER_NB, plane_count(split)) + align_up((size_t)(C + 1) * sizeof(float), 256) : 0;
+  if (math != MQ_MATH_TENSOR) return 0;
+  return plane_set_bytes(C, SUPER_NB, plane_count(split)) + align_up((size_t)(C + 1) * sizeof(float), 256) + panel_sync_bytes(C);
+}
+
+// One panel: the block and the rows above it (factor_panel_kernel).  Eight warps of RPW rows a CTA, one CTA per SM at most.
+static int launch_panel(bool chained, const PanelArgs& a, cudaStream_t st) {
+  auto launch = [&](auto* kernel, int rpw) {
+    const int64_t groups = ceil_div(a.nrows, PANEL_WARPS * rpw);
+    const unsigned grid = 1 + (unsigned)(groups < 147 ? groups : 147);
+    return launch_chained(chained, kernel, dim3(grid), dim3(PANEL_THREADS), kPanelSmem, st, a);
+  };
+  if (a.nrows <= 147 * PANEL_WARPS * 4) MQ_CUDA(launch(factor_panel_kernel<4>, 4));
+  else if (a.nrows <= 147 * PANEL_WARPS * 8) MQ_CUDA(launch(factor_panel_kernel<8>, 8));
+  else MQ_CUDA(launch(factor_panel_kernel<16>, 16));
+  return MQ_OK;
+}
+
+static int launch_solve(const float* dblk, int64_t ldh, float* rows, int nrows, int nb, uint16_t* planes, int64_t plane_stride, int split,
+                        bool half, bool compact, cudaStream_t st) {
+  // 32 rows per CTA (one group of four rows per warp); compact launches: 64 rows, half the CTAs
+  // and half the copies of the diagonal block (462 against 454-459 layers/s on eight streams)
+  const int grid = compact ? (int)ceil_div(nrows, 64) : (int)(ceil_div(nrows, 32) < 148 * 2 ? ceil_div(nrows, 32) : 148 * 2);
+  ProfScope prof(PROF_TRSM, (double)nrows * nb * nb, 0.0, st);
+  MQ_CUDA(launch_chained(true, trsm_rows_kernel<false>, dim3(grid, 1), dim3(256), kTrsmSmem, st, dblk, ldh, (int64_t)0, rows, ldh, (int64_t)0,
+                         nrows, nb, 0, planes, plane_stride, split, SUPER_NB, half ? 1 : 0));
+  MQ_LAUNCH_CHECK();
+  return MQ_OK;
 }
 
 static int equilibration(const float* H, int64_t C, int64_t ldh, float* eq, cudaStream_t st) {
@@ -566,7 +891,6 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
     MQ_TRY(copy_upper_scaled(H, ldh, H, ldh, C, own, st));
     eq = own;
   }
-  Engine eng(math, split, local, st);
   const int P = (int)ceil_div(C, NB);
   // Tensor path: the panel solve writes its result as planes too, and the rank-128 update
   // P P^T reads one plane set as both operands.
@@ -582,13 +906,24 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
     // plane set as both operands.
     PlaneSet pset;
     if (tensor) {
-      Workspace mine = eng.ws;
       const int planes = half ? 2 : split;
-      pset.base = mine.take<uint16_t>(plane_set_bytes(C, SUPER_NB, planes) / 2);
+      pset.base = local.take<uint16_t>(plane_set_bytes(C, SUPER_NB, planes) / 2);
       MQ_REQUIRE(pset.base, MQ_ERR_WORKSPACE, "factorisation: workspace too small for the panel planes");
       pset.planes = planes; pset.rows_pad = (int)pad_rows(C); pset.total_rows = pset.rows_pad; pset.K_pad = SUPER_NB;
       pset.fp16 = half;
     }
+    // A caller with several layers in flight gives each few SMs, and the solving CTAs would hold theirs while they wait.
+    const bool together = tensor && !compact && P > 1;
+    uint64_t* strips = nullptr;
+    int *tickets = nullptr, *fault = nullptr;
+    MQ_TRY(engine_fault_word(&fault));
+    if (together) {
+      strips = local.take<uint64_t>(panel_sync_bytes(C) / sizeof(uint64_t));
+      MQ_REQUIRE(strips, MQ_ERR_WORKSPACE, "factorisation: workspace too small for the panels' strips");
+      tickets = reinterpret_cast<int*>(strips + STRIP_WORDS);
+      MQ_CUDA(cudaMemsetAsync(strips, 0, panel_sync_bytes(C), st));
+    }
+    Engine eng(math, split, local, st);   // fp32 math
     for (int p = P - 1; p >= 0; --p) {
       const int p_lo = (p / SUPER_PANELS) * SUPER_PANELS;      // first (lowest) panel of this super-panel
       const int64_t k0 = (int64_t)p_lo * NB;                   // first column of the super-panel
@@ -596,22 +931,27 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
       const int nb = (int)((C - k1) < NB ? (C - k1) : NB);
       const int kwin = (p - p_lo) * NB;                        // this panel's k window in the plane buffer
       float* dblk = H + k1 * ldh + k1;
-      {
+      if (together && k1 > 0) {
+        PanelArgs pa;
+        pa.blk = dblk; pa.rows = H + k1; pa.ld = ldh;
+        pa.nb = nb; pa.nrows = (int)k1; pa.k_global = (int)k1;
+        pa.diag = diag + k1; pa.flags = flags;
+        pa.planes = pset.base + kwin; pa.plane_stride = pset.total_rows * (int64_t)SUPER_NB;
+        pa.n_planes = split; pa.plane_ld = SUPER_NB; pa.half = half ? 1 : 0;
+        pa.ticket = tickets + p; pa.strips = strips; pa.tag = (uint32_t)(p + 1);
+        pa.fault = fault;
+        ProfScope prof(PROF_CHOL_DIAG, (double)nb * nb * nb / 3.0 + (double)k1 * nb * nb, 0.0, st);
+        MQ_TRY(launch_panel(p < P - 1, pa, st));
+      } else {
         ProfScope prof(PROF_CHOL_DIAG, (double)nb * nb * nb / 3.0, 0.0, st);
-        MQ_CUDA(launch_chained(true, chol_diag_rev_kernel, dim3(1), dim3(DIAG_THREADS), kDiagSmem, st, dblk, ldh, nb, (int)k1, flags));
+        MQ_CUDA(launch_chained(true, chol_diag_rev_kernel, dim3(1), dim3(DIAG_THREADS), kDiagSmem, st, dblk, ldh, nb, (int)k1, diag + k1, flags, fault));
       }
       MQ_LAUNCH_CHECK();
       if (k1 == 0) break;
-      // 32 rows per CTA (one group of four rows per warp); compact launches: 64 rows, half the CTAs
-      // and half the copies of the diagonal block (462 against 454-459 layers/s on eight streams)
-      const int grid = compact ? (int)ceil_div(k1, 64) : (int)(ceil_div(k1, 32) < 148 * 2 ? ceil_div(k1, 32) : 148 * 2);
-      {
-        ProfScope prof(PROF_TRSM, (double)k1 * nb * nb, 0.0, st);
-        MQ_CUDA(launch_chained(true, trsm_rows_kernel<false>, dim3(grid, 1), dim3(256), kTrsmSmem, st, dblk, ldh, 0, H + k1, ldh, 0,
-                               (int)k1, nb, 0, tensor ? pset.base + kwin : nullptr, tensor ? pset.total_rows * (int64_t)SUPER_NB : 0,
-                               split, SUPER_NB, half ? 1 : 0));
+      if (!together) {
+        MQ_TRY(launch_solve(dblk, ldh, H + k1, (int)k1, nb, tensor ? pset.base + kwin : nullptr, tensor ? pset.total_rows * (int64_t)SUPER_NB : 0,
+                            split, half, compact != 0, st));
       }
-      MQ_LAUNCH_CHECK();
       if (!tensor) {
         GemmDesc g;
         g.A = H + k1; g.a_rs = ldh; g.a_cs = 1;
@@ -654,8 +994,6 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
     finish_diag_blocks_kernel<<<(unsigned)P, 1024, 0, st>>>(H, C, ldh, diag, eq);
     MQ_LAUNCH_CHECK();
   } else {
-    extract_diag_kernel<<<(unsigned)ceil_div(C, 256), 256, 0, st>>>(H, C, ldh, diag);
-    MQ_LAUNCH_CHECK();
     const unsigned gx = (unsigned)(ceil_div(C, 256) < 8 ? ceil_div(C, 256) : 8);
     scale_columns_kernel<<<dim3(gx, (unsigned)C), 256, 0, st>>>(H, C, ldh, diag, eq, upper_only ? 1 : 0);
     MQ_LAUNCH_CHECK();

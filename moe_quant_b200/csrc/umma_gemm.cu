@@ -31,6 +31,7 @@
 #include <cstring>
 
 #include "engine.cuh"
+#include "mbarrier.cuh"
 #include "profile.cuh"
 
 namespace mq {
@@ -77,43 +78,11 @@ struct UmmaParams {
 };
 
 // ---------------------------------------------------------------- PTX wrappers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 // Bounded wait: gives up after about one second and records `code`.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code) {
-  uint64_t t0 = 0;
-  for (uint32_t it = 0;; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((it & 255u) == 255u) {
-      // once any wait on this device has expired, every later wait gives up at once
-      if (*reinterpret_cast<volatile int*>(&g_engine_fault) != 0) return false;
-      uint64_t now;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > 1000000000ull) {
-        atomicCAS(&g_engine_fault, 0, code);
-        return false;
-      }
-    }
-  }
-}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code) { return mq::mbar_wait(bar, parity, &g_engine_fault, code); }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
@@ -1229,18 +1198,9 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
 }
 // A wait that only the clock ends (a fault elsewhere does not): for what is still under way after a wait was given up.
 __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
-  uint64_t t0, now;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-    if (ok || now - t0 > 100000000ull) return;
-  }
+  const uint64_t t0 = global_ns();
+  while (!mbar_try(bar, parity))
+    if (global_ns() - t0 > 100000000ull) return;
 }
 
 // DOT: nothing is stored; B is upper triangular (rows past a tile's last column hold nothing: k stops there), tiles are
@@ -2151,6 +2111,13 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
 }
 
 }  // namespace
+
+int engine_fault_word(int** out) {
+  void* p = nullptr;
+  MQ_CUDA(cudaGetSymbolAddress(&p, g_engine_fault));   // of the current device
+  *out = static_cast<int*>(p);
+  return MQ_OK;
+}
 
 int gemm_tensor_planes(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStream_t st) {
   if (d.M <= 0 || d.N <= 0 || d.batch <= 0) return MQ_OK;

@@ -754,6 +754,22 @@ def test_compact_sweep_is_bit_identical(cuda, R, C, g, dtype, math):
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1].float(), res[1][1].float())
 
 
+# ------------------------------------------------------------------ one launch per panel
+@pytest.mark.parametrize("C,tokens", [(136, 200), (392, 100), (1160, 1500), (4840, 1000), (9544, 700)])
+def test_panel_in_one_launch_is_bit_identical(cuda, C, tokens):
+    """The block and the solve in one launch against one launch each (compact): the same operations in the same order.
+    One, two and four groups of rows per warp (from 4705 and 9409 rows on), first panels of 8 and 72 columns."""
+    R = 24
+    W = synthetic.layer_weight(R, C, 3, torch.bfloat16).to(cuda)
+    X = synthetic.activations(tokens, C, 4, torch.bfloat16).to(cuda)
+    H = torch.zeros(C, C, device=cuda)
+    ops.hessian_accum(H, X, 0.0, 2.0 / tokens)
+    outs = [ops.quantize_layer([W], H.clone(), C, 4, 1e-2, want_dequantized=True, precision=ops.Precision(compact=c)) for c in (False, True)]
+    (c0, s0, d0, f0), (c1, s1, d1, f1) = outs
+    assert f0.tolist() == f1.tolist() and int(f0[3]) == 0
+    assert torch.equal(c0[0], c1[0]) and torch.equal(s0[0], s1[0]) and torch.equal(d0[0], d1[0])
+
+
 # ------------------------------------------------------------------ row groups of the sweep tile
 @pytest.mark.parametrize("R", [1, 7, 8, 9, 33, 1184, 1185, 4737, 9473])
 @pytest.mark.parametrize("C,g", [(24, 24), (136, 8), (256, 32)])
