@@ -133,6 +133,8 @@ __device__ __forceinline__ void factor_diag_block(const DiagShared sh, float* __
       // of the leaf itself, and those below it, run the row arithmetic too.  A pivot that is not positive
       // turns what follows into NaN; it is reported, and the whole factor is replaced.
       int fail = 0;
+      float* pb = sh.pan + (kt & 1) * 8 * PAN_LD;
+      const bool in[2] = {t < 8 * kt + 8, t + 64 < 8 * kt + 8};
 #pragma unroll
       for (int kk = 7; kk >= 0; --kk) {
         const float d = L[kk][kk];
@@ -153,34 +155,20 @@ __device__ __forceinline__ void factor_diag_block(const DiagShared sh, float* __
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float pv = x[h][kk] * r;
-          x[h][kk] = pv;
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             if (j < kk) x[h][j] = fmaf(-pv, L[j][kk], x[h][j]);
+          // A row of the leaf goes through the same operations as its copy in L: it is the factor from its diagonal on.
+          x[h][kk] = t + 64 * h > 8 * kt + kk ? 0.0f : pv;
+          if (in[h]) pb[kk * PAN_LD + (h ? p1 : p0)] = x[h][kk];
         }
       }
       if (t == 0 && fail != 0 && kt * 8 + fail - 1 < nb) atomicCAS(&flags->not_positive, 0, k_global + kt * 8 + fail);
-      // A row of the leaf has gone through the same operations as its copy in L: it is the factor from its diagonal on.
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int kk = 0; kk < 7; ++kk)
-          if (t + 64 * h > 8 * kt + kk) x[h][kk] = 0.0f;
-      float* pb = sh.pan + (kt & 1) * 8 * PAN_LD;
-      const bool in0 = t < 8 * kt + 8, in1 = t + 64 < 8 * kt + 8;
-      if (in0) {
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) pb[kk * PAN_LD + p0] = x[0][kk];
-      }
-      if (in1) {
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) pb[kk * PAN_LD + p1] = x[1][kk];
-      }
       if (kt > 0) bar_sync(2, CHAIN_THREADS + HELP_THREADS);
       // the strip is final
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        if (h ? in1 : in0) {
+        if (in[h]) {
           float* dst = sh.T + (t + 64 * h) * DIAG_LD + 8 * kt;
           *reinterpret_cast<float4*>(dst) = make_float4(x[h][0], x[h][1], x[h][2], x[h][3]);
           *reinterpret_cast<float4*>(dst + 4) = make_float4(x[h][4], x[h][5], x[h][6], x[h][7]);
@@ -542,12 +530,19 @@ __device__ __forceinline__ uint64_t* strip_words(uint64_t* strips, int kt, int q
 __device__ __forceinline__ void publish_strips(const DiagShared sh, const PanelArgs& p, int lane) {
   for (int kt = ((p.nb + 7) >> 3) - 1; kt >= 0; --kt) {
     if (!mbar_wait(smem_u32(sh.ready + kt), 0, p.fault, 64)) return;
+    // as the solve wants them: divided by the diagonal above it (times the reciprocal), the diagonal itself, zeros below
+    const int k = 8 * kt + (lane & 7);
+    const float mine = 1.0f / sh.T[k * (DIAG_LD + 1)];
+    float rd[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) rd[q] = __shfl_sync(0xffffffffu, mine, q);
     for (int row = lane; row < 8 * kt + 8; row += 32) {
       const float4 lo = *reinterpret_cast<const float4*>(sh.T + row * DIAG_LD + 8 * kt), hi = *reinterpret_cast<const float4*>(sh.T + row * DIAG_LD + 8 * kt + 4);
-      store_tagged(strip_words(p.strips, kt, 0, row), lo.x, lo.y, p.tag);
-      store_tagged(strip_words(p.strips, kt, 1, row), lo.z, lo.w, p.tag);
-      store_tagged(strip_words(p.strips, kt, 2, row), hi.x, hi.y, p.tag);
-      store_tagged(strip_words(p.strips, kt, 3, row), hi.z, hi.w, p.tag);
+      float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = row < 8 * kt + q ? v[q] * rd[q] : v[q];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) store_tagged(strip_words(p.strips, kt, q, row), v[2 * q], v[2 * q + 1], p.tag);
     }
   }
 }
@@ -582,26 +577,25 @@ __device__ __forceinline__ void fetch_strips(const PanelArgs& p, float* TT, floa
       if ((it & 255u) == 255u && lane == 0) gone = limit.expired(p.fault, 61);
       if (__shfl_sync(0xffffffffu, gone, 0)) return;   // the solving warps give up by themselves
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int kk = lane + 32 * i - 8 * kt;
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (q == kk) {
-          const float d = __uint_as_float((uint32_t)v[i][q]);
-          dg[8 * kt + kk] = d;
-          rdg[8 * kt + kk] = 1.0f / d;
-        }
-    }
-    __syncwarp();
-    const float4 r0 = *reinterpret_cast<const float4*>(rdg + 8 * kt), r1 = *reinterpret_cast<const float4*>(rdg + 8 * kt + 4);
-    const float rd[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+    float d = 1.0f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = lane + 32 * i;
       if (row >= 8 * kt + 8) continue;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) TT[(8 * kt + q) * TT_LD + row] = row < 8 * kt + q ? __uint_as_float((uint32_t)v[i][q]) * rd[q] : 0.0f;
+      for (int q = 0; q < 8; ++q) {
+        float x = __uint_as_float((uint32_t)v[i][q]);
+        if (row == 8 * kt + q) {
+          d = x;
+          x = 0.0f;
+        }
+        TT[(8 * kt + q) * TT_LD + row] = x;
+      }
+    }
+    if (((lane - 8 * kt) & 31) < 8) {   // the leaf's rows
+      const int k = 8 * kt + ((lane - 8 * kt) & 31);
+      dg[k] = d;
+      rdg[k] = 1.0f / d;
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(full0 + 8 * kt);
