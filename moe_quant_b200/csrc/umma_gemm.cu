@@ -13,10 +13,10 @@
 // Where operands can be scaled into fp16's range (the factorisation, the inverse-free sweep, the quadratic forms) a pair
 // of fp16 planes (split_half2) does with three products.
 //
-// Five kernels share the pieces below: umma_gemm_kernel (one tile per CTA, any K, planes,
-// batches), umma_gemm_persistent_kernel (one-plane GEMMs and the Hessian: one CTA per SM walks
-// 128 x 256 tiles, epilogue under the next tile's MMAs; 16-bit activations are read in place as
-// MN-major boxes), umma_panel_kernel (K <= 128, A stationary, C through the TMA unit),
+// Six kernels share the pieces below: umma_gemm_kernel (one tile per CTA, any K, planes,
+// batches), umma_gemm_persistent_kernel (one-plane GEMMs: one CTA per SM walks
+// 128 x 256 tiles, epilogue under the next tile's MMAs), umma_gram_kernel (the Hessian: 16-bit activations read in place as
+// MN-major boxes, two CTAs per tile), umma_panel_kernel (K <= 128, A stationary, C through the TMA unit),
 // umma_stream_kernel (deep updates on bf16 planes) and umma_pair_kernel (deep updates and quadratic forms on fp16
 // pairs, two CTAs per tile).
 // Structure of the first (one 128 x 128 output tile per CTA, 192 threads):
@@ -67,6 +67,7 @@ struct UmmaParams {
   int planes, nterms, stages;
   uint32_t idesc;
   int mirror;  // symmetric result: every block above the diagonal is also stored transposed
+  int vec;     // gram kernel: rows of C are 16-byte aligned and a multiple of four long
   int c_tma;   // panel kernel epilogue: 0 = loads/stores by the warps, 1 = TMA store (beta == 0), 2 = TMA add (beta == 1)
   int pairs;           // operands are pairs of fp16 planes: the leading product is summed per slab of k (see below)
   int all_products;    // pairs: lo lo as well
@@ -195,18 +196,6 @@ __device__ __forceinline__ uint64_t mnmajor_sw128_desc(uint32_t smem_addr, uint3
   d |= (uint64_t)1 << 46;                   // version
   d |= (uint64_t)2 << 61;                   // SWIZZLE_128B
   return d;
-}
-
-// One 64-wide K slab of a one-plane GEMM whose operands are MN-major boxes (8 KB per 64 rows of
-// m/n): a K step of 16 is two groups of 8 k, 2048 bytes.
-__device__ __forceinline__ void issue_slab_mn(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile, uint32_t idesc,
-                                              uint32_t& accumulate) {
-  const uint64_t a0 = mnmajor_sw128_desc(a_tile, 8192), b0 = mnmajor_sw128_desc(b_tile, 8192);
-#pragma unroll
-  for (int kk = 0; kk < SLAB_K / 16; ++kk) {
-    umma_bf16(tmem_d, a0 + (uint64_t)((kk * 2048) >> 4), b0 + (uint64_t)((kk * 2048) >> 4), idesc, accumulate);
-    accumulate = 1;
-  }
 }
 
 // All MMAs of one 64-wide K slab: for each of the four K16 steps, the products A_i B_j with
@@ -515,15 +504,13 @@ __global__ void __launch_bounds__(GEMM_THREADS) umma_gemm_kernel(const __grid_co
   }
 }
 
-// ---------------------------------------------------------------- persistent one-plane GEMM (the Hessian)
+// ---------------------------------------------------------------- persistent one-plane GEMM
 // 128 x 256 tiles, one plane per operand (bf16/fp16 activations), any K.  One CTA per SM walks the
 // list of kept tiles (index = blockIdx.x + i * gridDim.x): the operand ring keeps running across
 // tiles, the accumulator alternates between the two halves of tensor memory, and the epilogue of
-// tile i (read-modify-write of C and, for the symmetric Hessian, the transposed store) runs while
+// tile i (read-modify-write of C and, for a symmetric result, the transposed store) runs while
 // tile i+1 is multiplied.  With one tile per CTA the tensor pipe idled through every prologue and
 // epilogue.
-// (A short update of a 7168-channel Hessian, 126 tokens, takes 77 us for 309 MB.  Two sets of epilogue warps that take
-// turns: 82 us; transposed stores of 16-byte pieces instead of one 128-byte row per instruction: 92 us.)
 constexpr int PERSIST_TN = 256, PERSIST_STAGES = 4;
 
 // kept tile number w -> tile row ty, tile column tx (row-major over the kept tiles)
@@ -543,10 +530,6 @@ __device__ __forceinline__ void persistent_tile(const UmmaParams& p, int w, int 
   }
 }
 
-// DIRECT: the operands are not plane buffers but one row-major 16-bit matrix X (k x m, the
-// activations: tokens x channels) read in place through a 2-D map (map_a; map_b unused) with
-// 64 x 64 boxes, which arrive MN-major; C <- alpha X^T X + beta C.
-template <bool DIRECT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                             const __grid_constant__ CUtensorMap map_b,
                                                                             const UmmaParams p, const int n_work) {
@@ -594,20 +577,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_persistent_kernel(c
         if (lane == 0) {
           mbar_expect_tx(full0 + 8 * st, STAGE);
           const uint32_t dst = smem_base + (uint32_t)st * STAGE;
-          if (DIRECT) {
-            // boxes of 64 channels x 64 tokens, 8 KB each: two for A, four for B
-#pragma unroll
-            for (int h = 0; h < TILE_M / 64; ++h) tma_load_2d(dst + h * 8192, &map_a, full0 + 8 * st, a_row + h * 64, s * SLAB_K);
-#pragma unroll
-            for (int h = 0; h < TN / 64; ++h)
-              tma_load_2d(dst + PLANE_TILE_BYTES + h * 8192, &map_a, full0 + 8 * st, b_row + h * 64, s * SLAB_K);
-          } else {
             tma_load_3d(dst, &map_a, full0 + 8 * st, s * SLAB_K + p.a_k0, a_row, 0);
 #pragma unroll
             for (int h = 0; h < TN / TILE_M; ++h)  // the TMA box is 128 rows
               tma_load_3d(dst + PLANE_TILE_BYTES + h * PLANE_TILE_BYTES, &map_b, full0 + 8 * st, s * SLAB_K + p.b_k0,
                           b_row + h * TILE_M, 0);
-          }
         }
         __syncwarp();
       }
@@ -628,8 +602,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_persistent_kernel(c
         tc_fence_after();
         if (lane == 0) {
           const uint32_t a_base = smem_base + (uint32_t)st * STAGE;
-          if (DIRECT) issue_slab_mn(tmem_acc + (uint32_t)(acc * TN), a_base, a_base + PLANE_TILE_BYTES, p.idesc, accumulate);
-          else issue_slab<1>(tmem_acc + (uint32_t)(acc * TN), 0u, a_base, a_base + PLANE_TILE_BYTES, p.idesc, accumulate, unused_small);
+          issue_slab<1>(tmem_acc + (uint32_t)(acc * TN), 0u, a_base, a_base + PLANE_TILE_BYTES, p.idesc, accumulate, unused_small);
           umma_commit(empty0 + 8 * st);
         }
         __syncwarp();
@@ -1203,6 +1176,56 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
     if (global_ns() - t0 > 100000000ull) return;
 }
 
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem) {   // all 512 columns of both CTAs
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(dst_smem) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(taddr) : "memory");
+}
+
+// What the two CTAs must know of each other before they leave: a wait of either was given up, slabs multiplied and accumulators handed over (set in
+// both), slabs whose copies either producer has issued (the leader's).  With every wait satisfied nothing is under way at the end: the
+// producers have seen the last commits on `empty` (await_stages), the epilogue warps all of those on `acc_full`, and the cluster barrier orders
+// the arrivals on the leader's `acc_empty`.  After a wait that was given up what is under way comes to its end first (drain): the MMAs through
+// their commits, of which the last use of every barrier is known, the copies through the leader's `full` (a stage that one
+// producer alone has filled never completes; the copy lands long before that wait runs out).
+struct PairEnd {
+  int given_up, n_multiplied, n_accs, n_copied[2];
+  __device__ __forceinline__ void reset() { given_up = n_multiplied = n_accs = n_copied[0] = n_copied[1] = 0; }
+  __device__ __forceinline__ void give_up() {
+    set_in_cta(&given_up, 0, 1);
+    set_in_cta(&given_up, 1, 1);
+  }
+  __device__ __forceinline__ void multiplied(int slabs, int accs) {
+    for (int c = 0; c < 2; ++c) {
+      set_in_cta(&n_multiplied, c, slabs);
+      set_in_cta(&n_accs, c, accs);
+    }
+  }
+  __device__ __forceinline__ void copied_by(int rank, int slabs) { set_in_cta(&n_copied[rank], 0, slabs); }
+  // by the producers' warps: the last use of every stage has been read (so its copies had landed) and its commit has arrived in this CTA
+  template <int NST>
+  static __device__ __forceinline__ bool await_stages(uint32_t empty0, int slabs, bool ok, int code) {
+    for (int j = slabs > NST ? slabs - NST : 0; j < slabs && ok; ++j) ok = mbar_wait(empty0 + 8 * (j % NST), (j / NST) & 1, code);
+    return ok;
+  }
+  template <int NST>
+  __device__ __forceinline__ void drain(int rank, uint32_t full0, uint32_t empty0, uint32_t acc_full) const {
+    for (int j = n_multiplied > NST ? n_multiplied - NST : 0; j < n_multiplied; ++j) mbar_drain(empty0 + 8 * (j % NST), (j / NST) & 1);
+    for (int j = n_accs > 2 ? n_accs - 2 : 0; j < n_accs; ++j) mbar_drain(acc_full + 8 * (j & 1), (j >> 1) & 1);
+    if (rank != 0) return;
+    const int c = n_copied[0] > n_copied[1] ? n_copied[0] : n_copied[1];
+    for (int j = c > NST ? c - NST : 0; j < c; ++j) mbar_drain(full0 + 8 * (j % NST), (j / NST) & 1);
+  }
+};
+
 // DOT: nothing is stored; B is upper triangular (rows past a tile's last column hold nothing: k stops there), tiles are
 // taken from the right, longest first, and the epilogue sums the tile's products with A in fp64.
 __device__ __forceinline__ void pair_tile(TileWalk& w, int idx, int n_tiles, int m_tiles, bool dot, int upper) {
@@ -1232,9 +1255,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   __shared__ __align__(8) uint64_t bars[2 * PAIR_STAGES + 4];
   __shared__ uint32_t tmem_slot;
-  // for the end of the kernel: a wait of either CTA was given up, slabs multiplied (both set in both CTAs), slabs
-  // whose copies either producer has issued (the leader's)
-  __shared__ int given_up, n_multiplied, n_copied[2];
+  __shared__ PairEnd end;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[PAIR_STAGES]);
   // two accumulators of 256 columns, by slab & 1
   const uint32_t acc_full = smem_u32(&bars[2 * PAIR_STAGES]), acc_empty = smem_u32(&bars[2 * PAIR_STAGES + 2]);
@@ -1248,17 +1269,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
       mbar_init(acc_full + 8 * b, 1);
       mbar_init(acc_empty + 8 * b, 16);  // the leader's: eight epilogue warps of either CTA
     }
-    given_up = n_multiplied = n_copied[0] = n_copied[1] = 0;
+    end.reset();
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  auto give_up = [&]() {
-    set_in_cta(&given_up, 0, 1);
-    set_in_cta(&given_up, 1, 1);
-  };
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
+  if (warp == 1) tmem_alloc_pair(smem_u32(&tmem_slot));
   tc_fence_before();
   __syncthreads();
   cluster_sync();   // either CTA's barriers and tensor memory exist before the other signals or writes them
@@ -1294,13 +1308,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           __syncwarp();
         }
       }
-      // the last use of every stage: its MMAs have read it (so its copies had landed) and their commit has
-      // arrived in this CTA
-      for (int j = it > PAIR_STAGES ? it - PAIR_STAGES : 0; j < it && ok; ++j)
-        ok = mbar_wait(empty0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1, 55);
+      ok = PairEnd::await_stages<PAIR_STAGES>(empty0, it, ok, 55);
       if (lane == 0) {
-        set_in_cta(&n_copied[rank], 0, it);
-        if (!ok) give_up();
+        end.copied_by(rank, it);
+        if (!ok) end.give_up();
       }
     } else if (warp == 1) {
       if (rank == 0) {
@@ -1345,9 +1356,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           }
         }
         if (lane == 0) {
-          set_in_cta(&n_multiplied, 0, it);
-          set_in_cta(&n_multiplied, 1, it);
-          if (!ok) give_up();
+          end.multiplied(it, it);   // an accumulator per slab
+          if (!ok) end.give_up();
         }
       }
     }
@@ -1468,34 +1478,285 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     }
     if (lane == 0) {
       bulk_wait_read_all();  // the boxes have left shared memory; the writes land before the grid completes
-      if (!ok) give_up();
+      if (!ok) end.give_up();
     }
     __syncwarp();
   }
   tc_fence_before();
   __syncthreads();
   cluster_sync();   // neither CTA issues a copy, an MMA or an arrival any more
-  // With every wait satisfied nothing is under way either: the producers have seen the last commits on `empty`, the
-  // epilogue warps all of those on `acc_full`, and the barrier orders the arrivals on the leader's `acc_empty`.
-  // After a wait that was given up what is under way comes to its end first: the MMAs through their commits, of which the
-  // last use of every barrier is known, the copies through the leader's `full` (a stage that one producer alone
-  // has filled never completes; the copy lands long before that wait runs out).
-  if (given_up) {   // the same in both CTAs
-    if (warp == 0) {
-      const int n = n_multiplied;
-      for (int j = n > PAIR_STAGES ? n - PAIR_STAGES : 0; j < n; ++j) mbar_drain(empty0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1);
-      for (int j = n > 2 ? n - 2 : 0; j < n; ++j) mbar_drain(acc_full + 8 * (j & 1), (j >> 1) & 1);
-      if (rank == 0) {
-        const int c = n_copied[0] > n_copied[1] ? n_copied[0] : n_copied[1];
-        for (int j = c > PAIR_STAGES ? c - PAIR_STAGES : 0; j < c; ++j) mbar_drain(full0 + 8 * (j % PAIR_STAGES), (j / PAIR_STAGES) & 1);
-      }
-    }
+  if (end.given_up) {   // the same in both CTAs
+    if (warp == 0) end.drain<PAIR_STAGES>(rank, full0, empty0, acc_full);
     __syncthreads();
     cluster_sync();   // the other CTA's copies signal the leader's barriers
   }
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_acc) : "memory");
+    tmem_dealloc_pair(tmem_acc);
+  }
+}
+
+// ---------------------------------------------------------------- the Hessian: CTA pairs on the activations as they lie
+// C <- alpha X^T X + beta C for a row-major 16-bit X (tokens x channels), read in place through a 2-D map with boxes of 64
+// channels x 64 tokens, which arrive MN-major.  Two CTAs of a cluster share a 256 x 256 tile (cta_group::2), 128 rows of either operand
+// each: 32 KB of operands per 64 tokens and SM for 512 cycles of MMAs, 64 bytes a cycle; an SM draws 57 from the L2 when all do.
+// (One CTA per 128 x 256 tile needed 96.)  Both accumulators of a pair's 512 TMEM columns are in use: the epilogue of tile i runs
+// under the MMAs of tile i + 1.  Two updates of 4096 tokens, 7168 channels: 478 us with a tile per CTA, 435 now (at the power cap);
+// eight of about 126 tokens 670 and 640: there the read, the write and the transposed write of 206 MB bound it.
+//   warp 0 of either CTA : TMA, its own rows, a ring of six stages; the bytes of both count on the leader's barrier
+//   warp 1 of the leader : tcgen05.mma (M 256, N 256) for both SMs
+//   warps 4..7 / 8..11   : epilogue of the left / right 128 columns of the CTA's 128 rows
+constexpr int GRAM_STAGES = 6;
+constexpr uint32_t GRAM_STAGE_BYTES = 2 * PLANE_TILE_BYTES;
+constexpr size_t kGramSmem = (size_t)GRAM_STAGES * GRAM_STAGE_BYTES + 8 * 4096 + 1024;
+
+// 32 rows x 128 columns of the result by one warp, in 32 x 32 blocks (block row gr, block column gc).  The upper triangle is authoritative: a
+// block right of the diagonal is stored and stored transposed, one on it is symmetrised (A_i B_j and A_j B_i are summed in different
+// orders by the MMA), one left of it is left to its mirror image: C[n][m] == C[m][n] bit for bit.  Every global access is a run of
+// whole 128-byte row segments.  Two blocks of C are on their way while one is worked on, the first two from before the accumulator is waited for.
+// The block of a warp in shared memory: 32 x 32, quad j of row r at block_at(r, j) (rows and columns without bank conflicts).
+__device__ __forceinline__ int block_at(int r, int j) { return r * 32 + ((j ^ (r & 7)) << 2); }
+
+template <typename WaitFn, typename ReleaseFn>
+__device__ __forceinline__ bool gram_epilogue(const UmmaParams& p, const int y0, const int n0, const uint32_t tmem, float* stage, const int lane,
+                                              WaitFn wait_acc, ReleaseFn release_acc) {
+  const int N = p.N, gr = y0 >> 5;
+  const int64_t ldc = p.ldc;
+  const int r8 = lane >> 3, c4 = (lane & 7) * 4;
+  float* c0 = p.C + (int64_t)(y0 + r8) * ldc + n0 + c4;
+  float4 old[2][8];
+  auto kept = [&](int c) { return (n0 >> 5) + c >= gr && n0 + 32 * c < N && y0 < N; };
+  auto request = [&](int c) {
+    if (p.beta == 0.0f || !kept(c)) return;
+#pragma unroll
+    for (int it = 0; it < 8; ++it)
+      old[c & 1][it] = (y0 + 4 * it + r8 < N && n0 + 32 * c + c4 < N) ? *reinterpret_cast<const float4*>(c0 + (int64_t)(4 * it) * ldc + 32 * c)
+                                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  if (!p.vec) {
+    if (!wait_acc()) return false;
+    const int row = y0 + lane;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      float v[32];
+      tmem_ld32(tmem + (uint32_t)(c * 32), v);
+      if (c == 3) release_acc();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int col = n0 + 32 * c + j;
+        if (row >= N || col >= N || col < row) continue;
+        float* dst = p.C + (int64_t)row * ldc + col;
+        float o = p.alpha * v[j];
+        if (p.beta != 0.0f) o = fmaf(p.beta, *dst, o);
+        *dst = o;
+        if (col > row) p.C[(int64_t)col * ldc + row] = o;
+      }
+    }
+    return true;
+  }
+  request(0);
+  request(1);
+  if (!wait_acc()) return false;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const bool keep = kept(c);   // uniform in the warp
+    if (keep) {
+      float v[32];
+      tmem_ld32(tmem + (uint32_t)(c * 32), v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<float4*>(&stage[block_at(lane, j)]) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+    if (c == 3) release_acc();
+    if (!keep) {
+      if (c + 2 < 4) request(c + 2);
+      continue;
+    }
+    __syncwarp();
+    const int x0 = n0 + 32 * c, gc = x0 >> 5;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      float* sp = &stage[block_at(4 * it + r8, lane & 7)];
+      const float4 a4 = *reinterpret_cast<const float4*>(sp);
+      float4 o = make_float4(p.alpha * a4.x, p.alpha * a4.y, p.alpha * a4.z, p.alpha * a4.w);
+      if (p.beta != 0.0f) {
+        const float4 od = old[c & 1][it];
+        o.x = fmaf(p.beta, od.x, o.x); o.y = fmaf(p.beta, od.y, o.y);
+        o.z = fmaf(p.beta, od.z, o.z); o.w = fmaf(p.beta, od.w, o.w);
+      }
+      if (gc > gr && y0 + 4 * it + r8 < N && x0 + c4 < N) *reinterpret_cast<float4*>(c0 + (int64_t)(4 * it) * ldc + 32 * c) = o;
+      *reinterpret_cast<float4*>(sp) = o;
+    }
+    if (c + 2 < 4) request(c + 2);
+    __syncwarp();
+    if (gc == gr) {
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const int r = 4 * it + r8;
+        float e[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) e[t] = (c4 + t >= r) ? stage[block_at(r, lane & 7) + t] : stage[block_at(c4 + t, r >> 2) + (r & 3)];
+        if (y0 + r < N && x0 + c4 < N) *reinterpret_cast<float4*>(c0 + (int64_t)(4 * it) * ldc + 32 * c) = make_float4(e[0], e[1], e[2], e[3]);
+      }
+    } else {
+      // C[x0 + i][y0 + lane] = block[lane][i]: one 128-byte row segment per i
+      float* mq = p.C + (int64_t)x0 * ldc + y0 + lane;
+      const bool in = y0 + lane < N;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 f = *reinterpret_cast<const float4*>(&stage[block_at(lane, j)]);
+        if (in && x0 + 4 * j < N) {     // N % 4 == 0
+          mq[(int64_t)(4 * j) * ldc] = f.x;
+          mq[(int64_t)(4 * j + 1) * ldc] = f.y;
+          mq[(int64_t)(4 * j + 2) * ldc] = f.z;
+          mq[(int64_t)(4 * j + 3) * ldc] = f.w;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  return true;
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+    umma_gram_kernel(const __grid_constant__ CUtensorMap map_x, const UmmaParams p, const int total) {
+  const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
+  const int n_tiles = (p.N + PAIR_TILE - 1) / PAIR_TILE;
+  const int my_tiles = (total - pair + n_pairs - 1) / n_pairs;   // the host launches at most one pair per tile
+  const int n_slabs = (p.K + SLAB_K - 1) / SLAB_K;
+
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  __shared__ __align__(8) uint64_t bars[2 * GRAM_STAGES + 4];
+  __shared__ uint32_t tmem_slot;
+  __shared__ PairEnd end;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[GRAM_STAGES]);
+  // two accumulators of 256 columns, by tile & 1
+  const uint32_t acc_full = smem_u32(&bars[2 * GRAM_STAGES]), acc_empty = smem_u32(&bars[2 * GRAM_STAGES + 2]);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < GRAM_STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);    // the leader's: its producer's arrival, then the bytes of both CTAs
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full + 8 * b, 1);
+      mbar_init(acc_empty + 8 * b, 16);  // the leader's: eight epilogue warps of either CTA
+    }
+    end.reset();
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc_pair(smem_u32(&tmem_slot));
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // either CTA's barriers and tensor memory exist before the other signals or writes them
+  tc_fence_after();
+  const uint32_t tmem_acc = tmem_slot;
+  chain_wait();
+  chain_release();
+
+  if (warp == 0) {
+    const uint32_t full_leader = leader_addr(full0);
+    int it = 0;
+    bool ok = true;
+    for (int i = 0; i < my_tiles && ok; ++i) {
+      TileWalk w;
+      w.seek(pair + i * n_pairs, n_tiles, 1);
+      const int a_col = w.m * PAIR_TILE + rank * TILE_M, b_col = w.n * PAIR_TILE + rank * TILE_N;
+      for (int s = 0; s < n_slabs; ++s, ++it) {
+        const int st = it % GRAM_STAGES;
+        if (it >= GRAM_STAGES && !mbar_wait(empty0 + 8 * st, ((it / GRAM_STAGES) - 1) & 1, 71)) { ok = false; break; }
+        if (lane == 0) {
+          if (rank == 0) mbar_expect_tx(full0 + 8 * st, 2 * GRAM_STAGE_BYTES);
+          const uint32_t dst = smem_base + (uint32_t)st * GRAM_STAGE_BYTES;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            tma_load_2d_pair(dst + h * 8192, &map_x, full_leader + 8 * st, a_col + h * 64, s * SLAB_K);
+            tma_load_2d_pair(dst + PLANE_TILE_BYTES + h * 8192, &map_x, full_leader + 8 * st, b_col + h * 64, s * SLAB_K);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    ok = PairEnd::await_stages<GRAM_STAGES>(empty0, it, ok, 75);
+    if (lane == 0) {
+      end.copied_by(rank, it);
+      if (!ok) end.give_up();
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      int it = 0, accs = 0;
+      bool ok = true;
+      for (int i = 0; i < my_tiles && ok; ++i) {
+        const int b = i & 1;
+        if (i >= 2) ok = mbar_wait(acc_empty + 8 * b, ((i >> 1) - 1) & 1, 73);
+        if (!ok) break;
+        tc_fence_after();
+        for (int s = 0; s < n_slabs && ok; ++s, ++it) {
+          const int st = it % GRAM_STAGES;
+          ok = mbar_wait(full0 + 8 * st, (it / GRAM_STAGES) & 1, 72);
+          if (!ok) break;
+          tc_fence_after();
+          if (lane == 0) {
+            const uint32_t a_tile = smem_base + (uint32_t)st * GRAM_STAGE_BYTES;
+            // a K step of 16 is two groups of 8 tokens, 2048 bytes
+            const uint64_t a0 = mnmajor_sw128_desc(a_tile, 8192), b0 = mnmajor_sw128_desc(a_tile + PLANE_TILE_BYTES, 8192);
+#pragma unroll
+            for (int kk = 0; kk < SLAB_K / 16; ++kk)
+              umma_f16_pair(tmem_acc + (uint32_t)(b * PAIR_TILE), a0 + (uint64_t)((kk * 2048) >> 4), b0 + (uint64_t)((kk * 2048) >> 4), p.idesc,
+                            (s > 0 || kk > 0) ? 1u : 0u);
+            umma_commit_pair(empty0 + 8 * st);
+          }
+          __syncwarp();
+        }
+        if (ok) {
+          if (lane == 0) umma_commit_pair(acc_full + 8 * b);
+          ++accs;
+        }
+        __syncwarp();
+      }
+      if (lane == 0) {
+        end.multiplied(it, accs);
+        if (!ok) end.give_up();
+      }
+    }
+  } else if (warp >= 4) {
+    const int h = (warp - 4) >> 2, q = warp & 3;   // half of the columns, TMEM lane quadrant
+    const uint32_t empty_leader = leader_addr(acc_empty);
+    const uint32_t t_lane = tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * TILE_N);
+    float* stage = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + GRAM_STAGES * GRAM_STAGE_BYTES) + (warp - 4) * 1024;
+    bool ok = true;
+    for (int i = 0; i < my_tiles && ok; ++i) {
+      TileWalk w;
+      w.seek(pair + i * n_pairs, n_tiles, 1);
+      const int b = i & 1;
+      ok = gram_epilogue(
+          p, w.m * PAIR_TILE + rank * TILE_M + q * 32, w.n * PAIR_TILE + h * TILE_N, t_lane + (uint32_t)(b * PAIR_TILE), stage, lane,
+          [&]() {
+            const bool there = mbar_wait(acc_full + 8 * b, (uint32_t)((i >> 1) & 1), 74);
+            tc_fence_after();
+            return there;
+          },
+          [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * b);
+          });
+    }
+    if (lane == 0 && !ok) end.give_up();
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // neither CTA issues a copy, an MMA or an arrival any more
+  if (end.given_up) {
+    if (warp == 0) end.drain<GRAM_STAGES>(rank, full0, empty0, acc_full);
+    __syncthreads();
+    cluster_sync();   // the other CTA's copies signal the leader's barriers
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_acc);
   }
 }
 
@@ -1968,8 +2229,8 @@ int configure_once() {
   MQ_CUDA(cudaGetDevice(&dev));
   if (!done[dev & 63]) {
     MQ_CUDA(cudaFuncSetAttribute(umma_gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    MQ_CUDA(cudaFuncSetAttribute(umma_gemm_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
-    MQ_CUDA(cudaFuncSetAttribute(umma_gemm_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
+    MQ_CUDA(cudaFuncSetAttribute(umma_gemm_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
+    MQ_CUDA(cudaFuncSetAttribute(umma_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGramSmem));
     MQ_CUDA(cudaFuncSetAttribute(umma_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
     MQ_CUDA(cudaFuncSetAttribute(umma_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
     MQ_CUDA(cudaFuncSetAttribute(umma_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
@@ -2101,7 +2362,7 @@ int launch_umma(const GemmDesc& d, const PlaneSet& A, const PlaneSet& B, cudaStr
         if (nx_tiles > tx0) n_work += nx_tiles - tx0;
       }
       const size_t wsmem = (size_t)PERSIST_STAGES * (PLANE_TILE_BYTES + PERSIST_TN * SLAB_K * 2) + STAGE_BYTES + 1024;
-      umma_gemm_persistent_kernel<false><<<(unsigned)(n_work < 148 ? n_work : 148), GEMM_THREADS, wsmem, st>>>(map_a, map_b, p, (int)n_work);
+      umma_gemm_persistent_kernel<<<(unsigned)(n_work < 148 ? n_work : 148), GEMM_THREADS, wsmem, st>>>(map_a, map_b, p, (int)n_work);
     } else {
       umma_gemm_kernel<128><<<grid, GEMM_THREADS, smem, st>>>(map_a, map_b, p);
     }
@@ -2266,7 +2527,7 @@ size_t hessian_accum_tensor_workspace_bytes(int x_dtype, int64_t m, int64_t C, i
 int hessian_accum_tensor(const void* X, int x_dtype, int64_t m, int64_t C, int64_t ldx, float* H, int64_t ldh, float beta,
                          float alpha, int split, Workspace& ws, cudaStream_t st) {
   MQ_REQUIRE(split >= 1 && split <= 3, MQ_ERR_ARGUMENT, "mq_hessian_accum: split must be 1, 2 or 3 (got %d)", split);
-  if (x_dtype != MQ_F32 && m > 0 && C >= PERSIST_TN && (ldx & 7) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
+  if (x_dtype != MQ_F32 && m > 0 && C >= PERSIST_TN && (ldx & 7) == 0 && aligned(X, 16)) {
     // 16-bit activations are read where they lie: no transposed copy, no workspace
     MQ_TRY(configure_once());
     EncodeTiledFn enc;
@@ -2285,22 +2546,15 @@ int hessian_accum_tensor(const void* X, int x_dtype, int64_t m, int64_t C, int64
     p.C = H; p.ldc = ldh;
     p.M = (int)C; p.N = (int)C; p.K = (int)m;
     p.alpha = alpha; p.beta = beta;
-    p.upper_tiles_only = 1; p.mirror = 1;
-    p.planes = 1; p.nterms = 1; p.stages = PERSIST_STAGES;
+    p.vec = (C & 3) == 0 && (ldh & 3) == 0 && aligned(H, 16) ? 1 : 0;
     const uint32_t fmt = x_dtype == MQ_F16 ? 0u : 1u;
     // both operands MN-major (bits 15 and 16)
-    p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(PERSIST_TN >> 3) << 17) |
-              ((uint32_t)(TILE_M >> 4) << 24);
-    const int my_tiles = (int)ceil_div(C, TILE_M), nx_tiles = (int)ceil_div(C, PERSIST_TN);
-    long long n_work = 0;
-    for (int ty = 0; ty < my_tiles; ++ty) {
-      const int tx0 = (ty * TILE_M) / PERSIST_TN;
-      if (nx_tiles > tx0) n_work += nx_tiles - tx0;
-    }
-    const size_t wsmem = (size_t)PERSIST_STAGES * (PLANE_TILE_BYTES + PERSIST_TN * SLAB_K * 2) + STAGE_BYTES + 1024;
-    ProfScope prof(PROF_UMMA_GEMM, (double)m * C * (C + 1), 2.0 * (double)n_work * TILE_M * PERSIST_TN * pad_to((int)m, SLAB_K), st);
-    umma_gemm_persistent_kernel<true><<<(unsigned)(n_work < 148 ? n_work : 148), GEMM_THREADS, wsmem, st>>>(map_x, map_x, p,
-                                                                                                          (int)n_work);
+    p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(PAIR_TILE >> 3) << 17) |
+              ((uint32_t)(PAIR_TILE >> 4) << 24);
+    const int64_t n_tiles = ceil_div(C, PAIR_TILE), tiles = n_tiles * (n_tiles + 1) / 2;
+    ProfScope prof(PROF_UMMA_GEMM, (double)m * C * (C + 1), 2.0 * (double)tiles * PAIR_TILE * PAIR_TILE * pad_to((int)m, SLAB_K), st);
+    MQ_CUDA(launch_chained(true, umma_gram_kernel, dim3((unsigned)(2 * (tiles < 74 ? tiles : 74))), dim3(PAIR_THREADS), kGramSmem, st, map_x, p,
+                           (int)tiles));
     MQ_LAUNCH_CHECK();
     return MQ_OK;
   }

@@ -172,6 +172,26 @@ def test_hessian_accum_first_batch_reads_nothing(cuda, precision, C, dtype):
             assert torch.equal(got, got.t())
 
 
+@pytest.mark.parametrize("C,pad", [(256, 0), (264, 8), (3335, 9), (3336, 0)])
+@pytest.mark.parametrize("m", [1, 320, 1100])
+@pytest.mark.parametrize("beta", [0.0, 0.25])
+def test_hessian_accum_in_tile_pairs(cuda, C, pad, m, beta):
+    """One tile, a ragged last tile, rows of the Hessian that are not 16-byte aligned, and 105 tiles for 74 pairs of CTAs with one,
+    five and eighteen slabs of tokens for a ring of six.  fp32 sums of m products: 2^-24 m of the sum of their sizes at most."""
+    gen = torch.Generator().manual_seed(C + m)
+    big = torch.randn(m, C + pad, generator=gen).to(torch.bfloat16)
+    H0 = torch.randn(C, C, generator=gen)
+    H0 = H0 + H0.t()
+    H = H0.to(cuda) if beta else torch.full((C, C), float("nan"), device=cuda)
+    ops.hessian_accum(H, big.to(cuda)[:, :C], beta, 0.5)
+    x = big[:, :C].to(cuda).double()
+    want, size = 0.5 * (x.t() @ x), 0.5 * (x.abs().t() @ x.abs())
+    if beta:
+        want, size = want + beta * H0.to(cuda).double(), size + beta * H0.to(cuda).double().abs()
+    assert bool(((H.double() - want).abs() <= 2.0 ** -24 * (m + 3) * size).all())
+    assert torch.equal(H, H.t())
+
+
 # ------------------------------------------------------------------ prepare
 def test_prepare_golden(cuda, golden):
     H = golden.t("H_final").clone().to(cuda)
