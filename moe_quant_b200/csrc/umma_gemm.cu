@@ -67,7 +67,7 @@ struct UmmaParams {
   int planes, nterms, stages;
   uint32_t idesc;
   int mirror;  // symmetric result: every block above the diagonal is also stored transposed
-  int vec;     // gram kernel: rows of C are 16-byte aligned and a multiple of four long
+  int vec;     // gram kernel and DOT form: the rows of C (of the form's operands) are 16-byte aligned and a multiple of four long
   int c_tma;   // panel kernel epilogue: 0 = loads/stores by the warps, 1 = TMA store (beta == 0), 2 = TMA add (beta == 1)
   int pairs;           // operands are pairs of fp16 planes: the leading product is summed per slab of k (see below)
   int all_products;    // pairs: lo lo as well
@@ -1399,41 +1399,52 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
       const int mb = 2 * w.m + rank, nb = 2 * w.n + h;          // 128-blocks
       const int y = mb * TILE_M + q * 32, n0 = nb * TILE_N;
       if constexpr (DOT) {
-        // this lane's row of A against its 128 sums, 32 columns at a time: the block of A is read along its rows
-        // (a load is one 128-byte segment) and turned through a swizzled tile of this warp
+        // This lane's row of A against its 128 sums.  Every lane reads its own row, whole sectors in loads that follow one another; the
+        // columns' factors come a lane each and go round by shuffles.  (Rows read in 128-byte segments and turned through a tile of 4 KB,
+        // and factors read by all lanes where they are used, one after the other: 62000 cycles at the end of a tile instead of 43000.)
         const bool two = y >= p.dot.second;                  // forms begin at whole tiles: uniform in the warp
         const int r_first = two ? y - p.dot.second : y;
-        const float* a0 = two ? p.dot.x1 + (int64_t)r_first * p.dot.ld1 : p.dot.x0 + (int64_t)r_first * p.dot.ld0;
-        const int64_t ld0 = two ? p.dot.ld1 : p.dot.ld0;
-        const float* a1 = (two || p.dot.x1 == nullptr) ? nullptr : p.dot.x1 + (int64_t)r_first * p.dot.ld1;
-        float* boxf = reinterpret_cast<float*>(smem_raw + (box - smem_u32(smem_raw)));
-        double sum = 0.0;
+        const bool in = r_first + lane < p.dot.rows;
+        const float* a0 = two ? p.dot.x1 + (int64_t)(r_first + lane) * p.dot.ld1 : p.dot.x0 + (int64_t)(r_first + lane) * p.dot.ld0;
+        const float* a1 = (two || p.dot.x1 == nullptr) ? nullptr : p.dot.x1 + (int64_t)(r_first + lane) * p.dot.ld1;
+        double sum[2] = {0.0, 0.0};
 #pragma unroll
         for (int c = 0; c < TILE_N / 32; ++c) {
-          const int x = n0 + c * 32;
-          const bool col_in = x + lane < p.N;
-#pragma unroll 8
-          for (int r = 0; r < 32; ++r) {
-            const bool in = col_in && r_first + r < p.dot.rows;
-            float v = in ? __ldg(a0 + (int64_t)r * ld0 + x + lane) : 0.0f;
-            if (a1 && in) v -= __ldg(a1 + (int64_t)r * p.dot.ld1 + x + lane);
-            boxf[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)] = v;
-          }
-          __syncwarp();
+          const int x0 = n0 + c * 32;
+          const float my_f = x0 + lane < p.N ? __ldg(p.col_f + x0 + lane) : 0.0f;   // columns past the end have no sum
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 v = *reinterpret_cast<const float4*>(boxf + lane * 32 + ((j ^ (lane & 7)) << 2));
-            const float av[4] = {v.x, v.y, v.z, v.w};
+          for (int h2 = 0; h2 < 2; ++h2) {
+            const int x = x0 + h2 * 16;
+            float av[16];
+            if (p.vec) {                                     // 16-byte aligned rows, N % 4 == 0
 #pragma unroll
-            for (int t = 0; t < 4; ++t)
-              if (x + 4 * j + t < p.N) sum += (double)acc[c * 32 + 4 * j + t] * (double)__ldg(p.col_f + x + 4 * j + t) * (double)av[t];
+              for (int j = 0; j < 4; ++j) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in && x + 4 * j < p.N) {
+                  v = __ldg(reinterpret_cast<const float4*>(a0 + x + 4 * j));
+                  if (a1) {
+                    const float4 u = __ldg(reinterpret_cast<const float4*>(a1 + x + 4 * j));
+                    v = make_float4(v.x - u.x, v.y - u.y, v.z - u.z, v.w - u.w);
+                  }
+                }
+                av[4 * j] = v.x; av[4 * j + 1] = v.y; av[4 * j + 2] = v.z; av[4 * j + 3] = v.w;
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                av[j] = in && x + j < p.N ? __ldg(a0 + x + j) : 0.0f;
+                if (a1 && in && x + j < p.N) av[j] -= __ldg(a1 + x + j);
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              sum[j & 1] += (double)acc[c * 32 + h2 * 16 + j] * (double)__shfl_sync(0xffffffffu, my_f, h2 * 16 + j) * (double)av[j];
           }
-          __syncwarp();
         }
         if (r_first + lane < p.dot.rows) {
           const double f = (double)__ldg(p.row_f + y + lane);
-          if (two) total1 += sum * f;
-          else total0 += sum * f;
+          if (two) total1 += (sum[0] + sum[1]) * f;
+          else total0 += (sum[0] + sum[1]) * f;
         }
         continue;
       }
@@ -2484,6 +2495,7 @@ int quadratic_forms(const float* X0, int64_t ld0, const float* X1, int64_t ld1, 
   p.planes = 2; p.pairs = 1;
   p.row_f = row_f; p.col_f = col_f;
   p.dot = f;
+  p.vec = C % 4 == 0 && ld0 % 4 == 0 && aligned(X0, 16) && (!X1 || (ld1 % 4 == 0 && aligned(X1, 16))) ? 1 : 0;
   p.idesc = (1u << 4) | ((uint32_t)(PAIR_TILE >> 3) << 17) | ((uint32_t)(PAIR_TILE >> 4) << 24);
   const long long tiles = (long long)(A.total_rows / PAIR_TILE) * ceil_div(C, PAIR_TILE);
   ProfScope prof(PROF_UMMA_DEEP, (double)forms * R * C * (C + 1), 3.0 * forms * R * C * (C + 1), st);
