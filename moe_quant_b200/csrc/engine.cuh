@@ -90,6 +90,12 @@ inline bool uses_pairs(int64_t C, int math, int split) {
 }
 inline int plane_count(int split) { return split == 4 ? 3 : split; }
 
+// Columns whose update of everything behind them (in front of them, in the factorisation) is applied together where operands are pairs.
+constexpr int64_t PAIR_FAR_COLUMNS = 1024;
+// ... provided that the first half's update by itself, `tiles` of 256 x 256, is more than one for each of the 74 CTA pairs.  Otherwise an update takes as long
+// as one tile, and one tile of 1024 takes longer than one of 512 (1056 columns: 544 us instead of 535).
+inline bool joint_update(long long tiles) { return tiles > 74; }
+
 // Tensor-core GEMM whose operands are already planes (d.A / d.B and their strides are ignored;
 // d.K is the reduction length starting at k0 of each set).  Both sets must have the same
 // number of planes.

@@ -14,10 +14,10 @@
 //   1. the 128x128 diagonal block, one CTA, and
 //   2. the panel above it, substitution against that block: both in one launch (factor_panel_kernel) when the
 //                              layer has the GPU to itself, else chol_diag_rev_kernel and trsm_rows_kernel;
-//   3. GEMMs (GemmDesc)      : trailing update of the upper triangle; on the tensor path in two
+//   3. GEMMs (GemmDesc)      : trailing update of the upper triangle; on the tensor path in
 //                              levels (the rest of the panel's 512-column super-panel at once,
-//                              everything in front of the super-panel once per super-panel with
-//                              all 512 columns in the contraction).
+//                              what lies in front of it once per super-panel or two, with
+//                              all of their columns in the contraction).
 // The inverse is built by inverting the 128x128 diagonal blocks (same substitution
 // kernel on identity rows) and then merging neighbouring blocks pairwise,
 //   inv([A B; 0 D]) = [A^-1, -A^-1 B D^-1; 0, D^-1],
@@ -32,7 +32,7 @@ namespace mq {
 namespace {
 
 constexpr int NB = 128;  // panel width
-constexpr int SUPER_PANELS = 4;               // panels whose far update is applied together
+constexpr int SUPER_PANELS = 4;               // panels whose update of what lies in front of them is applied together
 constexpr int SUPER_NB = SUPER_PANELS * NB;   // 512
 
 // ------------------------------------------------------------------ diagonal block
@@ -801,6 +801,19 @@ int configure_once() {
 
 }  // namespace
 
+static long long upper_pair_tiles(int64_t C) {
+  const int64_t n = ceil_div(C, 256);
+  return n * (n + 1) / 2;
+}
+
+// Columns whose update of everything in front of them is applied together.  1024 with pairs: what bounds those updates is the way of
+// every tile out of its SM, whatever their depth (see umma_pair_kernel); with the sweep's, an attention block
+// takes 28.5 instead of 30.0 ms, four experts 13.0 instead of 13.6.  The factor's error against fp64 is 0.98 to 1.00 of that with 512 where tokens are at
+// least half the columns, but 1.00 to 1.02 with a sixth as many: callers that ask for all four products, as few tokens do, stay at 512.
+static int far_columns(int64_t C, int math, int split) {
+  return uses_pairs(C, math, split) && split == 3 ? (int)PAIR_FAR_COLUMNS : SUPER_NB;
+}
+
 // what the CTAs of factor_panel_kernel tell one another: the strips of the block in flight, a ticket per panel
 static size_t panel_sync_bytes(int64_t C) {
   return align_up(STRIP_WORDS * sizeof(uint64_t) + (size_t)ceil_div(C, NB) * sizeof(int), 256);
@@ -808,7 +821,7 @@ static size_t panel_sync_bytes(int64_t C) {
 
 size_t factor_workspace_bytes(int64_t C, int math, int split) {
   if (math != MQ_MATH_TENSOR) return 0;
-  return plane_set_bytes(C, SUPER_NB, plane_count(split)) + align_up((size_t)(C + 1) * sizeof(float), 256) + panel_sync_bytes(C);
+  return plane_set_bytes(C, far_columns(C, math, split), uses_pairs(C, math, split) ? 2 : plane_count(split)) + align_up((size_t)(C + 1) * sizeof(float), 256) + panel_sync_bytes(C);
 }
 
 // One panel: the block and the rows above it (factor_panel_kernel).  Eight warps of RPW rows a CTA, one CTA per SM at most.
@@ -825,13 +838,13 @@ static int launch_panel(bool chained, const PanelArgs& a, cudaStream_t st) {
 }
 
 static int launch_solve(const float* dblk, int64_t ldh, float* rows, int nrows, int nb, uint16_t* planes, int64_t plane_stride, int split,
-                        bool half, bool compact, cudaStream_t st) {
+                        bool half, int plane_ld, bool compact, cudaStream_t st) {
   // 32 rows per CTA (one group of four rows per warp); compact launches: 64 rows, half the CTAs
   // and half the copies of the diagonal block (462 against 454-459 layers/s on eight streams)
   const int grid = compact ? (int)ceil_div(nrows, 64) : (int)(ceil_div(nrows, 32) < 148 * 2 ? ceil_div(nrows, 32) : 148 * 2);
   ProfScope prof(PROF_TRSM, (double)nrows * nb * nb, 0.0, st);
   MQ_CUDA(launch_chained(true, trsm_rows_kernel<false>, dim3(grid, 1), dim3(256), kTrsmSmem, st, dblk, ldh, (int64_t)0, rows, ldh, (int64_t)0,
-                         nrows, nb, 0, planes, plane_stride, split, SUPER_NB, half ? 1 : 0));
+                         nrows, nb, 0, planes, plane_stride, split, plane_ld, half ? 1 : 0));
   MQ_LAUNCH_CHECK();
   return MQ_OK;
 }
@@ -873,6 +886,7 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
   MQ_REQUIRE(math != MQ_MATH_TENSOR || (split >= 1 && split <= 4), MQ_ERR_ARGUMENT, "factorisation: split must be 1, 2, 3 or 4 (got %d)", split);
   const bool half = uses_pairs(C, math, split);   // pairs of fp16 planes (split_half2)
   const int all_products = half && split == 4 ? 1 : 0;
+  const int far_nb = far_columns(C, math, split), far_panels = far_nb / NB;
   split = plane_count(split);
   MQ_REQUIRE(!eq || half, MQ_ERR_ARGUMENT, "factorisation: an equilibrated matrix needs pairs of planes");
   Workspace local(ws.base ? ws.base + ws.used : nullptr, ws.base ? ws.size - ws.used : 0);
@@ -890,20 +904,20 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
   // P P^T reads one plane set as both operands.
   const bool tensor = math == MQ_MATH_TENSOR;
   {
-    // ---- right-looking in two levels, last panel first.  Four panels form a super-panel of 512
+    // ---- right-looking in levels, last panel first.  Four panels form a super-panel of 512
     // columns.  Behind each panel only the columns of its own super-panel that are still to be
-    // factored take their rank-128 update at once (a strip at most 384 wide); everything in
-    // front of the super-panel is updated once per super-panel, with all 512 columns of it in one
-    // contraction, so a tile of the trailing matrix is read and written once per 512 instead of
-    // once per 128 eliminated columns.  Tensor path: the panel solve writes its result as bf16
-    // planes too (k window of its panel inside a 512-wide plane buffer), and the updates read one
+    // factored take their rank-128 update at once (a strip at most 384 wide); what lies in
+    // front of the super-panel is updated with all 512 columns of it in one contraction.  Where far_columns says so
+    // two super-panels go together: behind the first only the second takes its update (512 deep), and everything
+    // in front of both takes one with all 1024 columns, so a tile of the trailing matrix moves once per 1024 columns.  Tensor path: the panel solve writes its result as operand
+    // planes too (k window of its panel inside the plane buffer), and the updates read one
     // plane set as both operands.
     PlaneSet pset;
     if (tensor) {
       const int planes = half ? 2 : split;
-      pset.base = local.take<uint16_t>(plane_set_bytes(C, SUPER_NB, planes) / 2);
+      pset.base = local.take<uint16_t>(plane_set_bytes(C, far_nb, planes) / 2);
       MQ_REQUIRE(pset.base, MQ_ERR_WORKSPACE, "factorisation: workspace too small for the panel planes");
-      pset.planes = planes; pset.rows_pad = (int)pad_rows(C); pset.total_rows = pset.rows_pad; pset.K_pad = SUPER_NB;
+      pset.planes = planes; pset.rows_pad = (int)pad_rows(C); pset.total_rows = pset.rows_pad; pset.K_pad = far_nb;
       pset.fp16 = half;
     }
     // A caller with several layers in flight gives each few SMs, and the solving CTAs would hold theirs while they wait.
@@ -923,15 +937,16 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
       const int64_t k0 = (int64_t)p_lo * NB;                   // first column of the super-panel
       const int64_t k1 = (int64_t)p * NB;
       const int nb = (int)((C - k1) < NB ? (C - k1) : NB);
-      const int kwin = (p - p_lo) * NB;                        // this panel's k window in the plane buffer
+      const int f_lo = (p / far_panels) * far_panels;          // first panel of those whose far update is applied together
+      const int kwin = (p - f_lo) * NB;                        // this panel's k window in the plane buffer
       float* dblk = H + k1 * ldh + k1;
       if (together && k1 > 0) {
         PanelArgs pa;
         pa.blk = dblk; pa.rows = H + k1; pa.ld = ldh;
         pa.nb = nb; pa.nrows = (int)k1; pa.k_global = (int)k1;
         pa.diag = diag + k1; pa.flags = flags;
-        pa.planes = pset.base + kwin; pa.plane_stride = pset.total_rows * (int64_t)SUPER_NB;
-        pa.n_planes = split; pa.plane_ld = SUPER_NB; pa.half = half ? 1 : 0;
+        pa.planes = pset.base + kwin; pa.plane_stride = pset.total_rows * (int64_t)far_nb;
+        pa.n_planes = split; pa.plane_ld = far_nb; pa.half = half ? 1 : 0;
         pa.ticket = tickets + p; pa.strips = strips; pa.tag = (uint32_t)(p + 1);
         pa.fault = fault;
         ProfScope prof(PROF_CHOL_DIAG, (double)nb * nb * nb / 3.0 + (double)k1 * nb * nb, 0.0, st);
@@ -943,8 +958,8 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
       MQ_LAUNCH_CHECK();
       if (k1 == 0) break;
       if (!together) {
-        MQ_TRY(launch_solve(dblk, ldh, H + k1, (int)k1, nb, tensor ? pset.base + kwin : nullptr, tensor ? pset.total_rows * (int64_t)SUPER_NB : 0,
-                            split, half, compact != 0, st));
+        MQ_TRY(launch_solve(dblk, ldh, H + k1, (int)k1, nb, tensor ? pset.base + kwin : nullptr, tensor ? pset.total_rows * (int64_t)far_nb : 0,
+                            split, half, far_nb, compact != 0, st));
       }
       if (!tensor) {
         GemmDesc g;
@@ -970,16 +985,34 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
         b.k0 = kwin; b.row0 = k0;
         MQ_TRY(gemm_tensor_planes(g, a, b, st));
       } else if (k0 > 0) {
-        // far: H[0:k0, 0:k0] -= P_S P_S^T over all columns of the super-panel, tiles on and above the diagonal
+        const int64_t f0 = (int64_t)f_lo * NB;
         const int p_hi = (p_lo + SUPER_PANELS - 1) < (P - 1) ? (p_lo + SUPER_PANELS - 1) : (P - 1);
+        const int f_hi = (f_lo + far_panels - 1) < (P - 1) ? (f_lo + far_panels - 1) : (P - 1);
         GemmDesc g;
-        g.C = H; g.ldc = ldh;
-        g.M = (int)k0; g.N = (int)k0; g.K = (p_hi - p_lo + 1) * NB;
+        g.ldc = ldh;
         g.alpha = -1.0f; g.beta = 1.0f;
-        g.upper_tiles_only = 1;
         g.all_products = all_products;
         g.k_round = NB;   // partial sums per panel meet in round-to-nearest adds, as in a one-level loop
-        MQ_TRY(gemm_tensor_planes(g, pset, pset, st));
+        PlaneSet a = pset, b = pset;
+        a.k0 = b.k0 = (p_lo - f_lo) * NB;
+        const bool joint = far_nb > SUPER_NB && joint_update(upper_pair_tiles((int64_t)(f_lo + SUPER_PANELS) * NB));
+        if (!joint) {
+          // H[0:k0, 0:k0] -= P_S P_S^T over the columns of this super-panel, tiles on and above the diagonal
+          g.C = H;
+          g.M = (int)k0; g.N = (int)k0; g.K = (p_hi - p_lo + 1) * NB;
+          g.upper_tiles_only = 1;
+        } else if (p_lo > f_lo) {
+          // H[0:k0, f0:k0] -= P_S P_S[f0:k0]^T over the columns of this super-panel: the rest of those that go together
+          g.C = H + f0;
+          g.M = (int)k0; g.N = (int)(k0 - f0); g.K = (p_hi - p_lo + 1) * NB;
+          b.row0 = f0;
+        } else {
+          // H[0:k0, 0:k0] -= P P^T over all columns of those, tiles on and above the diagonal
+          g.C = H;
+          g.M = (int)k0; g.N = (int)k0; g.K = (f_hi - f_lo + 1) * NB;
+          g.upper_tiles_only = 1;
+        }
+        MQ_TRY(gemm_tensor_planes(g, a, b, st));
       }
     }
   }

@@ -396,7 +396,7 @@ int configure_once() {
 size_t sweep_workspace_bytes(int64_t R, int64_t C, int math, int split, bool inverse_free) {
   if ((math & ~MQ_MATH_COMPACT) != MQ_MATH_TENSOR) return align_up((size_t)R * TILE * sizeof(float), 256);
   if (inverse_free && uses_pairs(C, math, split))
-    return plane_set_bytes(R, SUPER, 2) + plane_set_bytes(C, C, 2) + align_up((size_t)R * (SUPER / TILE) * sizeof(float), 256) +
+    return plane_set_bytes(R, PAIR_FAR_COLUMNS, 2) + plane_set_bytes(C, C, 2) + align_up((size_t)R * (PAIR_FAR_COLUMNS / TILE) * sizeof(float), 256) +
            align_up((size_t)C * 2 * sizeof(float), 256);
   return plane_set_bytes(R, SUPER, plane_count(split)) + plane_set_bytes(C, C, plane_count(split));
 }
@@ -430,16 +430,17 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   // other form, which propagates y - x against the inverse, keeps three bf16 planes.
   const bool half = uses_pairs(C, math, split) && Worig != nullptr;
   MQ_REQUIRE(!eq || half || !tensor, MQ_ERR_ARGUMENT, "mq_gptq_sweep: an equilibrated factor needs the inverse-free form");
+  const int64_t far = half ? PAIR_FAR_COLUMNS : SUPER;   // columns whose update of everything behind them is applied together
   PlaneSet err_set, u_set;
   float *row_f = nullptr, *col_f = nullptr;
   if (half) {
-    uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, SUPER, 2) / 2);
+    uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, far, 2) / 2);
     uint16_t* up = ws.take<uint16_t>(plane_set_bytes(C, C, 2) / 2);
-    row_f = ws.take<float>((size_t)R * (SUPER / TILE));
+    row_f = ws.take<float>((size_t)R * (far / TILE));
     col_f = ws.take<float>((size_t)C * 2);
     MQ_REQUIRE(ep && up && row_f && col_f, MQ_ERR_WORKSPACE, "mq_gptq_sweep: workspace too small for the operand planes");
     err_set.base = ep; err_set.planes = 2; err_set.rows_pad = (int)pad_rows(R); err_set.total_rows = err_set.rows_pad;
-    err_set.K_pad = SUPER; err_set.fp16 = true;
+    err_set.K_pad = (int)far; err_set.fp16 = true;
     MQ_TRY(make_factor_planes_half(Uhat, ldu, (int)C, up, col_f, col_div, eq, eq_bounds, &u_set, st));
   } else if (tensor) {
     uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, SUPER, split) / 2);
@@ -461,9 +462,9 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   sa.deq = deq; sa.err = err;
   sa.Worig = Worig; sa.ldwo = ldwo;
   sa.err_planes = nullptr;
-  sa.plane_stride = tensor ? err_set.total_rows * (int64_t)SUPER : 0;
+  sa.plane_stride = tensor ? err_set.total_rows * far : 0;
   sa.n_planes = half ? 2 : split;
-  sa.err_ld = tensor ? SUPER : TILE;
+  sa.err_ld = tensor ? (int)far : TILE;
   const bool uniform = group % SUB == 0;
   // Rows per CTA: the chain costs the same for 1 row and for 64, so a tile of 2048 rows takes 16.5 us on 148 SMs,
   // 17.4 on 74 and 19.0 on 48.  Alone, one CTA per SM; a caller with several layers in flight gives each
@@ -483,8 +484,8 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       // bytes the tile must move: W in, codes out, errors out, the triangle of Uhat once
       ProfScope prof(PROF_SWEEP_TILE, (double)R * nb * (4.0 + 1.0 + 4.0) + 2.0 * nb * nb, (double)R * nb * (nb - 1), st);
       sa.i1 = (int)i1; sa.nb = nb;
-      if (tensor) sa.err_planes = err_set.base + (i1 % SUPER);
-      sa.row_f = half ? row_f + (i1 % SUPER) / TILE * R : nullptr;
+      if (tensor) sa.err_planes = err_set.base + (i1 % far);
+      sa.row_f = half ? row_f + (i1 % far) / TILE * R : nullptr;
       switch (out_dtype) {
         case MQ_F32: MQ_TRY(launch_sweep_tile<MQ_F32>(chained, uniform, grid, rows, st, sa)); break;
         case MQ_BF16: MQ_TRY(launch_sweep_tile<MQ_BF16>(chained, uniform, grid, rows, st, sa)); break;
@@ -516,20 +517,27 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
       g.all_products = all_products;
       g.row_f = sa.row_f; g.col_f = col_f ? col_f + i2 : nullptr;
       PlaneSet a = err_set, b = u_set;
-      a.k0 = (int)(i1 - s0);
+      a.k0 = (int)(i1 % far);
       b.row0 = i2; b.k0 = (int)i1;
       MQ_TRY(gemm_tensor_planes(g, a, b, st));
     } else {
-      // far: W[:, s1:] += E_super Uhat[s0:s1, s1:], all errors of the super-block in one contraction
+      // The super-block is done.  By itself: W[:, s1:] += E_super Uhat[s0:s1, s1:], all errors of the super-block in one contraction.
+      // Where two go together, behind the first only the second takes its update, W[:, s1:f1] += E_super Uhat[s0:s1, s1:f1], and
+      // everything behind both takes the errors of both: W[:, s1:] += E Uhat[f0:s1, s1:].
+      const int64_t f0 = i1 / far * far, f1 = (f0 + far) < C ? (f0 + far) : C;
+      const bool joint = far > SUPER && joint_update(ceil_div(R, 256) * ceil_div(C - f0 - SUPER, 256));
+      const bool rest = joint && s1 < f1;
+      const int64_t from = joint && !rest ? f0 : s0;
       GemmDesc g;
       g.C = W + s1; g.ldc = ldw;
-      g.M = (int)R; g.N = (int)(C - s1); g.K = (int)(s1 - s0);
+      g.M = (int)R; g.N = (int)((rest ? f1 : C) - s1); g.K = (int)(s1 - from);
       g.alpha = 1.0f; g.beta = 1.0f;
       g.all_products = all_products;
-      g.row_f = row_f; g.row_f_step = R; g.col_f = col_f ? col_f + s1 : nullptr;
-      PlaneSet b = u_set;
-      b.row0 = s1; b.k0 = (int)s0;
-      MQ_TRY(gemm_tensor_planes(g, err_set, b, st));
+      g.row_f = half ? row_f + (from - f0) / TILE * R : nullptr; g.row_f_step = R; g.col_f = col_f ? col_f + s1 : nullptr;
+      PlaneSet a = err_set, b = u_set;
+      a.k0 = (int)(from - f0);
+      b.row0 = s1; b.k0 = (int)from;
+      MQ_TRY(gemm_tensor_planes(g, a, b, st));
     }
   }
   return MQ_OK;

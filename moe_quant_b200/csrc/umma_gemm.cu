@@ -1129,8 +1129,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_stream_kernel(const __gr
 // 7168-column Hessian against fp64 (2-norm, relative), three bf16 planes with one accumulator per 128 of k / this:
 // 9.0e-7 / 8.6e-7 after 4096 tokens, 5.4e-7 / 5.0e-7 after 7168, 3.8e-7 / 3.5e-7 after 14000.  All 26 deep updates
 // of a 2048 x 7168 layer: 1270 us / 855 us; of an attention block (widest layer 7168 x 16384) 18.5 ms / 10.5 ms.
-// Inside a tile the tensor pipe runs at its rate (1536 cycles per slab); what is left is the end of a tile, where
-// all SMs add 19 MB at once and the L2 takes them at about 5 TB/s.
+// Inside a tile the tensor pipe runs at its rate (1536 cycles per slab) and never waits for operands; what is left is the end of a tile, some 8000
+// cycles of which the next tile's first slabs cover 3000.  It takes as long whether the adds of all SMs come together or not (staggered starts), with
+// one box per warp under way or three (in a stage lent by the ring), and as loads, sums in shared memory and stores: the 128 KB of an SM leave
+// it at 16 bytes a cycle.  So the callers go deeper where they can (PAIR_FAR_COLUMNS).
 constexpr int PAIR_TILE = 256, PAIR_STAGES = 3, PAIR_THREADS = 384;
 constexpr uint32_t PAIR_STAGE_BYTES = 4 * PLANE_TILE_BYTES;
 constexpr size_t kPairSmem = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 8 * 4096 + 1024;

@@ -562,6 +562,49 @@ def test_sweep_running_values_against_fp64(cuda, C, g, kind, split):
         assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
 
 
+@pytest.mark.parametrize("R,C", [(2600, 2600), (7000, 1800)])
+def test_sweep_running_values_where_super_blocks_go_together(cuda, R, C):
+    """As above, with enough rows that two super-blocks of 512 columns share an update (and a last one that does not)."""
+    g = 8
+    W = synthetic.layer_weight(R, C, 5, torch.float32).to(cuda)
+    X = synthetic.activations(2 * C, C, 6, torch.bfloat16).to(cuda).double()
+    H = X.T @ X / C
+    H.diagonal().add_(0.01 * H.diagonal().mean())
+    T = torch.linalg.cholesky(H.flip(0, 1)).flip(0, 1)
+    U = (T / T.diagonal()[None, :]).float().contiguous()
+    run = W.clone()
+    scale = ops.absmax_scales(W, g, 4, torch.float32)
+    _, deq = ops.gptq_sweep(run, U, scale, None, g, C // g, 1, 4, torch.float32, True, ops.Precision(), W_original=W)
+    E, U64 = (W - deq).double(), U.double()
+    for j in range(128, C, 128):
+        e, u = E[:, :j], U64[:j, j : j + 128]
+        size = e.abs() @ u.abs()
+        want = W[:, j : j + 128].double() + e @ u
+        bound = 2.0 ** -20 * size + (C // 128 + 3) * 2.0 ** -24 * (W[:, j : j + 128].abs().double() + size)
+        assert bool(((run[:, j : j + 128].double() - want).abs() <= bound).all()), j
+
+
+@pytest.mark.parametrize("C", [3592, 4104, 5640])
+def test_factor_where_super_panels_go_together(cuda, C):
+    """Updates 1024 columns deep (three products, as many tokens as columns) against those of 512 (all four products) and fp64: the sums of 64
+    of k are the same, and one rounding of the trailing matrix less counts for more than the product that is left out."""
+    gen = torch.Generator(device=cuda).manual_seed(C)
+    X = torch.randn(C, C, generator=gen, device=cuda, dtype=torch.float64) * torch.exp(torch.randn(C, generator=gen, device=cuda, dtype=torch.float64))
+    H = X.T @ X * (2.0 / C)
+    H.diagonal().add_(0.01 * H.diagonal().mean())
+    H = H.float()
+    T = torch.linalg.cholesky(H.double().flip(0, 1)).flip(0, 1)
+    U64 = T / T.diagonal()[None, :]
+
+    def error(split):
+        U = H.clone()
+        flags, _ = ops.chol_unit_factor(U, ops.Precision(split_hinv=split))
+        assert int(flags[3]) == 0 and not bool(torch.tril(U, -1).any())
+        return float((U.double() - U64).norm() / torch.triu(U64, 1).norm())
+
+    assert error(3) < 1.1 * error(4) < 1e-6
+
+
 @pytest.mark.parametrize("C,tokens", [(648, 110), (1024, 174), (1544, 260)])
 def test_all_products_where_the_sums_cancel(cuda, C, tokens):
     """A Hessian of few tokens: the product of the low pieces takes error off the factor (its 2^-22 per product is most of
