@@ -60,7 +60,7 @@ typedef enum { MQ_MATH_FP32 = 0, MQ_MATH_TENSOR = 1 } mq_math;
  * their *_workspace_bytes): the caller processes several layers at once on different streams
  * (gptq.quantize_many).  The library then prefers launch shapes that occupy few SMs over the
  * lowest latency of a single layer: the sweep's tiles take more rows per CTA (R/44
- * instead of R/148, at most 64), a CTA of a rank-128 strip update walks a whole
+ * instead of R/148, at most 64; R/74 where a launch takes 512 columns), a CTA of a rank-128 strip update walks a whole
  * row of output tiles, a CTA of a panel solve takes 64 rows instead of 32.  Results are bit-identical with and without it. */
 #define MQ_MATH_COMPACT 0x100
 

@@ -32,7 +32,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
                void* deq, const float* Worig, int64_t ldwo, int math, int split, Workspace& ws, cudaStream_t st,
                const float* col_div, const float* eq, bool eq_bounds, int32_t* packed);
 int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, int split, mq_layer_flags* flags,
-                     Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled, const float* eq);
+                     Workspace& ws, cudaStream_t st, bool upper_only, int unscaled, const float* eq);
 int copy_upper_scaled(const float* src, int64_t lds, float* dst, int64_t ldd, int64_t C, const float* eq, cudaStream_t st);
 int hessian_accum_tensor(const void* X, int x_dtype, int64_t m, int64_t C, int64_t ldx, float* H, int64_t ldh, float beta,
                          float alpha, int split, Workspace& ws, cudaStream_t st);
@@ -163,7 +163,7 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   // pairs).  The sweep takes an equilibrated factor only where it works on such pairs itself; otherwise the
   // factorisation gives its result back in H's units.
   const bool pairs = uses_pairs(C, math, split_hinv) && uses_pairs(C, math, split_sweep);
-  const bool unscaled = math == MQ_MATH_TENSOR && (pairs || !uses_pairs(C, math, split_hinv));
+  const int unscaled = math == MQ_MATH_TENSOR && (pairs || !uses_pairs(C, math, split_hinv)) ? (sweep_by_super_blocks(R, math) ? SUPER_COLUMNS : 128) : 0;
   // W.clone().float(), pre-step, masking and damping, grid; driven by the first layer's weight: the handle that
   // owns H.  A tied handle meets an H that is already regularised and changes neither H nor its own
   // weight (src/gptq.py:129-136, 227).       src/gptq.py:140-152, 224-234, src/quant_utils.py:75-101

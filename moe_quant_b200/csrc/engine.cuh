@@ -90,11 +90,21 @@ inline bool uses_pairs(int64_t C, int math, int split) {
 }
 inline int plane_count(int split) { return split == 4 ? 3 : split; }
 
+// Columns of a super-block of the sweep and of a super-panel of the factorisation.
+constexpr int SUPER_COLUMNS = 512;
 // Columns whose update of everything behind them (in front of them, in the factorisation) is applied together where operands are pairs.
 constexpr int64_t PAIR_FAR_COLUMNS = 1024;
 // ... provided that the first half's update by itself, `tiles` of 256 x 256, is more than one for each of the 74 CTA pairs.  Otherwise an update takes as long
 // as one tile, and one tile of 1024 takes longer than one of 512 (1056 columns: 544 us instead of 535).
 inline bool joint_update(long long tiles) { return tiles > 74; }
+
+// Whether a sweep takes a super-block of SUPER_COLUMNS per launch (sweep_super.cu) instead of a 128-column tile and the update behind it.
+// The factor's diagonal blocks of that size are then scaled as a whole.  Of one layer with 4096 columns (its quantization, us, tiles /
+// super-blocks) 512 rows take 1574 / 1462, 1024 rows 1598 / 1485, 2048 rows 1670 / 1558; but with several layers in flight the super-blocks'
+// SM time counts, and the two must agree to the last bit there: four experts of 512 x 4096 take 6.66 / 5.80 ms, 1024 x 4096 6.38 / 6.38,
+// 1024 x 7168 11.53 / 11.57, 1536 x 7168 12.46 / 12.87, 2048 x 7168 13.9 / 15.3.
+constexpr int64_t SUPER_BLOCK_ROWS = 1024;
+inline bool sweep_by_super_blocks(int64_t R, int math) { return (math & ~MQ_MATH_COMPACT) == MQ_MATH_TENSOR && R <= SUPER_BLOCK_ROWS; }
 
 // Tensor-core GEMM whose operands are already planes (d.A / d.B and their strides are ignored;
 // d.K is the reduction length starting at k0 of each set).  Both sets must have the same
@@ -114,10 +124,10 @@ int make_planes_f32(const float* src, int64_t rs, int64_t cs, int rows, int K, i
 // t_j a power of two that brings the column's entries under 2^14: from the column's maximum (a pass of its own), or, where
 // eq_bounds says that this is near enough, with the C factors eq of an equilibration followed by the smallest of them, from the
 // bound 2^14 / eq[C] that every entry of U[i][j] / eq[i] keeps.  inv_t (2 C floats)
-// receives 1 / t_j in its first half, the second is scratch.  Only k in 128-blocks in front of the row's own
-// block are written.
+// receives 1 / t_j in its first half, the second is scratch.  Only k in the blocks of `own` columns (128 or SUPER_COLUMNS) in
+// front of the row's own are written (and read), inv_t from the second such block on.
 int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, float* inv_t, const float* col_div, const float* eq,
-                            bool eq_bounds, PlaneSet* out, cudaStream_t st);
+                            bool eq_bounds, int own, PlaneSet* out, cudaStream_t st);
 
 // Whether that bound is near enough, by the damping: diag(T) is at least sqrt(rel_damp mean(diag H)), so the bound exceeds Utilde's unit
 // diagonal by at most 2 sqrt(C / rel_damp), 2^11.5 here, and what a pair of fp16 planes drops (2^-39 of it) stays below

@@ -33,7 +33,8 @@ namespace {
 
 constexpr int NB = 128;  // panel width
 constexpr int SUPER_PANELS = 4;               // panels whose update of what lies in front of them is applied together
-constexpr int SUPER_NB = SUPER_PANELS * NB;   // 512
+constexpr int SUPER_NB = SUPER_PANELS * NB;
+static_assert(SUPER_NB == SUPER_COLUMNS, "a super-panel");
 
 // ------------------------------------------------------------------ diagonal block
 // D (nb x nb, upper triangle valid) -> T_d upper with D = T_d T_d^T, by one CTA, eight pivots at a time (a "leaf", columns
@@ -703,20 +704,14 @@ __device__ __forceinline__ void scale_quad(float* __restrict__ H, int64_t ld, co
   *reinterpret_cast<float4*>(H + r * ld + c) = o;
 }
 
-// The end of an unscaled factorisation, one CTA per diagonal 128-block: the block divided by diag(T)
-// (the sweep tiles read the diagonal blocks; the blocks above are divided by whoever splits them into planes).
-__global__ void __launch_bounds__(1024) finish_diag_blocks_kernel(float* __restrict__ H, int64_t C, int64_t ld,
-                                                                 const float* __restrict__ diag, const float* __restrict__ eq) {
-  __shared__ __align__(16) float d[NB];
-  const int64_t k0 = (int64_t)blockIdx.x * NB;
-  const int nb = C - k0 < NB ? (int)(C - k0) : NB;
-  const int t = threadIdx.x;
-  if (t < nb) d[t] = diag[k0 + t];
-  __syncthreads();
-  for (int idx = t; idx < nb * (NB / 4); idx += blockDim.x) {
-    const int r = idx >> 5, c = (idx & 31) * 4;
-    if (c < nb && c + 3 >= r) scale_quad(H, ld, d - k0, eq, k0 + r, k0 + c);   // C % 8 == 0: quads are whole
-  }
+// The end of an unscaled factorisation: the diagonal blocks of `own` columns divided by diag(T)
+// (the sweep kernels read them; the blocks above are divided by whoever splits them into planes).  A warp takes a row.
+__global__ void __launch_bounds__(256) finish_diag_blocks_kernel(float* __restrict__ H, int64_t C, int64_t ld, int own,
+                                                                const float* __restrict__ diag, const float* __restrict__ eq) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= C) return;
+  const int64_t end = (r / own + 1) * own < C ? (r / own + 1) * own : C;   // C % 8 == 0: quads are whole
+  for (int64_t c = r / 4 * 4 + (threadIdx.x & 31) * 4; c < end; c += 128) scale_quad(H, ld, diag, eq, r, c);
 }
 
 __global__ void __launch_bounds__(256) scale_columns_kernel(float* __restrict__ H, int64_t C, int64_t ld,
@@ -872,14 +867,14 @@ size_t hinv_workspace_bytes(int64_t C, int math, int split) {
 
 // H (damped, symmetric; upper triangle read) -> unit upper factor Utilde = T diag(T)^-1 in place,
 // zeros below the diagonal (upper_only: the part below the diagonal blocks is neither read nor written;
-// unscaled: only the diagonal blocks are scaled; above them T itself is left in place and the caller
+// unscaled, if not 0: only the diagonal blocks of that many columns are scaled; above them T itself is left in place and the caller
 // divides column c by diag[c] where it reads it).  diag (C floats, device) receives diag(T).  On a non-positive pivot
 // flags->not_positive is set and the result is replaced by I.
 // eq (uses_pairs only): H has been equilibrated by the caller (copy_upper_scaled) with these
 // factors; unscaled then leaves the equilibrated factor above the diagonal blocks and its diagonal in diag.
 // Null: where pairs are used the matrix is equilibrated here and everything is given back in H's own units.
 int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, int split, mq_layer_flags* flags,
-                     Workspace& ws, cudaStream_t st, bool upper_only, bool unscaled, const float* eq) {
+                     Workspace& ws, cudaStream_t st, bool upper_only, int unscaled, const float* eq) {
   MQ_TRY(configure_once());
   const int compact = (math & MQ_MATH_COMPACT) ? 1 : 0;   // the panel solves and the rank-128 strips look at it
   math &= ~MQ_MATH_COMPACT;
@@ -1018,7 +1013,7 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
   }
   // ---- T -> unit-diagonal factor
   if (unscaled) {
-    finish_diag_blocks_kernel<<<(unsigned)P, 1024, 0, st>>>(H, C, ldh, diag, eq);
+    finish_diag_blocks_kernel<<<(unsigned)ceil_div(C, 8), 256, 0, st>>>(H, C, ldh, unscaled, diag, eq);
     MQ_LAUNCH_CHECK();
   } else {
     const unsigned gx = (unsigned)(ceil_div(C, 256) < 8 ? ceil_div(C, 256) : 8);
@@ -1041,7 +1036,7 @@ int hinv_upper(float* H, int64_t C, int64_t ldh, float* Uhat, int64_t ldu, float
   MQ_REQUIRE(diag && scratch, MQ_ERR_WORKSPACE, "mq_hinv_upper: workspace too small");
   // The factor is the result here and no sweep averages its error: with three products it is 1.00 to 1.02 of that of three planes
   // (648 to 4096 columns, as many tokens), with all four 0.98 to 1.00.
-  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split == 3 ? 4 : split, flags, ws, st, false, false, nullptr));
+  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split == 3 ? 4 : split, flags, ws, st, false, 0, nullptr));
   if (diag_out) MQ_CUDA(cudaMemcpyAsync(diag_out, diag, C * sizeof(float), cudaMemcpyDeviceToDevice, st));
   Engine eng(math, plane_count(split), ws, st);
   const int P = (int)ceil_div(C, NB);
@@ -1114,7 +1109,7 @@ extern "C" int mq_chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag
   float* diag = ws.take<float>(C);
   MQ_REQUIRE(diag, MQ_ERR_WORKSPACE, "mq_chol_unit_factor: workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split, flags, ws, st, false, false, nullptr));
+  MQ_TRY(chol_unit_factor(H, C, ldh, diag, math, split, flags, ws, st, false, 0, nullptr));
   if (diag_out) MQ_CUDA(cudaMemcpyAsync(diag_out, diag, C * sizeof(float), cudaMemcpyDeviceToDevice, st));
   return MQ_OK;
 }

@@ -2,6 +2,8 @@
 // reference's captured loop (src/gptq_loop.py:141-148) with, per 128-column tile,
 // ONE sweep kernel plus ONE GEMM.
 //
+// (Up to 1024 rows a launch takes 512 columns instead: sweep_super.cu.)
+//
 // Sweep kernel: a CTA takes up to 64 weight rows through the tile in sub-blocks of sixteen columns.
 // Column j is quantized as
 //   q = clamp(floor(x/s + z + 0.5), 0, maxq)   y = round_to_dtype((q - z) s)   e = y - x
@@ -19,6 +21,7 @@
 // written straight into the (R, C) uint8 result, so the transposes of src/gptq.py:191-199
 // never happen.
 #include "engine.cuh"
+#include "mbarrier.cuh"
 #include "profile.cuh"
 #include "sweep.cuh"
 
@@ -36,7 +39,7 @@ constexpr int W_LD = TILE + 4;          // row stride of the running weights: a 
 // super-block takes the rank-128 update at once; the columns behind the super-block are updated
 // once per super-block with all 512 errors of a row in one contraction, so a tile of W is read
 // and written once per 512 instead of once per 128 swept columns.
-constexpr int SUPER = 4 * TILE;
+constexpr int SUPER = SUPER_COLUMNS;
 
 constexpr size_t sweep_smem_bytes(int rows, bool uniform) {
   return (size_t)(TILE * TILE + rows * W_LD + rows * (uniform ? N_SUB : 2 * SUB) * 4) * sizeof(float);
@@ -309,49 +312,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
     for (int idx = tid; idx < rows * (TILE / 8); idx += SWEEP_THREADS) {
       const int r = idx >> 4, k = (idx & 15) * 8;
       const float4 lo4 = *reinterpret_cast<const float4*>(ws + r * W_LD + k), hi4 = *reinterpret_cast<const float4*>(ws + r * W_LD + k + 4);
-      const float e[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
-      const int64_t gr = row0 + r;
-      if (!a.err_planes) {
-        float4* dst = reinterpret_cast<float4*>(a.err + gr * a.err_ld + k);
-        dst[0] = lo4;
-        dst[1] = hi4;
-        continue;
-      }
-      uint32_t p0[4], p1[4], p2[4];
-      if (a.row_f) {
-        // The largest error of the row's 128 comes just under 2^14, so that a pair holds 22 bits of every error down to 2^-17 of
-        // it; the sixteen lanes of a row agree on it.  (One power of two per row of the matrix cost a row whose groups differ
-        // by 2^20 the last bits of its small groups: 13 to 16 times the error of three bf16 planes there.)
-        float m = 0.0f;
-#pragma unroll
-        for (int t = 0; t < 8; ++t) m = fmaxf(m, fabsf(e[t]));
-        const unsigned half_warp = 0xffffu << (lane & 16);
-        for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(half_warp, m, o));
-        const float rho = scale_below_2_14(m);
-        if ((lane & 15) == 0) a.row_f[gr] = 1.0f / rho;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          uint16_t h0, l0, h1, l1;
-          split_half2(e[2 * t] * rho, h0, l0);
-          split_half2(e[2 * t + 1] * rho, h1, l1);
-          p0[t] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-          p1[t] = (uint32_t)l0 | ((uint32_t)l1 << 16);
-        }
-      } else {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          uint16_t h0, m0, l0, h1, m1, l1;
-          split_bf16x3(e[2 * t], h0, m0, l0);
-          split_bf16x3(e[2 * t + 1], h1, m1, l1);
-          p0[t] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-          p1[t] = (uint32_t)m0 | ((uint32_t)m1 << 16);
-          p2[t] = (uint32_t)l0 | ((uint32_t)l1 << 16);
-        }
-      }
-      uint16_t* dst = a.err_planes + gr * a.err_ld + k;
-      *reinterpret_cast<uint4*>(dst) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
-      if (a.n_planes > 1) *reinterpret_cast<uint4*>(dst + a.plane_stride) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-      if (a.n_planes > 2) *reinterpret_cast<uint4*>(dst + 2 * a.plane_stride) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+      write_errors(a, row0 + r, k, lo4, hi4, lane);
     }
     __syncthreads();   // the next group's weights replace the errors
   }
@@ -407,7 +368,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
                const float* col_div, const float* eq, bool eq_bounds, int32_t* packed) {
   // col_div (tensor math only): above its diagonal 128-blocks Uhat holds the factor before its
   // columns were divided by col_div; the plane split divides where it reads it.  The diagonal
-  // blocks, which the tiles read, are already scaled.  eq (with col_div): what lies above is the factor
+  // blocks, which the tiles read, are already scaled (blocks of SUPER columns where sweep_by_super_blocks says so).  eq (with col_div): what lies above is the factor
   // of the equilibrated matrix, entry (i, j) times eq[j] / eq[i] is the one of the matrix itself; eq_bounds: see
   // make_factor_planes_half.
   MQ_TRY(configure_once());
@@ -430,6 +391,8 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   // other form, which propagates y - x against the inverse, keeps three bf16 planes.
   const bool half = uses_pairs(C, math, split) && Worig != nullptr;
   MQ_REQUIRE(!eq || half || !tensor, MQ_ERR_ARGUMENT, "mq_gptq_sweep: an equilibrated factor needs the inverse-free form");
+  const bool by_super = sweep_by_super_blocks(R, math);
+  const int own = by_super ? SUPER : TILE;               // diagonal blocks of this size are already divided by col_div, and need no planes
   const int64_t far = half ? PAIR_FAR_COLUMNS : SUPER;   // columns whose update of everything behind them is applied together
   PlaneSet err_set, u_set;
   float *row_f = nullptr, *col_f = nullptr;
@@ -441,8 +404,8 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
     MQ_REQUIRE(ep && up && row_f && col_f, MQ_ERR_WORKSPACE, "mq_gptq_sweep: workspace too small for the operand planes");
     err_set.base = ep; err_set.planes = 2; err_set.rows_pad = (int)pad_rows(R); err_set.total_rows = err_set.rows_pad;
     err_set.K_pad = (int)far; err_set.fp16 = true;
-    MQ_TRY(make_factor_planes_half(Uhat, ldu, (int)C, up, col_f, col_div, eq, eq_bounds, &u_set, st));
-  } else if (tensor) {
+    MQ_TRY(make_factor_planes_half(Uhat, ldu, (int)C, up, col_f, col_div, eq, eq_bounds, own, &u_set, st));
+  } else if (tensor && !(by_super && C <= SUPER)) {   // (a single super-block has no updates)
     uint16_t* ep = ws.take<uint16_t>(plane_set_bytes(R, SUPER, split) / 2);
     uint16_t* up = ws.take<uint16_t>(plane_set_bytes(C, C, split) / 2);
     MQ_REQUIRE(ep && up, MQ_ERR_WORKSPACE, "mq_gptq_sweep: workspace too small for the operand planes");
@@ -460,6 +423,7 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   sa.codes = codes; sa.C = C;
   sa.packed = packed;
   sa.deq = deq; sa.err = err;
+  MQ_TRY(engine_fault_word(&sa.fault));
   sa.Worig = Worig; sa.ldwo = ldwo;
   sa.err_planes = nullptr;
   sa.plane_stride = tensor ? err_set.total_rows * far : 0;
@@ -475,21 +439,27 @@ int gptq_sweep(float* W, int64_t R, int64_t C, int64_t ldw, const float* Uhat, i
   const int64_t row_groups = ceil_div(R, rows);
   const int grid = (int)(row_groups < 148 ? row_groups : 148);
 
-  for (int64_t i1 = 0; i1 < C; i1 += TILE) {
-    const int nb = (int)((C - i1) < TILE ? (C - i1) : TILE);
+  const int64_t step = by_super ? SUPER : TILE;
+  for (int64_t i1 = 0; i1 < C; i1 += step) {
+    const int nb = (int)((C - i1) < step ? (C - i1) : step);
     {
-      // The kernel stages its tile of the factor before it waits for its predecessor: only a launch
+      // The kernels stage their part of the factor before they wait for their predecessor: only a launch
       // that follows this loop's own update (which writes W, never the factor) may be chained.
       const bool chained = i1 > 0;
-      // bytes the tile must move: W in, codes out, errors out, the triangle of Uhat once
+      // bytes the launch must move: W in, codes out, errors out, the triangle of Uhat once
       ProfScope prof(PROF_SWEEP_TILE, (double)R * nb * (4.0 + 1.0 + 4.0) + 2.0 * nb * nb, (double)R * nb * (nb - 1), st);
       sa.i1 = (int)i1; sa.nb = nb;
       if (tensor) sa.err_planes = err_set.base + (i1 % far);
       sa.row_f = half ? row_f + (i1 % far) / TILE * R : nullptr;
-      switch (out_dtype) {
-        case MQ_F32: MQ_TRY(launch_sweep_tile<MQ_F32>(chained, uniform, grid, rows, st, sa)); break;
-        case MQ_BF16: MQ_TRY(launch_sweep_tile<MQ_BF16>(chained, uniform, grid, rows, st, sa)); break;
-        default: MQ_TRY(launch_sweep_tile<MQ_F16>(chained, uniform, grid, rows, st, sa));
+      if (by_super) {
+        if (i1 + nb >= C) sa.err_planes = nullptr;   // nothing behind it
+        MQ_TRY(sweep_super_block(chained, uniform, compact, out_dtype, sa, st));
+      } else {
+        switch (out_dtype) {
+          case MQ_F32: MQ_TRY(launch_sweep_tile<MQ_F32>(chained, uniform, grid, rows, st, sa)); break;
+          case MQ_BF16: MQ_TRY(launch_sweep_tile<MQ_BF16>(chained, uniform, grid, rows, st, sa)); break;
+          default: MQ_TRY(launch_sweep_tile<MQ_F16>(chained, uniform, grid, rows, st, sa));
+        }
       }
     }
     MQ_LAUNCH_CHECK();

@@ -1894,14 +1894,14 @@ __global__ void __launch_bounds__(256) split_transposed_f32_kernel(SplitParams p
 }
 
 // Column maxima of the factor's blocks above the diagonal: colmax[j] = max_i |U[i][j]| over the rows in
-// front of column j's 128-block, as the bits of a non-negative float (they order like integers); with eq of |U[i][j]| / eq[i].
+// front of column j's block of `own` columns, as the bits of a non-negative float (they order like integers); with eq of |U[i][j]| / eq[i].
 // One CTA takes 128 columns x `rows_per` rows: a warp reads 512 bytes of a row at a time, four in flight.
-__global__ void __launch_bounds__(256) factor_colmax_kernel(const float* __restrict__ U, int64_t ldu, int C, int rows_per,
+__global__ void __launch_bounds__(256) factor_colmax_kernel(const float* __restrict__ U, int64_t ldu, int C, int rows_per, int own,
                                                             const float* __restrict__ eq, int* __restrict__ colmax) {
   __shared__ float part[8][TILE_N];
-  const int j0 = ((int)blockIdx.x + 1) * TILE_N;   // the first block of columns has nothing above it
-  const int r_begin = (int)blockIdx.y * rows_per;
-  const int r_end = r_begin + rows_per < j0 ? r_begin + rows_per : j0;
+  const int j0 = own + (int)blockIdx.x * TILE_N;   // the first block of columns has nothing above it
+  const int above = j0 / own * own, r_begin = (int)blockIdx.y * rows_per;
+  const int r_end = r_begin + rows_per < above ? r_begin + rows_per : above;
   if (r_begin >= r_end) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = j0 + lane * 4;
@@ -1937,10 +1937,10 @@ __global__ void __launch_bounds__(256) factor_colmax_kernel(const float* __restr
 __global__ void __launch_bounds__(256) split_factor_half_kernel(const float* __restrict__ U, int64_t ldu, int C, int rows_pad, int K_pad,
                                                                 const float* __restrict__ col_div, const float* __restrict__ eq,
                                                                 const int* __restrict__ colmax, float* __restrict__ inv_t,
-                                                                uint16_t* __restrict__ dst, int64_t plane_stride) {
+                                                                int own, uint16_t* __restrict__ dst, int64_t plane_stride) {
   __shared__ float tile[64][65];  // tile[k][r]
   const int r0 = blockIdx.y * 64, k0 = blockIdx.x * 64;
-  if (k0 >= (r0 / TILE_M) * TILE_M) return;
+  if (k0 >= r0 / own * own) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -2425,7 +2425,7 @@ int make_planes_f32(const float* src, int64_t rs, int64_t cs, int rows, int K, i
 }
 
 int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, float* inv_t, const float* col_div, const float* eq,
-                            bool eq_bounds, PlaneSet* out, cudaStream_t st) {
+                            bool eq_bounds, int own, PlaneSet* out, cudaStream_t st) {
   PlaneSet ps;
   ps.planes = 2;
   ps.rows_pad = pad_to(C, TILE_M);
@@ -2434,18 +2434,18 @@ int make_factor_planes_half(const float* U, int64_t ldu, int C, uint16_t* dst, f
   ps.fp16 = true;
   ps.base = dst;
   *out = ps;
-  if (C <= TILE_M) return MQ_OK;   // no block above the diagonal
+  if (C <= own) return MQ_OK;   // no block above the diagonal
   int* colmax = eq && eq_bounds ? nullptr : reinterpret_cast<int*>(inv_t + C);
   ProfScope prof(PROF_SPLIT, (double)C * C * 0.5 * (4.0 + 4.0), 0.0, st);
   if (colmax) {
     MQ_CUDA(cudaMemsetAsync(colmax, 0, (size_t)C * sizeof(int), st));
-    const int col_blocks = (int)ceil_div(C, TILE_N) - 1;
+    const int col_blocks = (int)ceil_div(C - own, TILE_N);
     const int rows_per = 128;
-    factor_colmax_kernel<<<dim3((unsigned)col_blocks, (unsigned)ceil_div(C, rows_per)), 256, 0, st>>>(U, ldu, C, rows_per, eq, colmax);
+    factor_colmax_kernel<<<dim3((unsigned)col_blocks, (unsigned)ceil_div(C, rows_per)), 256, 0, st>>>(U, ldu, C, rows_per, own, eq, colmax);
     MQ_LAUNCH_CHECK();
   }
   split_factor_half_kernel<<<dim3((unsigned)(ps.K_pad / 64), (unsigned)ceil_div(ps.rows_pad, 64)), 256, 0, st>>>(
-      U, ldu, C, ps.rows_pad, ps.K_pad, col_div, eq, colmax, inv_t, dst, ps.total_rows * (int64_t)ps.K_pad);
+      U, ldu, C, ps.rows_pad, ps.K_pad, col_div, eq, colmax, inv_t, own, dst, ps.total_rows * (int64_t)ps.K_pad);
   MQ_LAUNCH_CHECK();
   return MQ_OK;
 }

@@ -857,6 +857,36 @@ def test_sweep_tile_row_groups(cuda, R, C, g):
     assert torch.equal(got, sweep(W.to(cuda), ops.Precision(compact=True)))
 
 
+# ------------------------------------------------------------------ super-blocks of the sweep
+@pytest.mark.parametrize("R", [1, 9, 1024, 1025])
+@pytest.mark.parametrize("C,g", [(24, 8), (136, 136), (520, 8), (1160, 40), (1536, 128)])
+@pytest.mark.parametrize("inverse_free", [True, False])
+def test_sweep_by_super_blocks(cuda, R, C, g, inverse_free):
+    """Up to 1024 rows a launch takes 512 columns: last blocks of eight columns and of one tile, CTAs that are not full, scales per
+    sub-block and per column with zero points of their own, both recurrences, and the row behind the last that goes this way.
+    Codes as on the fp32 CUDA cores, the compact launch's bits."""
+    W = synthetic.layer_weight(R, C, 5, torch.bfloat16).float().to(cuda)
+    X = synthetic.activations(2 * C, C, 6, torch.bfloat16).double()
+    H = X.T @ X / C
+    H.diagonal().add_(0.01 * H.diagonal().mean())
+    U = H.float().to(cuda)
+    if inverse_free:
+        ops.chol_unit_factor(U)
+    else:
+        U = ops.hinv_upper(U)[0]
+    scale = ops.absmax_scales(W, g, 4, torch.bfloat16)
+    zero = (8 - torch.arange(scale.numel(), device=cuda).reshape(scale.shape) % 3).float().contiguous()
+
+    def sweep(precision):
+        return ops.gptq_sweep(W.clone(), U, scale, zero, g, C // g, 1, 4, torch.bfloat16, True, precision, W_original=W if inverse_free else None)
+
+    (q, deq), (q0, _), (q1, deq1) = sweep(ops.Precision()), sweep(ops.Precision(math=MATH_FP32)), sweep(ops.Precision(compact=True))
+    # a code on a rounding boundary takes others of its row along: of few codes those of one row in a hundred may differ
+    assert int((q != q0).sum()) <= max(0.005 * q.numel(), 0.01 * C)
+    assert torch.equal(q, q1) and torch.equal(deq, deq1)
+    assert torch.equal(deq, ops.dequantize(q, scale, zero, g, 4, torch.bfloat16))
+
+
 # ------------------------------------------------------------------ the weights' way in, the diagonal pass
 @pytest.mark.parametrize("R,C,g", [(1, 8, 8), (65, 136, 8), (7, 160, 32), (64, 192, 64), (130, 1152, 128), (3, 9216, 64)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
