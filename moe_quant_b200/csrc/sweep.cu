@@ -41,8 +41,8 @@ constexpr int W_LD = TILE + 4;          // row stride of the running weights: a 
 // and written once per 512 instead of once per 128 swept columns.
 constexpr int SUPER = SUPER_COLUMNS;
 
-constexpr size_t sweep_smem_bytes(int rows, bool uniform) {
-  return (size_t)(TILE * TILE + rows * W_LD + rows * (uniform ? N_SUB : 2 * SUB) * 4) * sizeof(float);
+constexpr size_t sweep_smem_bytes(int rows, bool uniform, bool inverse_free) {
+  return (size_t)(TILE * TILE + rows * W_LD * (inverse_free ? 2 : 1) + rows * (uniform ? N_SUB : 2 * SUB) * 4) * sizeof(float);
 }
 
 // One 128 x 128 tile of the factor (top-left element at `src`) -> shared memory, row-major, by
@@ -88,9 +88,10 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
   extern __shared__ __align__(16) float sweep_smem[];
   float* us = sweep_smem;                            // [TILE][TILE], strict upper triangle
   float* ws = sweep_smem + TILE * TILE;              // [group_rows][W_LD]: running weights, replaced by the errors as they become known
+  float* wos = ws + group_rows * W_LD;               // INVERSE_FREE: [group_rows][W_LD], original weights
   // the grid of every row (scale, its reciprocal, zero point): UNIFORM [N_SUB][group_rows], one per sub-block;
   // otherwise [2][SUB][group_rows], the columns of two sub-blocks by turns
-  float4* gs = reinterpret_cast<float4*>(ws + group_rows * W_LD);
+  float4* gs = reinterpret_cast<float4*>(ws + group_rows * W_LD * (INVERSE_FREE ? 2 : 1));
   const int nb = a.nb, i1 = a.i1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // The factor is constant during the sweep: its tile is staged before this grid waits for the
   // rank-128 update that precedes it in the stream (only W depends on that update).
@@ -110,6 +111,10 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
       const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&ws[r * W_LD + k4]);
       const float* g = a.W + (int64_t)(row0 + r) * a.ldw + i1 + (keep ? k4 : 0);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(g), "r"(keep ? 16 : 0) : "memory");
+      if constexpr (INVERSE_FREE) {
+        const float* go = a.Worig + (int64_t)(row0 + r) * a.ldwo + i1 + (keep ? k4 : 0);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + group_rows * W_LD * 4), "l"(go), "r"(keep ? 16 : 0) : "memory");
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     auto grid_of = [&](int r, int j) {   // column j of the tile
@@ -139,17 +144,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
       const int r = valid ? tid : rows - 1;
       const int64_t row = row0 + r;
       float* wrow = ws + r * W_LD;
-      const float* worow = INVERSE_FREE ? a.Worig + row * a.ldwo + i1 : nullptr;
-      float w[SUB], wo[SUB];
-      auto fetch_original = [&](int j0) {
-#pragma unroll
-        for (int qd = 0; qd < SUB / 4; ++qd) {
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (INVERSE_FREE && j0 + 4 * qd < nb) v = __ldg(reinterpret_cast<const float4*>(worow + j0 + 4 * qd));
-          wo[4 * qd] = v.x; wo[4 * qd + 1] = v.y; wo[4 * qd + 2] = v.z; wo[4 * qd + 3] = v.w;
-        }
-      };
-      fetch_original(0);
+      const float* worow = wos + r * W_LD;
+      float w[SUB];
 #pragma unroll
       for (int qd = 0; qd < SUB / 4; ++qd) {
         const float4 v = *reinterpret_cast<const float4*>(wrow + 4 * qd);
@@ -172,6 +168,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
         }
         float e[SUB];
         uint32_t cw[SUB / 4];
+        float4 wo = make_float4(0.f, 0.f, 0.f, 0.f);
         const float* ud = us + j0 * TILE + j0;   // the sub-block's own 16 x 16 block of the factor
 #pragma unroll
         for (int t = 0; t < SUB; ++t) {
@@ -192,7 +189,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
           const float big = __fadd_rd(v, 8388608.0f);
           const float q = big - 8388608.0f;
           const float y = round_through<DT>((q - z_t) * s_t);
-          const float et = INVERSE_FREE ? (wo[t] - y) : (y - x);
+          if (INVERSE_FREE && (t & 3) == 0) wo = *reinterpret_cast<const float4*>(worow + j0 + t);
+          const float et = INVERSE_FREE ? ((t & 3) == 0 ? wo.x : (t & 3) == 1 ? wo.y : (t & 3) == 2 ? wo.z : wo.w) - y : y - x;
           e[t] = et;
           const uint32_t code = __float_as_uint(big) & 0xFFu;
           if ((t & 3) == 0) cw[t >> 2] = code;
@@ -214,7 +212,6 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
             w[4 * qd] = p01.x; w[4 * qd + 1] = p01.y; w[4 * qd + 2] = p23.x; w[4 * qd + 3] = p23.y;
           }
         }
-        if (c + 1 < N_SUB) fetch_original(j0 + SUB);
         if (valid) {
 #pragma unroll
           for (int qd = 0; qd < SUB / 4; ++qd)
@@ -324,13 +321,13 @@ int launch_sweep_tile(bool chained, bool uniform, int grid, int rows, cudaStream
   const bool free = args.Worig != nullptr;
   auto* kernel = uniform ? (free ? sweep_tile_kernel<DT, true, true> : sweep_tile_kernel<DT, true, false>)
                          : (free ? sweep_tile_kernel<DT, false, true> : sweep_tile_kernel<DT, false, false>);
-  MQ_CUDA(launch_chained(chained, kernel, dim3(grid), dim3(SWEEP_THREADS), sweep_smem_bytes(rows, uniform), st, args, rows));
+  MQ_CUDA(launch_chained(chained, kernel, dim3(grid), dim3(SWEEP_THREADS), sweep_smem_bytes(rows, uniform, free), st, args, rows));
   return MQ_OK;
 }
 
 template <int DT>
 int configure_dtype() {
-  constexpr int bytes = (int)sweep_smem_bytes(MAX_ROWS, false);
+  constexpr int bytes = (int)sweep_smem_bytes(MAX_ROWS, false, true);
   MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   MQ_CUDA(cudaFuncSetAttribute(sweep_tile_kernel<DT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
