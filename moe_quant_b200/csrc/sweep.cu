@@ -72,11 +72,11 @@ __device__ __forceinline__ void stage_factor_tile(float* us, const float* __rest
 // warps have added everything up to c - 1 there.  Every element so takes the errors in increasing column order
 // with one FMA each, as a column-at-a-time recurrence does.
 // What bounds a tile is the chain, 128 steps of 84 cycles whatever the number of rows (5.6 us), and handing the
-// sub-blocks over, 800 to 1100 cycles each (3.7 us).  (With
+// sub-blocks over, 700 to 1000 cycles each (3.4 us).  (Original weights that the chain loaded itself, a sub-block ahead, cost a sweep of
+// 2048 x 7168 45 us of 1485, and staging them behind the wait for the update in front another 8; the scales are as well off behind it.  With
 // sixteen or eight lanes per row and the row's tile in their registers, the owner of a chunk ran its chain while
 // the others waited, and both the chain and the rest were one serial instruction stream: 19 us for 2048 rows,
-// 36 us for 7168; one row per thread for everything, 30 us.  Now 16.5 and 20 us, and 15.7 instead of 20.3 us
-// with a scale per column.)
+// 36 us for 7168; one row per thread for everything, 30 us.  Now 15.7 and 19 us.)
 // UNIFORM: the columns of a sub-block lie in one quantization group (group % 16 == 0).
 // INVERSE_FREE (a.Worig given): U is the unit factor Utilde = Uhat^-1 and what is propagated is minus the
 // total change of the column, -(y - w_original), instead of the error against the running value;
@@ -93,48 +93,51 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
   // otherwise [2][SUB][group_rows], the columns of two sub-blocks by turns
   float4* gs = reinterpret_cast<float4*>(ws + group_rows * W_LD * (INVERSE_FREE ? 2 : 1));
   const int nb = a.nb, i1 = a.i1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // The factor is constant during the sweep: its tile is staged before this grid waits for the
-  // rank-128 update that precedes it in the stream (only W depends on that update).
-  stage_factor_tile(us, a.U + (int64_t)i1 * a.ldu + i1, a.ldu, nb);
-  chain_wait();
-  chain_release();
   const float maxq = a.maxq;
   const bool wide_codes = (a.C & 15) == 0 && (reinterpret_cast<uintptr_t>(a.codes) & 15) == 0;
   const uint32_t group = (uint32_t)a.group;
-
-  for (int row0 = blockIdx.x * group_rows; row0 < a.R; row0 += gridDim.x * group_rows) {
-    const int rows = a.R - row0 < group_rows ? a.R - row0 : group_rows;
-    const int chain_warps = (rows + 31) >> 5;
+  int row0 = blockIdx.x * group_rows, rows = a.R - row0 < group_rows ? a.R - row0 : group_rows;   // the grid has no CTA without rows
+  auto grid_of = [&](int r, int j) {   // column j of the tile
+    float s = 1.0f, z = a.zero_default;
+    if (j < nb) {
+      const int64_t off = (int64_t)(row0 + r) * a.s_rs + (int64_t)((uint32_t)(i1 + j) / group) * a.s_gs;
+      s = __ldg(a.scale + off);
+      if (a.zero) z = __ldg(a.zero + off);
+    }
+    return make_float4(s, 1.0f / s, z, 0.0f);
+  };
+  auto fill_columns = [&](int c, int from, int step) {   // !UNIFORM: the sixteen columns of sub-block c
+    for (int idx = from; idx < rows * SUB; idx += step)
+      gs[((c & 1) * SUB + (idx & (SUB - 1))) * group_rows + idx / SUB] = grid_of(idx / SUB, c * SUB + (idx & (SUB - 1)));
+  };
+  auto stage_rows = [&](float* dst, const float* __restrict__ src, int64_t ld) {   // this tile's columns of the group
     for (int idx = tid; idx < rows * (TILE / 4); idx += SWEEP_THREADS) {
       const int r = idx >> 5, k4 = (idx & 31) * 4;
       const bool keep = k4 < nb;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&ws[r * W_LD + k4]);
-      const float* g = a.W + (int64_t)(row0 + r) * a.ldw + i1 + (keep ? k4 : 0);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(g), "r"(keep ? 16 : 0) : "memory");
-      if constexpr (INVERSE_FREE) {
-        const float* go = a.Worig + (int64_t)(row0 + r) * a.ldwo + i1 + (keep ? k4 : 0);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + group_rows * W_LD * 4), "l"(go), "r"(keep ? 16 : 0) : "memory");
-      }
+      const float* g = src + (int64_t)(row0 + r) * ld + i1 + (keep ? k4 : 0);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(&dst[r * W_LD + k4])), "l"(g), "r"(keep ? 16 : 0)
+                   : "memory");
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    auto grid_of = [&](int r, int j) {   // column j of the tile
-      float s = 1.0f, z = a.zero_default;
-      if (j < nb) {
-        const int64_t off = (int64_t)(row0 + r) * a.s_rs + (int64_t)((uint32_t)(i1 + j) / group) * a.s_gs;
-        s = __ldg(a.scale + off);
-        if (a.zero) z = __ldg(a.zero + off);
-      }
-      return make_float4(s, 1.0f / s, z, 0.0f);
-    };
-    auto fill_columns = [&](int c, int from, int step) {   // !UNIFORM: the sixteen columns of sub-block c
-      for (int idx = from; idx < rows * SUB; idx += step)
-        gs[((c & 1) * SUB + (idx & (SUB - 1))) * group_rows + idx / SUB] = grid_of(idx / SUB, c * SUB + (idx & (SUB - 1)));
-    };
+  };
+  auto fill_grid = [&] {
     if constexpr (UNIFORM) {
       for (int idx = tid; idx < rows * N_SUB; idx += SWEEP_THREADS) gs[(idx & 7) * group_rows + (idx >> 3)] = grid_of(idx >> 3, (idx & 7) * SUB);
     } else {
       fill_columns(0, tid, SWEEP_THREADS);
     }
+  };
+  // The factor and the original weights are constant during the sweep: they are staged before this grid waits for the
+  // rank-128 update that precedes it in the stream (only W depends on that update).
+  stage_factor_tile(us, a.U + (int64_t)i1 * a.ldu + i1, a.ldu, nb);
+  if constexpr (INVERSE_FREE) stage_rows(wos, a.Worig, a.ldwo);
+  chain_wait();
+  chain_release();
+
+  for (;;) {
+    const int chain_warps = (rows + 31) >> 5;
+    stage_rows(ws, a.W, a.ldw);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    fill_grid();
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 
@@ -311,9 +314,12 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) sweep_tile_kernel(const Swee
       const float4 lo4 = *reinterpret_cast<const float4*>(ws + r * W_LD + k), hi4 = *reinterpret_cast<const float4*>(ws + r * W_LD + k + 4);
       write_errors(a, row0 + r, k, lo4, hi4, lane);
     }
+    row0 += gridDim.x * group_rows;
+    if (row0 >= a.R) break;
+    rows = a.R - row0 < group_rows ? a.R - row0 : group_rows;
     __syncthreads();   // the next group's weights replace the errors
+    if constexpr (INVERSE_FREE) stage_rows(wos, a.Worig, a.ldwo);
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");   // a CTA without rows leaves no copy behind
 }
 
 template <int DT>
