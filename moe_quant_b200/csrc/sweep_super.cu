@@ -26,7 +26,7 @@ constexpr int SLAB_FAULT = 65;          // code of a slab that did not arrive
 constexpr int WO_LD = SUB + 4;          // row stride of the original weights of a sub-block
 
 constexpr size_t super_smem_bytes(int rows, bool uniform) {
-  return (size_t)(SLOTS * SLAB + rows * W_LD + rows * 2 * WO_LD + rows * 2 * (uniform ? 1 : SUB) * 4) * sizeof(float);
+  return (size_t)(SLOTS * SLAB + rows * W_LD + rows * 2 * WO_LD + rows * 2 * ((uniform ? 1 : SUB) + 1) * 4) * sizeof(float);
 }
 static_assert(super_smem_bytes(MAX_ROWS, false) <= 227 * 1024 - 64, "shared memory of a CTA");
 
@@ -69,8 +69,8 @@ __device__ __forceinline__ void fma4(float4& v, const float4 u, const float e) {
 // The factor passes through three slabs of sixteen rows, 32 KB down to 1 KB each, fetched two sub-blocks ahead.
 //
 // What bounds a super-block is the chain, 512 steps of 94 cycles, and handing the sub-blocks over (the next one's sixteen columns 600 cycles,
-// more while the helpers read shared memory): 2900 cycles per sub-block, about 48 us, whatever the number of rows.  As four tiles and
-// three rank-128 updates the same columns take 4 x 16.5 + 3 x 8.5 us: 512 x 4096 is quantized in 1462 us instead of 1574, 500 x 1056 in 420
+// more while the helpers read shared memory): 2800 cycles per sub-block, about 46 us, whatever the number of rows.  As four tiles and
+// three rank-128 updates the same columns take 4 x 16.5 + 3 x 8.5 us: 512 x 4096 is quantized in 1450 us instead of 1574, 500 x 1056 in 419
 // instead of 533.  More rows: the helpers' FMAs take over (2048 rows on 74 SMs: 59 us), where the tensor cores' updates are the better
 // way; far products on mma.sync, from planes in shared memory, took longer still (49 rows per CTA: 141 us against 121).
 // UNIFORM: the columns of a sub-block lie in one quantization group (group % 16 == 0).
@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
   float* wos = ws + group_rows * W_LD;    // [2][group_rows][WO_LD]: original weights of two sub-blocks by turns
   // the grid of every row (scale, its reciprocal, zero point) for two sub-blocks by turns: UNIFORM [2][group_rows], otherwise [2][SUB][group_rows]
   float4* gs = reinterpret_cast<float4*>(wos + 2 * group_rows * WO_LD);
+  uint4* cs = reinterpret_cast<uint4*>(gs + 2 * group_rows * (UNIFORM ? 1 : SUB));   // [2][group_rows]: codes of two sub-blocks by turns
   const int nb = a.nb, i1 = a.i1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n_sub = (nb + SUB - 1) / SUB;
   const float* factor = a.U + (int64_t)i1 * a.ldu + i1;
@@ -216,6 +217,27 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
             asm volatile("cp.async.commit_group;" ::: "memory");
             fill_grid(c + 2, from, step);
           }
+          // codes (and packed words) leave; a narrow last tile ends on a multiple of eight columns.  (From the chain: a sweep of 512 x 4096
+          // took 562 us instead of 545.)
+          if (from < rows) {
+            const int j0 = c * SUB;
+            const int64_t row = row0 + from;
+            const uint4 code = cs[(c & 1) * group_rows + from];
+            const uint32_t cw[SUB / 4] = {code.x, code.y, code.z, code.w};
+            uint8_t* cdst = a.codes + row * a.C + i1 + j0;
+            if (wide_codes && j0 + SUB <= nb) {
+              *reinterpret_cast<uint4*>(cdst) = code;
+            } else {
+#pragma unroll
+              for (int qd = 0; qd < SUB / 4; ++qd)
+                if (j0 + 4 * qd < nb) *reinterpret_cast<uint32_t*>(cdst + 4 * qd) = cw[qd];
+            }
+            if (a.packed) {
+#pragma unroll
+              for (int h = 0; h < SUB / 8; ++h)
+                if (j0 + 8 * h < nb) a.packed[row * (a.C >> 3) + ((i1 + j0 + 8 * h) >> 3)] = (int32_t)pack_nibbles(cw[2 * h], cw[2 * h + 1]);
+            }
+          }
           constexpr int PER_TILE = TILE / SUB;
           if (errors_leave && c >= PER_TILE) {
             const int part = c % PER_TILE;
@@ -298,6 +320,7 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
         };
         if (!UNIFORM && valid) write_dequantized();   // behind the barrier the table belongs to sub-block c + 2
         if (valid) {
+          cs[(c & 1) * group_rows + r] = make_uint4(cw[0], cw[1], cw[2], cw[3]);
 #pragma unroll
           for (int qd = 0; qd < SUB / 4; ++qd)
             *reinterpret_cast<float4*>(wrow + j0 + 4 * qd) = make_float4(e[4 * qd], e[4 * qd + 1], e[4 * qd + 2], e[4 * qd + 3]);
@@ -324,23 +347,7 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
 #pragma unroll
           for (int qd = 0; qd < SUB / 4; ++qd) { w[4 * qd] = v[qd].x; w[4 * qd + 1] = v[qd].y; w[4 * qd + 2] = v[qd].z; w[4 * qd + 3] = v[qd].w; }
         }
-        // codes (and packed words) leave; a narrow last tile ends on a multiple of eight columns
-        if (valid) {
-          uint8_t* cdst = a.codes + row * a.C + i1 + j0;
-          if (wide_codes && j0 + SUB <= nb) {
-            *reinterpret_cast<uint4*>(cdst) = make_uint4(cw[0], cw[1], cw[2], cw[3]);
-          } else {
-#pragma unroll
-            for (int qd = 0; qd < SUB / 4; ++qd)
-              if (j0 + 4 * qd < nb) *reinterpret_cast<uint32_t*>(cdst + 4 * qd) = cw[qd];
-          }
-          if (a.packed) {
-#pragma unroll
-            for (int h = 0; h < SUB / 8; ++h)
-              if (j0 + 8 * h < nb) a.packed[row * (a.C >> 3) + ((i1 + j0 + 8 * h) >> 3)] = (int32_t)pack_nibbles(cw[2 * h], cw[2 * h + 1]);
-          }
-          if (UNIFORM) write_dequantized();
-        }
+        if (UNIFORM && valid) write_dequantized();
       }
       }
       end_group();
