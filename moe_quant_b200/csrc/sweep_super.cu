@@ -68,17 +68,19 @@ __device__ __forceinline__ void fma4(float4& v, const float4 u, const float e) {
 // comes next: the value goes back to W (which so holds every tile as it was when its turn came).
 // The factor passes through three slabs of sixteen rows, 32 KB down to 1 KB each, fetched two sub-blocks ahead.
 //
-// What bounds a super-block is the chain, 512 steps of 94 cycles, and handing the sub-blocks over (the next one's sixteen columns 600 cycles,
-// more while the helpers read shared memory): 2800 cycles per sub-block, about 47 us, whatever the number of rows.  As four tiles and
-// three rank-128 updates the same columns take 4 x 16.5 + 3 x 8.5 us: 512 x 4096 is quantized in 1450 us instead of 1574, 500 x 1056 in 419
-// instead of 533.  More rows: the helpers' FMAs take over (2048 rows on 74 SMs: 59 us), where the tensor cores' updates are the better
-// way; far products on mma.sync, from planes in shared memory, took longer still (49 rows per CTA: 141 us against 121).
+// What bounds a super-block is the chain, 512 steps of 94 cycles, and handing the sub-blocks over (the next one's sixteen columns take a lane
+// by itself 600 cycles, and 900 while the helpers read shared memory): 2800 cycles per sub-block, 47 us, whatever the number of rows;
+// 45 us with up to eight rows per CTA.  As four tiles and three rank-128 updates the same columns take 4 x 16.5 + 3 x 8.5 us: 512 x 4096 is
+// quantized in 1435 us instead of 1574, 500 x 1056 in 419 instead of 533.  More rows: the helpers' FMAs take over (2048 rows on 74 SMs:
+// 59 us), where the tensor cores' updates are the better way; far products on mma.sync, from planes in shared memory, took longer
+// still (49 rows per CTA: 141 us against 121).
 // UNIFORM: the columns of a sub-block lie in one quantization group (group % 16 == 0).
+// QUARTERS: at most eight rows (`next` by four lanes a row: a sweep of 512 x 4096 takes 534 us instead of 551).
 // INVERSE_FREE (a.Worig given): U is the unit factor Utilde = Uhat^-1 and what is propagated is minus the
 // total change of the column, -(y - w_original), instead of the error against the running value;
 // x_j = w_j - sum_{i<j} (y_i - w_i) Utilde[i,j] is the same number as the reference's running weight
 // (E Uhat = Y - W  <=>  E = (Y - W) Utilde).
-template <int DT, bool UNIFORM, bool INVERSE_FREE>
+template <int DT, bool UNIFORM, bool INVERSE_FREE, bool QUARTERS>
 __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const SweepArgs a, const int group_rows) {
   using T = typename StorageOf<DT>::type;
   extern __shared__ __align__(16) float sweep_smem[];
@@ -245,9 +247,11 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
           }
         }
       } else {
-      // ---- chains.  Lanes past the last row repeat it and store nothing.
-      const bool valid = tid < rows;
-      const int r = valid ? tid : rows - 1;
+      // ---- chains.  Lanes past the last row repeat it and store nothing.  QUARTERS: four lanes have the same row; each runs
+      // its chain, and brings a quad of the next columns up to date.
+      const int own_row = QUARTERS ? lane & 7 : lane;
+      const bool valid = lane < rows;
+      const int r = own_row < rows ? own_row : rows - 1;
       const int64_t row = row0 + r;
       float* wrow = ws + r * W_LD;
       float* wglobal = a.W + row * a.ldw + i1;
@@ -328,24 +332,42 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
         __syncthreads();
         if (c + 1 < n_sub) {
           // ---- next: this row's errors on the columns of the following sub-block
-          float4 v[SUB / 4];
+          if constexpr (QUARTERS) {
+            const int at = j0 + SUB + 4 * (lane >> 3);
+            float4 v = enters ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(wrow + at);
 #pragma unroll
-          for (int qd = 0; qd < SUB / 4; ++qd)
-            v[qd] = enters ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(wrow + j0 + SUB + 4 * qd);
-#pragma unroll
-          for (int t = 0; t < SUB; ++t)
-#pragma unroll
-            for (int qd = 0; qd < SUB / 4; ++qd) fma4(v[qd], *reinterpret_cast<const float4*>(ud + t * SUPER + SUB + 4 * qd), e[t]);
-          if (enters) {
+            for (int t = 0; t < SUB; ++t) fma4(v, *reinterpret_cast<const float4*>(ud + t * SUPER + at - j0), e[t]);
+            if (enters) {
+              const float4 got = *reinterpret_cast<const float4*>(wrow + at);
+              v = make_float4(got.x + v.x, got.y + v.y, got.z + v.z, got.w + v.w);
+              if (own_row < rows && at < nb) *reinterpret_cast<float4*>(wglobal + at) = v;
+            }
 #pragma unroll
             for (int qd = 0; qd < SUB / 4; ++qd) {
-              const float4 got = *reinterpret_cast<const float4*>(wrow + j0 + SUB + 4 * qd);
-              v[qd] = make_float4(got.x + v[qd].x, got.y + v[qd].y, got.z + v[qd].z, got.w + v[qd].w);
-              if (valid && j0 + SUB + 4 * qd < nb) *reinterpret_cast<float4*>(wglobal + j0 + SUB + 4 * qd) = v[qd];
+              const int from = own_row + 8 * qd;
+              w[4 * qd] = __shfl_sync(0xffffffffu, v.x, from); w[4 * qd + 1] = __shfl_sync(0xffffffffu, v.y, from);
+              w[4 * qd + 2] = __shfl_sync(0xffffffffu, v.z, from); w[4 * qd + 3] = __shfl_sync(0xffffffffu, v.w, from);
             }
-          }
+          } else {
+            float4 v[SUB / 4];
 #pragma unroll
-          for (int qd = 0; qd < SUB / 4; ++qd) { w[4 * qd] = v[qd].x; w[4 * qd + 1] = v[qd].y; w[4 * qd + 2] = v[qd].z; w[4 * qd + 3] = v[qd].w; }
+            for (int qd = 0; qd < SUB / 4; ++qd)
+              v[qd] = enters ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(wrow + j0 + SUB + 4 * qd);
+#pragma unroll
+            for (int t = 0; t < SUB; ++t)
+#pragma unroll
+              for (int qd = 0; qd < SUB / 4; ++qd) fma4(v[qd], *reinterpret_cast<const float4*>(ud + t * SUPER + SUB + 4 * qd), e[t]);
+            if (enters) {
+#pragma unroll
+              for (int qd = 0; qd < SUB / 4; ++qd) {
+                const float4 got = *reinterpret_cast<const float4*>(wrow + j0 + SUB + 4 * qd);
+                v[qd] = make_float4(got.x + v[qd].x, got.y + v[qd].y, got.z + v[qd].z, got.w + v[qd].w);
+                if (valid && j0 + SUB + 4 * qd < nb) *reinterpret_cast<float4*>(wglobal + j0 + SUB + 4 * qd) = v[qd];
+              }
+            }
+#pragma unroll
+            for (int qd = 0; qd < SUB / 4; ++qd) { w[4 * qd] = v[qd].x; w[4 * qd + 1] = v[qd].y; w[4 * qd + 2] = v[qd].z; w[4 * qd + 3] = v[qd].w; }
+          }
         }
         if (UNIFORM && valid) write_dequantized();
       }
@@ -440,20 +462,30 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
 template <int DT>
 int launch(bool chained, bool uniform, int grid, int rows, cudaStream_t st, const SweepArgs& args) {
   const bool free = args.Worig != nullptr;
-  auto* kernel = uniform ? (free ? sweep_super_kernel<DT, true, true> : sweep_super_kernel<DT, true, false>)
-                         : (free ? sweep_super_kernel<DT, false, true> : sweep_super_kernel<DT, false, false>);
+  auto pick = [&](auto quarters) {
+    constexpr bool Q = decltype(quarters)::value;
+    return uniform ? (free ? sweep_super_kernel<DT, true, true, Q> : sweep_super_kernel<DT, true, false, Q>)
+                   : (free ? sweep_super_kernel<DT, false, true, Q> : sweep_super_kernel<DT, false, false, Q>);
+  };
+  auto* kernel = rows <= 8 ? pick(std::true_type{}) : pick(std::false_type{});
   MQ_CUDA(launch_chained(chained, kernel, dim3(grid), dim3(SUPER_THREADS), super_smem_bytes(rows, uniform), st, args, rows));
+  return MQ_OK;
+}
+
+template <int DT, bool QUARTERS>
+int configure_kernels() {
+  constexpr int bytes = (int)super_smem_bytes(MAX_ROWS, true), by_column = (int)super_smem_bytes(MAX_ROWS, false);
+  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, true, true, QUARTERS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, true, false, QUARTERS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, false, true, QUARTERS>, cudaFuncAttributeMaxDynamicSharedMemorySize, by_column));
+  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, false, false, QUARTERS>, cudaFuncAttributeMaxDynamicSharedMemorySize, by_column));
   return MQ_OK;
 }
 
 template <int DT>
 int configure_dtype() {
-  constexpr int bytes = (int)super_smem_bytes(MAX_ROWS, true), by_column = (int)super_smem_bytes(MAX_ROWS, false);
-  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, by_column));
-  MQ_CUDA(cudaFuncSetAttribute(sweep_super_kernel<DT, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, by_column));
-  return MQ_OK;
+  MQ_TRY((configure_kernels<DT, true>()));
+  return configure_kernels<DT, false>();
 }
 
 int configure_once() {
