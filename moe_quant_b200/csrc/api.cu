@@ -114,7 +114,7 @@ extern "C" size_t mq_quantize_layer_workspace_bytes(int n_tied, int64_t R, int64
                                                     int split_sweep) {
   using namespace mq;
   if (n_tied <= 0 || R <= 0 || C <= 0) return 0;
-  math &= ~MQ_MATH_COMPACT;
+  math &= ~(MQ_MATH_COMPACT | MQ_MATH_MANY_TOKENS);
   size_t a = factor_workspace_bytes(C, math, split_hinv);            // factorisation: the planes of a super-panel
   size_t b = sweep_workspace_bytes(R, C, math, split_sweep, true);
   return layer_fixed_bytes(n_tied, R, C) + (a > b ? a : b);
@@ -141,9 +141,9 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
     MQ_REQUIRE(!packed || (packed[i] && bits == 4 && aligned(packed[i], 4)), MQ_ERR_UNSUPPORTED,
                "mq_quantize_layer: packed words need bits == 4 and a 4-byte aligned buffer per layer");
   }
-  const int sweep_math = math;   // the factorisation and the sweep honour MQ_MATH_COMPACT
-  math &= ~MQ_MATH_COMPACT;
-  MQ_REQUIRE(math == MQ_MATH_FP32 || math == MQ_MATH_TENSOR, MQ_ERR_ARGUMENT, "mq_quantize_layer: bad math %d", sweep_math);
+  const int factor_math = math, sweep_math = math & ~MQ_MATH_MANY_TOKENS;   // the factorisation and the sweep honour MQ_MATH_COMPACT
+  math &= ~(MQ_MATH_COMPACT | MQ_MATH_MANY_TOKENS);
+  MQ_REQUIRE(math == MQ_MATH_FP32 || math == MQ_MATH_TENSOR, MQ_ERR_ARGUMENT, "mq_quantize_layer: bad math %d", factor_math);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Workspace ws(workspace, workspace_bytes);
   float* U = ws.take<float>((size_t)C * C);
@@ -181,7 +181,7 @@ extern "C" int mq_quantize_layer(const void* const* Wsrc, int w_dtype, int n_tie
   MQ_TRY(copy_upper_scaled(H, ldh, U, C, C, pairs ? eq : nullptr, st));
   {
     Workspace sub(ws.base + ws.used, ws.size - ws.used);
-    MQ_TRY(chol_unit_factor(U, C, C, diag, sweep_math, split_hinv, flags, sub, st, true, unscaled, pairs ? eq : nullptr));
+    MQ_TRY(chol_unit_factor(U, C, C, diag, factor_math, split_hinv, flags, sub, st, true, unscaled, pairs ? eq : nullptr));
   }
   // sweep                                                       src/gptq_loop.py:141-148
   for (int i = 0; i < n_tied; ++i) {

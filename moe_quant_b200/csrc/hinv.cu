@@ -803,10 +803,12 @@ static long long upper_pair_tiles(int64_t C) {
 
 // Columns whose update of everything in front of them is applied together.  1024 with pairs: what bounds those updates is the way of
 // every tile out of its SM, whatever their depth (see umma_pair_kernel); with the sweep's, an attention block
-// takes 28.5 instead of 30.0 ms, four experts 13.0 instead of 13.6.  The factor's error against fp64 is 0.98 to 1.00 of that with 512 where tokens are at
-// least half the columns, but 1.00 to 1.02 with a sixth as many: callers that ask for all four products, as few tokens do, stay at 512.
-static int far_columns(int64_t C, int math, int split) {
-  return uses_pairs(C, math, split) && split == 3 ? (int)PAIR_FAR_COLUMNS : SUPER_NB;
+// takes 28.5 instead of 30.0 ms, four experts 13.0 instead of 13.6.  The factor's error against fp64 (4104 to 9224 columns, means of five
+// Hessians) is 0.985 to 0.998 of that with 512 where tokens are at least as many as columns, 0.988 to 1.009 with half to three quarters
+// as many, up to 1.034 with a twelfth: the partial sums of sixteen slabs outgrow what they leave of the matrix.  So only callers that
+// say so (many_tokens) go that deep.
+static int far_columns(int64_t C, int math, int split, bool many_tokens) {
+  return many_tokens && uses_pairs(C, math, split) && split == 3 ? (int)PAIR_FAR_COLUMNS : SUPER_NB;
 }
 
 // what the CTAs of factor_panel_kernel tell one another: the strips of the block in flight, a ticket per panel
@@ -814,9 +816,10 @@ static size_t panel_sync_bytes(int64_t C) {
   return align_up(STRIP_WORDS * sizeof(uint64_t) + (size_t)ceil_div(C, NB) * sizeof(int), 256);
 }
 
+// enough for either depth
 size_t factor_workspace_bytes(int64_t C, int math, int split) {
   if (math != MQ_MATH_TENSOR) return 0;
-  return plane_set_bytes(C, far_columns(C, math, split), uses_pairs(C, math, split) ? 2 : plane_count(split)) + align_up((size_t)(C + 1) * sizeof(float), 256) + panel_sync_bytes(C);
+  return plane_set_bytes(C, far_columns(C, math, split, true), uses_pairs(C, math, split) ? 2 : plane_count(split)) + align_up((size_t)(C + 1) * sizeof(float), 256) + panel_sync_bytes(C);
 }
 
 // One panel: the block and the rows above it (factor_panel_kernel).  Eight warps of RPW rows a CTA, one CTA per SM at most.
@@ -877,11 +880,12 @@ int chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag, int math, in
                      Workspace& ws, cudaStream_t st, bool upper_only, int unscaled, const float* eq) {
   MQ_TRY(configure_once());
   const int compact = (math & MQ_MATH_COMPACT) ? 1 : 0;   // the panel solves and the rank-128 strips look at it
-  math &= ~MQ_MATH_COMPACT;
+  const bool many_tokens = (math & MQ_MATH_MANY_TOKENS) != 0;
+  math &= ~(MQ_MATH_COMPACT | MQ_MATH_MANY_TOKENS);
   MQ_REQUIRE(math != MQ_MATH_TENSOR || (split >= 1 && split <= 4), MQ_ERR_ARGUMENT, "factorisation: split must be 1, 2, 3 or 4 (got %d)", split);
   const bool half = uses_pairs(C, math, split);   // pairs of fp16 planes (split_half2)
   const int all_products = half && split == 4 ? 1 : 0;
-  const int far_nb = far_columns(C, math, split), far_panels = far_nb / NB;
+  const int far_nb = far_columns(C, math, split, many_tokens), far_panels = far_nb / NB;
   split = plane_count(split);
   MQ_REQUIRE(!eq || half, MQ_ERR_ARGUMENT, "factorisation: an equilibrated matrix needs pairs of planes");
   Workspace local(ws.base ? ws.base + ws.used : nullptr, ws.base ? ws.size - ws.used : 0);
@@ -1094,7 +1098,7 @@ extern "C" int mq_hinv_upper(float* H, int64_t C, int64_t ldh, float* Uhat, int6
 
 extern "C" size_t mq_chol_unit_factor_workspace_bytes(int64_t C, int math, int split) {
   if (C <= 0) return 0;
-  return mq::align_up((size_t)C * sizeof(float), 256) + mq::factor_workspace_bytes(C, math, split);
+  return mq::align_up((size_t)C * sizeof(float), 256) + mq::factor_workspace_bytes(C, math & ~MQ_MATH_MANY_TOKENS, split);
 }
 
 extern "C" int mq_chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag_out, int math, int split,
@@ -1104,7 +1108,8 @@ extern "C" int mq_chol_unit_factor(float* H, int64_t C, int64_t ldh, float* diag
   MQ_REQUIRE(C > 0 && ldh >= C, MQ_ERR_ARGUMENT, "mq_chol_unit_factor: bad C=%lld ldh=%lld", (long long)C, (long long)ldh);
   MQ_REQUIRE(C % 8 == 0, MQ_ERR_UNSUPPORTED, "mq_chol_unit_factor: C=%lld must be a multiple of 8", (long long)C);
   MQ_REQUIRE(ldh % 4 == 0 && aligned(H, 16), MQ_ERR_ALIGNMENT, "mq_chol_unit_factor: H must be 16-byte aligned, ldh %% 4 == 0");
-  MQ_REQUIRE(math == MQ_MATH_FP32 || math == MQ_MATH_TENSOR, MQ_ERR_ARGUMENT, "mq_chol_unit_factor: bad math %d", math);
+  const int base_math = math & ~MQ_MATH_MANY_TOKENS;
+  MQ_REQUIRE(base_math == MQ_MATH_FP32 || base_math == MQ_MATH_TENSOR, MQ_ERR_ARGUMENT, "mq_chol_unit_factor: bad math %d", math);
   Workspace ws(workspace, workspace_bytes);
   float* diag = ws.take<float>(C);
   MQ_REQUIRE(diag, MQ_ERR_WORKSPACE, "mq_chol_unit_factor: workspace too small");

@@ -262,13 +262,17 @@ class GPTQ:
     def _layer_precision(self) -> ops.Precision:
         """The handle's precision; from fewer tokens than half the columns the factorisation takes all four products of
         its operand pairs (its sums cancel there: with three, the layer's error against fp64 is up to 1.08 of that of
-        three bf16 planes, with four 1.01; above half the columns three do: 0.97 and less).  What counts are the tokens of
-        all ranks behind the Hessian; the identity that stands in for no token at all has nothing to cancel."""
+        three bf16 planes, with four 1.01; above half the columns three do: 0.97 and less); from as many tokens as columns
+        on its updates may go deeper.  What counts are the tokens of all ranks behind the Hessian; the identity that stands in
+        for no token at all has nothing to cancel."""
         p = ops.DEFAULT_PRECISION if self.precision is None else self.precision
         owner = self if self.tied_gptq_handle is None else self.tied_gptq_handle
         tokens = max(owner.num_samples, owner._hessian_tokens)
-        if p.math == ops.MATH_TENSOR and p.split_hinv == 3 and 2 * tokens < self.d_col and not owner.issue_zero_samples:
-            return dataclasses.replace(p, split_hinv=4)
+        if p.math == ops.MATH_TENSOR and p.split_hinv == 3 and not owner.issue_zero_samples:
+            if 2 * tokens < self.d_col:
+                return dataclasses.replace(p, split_hinv=4)
+            if tokens >= self.d_col:
+                return dataclasses.replace(p, many_tokens=True)
         return p
 
     def _mse_search(self) -> bool:

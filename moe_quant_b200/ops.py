@@ -12,7 +12,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from ._lib import MATH_COMPACT, MATH_FP32, MATH_TENSOR, MoeQuantError, check, dtype_code, lib, ptr, require_cuda, require_one_device, stream_ptr
+from ._lib import MATH_COMPACT, MATH_FP32, MATH_MANY_TOKENS, MATH_TENSOR, MoeQuantError, check, dtype_code, lib, ptr, require_cuda, require_one_device, stream_ptr
 
 
 @dataclass
@@ -27,6 +27,8 @@ class Precision:
     of few tokens needs (a handle asks for it by itself).
     compact: several layers are in flight on different streams (quantize_many sets it): the sweep
     uses launch shapes that occupy few SMs (MQ_MATH_COMPACT); the results do not change.
+    many_tokens: the Hessian is of at least as many tokens as columns (a handle knows and says so by itself): with
+    split_hinv 3 the factorisation may apply deeper updates (MQ_MATH_MANY_TOKENS).
     """
 
     math: int = MATH_TENSOR
@@ -34,11 +36,22 @@ class Precision:
     split_hinv: int = 3
     split_sweep: int = 3
     compact: bool = False
+    many_tokens: bool = False
 
     @property
     def sweep_math(self) -> int:
-        """The `math` argument of the sweep and of the whole-layer entry point."""
+        """The `math` argument of the sweep."""
         return self.math | (MATH_COMPACT if self.compact else 0)
+
+    @property
+    def factor_math(self) -> int:
+        """The `math` argument of the factorisation by itself."""
+        return self.math | (MATH_MANY_TOKENS if self.many_tokens else 0)
+
+    @property
+    def layer_math(self) -> int:
+        """The `math` argument of the whole-layer entry point."""
+        return self.sweep_math | self.factor_math
 
 
 DEFAULT_PRECISION = Precision()
@@ -195,7 +208,7 @@ def chol_unit_factor(H: Tensor, precision: Optional[Precision] = None, flags: Op
     nbytes = L.mq_chol_unit_factor_workspace_bytes(C, p.math, p.split_hinv)
     ws = _lib.workspace(H.device, nbytes)
     with _lib.on_device(H.device):
-        check(L.mq_chol_unit_factor(ptr(H), C, H.stride(0), ptr(diag), p.math, p.split_hinv, ptr(flags), ptr(ws),
+        check(L.mq_chol_unit_factor(ptr(H), C, H.stride(0), ptr(diag), p.factor_math, p.split_hinv, ptr(flags), ptr(ws),
                                     ws.numel(), stream_ptr(H.device)))
     return flags, diag
 
@@ -265,7 +278,7 @@ def quantize_layer(weights: Sequence[Tensor], H: Tensor, group: int, bits: int, 
     p_arr = arr(*[t.data_ptr() for t in packed]) if packed is not None else None
     with _lib.on_device(dev):
         check(L.mq_quantize_layer(w_arr, dtype_code(dtype), n, R, C, ptr(H), H.stride(0), group, bits, rel_damp, c_arr,
-                                  p_arr, s_arr, d_arr, ptr(flags), p.sweep_math, p.split_hinv, p.split_sweep, ptr(ws), ws.numel(),
+                                  p_arr, s_arr, d_arr, ptr(flags), p.layer_math, p.split_hinv, p.split_sweep, ptr(ws), ws.numel(),
                                   stream_ptr(dev)))
     if want_packed:
         return codes, scales, deqs, flags, packed

@@ -133,6 +133,23 @@ def test_few_tokens_ask_for_all_products():
     assert gate._layer_precision() == ops.Precision(split_hinv=4, compact=True)
 
 
+def test_deep_updates_only_from_as_many_tokens_as_columns():
+    """Nobody but a handle that has counted them says many_tokens, and only where three products are taken."""
+    assert not ops.DEFAULT_PRECISION.many_tokens and ops.Precision().layer_math == ops.Precision().factor_math == ops.MATH_TENSOR
+    gate = GPTQ(_layer(C=1024), 8, True)
+    up = GPTQ(_layer(C=1024), 8, True, tied_gptq_handle=gate)
+    for tokens, many in ((10, False), (512, False), (1023, False), (1024, True), (5000, True)):
+        gate.num_samples = tokens
+        for p in (gate._layer_precision(), up._layer_precision()):
+            assert p.many_tokens == many
+            assert p.layer_math == p.factor_math == ops.MATH_TENSOR | (0x200 if many else 0) and p.sweep_math == ops.MATH_TENSOR
+    gate.precision = ops.Precision(compact=True)
+    assert gate._layer_precision() == ops.Precision(compact=True, many_tokens=True) and gate._layer_precision().layer_math == ops.MATH_TENSOR | 0x300
+    for p in (ops.Precision(split_hinv=4), ops.Precision(split_hinv=2), ops.Precision(math=ops.MATH_FP32)):
+        gate.precision = p
+        assert gate._layer_precision() == p
+
+
 def test_few_tokens_are_counted_over_all_ranks(monkeypatch):
     """A rank that holds a third of the tokens decides by all of them, as a single process with the same tokens would."""
     h = GPTQ(_layer(C=1024), 8, True, is_distributed=True)
@@ -162,7 +179,7 @@ def test_few_tokens_after_the_owner_was_reset():
 def test_no_token_at_all_has_nothing_to_cancel():
     h = GPTQ(_layer(C=1024), 8, True)
     h.quantization_pre_step()
-    assert h.issue_zero_samples and h._layer_precision().split_hinv == 3
+    assert h.issue_zero_samples and h._layer_precision().split_hinv == 3 and not h._layer_precision().many_tokens
 
 
 def test_asymmetric_is_refused():
