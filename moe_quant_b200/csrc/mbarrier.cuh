@@ -49,12 +49,18 @@ struct WaitLimit {
   }
 };
 
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* fault, int code) {
+// By one lane, or where nothing that the warp does together depends on the answer.
+__device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, int* fault, int code) {
   WaitLimit limit;
   for (uint32_t it = 0;; ++it) {
     if (mbar_try(bar, parity)) return true;
     if ((it & 255u) == 255u && limit.expired(fault, code)) return false;
   }
+}
+// By a whole warp.  Its lanes poll one by one, and a barrier may complete between the poll of one that gives up and that of the next:
+// they agree, so that what follows (shuffles, tensor memory loads) is entered by all of them or by none.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* fault, int code) {
+  return __all_sync(0xffffffffu, mbar_wait_lane(bar, parity, fault, code));
 }
 
 // The word on the current device that a wait records its code in (defined beside the tensor-core kernels).

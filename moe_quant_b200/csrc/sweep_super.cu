@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
     if (n_sub > 1) fetch_slab(us + SLAB, slab_full + 8, factor, a.ldu, nb, 1);
   };
   auto wait_slab = [&](int slot) {
-    if (!mbar_wait(slab_full + 8 * slot, (slab_phases >> slot) & 1, a.fault, SLAB_FAULT)) {
+    if (!mbar_wait_lane(slab_full + 8 * slot, (slab_phases >> slot) & 1, a.fault, SLAB_FAULT)) {
       // given up: what has been started still ends before the block does
       for (const uint64_t t0 = global_ns(); !mbar_try(slab_full + 8 * slot, (slab_phases >> slot) & 1) && global_ns() - t0 < 100000000ull;) {}
     }

@@ -82,8 +82,9 @@ struct UmmaParams {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Bounded wait: gives up after about one second and records `code`.
+// Bounded waits: they give up after about one second and record `code`.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code) { return mq::mbar_wait(bar, parity, &g_engine_fault, code); }
+__device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, int code) { return mq::mbar_wait_lane(bar, parity, &g_engine_fault, code); }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) umma_gemm_kernel(const __grid_co
       const int a_row = b * p.a_rows_pad + m0 + p.a_row0, b_row = b * p.b_rows_pad + n0 + p.b_row0;
       for (int s = 0; s < n_slabs; ++s) {
         const int st = s % p.stages;
-        if (s >= p.stages && !mbar_wait(empty0 + 8 * st, ((s / p.stages) - 1) & 1, 1)) break;
+        if (s >= p.stages && !mbar_wait_lane(empty0 + 8 * st, ((s / p.stages) - 1) & 1, 1)) break;
         mbar_expect_tx(full0 + 8 * st, stage_bytes);
         const uint32_t dst = smem_base + st * stage_bytes;
         const int k = k_lo + s * SLAB_K;
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) umma_gemm_kernel(const __grid_co
       bool ok = true;
       for (int s = 0; s < n_slabs && ok; ++s) {
         const int st = s % p.stages;
-        ok = mbar_wait(full0 + 8 * st, (s / p.stages) & 1, 2);
+        ok = mbar_wait_lane(full0 + 8 * st, (s / p.stages) & 1, 2);
         if (!ok) break;
         tc_fence_after();
         const uint32_t a_base = smem_base + st * stage_bytes;

@@ -3,7 +3,9 @@ issuer, one epilogue per CTA and an engine that lands copies, runs MMAs and deli
 schedules.  When the CTAs leave, no copy, MMA, commit or arrival may be under way, whether every wait was satisfied or
 one was given up: it would write into shared memory that belongs to the next CTA.
 """
+import os
 import random
+import re
 
 import pytest
 
@@ -151,3 +153,15 @@ def test_nothing_is_under_way_when_the_pair_leaves(slabs, gives_up):
 
     assert not any(runs(True))
     assert any(runs(False))     # without the waits at the end some schedule does leave something
+
+
+def test_a_whole_warp_gives_up_a_wait_or_none_of_it():
+    """What a warp does together behind a wait (shuffles, tensor memory loads) must be entered by all of its lanes: whole warps wait by
+    mbar_wait, which takes a vote.  Lanes decide by themselves only where one lane alone issues copies or MMAs (umma_gemm_kernel) and
+    where the answer decides about nothing but the lane's own further wait (a slab of the sweep)."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "moe_quant_b200", "csrc")
+    text = {name: open(os.path.join(csrc, name)).read() for name in sorted(os.listdir(csrc)) if name.endswith((".cu", ".cuh"))}
+    assert "return __all_sync(0xffffffffu, mbar_wait_lane(bar, parity, fault, code));" in text["mbarrier.cuh"]
+    alone = {name: len(re.findall(r"(?<!bool )(?<!mq::)\bmbar_wait_lane\(", body)) for name, body in text.items() if name != "mbarrier.cuh"}
+    assert {name: n for name, n in alone.items() if n} == {"sweep_super.cu": 1, "umma_gemm.cu": 2}
+    assert sum(len(re.findall(r"\bmbar_wait\(", body)) for body in text.values()) > 20
