@@ -18,7 +18,11 @@ constexpr int SUPER_THREADS = 384;
 constexpr int FETCHERS = 3, HELPERS = 8;
 constexpr int SUPER_REGS = 168, CHAIN_REGS = 248, HELPER_REGS = 128;   // a thread: at the launch, and how the warpgroups divide them
 static_assert((1 + FETCHERS) * CHAIN_REGS + HELPERS * HELPER_REGS <= SUPER_THREADS / 32 * SUPER_REGS, "the registers of the launch are all there are");
-constexpr int MAX_ROWS = 16;            // rows of a CTA
+// Rows of a CTA: eight; a caller with several layers in flight gives each half of the GPU (eight streams, four experts of
+// 4096 x 1024 at 74 / 148 CTAs: 6.38 / 7.08 ms).
+constexpr int ROWS = 8, COMPACT_CTAS = 74;
+constexpr int MAX_ROWS = ((int)SUPER_BLOCK_ROWS + COMPACT_CTAS - 1) / COMPACT_CTAS;
+static_assert(SUPER_BLOCK_ROWS <= 148 * ROWS && MAX_ROWS >= ROWS, "a CTA has one group of rows");
 constexpr int W_LD = SUPER + 4;         // row stride of the running weights: a warp's 16-byte reads of 8 rows hit 32 banks
 constexpr int SLOTS = 3;                // slabs (sixteen rows of the factor) in shared memory: one in use, one there, one on its way
 constexpr int SLAB = SUB * SUPER;
@@ -157,6 +161,9 @@ __global__ void __launch_bounds__(SUPER_THREADS, 1) sweep_super_kernel(const Swe
       }
     }
   };
+  // The launch has a CTA for every group of rows, so the loops over groups below end after the first.  They stay because
+  // without them the compiler spills 17 registers of the helpers' (227 KB of shared memory leave no L1): a sweep of 1024 x 4096 takes 610 us instead
+  // of 548, compact 699 instead of 598, 512 x 4096 568 instead of 536.
   auto begin_group = [&] {   // all warps: everything that the first two sub-blocks of rows row0 .. need
     rows = a.R - row0 < group_rows ? a.R - row0 : group_rows;
     if (warp == 3 && row0 != (int)blockIdx.x * group_rows) fetch_first_slabs();
@@ -467,7 +474,7 @@ int launch(bool chained, bool uniform, int grid, int rows, cudaStream_t st, cons
     return uniform ? (free ? sweep_super_kernel<DT, true, true, Q> : sweep_super_kernel<DT, true, false, Q>)
                    : (free ? sweep_super_kernel<DT, false, true, Q> : sweep_super_kernel<DT, false, false, Q>);
   };
-  auto* kernel = rows <= 8 ? pick(std::true_type{}) : pick(std::false_type{});
+  auto* kernel = rows <= ROWS ? pick(std::true_type{}) : pick(std::false_type{});
   MQ_CUDA(launch_chained(chained, kernel, dim3(grid), dim3(SUPER_THREADS), super_smem_bytes(rows, uniform), st, args, rows));
   return MQ_OK;
 }
@@ -505,13 +512,8 @@ int configure_once() {
 
 int sweep_super_block(bool chained, bool uniform, bool compact, int out_dtype, const SweepArgs& args, cudaStream_t st) {
   MQ_TRY(configure_once());
-  // Alone, as few rows per CTA as fill the GPU; a caller with several layers in flight gives each half of it (eight streams, four experts of
-  // 4096 x 1024 at 74 / 148 CTAs: 6.38 / 7.08 ms).  Eight at least.
-  int rows = (int)ceil_div(args.R, compact ? 74 : 148);
-  rows = rows < 8 ? 8 : rows;
-  if (rows > MAX_ROWS) rows = MAX_ROWS;
-  const int64_t groups = ceil_div(args.R, rows);
-  const int grid = (int)(groups < 148 ? groups : 148);
+  const int spread = (int)ceil_div(args.R, COMPACT_CTAS), rows = compact && spread > ROWS ? spread : ROWS;
+  const int grid = (int)ceil_div(args.R, rows);
   switch (out_dtype) {
     case MQ_F32: return launch<MQ_F32>(chained, uniform, grid, rows, st, args);
     case MQ_BF16: return launch<MQ_BF16>(chained, uniform, grid, rows, st, args);
