@@ -1,6 +1,7 @@
-"""The barriers of the CTA-pair kernel (csrc/umma_gemm.cu, umma_pair_kernel) as a model on the CPU: two producers, one MMA
+"""The barriers of the CTA-pair kernels (csrc/umma_gemm.cu) as a model on the CPU: two producers, one MMA
 issuer, one epilogue per CTA and an engine that lands copies, runs MMAs and delivers commits on its own, under random
-schedules.  When the CTAs leave, no copy, MMA, commit or arrival may be under way, whether every wait was satisfied or
+schedules.  umma_pair_kernel has three stages and hands an accumulator over per slab, umma_gram_kernel six stages and an
+accumulator per tile of several slabs.  When the CTAs leave, no copy, MMA, commit or arrival may be under way, whether every wait was satisfied or
 one was given up: it would write into shared memory that belongs to the next CTA.
 """
 import os
@@ -9,7 +10,7 @@ import re
 
 import pytest
 
-STAGES = 3
+PAIR_STAGES, GRAM_STAGES = 3, 6
 
 
 class Barrier:
@@ -37,14 +38,17 @@ def last_uses(count, slots):
     return range(max(0, count - slots), count)
 
 
-def under_way_at_exit(slabs, seed, tail, fault_at=None):
+def under_way_at_exit(slabs, seed, tail, fault_at=None, stages=PAIR_STAGES, per_tile=None):
+    """per_tile: slabs of a tile where an accumulator is handed over per tile; None: per slab."""
     rnd = random.Random(seed)
-    full = [Barrier(1) for _ in range(STAGES)]
-    empty = [[Barrier(1) for _ in range(STAGES)] for _ in range(2)]
+    per_acc = per_tile or 1
+    accs = slabs // per_acc
+    full = [Barrier(1) for _ in range(stages)]
+    empty = [[Barrier(1) for _ in range(stages)] for _ in range(2)]
     acc_full = [[Barrier(1) for _ in range(2)] for _ in range(2)]
     acc_empty = [Barrier(2) for _ in range(2)]
     engine, remote, mmas = [], [], []
-    end = {"given_up": False, "multiplied": 0, "copied": [0, 0]}
+    end = {"given_up": False, "multiplied": 0, "accs": 0, "copied": [0, 0]}
     fault = [False]
 
     def wait(bar, parity):
@@ -63,9 +67,9 @@ def under_way_at_exit(slabs, seed, tail, fault_at=None):
     def producer(rank):
         ok, it = True, 0
         while it < slabs:
-            s = it % STAGES
-            if it >= STAGES:
-                ok = yield from wait(empty[rank][s], (it // STAGES - 1) & 1)
+            s = it % stages
+            if it >= stages:
+                ok = yield from wait(empty[rank][s], (it // stages - 1) & 1)
                 if not ok:
                     break
             if rank == 0:
@@ -74,20 +78,24 @@ def under_way_at_exit(slabs, seed, tail, fault_at=None):
             it += 1
             yield
         if tail:
-            for j in last_uses(it, STAGES):
-                ok = ok and (yield from wait(empty[rank][j % STAGES], (j // STAGES) & 1))
+            for j in last_uses(it, stages):
+                ok = ok and (yield from wait(empty[rank][j % stages], (j // stages) & 1))
         end["copied"][rank] = it
         end["given_up"] |= not ok
 
     def issuer():
         ok, it = True, 0
         while it < slabs:
-            ok = yield from wait(full[it % STAGES], (it // STAGES) & 1)
-            if ok and it >= 2:
-                ok = yield from wait(acc_empty[it & 1], ((it >> 1) - 1) & 1)
+            acc, first, last = it // per_acc, it % per_acc == 0, it % per_acc == per_acc - 1
+            if per_tile and first and acc >= 2:
+                ok = yield from wait(acc_empty[acc & 1], ((acc >> 1) - 1) & 1)
+            ok = ok and (yield from wait(full[it % stages], (it // stages) & 1))
+            if not per_tile and ok and acc >= 2:
+                ok = yield from wait(acc_empty[acc & 1], ((acc >> 1) - 1) & 1)
             if not ok:
                 break
-            mmas.append(it)
+            mmas.append((it, acc if last else None))
+            end["accs"] += last
             it += 1
             yield
         end["multiplied"] = it
@@ -95,7 +103,7 @@ def under_way_at_exit(slabs, seed, tail, fault_at=None):
 
     def epilogue(rank):
         ok = True
-        for it in range(slabs):
+        for it in range(accs):
             ok = yield from wait(acc_full[rank][it & 1], (it >> 1) & 1)
             if not ok:
                 break
@@ -107,14 +115,13 @@ def under_way_at_exit(slabs, seed, tail, fault_at=None):
         end["given_up"] |= not ok
 
     def last_words(rank):
-        n = end["multiplied"]
-        for j in last_uses(n, STAGES):
-            yield from drain(empty[rank][j % STAGES], (j // STAGES) & 1)
-        for j in last_uses(n, 2):
+        for j in last_uses(end["multiplied"], stages):
+            yield from drain(empty[rank][j % stages], (j // stages) & 1)
+        for j in last_uses(end["accs"], 2):
             yield from drain(acc_full[rank][j & 1], (j >> 1) & 1)
         if rank == 0:
-            for j in last_uses(max(end["copied"]), STAGES):
-                yield from drain(full[j % STAGES], (j // STAGES) & 1)
+            for j in last_uses(max(end["copied"]), stages):
+                yield from drain(full[j % stages], (j // stages) & 1)
 
     def play(actors, step=0):
         while actors:
@@ -126,9 +133,11 @@ def under_way_at_exit(slabs, seed, tail, fault_at=None):
             if engine and k < 0.25:
                 engine.pop(rnd.randrange(len(engine)))()
             elif mmas and k < 0.45:
-                j = mmas.pop(0)
+                j, acc = mmas.pop(0)
                 for rank in range(2):
-                    engine.extend([empty[rank][j % STAGES].arrive, acc_full[rank][j & 1].arrive])
+                    engine.append(empty[rank][j % stages].arrive)
+                    if acc is not None:
+                        engine.append(acc_full[rank][acc & 1].arrive)
             elif remote and k < 0.6:
                 remote.pop(rnd.randrange(len(remote)))()
             else:
@@ -153,6 +162,19 @@ def test_nothing_is_under_way_when_the_pair_leaves(slabs, gives_up):
 
     assert not any(runs(True))
     assert any(runs(False))     # without the waits at the end some schedule does leave something
+
+
+@pytest.mark.parametrize("tiles,per_tile", [(1, 1), (1, 5), (1, 6), (1, 9), (2, 1), (2, 4), (3, 2), (3, 7), (5, 3), (6, 1)])
+@pytest.mark.parametrize("gives_up", [False, True])
+def test_nothing_is_under_way_when_the_pair_of_the_hessian_leaves(tiles, per_tile, gives_up):
+    slabs = tiles * per_tile
+
+    def runs(tail):
+        for seed in range(100):
+            yield under_way_at_exit(slabs, seed, tail, random.Random(seed).randrange(1, 60 * slabs) if gives_up else None, GRAM_STAGES, per_tile)
+
+    assert not any(runs(True))
+    assert any(runs(False))
 
 
 def test_a_whole_warp_gives_up_a_wait_or_none_of_it():
