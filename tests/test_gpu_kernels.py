@@ -11,8 +11,8 @@ import numpy as np
 import pytest
 import torch
 
-from moe_quant_b200 import ops, synthetic
-from moe_quant_b200._lib import MATH_FP32, MATH_TENSOR, MoeQuantError
+from moe_quant_b200 import _lib, ops, synthetic
+from moe_quant_b200._lib import MATH_FP32, MATH_TENSOR, MoeQuantError, lib
 from oracle import gptq_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -562,9 +562,10 @@ def test_sweep_running_values_against_fp64(cuda, C, g, kind, split):
         assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
 
 
-@pytest.mark.parametrize("R,C", [(2600, 2600), (7000, 1800)])
+@pytest.mark.parametrize("R,C", [(2600, 2600), (7000, 1800), (1024, 5640), (576, 7176)])
 def test_sweep_running_values_where_super_blocks_go_together(cuda, R, C):
-    """As above, with enough rows that two super-blocks of 512 columns share an update (and a last one that does not)."""
+    """As above, with enough tiles that two super-blocks of 512 columns share an update (and a last one that does not): tile by tile,
+    and by launches of 512 columns (up to 1024 rows)."""
     g = 8
     W = synthetic.layer_weight(R, C, 5, torch.float32).to(cuda)
     X = synthetic.activations(2 * C, C, 6, torch.bfloat16).to(cuda).double()
@@ -799,13 +800,11 @@ def test_mse_scales_skip_no_winner(cuda, R, C, g, factor, dtype, outliers):
                                               (333, 640, 32, torch.float32, MATH_TENSOR), (130, 512, 512, torch.bfloat16, MATH_FP32),
                                               (96, 392, 56, torch.float16, MATH_TENSOR), (2500, 256, 64, torch.bfloat16, MATH_TENSOR)])
 def test_compact_sweep_is_bit_identical(cuda, R, C, g, dtype, math):
-    """MQ_MATH_COMPACT only changes the launch shape of the sweep's full tiles (one weight row per
-    thread instead of eight lanes per row): codes, dequantized values, packed words and scales
-    must be the same bits, through the whole-layer call and through the sweep alone with zero
-    points and the factor of the inverse (the reference's form of the recurrence).  The last case
-    (group 56, C = 3 tiles + 8) has no tile the row kernel takes and a narrow last tile.  2500 rows
-    are more than the grid of the sixteen-lane shape holds at once: such layers take eight lanes
-    per row, and that case is also held to the CPU oracle."""
+    """MQ_MATH_COMPACT changes how a launch is laid out (rows per CTA, a panel of the factorisation in one launch or two): codes,
+    dequantized values, packed words and scales must be the same bits, through the whole-layer call and through the sweep
+    alone with zero points and the factor of the inverse (the reference's form of the recurrence).  Group 56 crosses
+    sub-blocks, 392 columns end on a tile of eight; 2500 rows are swept tile by tile, and that case is also held to the
+    CPU oracle."""
     W = synthetic.layer_weight(R, C, 3, dtype).to(cuda)
     X = synthetic.activations(2 * C, C, 4, dtype).to(cuda)
     H = torch.zeros(C, C, device=cuda)
@@ -846,9 +845,22 @@ def test_panel_in_one_launch_is_bit_identical(cuda, C, tokens):
     X = synthetic.activations(tokens, C, 4, torch.bfloat16).to(cuda)
     H = torch.zeros(C, C, device=cuda)
     ops.hessian_accum(H, X, 0.0, 2.0 / tokens)
-    outs = [ops.quantize_layer([W], H.clone(), C, 4, 1e-2, want_dequantized=True, precision=ops.Precision(compact=c)) for c in (False, True)]
-    (c0, s0, d0, f0), (c1, s1, d1, f1) = outs
+
+    def layer(compact):
+        # the call leaves the factor, and behind it its diagonal, at the front of its workspace
+        damped, nbytes = H.clone(), lib().mq_quantize_layer_workspace_bytes(1, R, C, MATH_TENSOR, 3, 3)
+        _lib.workspace(damped.device, nbytes).zero_()
+        out = ops.quantize_layer([W], damped, C, 4, 1e-2, want_dequantized=True, precision=ops.Precision(compact=compact))
+        words = _lib.workspace(damped.device, nbytes)[: 4 * C * (C + 1)].clone().view(torch.float32)
+        factor, diag = words[: C * C].view(C, C).triu(), words[C * C :]
+        # (the matrix is scaled by powers of two, and the last pivot is the root of its element)
+        scale = torch.log2(diag[-1] / damped[-1, -1].sqrt())
+        assert bool((diag > 0).all()) and abs(float(scale - scale.round())) < 1e-5 and int((factor != 0).sum()) > C * C // 3
+        return out, factor, diag
+
+    ((c0, s0, d0, f0), u0, t0), ((c1, s1, d1, f1), u1, t1) = layer(False), layer(True)
     assert f0.tolist() == f1.tolist() and int(f0[3]) == 0
+    assert torch.equal(u0, u1) and torch.equal(t0, t1)
     assert torch.equal(c0[0], c1[0]) and torch.equal(s0[0], s1[0]) and torch.equal(d0[0], d1[0])
 
 
@@ -902,6 +914,7 @@ def test_sweep_by_super_blocks(cuda, R, C, g, inverse_free):
     (q, deq), (q0, _), (q1, deq1) = sweep(ops.Precision()), sweep(ops.Precision(math=MATH_FP32)), sweep(ops.Precision(compact=True))
     # a code on a rounding boundary takes others of its row along: of few codes those of one row in a hundred may differ
     assert int((q != q0).sum()) <= max(0.005 * q.numel(), 0.01 * C)
+    assert R == 1 or int((q != q0).sum(0).max()) <= max(1, 0.1 * R)     # and no column is wrong as a whole
     assert torch.equal(q, q1) and torch.equal(deq, deq1)
     assert torch.equal(deq, ops.dequantize(q, scale, zero, g, 4, torch.bfloat16))
 
