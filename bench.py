@@ -19,7 +19,7 @@ Printed JSON (one line, rank 0):
   e2e        layers/s through the public handles with HOST buffers: per expert the calibration
              activations and the gate_proj / up_proj weights are copied from pinned memory, the
              Hessian is accumulated, both layers are quantized, codes and scales copied back
-  roofline   the tensor-core GEMMs take the largest share of a step; of that family the 512-deep
+  roofline   the tensor-core GEMMs take the largest share of a step; of that family the deep
              update (nine tenths of a layer's flop), timed with CUDA events on its launching stream
              by the library's measurement hooks in a separate pass; the family's other member
              follows in roofline.others and every family's share in kernel_time_shares
@@ -47,12 +47,28 @@ sys.path.insert(0, ROOT)
 R, C, TOKENS, GROUP, BITS = 2048, 7168, 4096, 128, 4
 WORKLOAD = "deepseek_v3_routed_expert_gate_proj_2048x7168_bf16_g128 (one rank's expert shard, Hessian resident)"
 METRIC = "GPTQ layers/sec (2048x7168, 4b g128)"
-# DRAM traffic of one 128 x 128 output tile of a 512-deep update: 104 MB read and 33 MB written over the 1378 tiles on and above
-# the diagonal of a 6656 x 6656 one (ncu, profiles/umma_pair_kernel_far_update.md).  C in and out alone is 128 KB: part of the
-# matrix stays in the L2
-DEEP_DRAM_BYTES_PER_TILE = 99.4e3
+# DRAM traffic of one 128 x 128 output tile of a deep update: 104 MB read and 33 MB written over the 1378 tiles on and above
+# the diagonal of a 6656 x 6656 one, 512 deep (ncu, profiles/umma_pair_kernel_far_update.md).  13.6 MB of it are the operands, once, which grow
+# with the depth; the rest is C (in and out alone would be 128 KB a tile: part of the matrix stays in the L2)
+DEEP_C_BYTES_PER_TILE, DEEP_OPERAND_BYTES_PER_TILE_512 = 89.5e3, 9.9e3
 CONFIG = {"workload": WORKLOAD, "rows": R, "cols": C, "bits": BITS, "group_size": GROUP, "rel_damp": 1e-2,
           "weight_dtype": "bf16", "calibration_tokens_mean": TOKENS}
+
+
+def deep_updates(rows, cols):
+    """(128 x 128 output tiles, columns deep) of every deep update of a layer with fewer tokens than columns: 512 in the factorisation; in the
+    sweep two super-blocks share one of 1024 where the first one's alone would be more than a wave of 74 tiles of 256 x 256."""
+    def up(a, b):
+        return -(-a // b)
+
+    out = [(up(k0, 128) * (up(k0, 128) + 1) // 2, min(512, cols - k0)) for k0 in range(512, cols, 512)]
+    for s0 in range(0, cols - 512, 512):
+        s1, f0 = s0 + 512, s0 // 1024 * 1024
+        f1 = min(f0 + 1024, cols)
+        joint = up(rows, 256) * up(cols - f0 - 512, 256) > 74
+        rest = joint and s1 < f1
+        out.append((up(rows, 128) * up((f1 if rest else cols) - s1, 128), s1 - (f0 if joint and not rest else s0)))
+    return out
 
 
 def _peaks():
@@ -408,7 +424,7 @@ def headline(cx):
         shares = {k: round(v["ms"] / tot, 4) for k, v in kinds.items()}
         per_layer_us = {k: round(v["ms"] / n_prof * 1e3, 1) for k, v in kinds.items()}
         # The tensor-core GEMMs (rank-128 updates inside a 512-column super-block: umma_gemm; the
-        # 512-deep updates behind it: umma_deep) are one family; when it has the largest share of the
+        # updates behind it, 512 or 1024 columns deep: umma_deep) are one family; when it has the largest share of the
         # kernel time the roofline is that of its member with the most work, the deep update (nine
         # tenths of a layer's flop, and the largest single share of a step once several layers run
         # side by side and the latency-bound kernels overlap).  The other members follow in
@@ -431,12 +447,12 @@ def headline(cx):
 
         if top in ("umma_gemm", "umma_deep", "simt_gemm"):
             roofline = tensor_line(top, v)
-            products = 1.0 if top == "simt_gemm" else 3.0
-            out_tiles = v["work2"] / v["launches"] / (2.0 * 128 * 128 * products)   # output tiles x k per launch
-            if top == "umma_deep":
-                roofline["traffic"] = DEEP_DRAM_BYTES_PER_TILE * out_tiles / 512.0
-                roofline["traffic_source"] = ("scaled by output tiles from an ncu capture of one 512-deep update "
-                                              "(profiles/umma_pair_kernel_far_update.md), not measured in this run")
+            deep = deep_updates(R, C)
+            if top == "umma_deep" and len(deep) * n_prof == v["launches"]:
+                roofline["depths"] = {str(k): sum(1 for _, d in deep if d == k) for k in sorted({d for _, d in deep})}
+                roofline["traffic"] = sum(t * (DEEP_C_BYTES_PER_TILE + DEEP_OPERAND_BYTES_PER_TILE_512 * k / 512.0) for t, k in deep) / len(deep)
+                roofline["traffic_source"] = ("from an ncu capture of one 512-deep update (profiles/umma_pair_kernel_far_update.md): C by output "
+                                              "tiles, operands by depth; not measured in this run")
             else:
                 roofline["traffic"] = None
             roofline["note"] = ("algorithmic work of the GEMM on pairs of fp16 planes: 2MNK on the kept tiles x 3 fp16 tensor products "
