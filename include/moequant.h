@@ -61,7 +61,9 @@ typedef enum { MQ_MATH_FP32 = 0, MQ_MATH_TENSOR = 1 } mq_math;
  * (gptq.quantize_many).  The library then prefers launch shapes that occupy few SMs over the
  * lowest latency of a single layer: the sweep's tiles take more rows per CTA (R/44
  * instead of R/148, at most 64; R/74 where a launch takes 512 columns), a CTA of a rank-128 strip update walks a whole
- * row of output tiles, a CTA of a panel solve takes 64 rows instead of 32.  Results are bit-identical with and without it. */
+ * row of output tiles, a CTA of a panel solve takes 64 rows instead of 32.  It also chooses between two forms of the
+ * factorisation: without it a panel is one launch whose CTAs hold up to all SMs while one of them factors the diagonal block,
+ * with it two launches, block and solve, none of whose CTAs waits for another.  Results are bit-identical with and without it. */
 #define MQ_MATH_COMPACT 0x100
 
 /* Flag that may be OR-ed into the `math` argument of mq_quantize_layer and mq_chol_unit_factor: H is the Hessian of at

@@ -100,7 +100,7 @@ inline bool joint_update(long long tiles) { return tiles > 74; }
 
 // Whether a sweep takes a super-block of SUPER_COLUMNS per launch (sweep_super.cu) instead of a 128-column tile and the update behind it.
 // The factor's diagonal blocks of that size are then scaled as a whole.  Of one layer with 4096 columns (its quantization, us, tiles /
-// super-blocks) 512 rows take 1574 / 1462, 1024 rows 1598 / 1485, 2048 rows 1670 / 1558; but with several layers in flight the super-blocks'
+// super-blocks with one lane a row; four lanes take another 14 us off) 512 rows take 1574 / 1462, 1024 rows 1598 / 1485, 2048 rows 1670 / 1558; but with several layers in flight the super-blocks'
 // SM time counts, and the two must agree to the last bit there: four experts of 512 x 4096 take 6.66 / 5.80 ms, 1024 x 4096 6.38 / 6.38,
 // 1024 x 7168 11.53 / 11.57, 1536 x 7168 12.46 / 12.87, 2048 x 7168 13.9 / 15.3.
 constexpr int64_t SUPER_BLOCK_ROWS = 1024;

@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(DIAG_THREADS, 1) chol_diag_rev_kernel(float* _
 // yields T^-1 (upper triangular) in `rows`.
 constexpr int TT_LD = NB + 4;
 
-// a / d through the reciprocal and one correction step (the last stage of a correctly rounded division)
+// a / d through the reciprocal and one residual correction (Markstein 1990)
 __device__ __forceinline__ float quotient(float a, float d, float rd) {
   const float q = a * rd;
   return fmaf(fmaf(-d, q, a), rd, q);
@@ -487,10 +487,12 @@ __global__ void __launch_bounds__(256) trsm_rows_kernel(const float* __restrict_
 // behind it.
 // Which CTA factors is settled by a ticket, so that it is one that runs: the others wait for it, it waits for nobody.  Waits are bounded.
 // The arithmetic is that of trsm_rows_kernel, column by column: a_j -= a_k (T[j,k] / T[k,k]), the quotients at the end.
-// A panel takes 21 us with 32 rows per CTA, 25.7 with 64 (4705 rows and more), where the two launches took 15 + 12.9 and the gap between
-// them: 2048 x 7168 4242 -> 3693 us, 7168 x 2048 1154 -> 1025.  One warp that fetches the strips is not enough (46 us a panel: a strip is under way
-// for 2 to 3 us, poll and load, and a new one is there every 0.7).  With several layers in flight the solving CTAs would hold
-// their SMs while they wait, so compact launches keep the two kernels.
+// A panel takes 16.9 us with 32 rows per CTA, 19.0 with 64 (4705 rows and more), where the two launches took 21.4 + 12.9 (the block now takes 15.0)
+// and the gap between them: 2048 x 7168 4242 -> 3498 us, 7168 x 2048 1154 -> 978.  One warp that fetches the strips is not enough (46 us a panel: a
+// strip is under way for 2 to 3 us, poll and load, and a new one is there every 0.7).  With several layers in flight the solving CTAs hold
+// their SMs while they wait, so compact launches keep the two kernels.  (Callers that run layers on streams of their own without saying so
+// are still better off than with two kernels: 2048 x 7168 on two / eight streams 2358 / 2095 us a layer against 2810 / 2190, 1024 x 4096 964 / 771
+// against 1221 / 816, the other steps since then included.)
 constexpr int PANEL_WARPS = 8;                             // of a solving CTA
 constexpr int FETCH_WARPS = 4;                             // the strips' way takes longer than the next strip: several fetch, by turns
 constexpr int PANEL_THREADS = (PANEL_WARPS + FETCH_WARPS) * 32;

@@ -75,7 +75,7 @@ __device__ __forceinline__ void fma4(float4& v, const float4 u, const float e) {
 // What bounds a super-block is the chain, 512 steps of 94 cycles, and handing the sub-blocks over (the next one's sixteen columns take a lane
 // by itself 600 cycles, and 900 while the helpers read shared memory): 2800 cycles per sub-block, 47 us, whatever the number of rows;
 // 45 us with up to eight rows per CTA.  As four tiles and three rank-128 updates the same columns take 4 x 16.5 + 3 x 8.5 us: 512 x 4096 is
-// quantized in 1435 us instead of 1574, 500 x 1056 in 419 instead of 533.  More rows: the helpers' FMAs take over (2048 rows on 74 SMs:
+// quantized in 1452 us instead of 1574, 500 x 1056 in 417 instead of 533.  With more rows per CTA than are taken now the helpers' FMAs take over (2048 rows on 74 SMs:
 // 59 us), where the tensor cores' updates are the better way; far products on mma.sync, from planes in shared memory, took longer
 // still (49 rows per CTA: 141 us against 121).
 // UNIFORM: the columns of a sub-block lie in one quantization group (group % 16 == 0).

@@ -578,11 +578,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_persistent_kernel(c
         if (lane == 0) {
           mbar_expect_tx(full0 + 8 * st, STAGE);
           const uint32_t dst = smem_base + (uint32_t)st * STAGE;
-            tma_load_3d(dst, &map_a, full0 + 8 * st, s * SLAB_K + p.a_k0, a_row, 0);
+          tma_load_3d(dst, &map_a, full0 + 8 * st, s * SLAB_K + p.a_k0, a_row, 0);
 #pragma unroll
-            for (int h = 0; h < TN / TILE_M; ++h)  // the TMA box is 128 rows
-              tma_load_3d(dst + PLANE_TILE_BYTES + h * PLANE_TILE_BYTES, &map_b, full0 + 8 * st, s * SLAB_K + p.b_k0,
-                          b_row + h * TILE_M, 0);
+          for (int h = 0; h < TN / TILE_M; ++h)  // the TMA box is 128 rows
+            tma_load_3d(dst + PLANE_TILE_BYTES + h * PLANE_TILE_BYTES, &map_b, full0 + 8 * st, s * SLAB_K + p.b_k0,
+                        b_row + h * TILE_M, 0);
         }
         __syncwarp();
       }
